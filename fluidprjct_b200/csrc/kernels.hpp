@@ -195,6 +195,26 @@ void launch_pack(const float* pos, const float* vel, int64_t np, float4* pos4, f
                  cudaStream_t st);
 
 // -------- generic CSR CG with FP64 vectors (kernels_pressure.cu) --------
+// Control block and results of one CSR solve on the device.
+struct CsrCtl {
+    GridBar bar;
+    int status;  // DEV_*
+    // 1: the check found malformed offsets, or columns; no solve ran.  Two words: a block may still be
+    // reading the first while another already checks columns.
+    int bad_off, bad_col;
+    int iters;
+    double rr, bb;  // ||r||^2 and ||b||^2
+};
+constexpr int kCsrVectors = 6;  // work vectors of launch_csr_cg
+constexpr int kCsrMaxBlocks = 256;
+constexpr int kCsrPartials = 4 * kCsrMaxBlocks;  // doubles in part
+// Queues the whole solve (two launches): device arrays, work vector i at
+// work + i * stride (stride >= n); results in *ctl.  check: validate offsets
+// and columns first (x is written only if they pass).  Returns 0 or a
+// cudaError_t value.
+int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, const double* b, double* x, double* work,
+                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st);
+// The same from host arrays, complete on return.
 int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x, double tol,
                  int maxit, int* iters, double* relres, cudaStream_t st);
 

@@ -17,6 +17,8 @@
 // updates, FP64 dot products reduced per CTA and then summed by every CTA in
 // a fixed order (deterministic, no host round trip per iteration), and a
 // bounded software grid barrier that reports a timeout instead of hanging.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 
 #include "device_memo.hpp"
@@ -461,45 +463,175 @@ __global__ void k_project(float* __restrict__ u, float* __restrict__ v, float* _
 }
 
 // ---------------------------------------------------------------- CSR CG (FP64)
-// Symmetric matrix from its upper triangle: y = U x + U^T x - diag(U) x.
-__global__ void k_csr_sym_spmv(int n, const int* __restrict__ off, const int* __restrict__ cols,
-                               const double* __restrict__ vals, const double* __restrict__ x, double* __restrict__ y) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = 0.0;
-    for (int e = off[i]; e < off[i + 1]; ++e) {
-        int c = cols[e];
-        s += vals[e] * x[c];
-        if (c != i) atomicAdd(&y[c], vals[e] * x[i]);
+// Jacobi-preconditioned CG on a symmetric matrix stored as its upper triangle,
+// y = U x + U^T x - diag(U) x, as one cooperative launch.
+//
+// Bound: latency.  A solve of 64,000 unknowns touches 4 MB, all of it in L2,
+// so its time is the number of dependent steps.  As separate kernels with the
+// scalars read back (ten launches and three host waits per iteration) 40^3
+// unknowns to 1e-12 (202 iterations) took 18.0 ms on a B200; this kernel takes
+// 1.52 ms, 7.5 us per iteration.  An iteration is two passes and two grid
+// barriers:
+//   pass 1 forms the row's new direction d = z + beta d_old, and its
+//     neighbours' with the same fused multiply-add (so d needs no pass of its
+//     own and no barrier between it and the product), adds the row's products
+//     into q with FP64 reductions, and sums (d, A d) from the products it
+//     makes: an entry (i, c) off the diagonal counts twice;
+//   pass 2 updates x, r, z of the row, clears its q, and sums (r, z), (r, r).
+// d is double-buffered, because pass 1 reads the old directions of other rows
+// while their owners write the new ones.
+constexpr int CSR_THREADS = 512;
+
+struct CsrCgArgs {
+    int n, check, maxit;
+    double tol;
+    const int *off, *cols;
+    const double *vals, *b;
+    double *x, *dg, *r, *z, *q, *d[2];
+    double* part;  // [2][2][gridDim.x]
+    CsrCtl* ctl;
+};
+
+// +0 computed from v, so that its store waits for the load of v (a store of a
+// constant to an address with a load in flight stalls in the memory pipeline).
+__device__ __forceinline__ double zero_after(double v) { return fmin(fabs(v), 0.0); }
+
+// Entries e .. e + CSR_BATCH - 1 of a row that ends at e1; c = -1 past its end.
+// A batch's loads are issued together; four hold a row of the 7-point operator.
+// The first row's first batch stays in registers for the whole solve (the
+// barriers' acquires empty L1); entry by entry, a row took one L2 round trip
+// for each of them (2.03 ms for the solve above).
+constexpr int CSR_BATCH = 4;
+struct Entries {
+    int c[CSR_BATCH];
+    double v[CSR_BATCH];
+};
+__device__ __forceinline__ void load_entries(const CsrCgArgs& a, int e, int e1, Entries& k) {
+#pragma unroll
+    for (int u = 0; u < CSR_BATCH; ++u) {
+        k.c[u] = e + u < e1 ? __ldg(a.cols + e + u) : -1;
+        k.v[u] = e + u < e1 ? __ldg(a.vals + e + u) : 0.0;
     }
-    atomicAdd(&y[i], s);
 }
-__global__ void k_csr_diag(int n, const int* __restrict__ off, const int* __restrict__ cols,
-                           const double* __restrict__ vals, double* __restrict__ dg) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double d = 1.0;
-    for (int e = off[i]; e < off[i + 1]; ++e) if (cols[e] == i) d = vals[e];
-    dg[i] = d;
+
+__global__ void __launch_bounds__(CSR_THREADS) k_csr_cg(CsrCgArgs a) {
+    const int nb = int(gridDim.x);
+    const int t0 = int(blockIdx.x) * CSR_THREADS + threadIdx.x, st = nb * CSR_THREADS;
+    CsrCtl* ctl = a.ctl;
+    int red = 0;
+    auto reduce = [&](double (&v)[2]) {
+        return grid_reduce(v, a.part + (red++ & 1) * 2 * nb, &ctl->bar, nb, &ctl->status);
+    };
+    if (a.check) {
+        // row offsets start at 0 and never decrease; then the columns, whose loop bounds that makes safe
+        for (int i = t0; i < a.n; i += st)
+            if ((i == 0 && a.off[0] != 0) || a.off[i + 1] < a.off[i]) ctl->bad_off = 1;
+        if (!grid_barrier(&ctl->bar, unsigned(nb), &ctl->status)) return;
+        if (__ldcg(&ctl->bad_off)) return;
+        for (int i = t0; i < a.n; i += st)
+            for (int e = a.off[i]; e < a.off[i + 1]; ++e)
+                if (a.cols[e] < 0 || a.cols[e] >= a.n) ctl->bad_col = 1;
+        if (!grid_barrier(&ctl->bar, unsigned(nb), &ctl->status)) return;
+        if (__ldcg(&ctl->bad_col)) return;
+    }
+    double sum[2] = {0.0, 0.0};
+    for (int i = t0; i < a.n; i += st) {
+        double d = 1.0;
+        for (int e = a.off[i]; e < a.off[i + 1]; ++e)
+            if (a.cols[e] == i) d = a.vals[e];
+        const double r = a.b[i], z = r / d;
+        a.dg[i] = d;
+        a.r[i] = r;
+        a.z[i] = z;
+        a.x[i] = 0.0;
+        a.q[i] = 0.0;
+        a.d[1][i] = 0.0;
+        sum[0] += r * z;
+        sum[1] += r * r;
+    }
+    // the thread's first row: offsets and entries, -1 past its end
+    int e_first = 0, e_last = 0;
+    Entries first;
+    if (t0 < a.n) {
+        e_first = a.off[t0];
+        e_last = a.off[t0 + 1];
+        load_entries(a, e_first, e_last, first);
+    }
+    if (!reduce(sum)) return;
+    double rz = sum[0], rr = sum[1], beta = 0.0;
+    const double bb = rr;
+    int it = 0;
+    while (bb > 0.0 && rr > a.tol * a.tol * bb && it < a.maxit) {
+        double* dn = a.d[it & 1];
+        const double* dold = a.d[(it & 1) ^ 1];
+        sum[0] = sum[1] = 0.0;
+        for (int i = t0; i < a.n; i += st) {
+            const bool f = i == t0;
+            const int e0 = f ? e_first : __ldg(a.off + i), e1 = f ? e_last : __ldg(a.off + i + 1);
+            double di = 0.0, s = 0.0, pair = 0.0, own = 0.0;
+            for (int e = e0;; e += CSR_BATCH) {
+                Entries k = first;
+                if (!(f && e == e0)) load_entries(a, e, e1, k);
+                double zc[CSR_BATCH], dc[CSR_BATCH];
+#pragma unroll
+                for (int u = 0; u < CSR_BATCH; ++u) {
+                    const int c = k.c[u] < 0 ? i : k.c[u];
+                    zc[u] = a.z[c];
+                    dc[u] = dold[c];
+                }
+                if (e == e0) di = __fma_rn(beta, dold[i], a.z[i]);
+#pragma unroll
+                for (int u = 0; u < CSR_BATCH; ++u) {
+                    if (k.c[u] < 0) continue;
+                    if (k.c[u] == i) {
+                        own += k.v[u] * di;
+                        continue;
+                    }
+                    const double t = k.v[u] * __fma_rn(beta, dc[u], zc[u]);
+                    s += t;
+                    pair += t;
+                    atomicAdd(&a.q[k.c[u]], k.v[u] * di);
+                }
+                if (e + CSR_BATCH >= e1) break;
+            }
+            dn[i] = di;
+            atomicAdd(&a.q[i], s + own);
+            sum[0] += di * (own + 2.0 * pair);
+        }
+        if (!reduce(sum)) return;
+        if (!(sum[0] > 0.0)) break;
+        const double alpha = rz / sum[0];
+        sum[0] = sum[1] = 0.0;
+        for (int i = t0; i < a.n; i += st) {
+            const double q = __ldcg(a.q + i);  // summed in L2
+            const double r = a.r[i] - alpha * q, z = r / a.dg[i];
+            a.x[i] += alpha * dn[i];
+            a.r[i] = r;
+            a.z[i] = z;
+            a.q[i] = zero_after(q);
+            sum[0] += r * z;
+            sum[1] += r * r;
+        }
+        if (!reduce(sum)) return;
+        beta = sum[0] / rz;
+        rz = sum[0];
+        rr = sum[1];
+        ++it;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->iters = it;
+        ctl->rr = rr;
+        ctl->bb = bb;
+    }
 }
-__global__ void k_dot(int n, const double* __restrict__ a, const double* __restrict__ b, double2* part) {
-    double s = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
-    double2 r = block_sum2(s, 0.0);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
-}
-__global__ void k_axpy2(int n, double alpha, const double* __restrict__ d, const double* __restrict__ q,
-                        double* __restrict__ x, double* __restrict__ r, const double* __restrict__ dg,
-                        double* __restrict__ z) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    x[i] += alpha * d[i];
-    r[i] -= alpha * q[i];
-    z[i] = r[i] / dg[i];
-}
-__global__ void k_xpby(int n, const double* __restrict__ z, double beta, double* __restrict__ d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) d[i] = z[i] + beta * d[i];
+
+__global__ void k_csr_reset(CsrCtl* ctl, unsigned limit) {
+    ctl->bar.count = 0;
+    ctl->bar.limit = limit;
+    ctl->status = DEV_OK;
+    ctl->bad_off = ctl->bad_col = 0;
+    ctl->iters = 0;
+    ctl->rr = ctl->bb = 0.0;
 }
 
 }  // namespace
@@ -628,66 +760,59 @@ void launch_project(float* u, float* v, float* w, const float* p, const uint8_t*
     k_project<<<grd, blk, 0, st>>>(u, v, w, p, labels, g, scale, inv, b, guard);
 }
 
+int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, const double* b, double* x, double* work,
+                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st) {
+    static DeviceMemo memo;
+    const int resident = memo.get([](int dev) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return std::min(sms, kCsrMaxBlocks);
+    });
+    // One row per thread while that fits one CTA per SM (a one-CTA grid's barrier is a block barrier).
+    const int nb = std::max(1, std::min(resident, (n - 1) / CSR_THREADS + 1));
+    k_csr_reset<<<1, 1, 0, st>>>(ctl, kDefaultWaitPolls);
+    CsrCgArgs a{};
+    a.n = n; a.check = check; a.maxit = maxit; a.tol = tol;
+    a.off = off; a.cols = cols; a.vals = vals; a.b = b; a.x = x;
+    double** v[kCsrVectors] = {&a.dg, &a.r, &a.z, &a.q, &a.d[0], &a.d[1]};
+    for (int i = 0; i < kCsrVectors; ++i) *v[i] = work + i * stride;
+    a.part = part;
+    a.ctl = ctl;
+    void* args[] = {&a};
+    return int(cudaLaunchCooperativeKernel((const void*)k_csr_cg, dim3(nb), dim3(CSR_THREADS), args, 0, st));
+}
+
 int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x, double tol,
                  int maxit, int* iters, double* relres, cudaStream_t st) {
     if (n <= 0) return -1;
-    int nnz = offsets[n];
-    int *d_off = nullptr, *d_cols = nullptr;
-    double *d_vals = nullptr, *d_x = nullptr, *d_r = nullptr, *d_d = nullptr, *d_q = nullptr, *d_z = nullptr,
-           *d_dg = nullptr;
-    double2* d_part = nullptr;
-    cudaError_t e = cudaSuccess;
+    const size_t nnz = size_t(offsets[n]), N = size_t(n);
+    // one allocation: doubles (values, b, x, the work vectors), the partials and the control block, then the integers
+    const size_t nd = nnz + (2 + kCsrVectors) * N;
+    const size_t bytes = sizeof(double) * (nd + kCsrPartials) + sizeof(CsrCtl) + sizeof(int) * (N + 1 + nnz);
+    unsigned char* base = nullptr;
+    cudaError_t e = cudaMalloc(&base, bytes);
+    if (e != cudaSuccess) return int(e);
+    double* d_vals = reinterpret_cast<double*>(base);
+    double *d_b = d_vals + nnz, *d_x = d_b + N, *work = d_x + N;
+    double* part = d_vals + nd;
+    CsrCtl* ctl = reinterpret_cast<CsrCtl*>(part + kCsrPartials);
+    int* d_off = reinterpret_cast<int*>(ctl + 1);
+    int* d_cols = d_off + N + 1;
     auto ck = [&](cudaError_t r) { if (r != cudaSuccess && e == cudaSuccess) e = r; };
-    ck(cudaMalloc(&d_off, sizeof(int) * (n + 1)));
-    ck(cudaMalloc(&d_cols, sizeof(int) * nnz));
-    ck(cudaMalloc(&d_vals, sizeof(double) * nnz));
-    for (double** p : {&d_x, &d_r, &d_d, &d_q, &d_z, &d_dg}) ck(cudaMalloc(p, sizeof(double) * n));
-    ck(cudaMalloc(&d_part, sizeof(double2) * 65));
-    if (e != cudaSuccess) goto done;
-    ck(cudaMemcpyAsync(d_off, offsets, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
+    ck(cudaMemcpyAsync(d_off, offsets, sizeof(int) * (N + 1), cudaMemcpyHostToDevice, st));
     ck(cudaMemcpyAsync(d_cols, cols, sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
     ck(cudaMemcpyAsync(d_vals, vals, sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
-    ck(cudaMemcpyAsync(d_r, b, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-    ck(cudaMemsetAsync(d_x, 0, sizeof(double) * n, st));
-    {
-        const int blk = 128, grd = (n + blk - 1) / blk;
-        k_csr_diag<<<grd, blk, 0, st>>>(n, d_off, d_cols, d_vals, d_dg);
-        auto dot = [&](const double* a, const double* bb) {
-            double h[2];
-            k_dot<<<64, 128, 0, st>>>(n, a, bb, d_part);
-            k_sum_partials<<<1, 32, 0, st>>>(d_part, 64, reinterpret_cast<double*>(d_part + 64));
-            cudaMemcpyAsync(h, reinterpret_cast<double*>(d_part + 64), sizeof(double) * 2, cudaMemcpyDeviceToHost, st);
-            cudaStreamSynchronize(st);
-            return h[0];
-        };
-        // z = r/diag, d = z
-        k_axpy2<<<grd, blk, 0, st>>>(n, 0.0, d_d, d_d, d_x, d_r, d_dg, d_z);
-        ck(cudaMemcpyAsync(d_d, d_z, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-        const double bb = dot(d_r, d_r);
-        double rz = dot(d_r, d_z), rr = bb;
-        int it = 0;
-        while (bb > 0 && rr > tol * tol * bb && it < maxit) {
-            ck(cudaMemsetAsync(d_q, 0, sizeof(double) * n, st));
-            k_csr_sym_spmv<<<grd, blk, 0, st>>>(n, d_off, d_cols, d_vals, d_d, d_q);
-            double dq = dot(d_d, d_q);
-            if (!(dq > 0)) break;
-            double alpha = rz / dq;
-            k_axpy2<<<grd, blk, 0, st>>>(n, alpha, d_d, d_q, d_x, d_r, d_dg, d_z);
-            double rz2 = dot(d_r, d_z);
-            rr = dot(d_r, d_r);
-            k_xpby<<<grd, blk, 0, st>>>(n, d_z, rz2 / rz, d_d);
-            rz = rz2;
-            ++it;
-        }
-        if (iters) *iters = it;
-        if (relres) *relres = bb > 0 ? sqrt(rr / bb) : 0.0;
-        ck(cudaMemcpyAsync(x, d_x, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-        ck(cudaStreamSynchronize(st));
-    }
-done:
-    cudaFree(d_off); cudaFree(d_cols); cudaFree(d_vals);
-    for (double* p : {d_x, d_r, d_d, d_q, d_z, d_dg}) cudaFree(p);
-    cudaFree(d_part);
+    ck(cudaMemcpyAsync(d_b, b, sizeof(double) * N, cudaMemcpyHostToDevice, st));
+    if (e == cudaSuccess)
+        ck(cudaError_t(launch_csr_cg(n, d_off, d_cols, d_vals, d_b, d_x, work, int64_t(N), part, ctl, 0, tol, maxit, st)));
+    CsrCtl h{};
+    ck(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, st));
+    ck(cudaMemcpyAsync(x, d_x, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+    ck(cudaStreamSynchronize(st));
+    if (e == cudaSuccess && h.status != DEV_OK) e = cudaErrorUnknown;  // a bounded wait gave up
+    if (iters) *iters = h.iters;
+    if (relres) *relres = h.bb > 0 ? sqrt(h.rr / h.bb) : 0.0;
+    cudaFree(base);
     return e == cudaSuccess ? 0 : int(e);
 }
 

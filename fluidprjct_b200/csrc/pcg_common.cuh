@@ -114,6 +114,65 @@ __device__ __forceinline__ double2 grid_sum2(const double2* part, int nb) {
     return r;
 }
 
+// Grid-wide sums of N doubles per thread, the same bits in every thread of
+// every block, around one grid barrier: block partials to part[N][nb] (two
+// buffers that alternate from call to call suffice), the barrier, then mid()
+// -- loads that wait on the barrier but not on the sums, so that their round
+// trip overlaps the partials' -- and the total, one warp per sum with all its
+// loads issued together.  Returns false if the barrier gave up.  Fixed order
+// throughout.  (Against block_sum3 + grid_barrier + grid_sum3, whose total is
+// a two-level tree over the whole block: one block barrier and half of the
+// shuffle steps fewer per reduction.)
+template <int N, class Mid>
+__device__ __forceinline__ bool grid_reduce(double (&v)[N], double* part, GridBar* bar, int nb, int* status, Mid mid) {
+    __shared__ double sh[N][32];
+    __shared__ double res[N];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = int(blockDim.x >> 5);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < N; ++k) sh[k][wid] = v[k];
+    __syncthreads();
+    double x = 0.0;
+    if (wid < N) {
+        x = lane < nw ? sh[wid][lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) {
+            if (nb == 1) res[wid] = x;
+            else part[wid * nb + int(blockIdx.x)] = x;
+        }
+    }
+    if (!grid_barrier(bar, unsigned(nb), status)) return false;
+    mid();
+    if (nb > 1 && wid < N) {
+        // written by other CTAs in this launch: read through L2
+        constexpr int B = 5;  // 160 CTAs in one batch of loads
+        x = 0.0;
+        for (int t0 = lane; t0 < nb; t0 += 32 * B) {
+            double y[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) y[b] = t0 + 32 * b < nb ? __ldcg(part + wid * nb + t0 + 32 * b) : 0.0;
+#pragma unroll
+            for (int b = 0; b < B; ++b) x += y[b];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) res[wid] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = res[k];
+    return true;
+}
+template <int N>
+__device__ __forceinline__ bool grid_reduce(double (&v)[N], double* part, GridBar* bar, int nb, int* status) {
+    return grid_reduce<N>(v, part, bar, nb, status, [] {});
+}
+
 // Sum of three per-block partial arrays part[0..nb), part[nb..2nb),
 // part[2nb..3nb), returned to every thread of every block.  All threads load
 // (one L2 round trip when nb <= blockDim) and reduce with a fixed tree, so

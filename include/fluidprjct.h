@@ -340,9 +340,9 @@ int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double*
  *     must be 0, offsets must not decrease, columns must lie in [0, n);
  *   - like fp_solve_csr_upper it returns FP_OK when CG stops at max_iters or
  *     breaks down: check *relres against tol;
- *   - the call is synchronous (it reads scalars back every iteration and
- *     drains its stream before returning), so it must not be issued on a
- *     stream that is being captured;
+ *   - the call is synchronous (it reads its result back and drains its
+ *     stream before returning), so it must not be issued on a stream that is
+ *     being captured;
  *   - all calls on a device share the array, so they take turns: a call
  *     holds a per-device host lock until its stream has drained, and calls
  *     from several host threads are serialised;
