@@ -25,6 +25,7 @@ SOURCES = [
     "kernels_sort.cu",
     "kernels_p2g.cu",
     "kernels_pressure.cu",
+    "kernels_pcg.cu",
     "kernels_advect.cu",
     "kernels_body.cu",
     "kernels_mg.cu",

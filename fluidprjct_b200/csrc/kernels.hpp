@@ -25,7 +25,9 @@ struct PcgOut {
     double rr;      // ||r||^2 of the recurrence at exit
     double bb;      // ||b||^2
     double rz;
-    double rr0;     // ||b - A x0||^2 of the initial iterate (MG kernel)
+    double rr0;     // ||b - A x0||^2 of the initial iterate (MG and mixed)
+    int outer;      // refinement loops (plain PCG: 1; MG leaves it alone)
+    int pad_;
 };
 
 // Device buffers of the pressure system.  Compact arrays are indexed by the
@@ -38,14 +40,14 @@ struct PressureBufs {
     uint8_t* diag;        // [nc] diagonal of the unit operator (compact)
     float* b;             // [nc] right-hand side (compact)
     float* bin;           // [nc] right-hand side of an inner refinement solve
-    void* R[2];           // padded dense residual (double-buffered)
+    void* R[2];           // padded dense residual (double-buffered); R[0] also u = M^-1 r
     void* Wv[2];          // padded dense w = A M^-1 r
     void* S[2];           // padded dense s = A p
     void* invd;           // padded dense 1/diag
     void* P;              // [nc] compact search direction
     void* X;              // [nc] compact solution
     double* x64;          // [nc] refinement accumulator (compact)
-    double* xd;           // padded dense FP64 copy of x64
+    double* xd;           // padded dense FP64 iterate
     double* part;         // [6 * max_blocks] per-block partial sums
     GridBar* bar;         // [1]
     PcgOut* out;          // [1]
@@ -120,29 +122,24 @@ void launch_copy(const float* src, float* dst, int64_t n, cudaStream_t st);
 // computed rhs (caller-provided system).
 void launch_pressure_setup(const uint8_t* labels, const float* u, const float* v, const float* w, Dims g, float dt,
                            BodyKin body, const float* rhs_dense, float* p, PressureBufs& pb, cudaStream_t st);
-// Persistent cooperative Jacobi PCG (Chronopoulos-Gear form, one grid barrier
-// per iteration) from x0 = 0 for A x = rhs to ||r||/||rhs|| <= tol; vectors in
-// FP64 (fp64 = 1) or FP32 (0), reductions always FP64.  Solution in pb.X,
-// diagnostics in pb.out.  The padded work grids must be zero on entry;
-// launch_pcg_clear restores that after a solve.
-int launch_pcg(Dims g, PressureBufs& pb, const float* rhs, int fp64, double tol, int maxit, cudaStream_t st,
+
+// -------- plain and mixed-precision PCG (kernels_pcg.cu) --------
+// Jacobi PCG with FP64 vectors from x0 = 0 for A x = b (the system of
+// launch_pressure_setup) to ||r||/||b|| <= tol.  Dense pressure to pout (its
+// non-FLUID cells must be zero), the true residual's ||b - A x||^2 and ||b||^2
+// to pb.red, diagnostics to pb.out.  The padded work grids must be zero on
+// entry and are zero again on exit, unless a wait gave up.
+int launch_pcg(Dims g, PressureBufs& pb, double tol, int maxit, float* pout, cudaStream_t st,
                unsigned wait_polls = kDefaultWaitPolls);
-void launch_pcg_clear(PressureBufs& pb, int fp64, int with_invd, cudaStream_t st);
+// The same by FP64 iterative refinement around FP32-vector PCG solves, from
+// x = 0 or from the compact guess x0 scaled by its energy-optimal factor
+// (x0, b) / (x0, A x0).
+int launch_pcg_mixed(Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout, cudaStream_t st,
+                     unsigned wait_polls = kDefaultWaitPolls);
 // Barrier word to zero with its poll limit, status word to DEV_OK (before
 // every persistent-solver launch).
 void launch_reset_barrier(GridBar* bar, int* status, unsigned wait_polls, cudaStream_t st);
 int pcg_max_blocks();
-// p[cell] = X[n] (src 0: FP32 X, 1: FP64 X, 2: x64).
-void launch_scatter_p(const PressureBufs& pb, float* p, int src, Dims g, cudaStream_t st);
-// ||b - A X||^2 and ||b||^2 in FP64 into pb.red[0..1] (uses R[0] as scratch).
-void launch_true_residual(PressureBufs& pb, int fp64, Dims g, cudaStream_t st);
-// Iterative refinement: bin = float(b - A x64) with the FP64 residual norms in
-// pb.red; x64 += X (FP32) and its padded copy xd.
-void launch_ir_residual(PressureBufs& pb, Dims g, cudaStream_t st);
-void launch_ir_update(PressureBufs& pb, Dims g, cudaStream_t st);
-// Scales the refinement's starting point x64 (and xd) by its energy-optimal
-// factor (x, b) / (x, A x), computed in FP64 on the device (3 launches).
-void launch_guess_scale(PressureBufs& pb, Dims g, cudaStream_t st);
 
 // -------- projection (kernels_pressure.cu) --------
 // guard: the status word of the solve that produced p, or null; the kernel

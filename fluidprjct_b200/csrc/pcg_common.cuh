@@ -66,54 +66,6 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nblocks, int
     return s_ok != 0;
 }
 
-// Block sum of two doubles (fixed tree, deterministic); result valid in thread 0.
-__device__ __forceinline__ double2 block_sum2(double a, double b) {
-    __shared__ double2 sh[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = make_double2(a, b);
-    __syncthreads();
-    double2 r = make_double2(0.0, 0.0);
-    if (wid == 0) {
-        r = lane < int(blockDim.x >> 5) ? sh[lane] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            r.x += __shfl_down_sync(0xffffffffu, r.x, o);
-            r.y += __shfl_down_sync(0xffffffffu, r.y, o);
-        }
-    }
-    __syncthreads();
-    return r;
-}
-
-// Sum of per-block partials part[0..nb) (pairs), identical in every block.
-__device__ __forceinline__ double2 grid_sum2(const double2* part, int nb) {
-    __shared__ double2 res;
-    if (threadIdx.x < 32) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int t = threadIdx.x; t < nb; t += 32) {
-            // Written by other CTAs in this launch: read through L2.
-            double2 v = __ldcg(part + t);
-            s.x += v.x;
-            s.y += v.y;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s.x += __shfl_down_sync(0xffffffffu, s.x, o);
-            s.y += __shfl_down_sync(0xffffffffu, s.y, o);
-        }
-        if (threadIdx.x == 0) res = s;
-    }
-    __syncthreads();
-    double2 r = res;
-    __syncthreads();
-    return r;
-}
-
 // Grid-wide sums of N doubles per thread, the same bits in every thread of
 // every block, around one grid barrier: block partials to part[N][nb] (two
 // buffers that alternate from call to call suffice), the barrier, then mid()

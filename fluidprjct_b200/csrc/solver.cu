@@ -437,198 +437,101 @@ void phase_save(fp_solver* s) {
     launch_copy(s->d_w, s->d_ws, s->g.nw(), s->st);
 }
 
+int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float pcg_ms, float learned_ms,
+               float guess_relres, int fallback);
+
+bool mg_solver(const fp_solver* s) { return s->cfg.solver == FP_SOLVER_PCG_MG || s->cfg.solver == FP_SOLVER_PCG_LEARNED; }
+bool mixed_solver(const fp_solver* s) {
+    return s->cfg.solver == FP_SOLVER_PCG_MIXED || s->cfg.solver == FP_SOLVER_PCG_LEARNED_MIXED;
+}
+bool learned_solver(const fp_solver* s) {
+    return s->cfg.solver == FP_SOLVER_PCG_LEARNED || s->cfg.solver == FP_SOLVER_PCG_LEARNED_MIXED;
+}
+// ||b - A x0|| / ||b|| of the solve read back in h_out.
+float guess_of(const fp_solver* s) {
+    return s->h_out->bb > 0 ? float(std::sqrt(s->h_out->rr0 / s->h_out->bb)) : 0.0f;
+}
+int outer_of(const fp_solver* s) { return mixed_solver(s) ? s->h_out->outer : 1; }
+
 // Pressure solve of the system already set up in s->pb (fidx, diag, b); writes
 // the dense solution to p_out and the diagnostics to s->stats.
 //   FP_SOLVER_PCG       one FP64-vector PCG to tol (the FP64 path);
 //   FP_SOLVER_PCG_MIXED FP64 iterative refinement: r = b - A x in FP64, an
-//                       FP32-vector PCG solves A c = r loosely, x += c.
-int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float pcg_ms, float learned_ms,
-               float guess_relres, int fallback);
-
-// defer: for the plain PCG and MG solvers, queue the read-back of the solve's
+//                       FP32-vector PCG solves A c = r loosely, x += c;
+//   FP_SOLVER_PCG_MG    flexible PCG with the multigrid V-cycle;
+//   the learned variants of the last two, with the plain PCG as fallback.
+// Each is one persistent launch that also writes p_out, the true residual and
+// its own clean-up.
+// defer: for the solvers without a network, queue the read-back of the solve's
 // statistics behind ev[9] and return without waiting; solve_finalize then
 // waits and fills them (one_step issues the projection and advection first).
 int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     PressureBufs& pb = s->pb;
     const double tol = s->cfg.tol;
     const int maxit = s->cfg.max_iters;
-    int outer = 0, inner_total = 0;
-    int dev_status = DEV_OK;
-    float pcg_ms = 0.0f;
-    cudaError_t ce;
-    float learned_ms = 0.0f, guess_relres = 1.0f;
-    int fallback = 0;
-    if (s->cfg.solver == FP_SOLVER_PCG || s->cfg.solver == FP_SOLVER_PCG_MG ||
-        s->cfg.solver == FP_SOLVER_PCG_LEARNED) {
-        const bool learned = s->cfg.solver == FP_SOLVER_PCG_LEARNED;
-        const bool mg = s->cfg.solver != FP_SOLVER_PCG;
-        if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
-        if (mg) {
-            s->launches += launch_mg_setup(s->d_labels, s->g, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->st);
-        }
-        cudaEventRecord(s->ev_pcg[0], s->st);
-        const float* x0 = nullptr;
-        if (learned) {
-            const unet::Lvl real{s->W, s->H, s->D};
-            unet::launch_rhs_dense(pb.nf, pb.fidx, real, pb.b, s->d_rhs_dense, s->st);
-            if (unet::forward_on(s->net, s->d_labels, s->d_rhs_dense, s->st))
-                return s->cuda_fail(cudaGetLastError(), "U-Net forward");
-            unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
-                                        unet::net_scal(s->net), s->d_x0c, s->st);
-            s->launches += 1 + 16 + 1;  // rhs scatter, network (2 scale/input, 10 conv, 2 pool, 2 concat), guess
-            cudaEventRecord(s->ev_net, s->st);
-            x0 = s->d_x0c;
-        }
-        // A learned solve that has not converged after kLearnedMaxit iterations
-        // counts as stalled and hands over to the plain PCG.
-        constexpr int kLearnedMaxit = 300;
-        int e = mg ? launch_pcg_mg(s->g, pb, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->d_mgp, s->d_mgq, s->d_mgx,
-                                   s->d_mgr, pb.b, tol, learned ? std::min(maxit, kLearnedMaxit) : maxit, s->st, x0,
-                                   s->cfg.mg_sweeps > 0 ? s->cfg.mg_sweeps : 2,
-                                   s->cfg.warm_start && p_out == s->d_p ? p_out : nullptr, p_out, s->wait_polls)
-                   : launch_pcg(s->g, pb, pb.b, 1, tol, maxit, s->st, s->wait_polls);
-        cudaEventRecord(s->ev_pcg[1], s->st);
-        if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
-        // FP64 solution to p, its true residual, then clear the work grids at
-        // this solve's FLUID cells (the residual check leaves x in R[0]); the
-        // MG kernel does all three itself
-        auto finish_launch = [&](bool jacobi) {
-            if (jacobi) {
-                launch_scatter_p(pb, p_out, 1, s->g, s->st);
-                launch_true_residual(pb, 1, s->g, s->st);
-                launch_pcg_clear(pb, 1, 1, s->st);
-                s->launches += 1 + 1 + 1 + 3 + 1;  // reset + pcg, scatter, residual (3), clear
-            } else {
-                s->launches += 1;  // the MG kernel
-            }
-            cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);  // out, red and nf
-        };
-        auto finish = [&](bool jacobi) -> cudaError_t {
-            finish_launch(jacobi);
-            return cudaStreamSynchronize(s->st);
-        };
-        if (defer && !learned) {
-            finish_launch(!mg);
-            cudaEventRecord(s->ev[9], s->st);
-            s->solve_pending = true;
-            s->pending_guess = mg && s->cfg.warm_start && p_out == s->d_p;
-            return FP_OK;
-        }
-        if (learned)
-            cudaMemcpyAsync(s->h_bad, unet::net_status(s->net), sizeof(int), cudaMemcpyDeviceToHost, s->st);
-        ce = finish(!mg);
-        if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
-        if (learned && *s->h_bad) return s->fail(FP_ERR_TIMEOUT, "U-Net forward: a bounded tensor-core wait gave up");
-        inner_total = s->h_out->iters;
-        dev_status = s->h_out->status;
-        outer = 1;
-        cudaEventElapsedTime(&pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
-        if (mg && (learned || (s->cfg.warm_start && p_out == s->d_p)))
-            guess_relres = s->h_out->bb > 0 ? float(std::sqrt(s->h_out->rr0 / s->h_out->bb)) : 0.0f;
-        if (learned) {
-            cudaEventElapsedTime(&learned_ms, s->ev_pcg[0], s->ev_net);
-            const double rel = s->h_red[1] > 0 ? std::sqrt(s->h_red[0] / s->h_red[1]) : 0.0;
-            if (*s->h_nf > 0 && dev_status != DEV_TIMEOUT && (dev_status != DEV_OK || !(rel <= tol))) {
-                // fallback: the plain FP64 PCG from x = 0
-                fallback = 1;
-                cudaEventRecord(s->ev_pcg[0], s->st);
-                e = launch_pcg(s->g, pb, pb.b, 1, tol, maxit, s->st, s->wait_polls);
-                cudaEventRecord(s->ev_pcg[1], s->st);
-                if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
-                ce = finish(true);
-                if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve (fallback)");
-                inner_total += s->h_out->iters;
-                dev_status = s->h_out->status;
-                outer = 2;
-                float ms = 0.0f;
-                cudaEventElapsedTime(&ms, s->ev_pcg[0], s->ev_pcg[1]);
-                pcg_ms += ms;
-            }
-        }
-    } else {
-        // FP_SOLVER_PCG_MIXED, or FP_SOLVER_PCG_LEARNED_MIXED: the same
-        // refinement started from the network's guess (energy-optimally scaled)
-        const bool learned = s->cfg.solver == FP_SOLVER_PCG_LEARNED_MIXED;
-        if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
-        cudaMemsetAsync(pb.x64, 0, sizeof(double) * s->g.nc(), s->st);
-        if (learned) {
-            cudaEventRecord(s->ev_pcg[0], s->st);
-            const unet::Lvl real{s->W, s->H, s->D};
-            unet::launch_rhs_dense(pb.nf, pb.fidx, real, pb.b, s->d_rhs_dense, s->st);
-            if (unet::forward_on(s->net, s->d_labels, s->d_rhs_dense, s->st))
-                return s->cuda_fail(cudaGetLastError(), "U-Net forward");
-            unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
-                                        unet::net_scal(s->net), s->d_x0c, s->st);
-            // x64 = xd = guess (xd is zero between solves), then scaled by (x, b) / (x, A x)
-            cudaMemcpyAsync(pb.X, s->d_x0c, sizeof(float) * size_t(s->g.nc()), cudaMemcpyDeviceToDevice, s->st);
-            launch_ir_update(pb, s->g, s->st);
-            launch_guess_scale(pb, s->g, s->st);
-            cudaEventRecord(s->ev_net, s->st);
-            s->launches += 1 + 16 + 1 + 1 + 3;  // rhs scatter, network, guess, copy-in, scaling
-            cudaMemcpyAsync(s->h_bad, unet::net_status(s->net), sizeof(int), cudaMemcpyDeviceToHost, s->st);
-        }
-        launch_ir_residual(pb, s->g, s->st);  // bin = b - A x64 (= b from x64 = 0)
-        s->launches += 3;
-        cudaMemcpyAsync(s->h_red, pb.red, sizeof(double) * 2, cudaMemcpyDeviceToHost, s->st);
-        cudaMemcpyAsync(s->h_nf, pb.nf, sizeof(int), cudaMemcpyDeviceToHost, s->st);
-        ce = cudaStreamSynchronize(s->st);
-        if (ce != cudaSuccess) return s->cuda_fail(ce, "refinement residual");
-        if (learned && *s->h_bad) return s->fail(FP_ERR_TIMEOUT, "U-Net forward: a bounded tensor-core wait gave up");
-        if (learned) cudaEventElapsedTime(&learned_ms, s->ev_pcg[0], s->ev_net);
-        const double bb = s->h_red[1];
-        double relres = bb > 0 ? std::sqrt(s->h_red[0] / bb) : 0.0;
-        if (learned) guess_relres = float(relres);
-        while (relres > tol && outer < 12 && inner_total < maxit) {
-            // Inner accuracy: enough to land below tol after this update, but
-            // not below what FP32 vectors can resolve.
-            const double inner_tol = std::min(0.1, std::max(2e-4, 0.5 * tol / relres));
-            cudaEventRecord(s->ev_pcg[0], s->st);
-            int e = launch_pcg(s->g, pb, pb.bin, 0, inner_tol, maxit - inner_total, s->st, s->wait_polls);
-            cudaEventRecord(s->ev_pcg[1], s->st);
-            if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
-            launch_ir_update(pb, s->g, s->st);
-            launch_pcg_clear(pb, 0, 0, s->st);
-            launch_ir_residual(pb, s->g, s->st);
-            s->launches += 2 + 1 + 1 + 2;  // reset + pcg, update, clear, residual (2)
-            cudaMemcpyAsync(s->h_out, pb.out, sizeof(PcgOut), cudaMemcpyDeviceToHost, s->st);
-            cudaMemcpyAsync(s->h_red, pb.red, sizeof(double) * 2, cudaMemcpyDeviceToHost, s->st);
-            ce = cudaStreamSynchronize(s->st);
-            if (ce != cudaSuccess) return s->cuda_fail(ce, "refinement step");
-            inner_total += s->h_out->iters;
-            ++outer;
-            float ms = 0.0f;
-            cudaEventElapsedTime(&ms, s->ev_pcg[0], s->ev_pcg[1]);
-            pcg_ms += ms;
-            if (s->h_out->status == DEV_TIMEOUT || s->h_out->status == DEV_NAN) { dev_status = s->h_out->status; break; }
-            const double nr = bb > 0 ? std::sqrt(s->h_red[0] / bb) : 0.0;
-            if (!(nr < relres)) { relres = nr; dev_status = DEV_BREAKDOWN; break; }  // refinement stalled
-            relres = nr;
-        }
-        launch_pcg_clear(pb, 0, 1, s->st);  // 1/diag grid
-        launch_scatter_p(pb, p_out, 2, s->g, s->st);
-        s->launches += 2;
-        s->h_red[0] = relres * relres * bb;
-        s->h_red[1] = bb;
-        if (relres > tol && dev_status == DEV_OK) dev_status = DEV_MAXIT;
-        // xd must be zero at the start of the next solve
-        cudaMemsetAsync(pb.xd, 0, sizeof(double) * size_t(s->padded), s->st);
-        pcg_ms += learned_ms;
-        if (learned && *s->h_nf > 0 && dev_status != DEV_TIMEOUT && dev_status != DEV_OK) {
-            // the refinement from the learned guess stalled: plain FP64 PCG from zero
+    const bool learned = learned_solver(s), mg = mg_solver(s), mixed = mixed_solver(s);
+    const bool warm = s->cfg.solver == FP_SOLVER_PCG_MG && s->cfg.warm_start && p_out == s->d_p;
+    if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
+    if (mg) s->launches += launch_mg_setup(s->d_labels, s->g, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->st);
+    cudaEventRecord(s->ev_pcg[0], s->st);
+    const float* x0 = nullptr;
+    if (learned) {
+        const unet::Lvl real{s->W, s->H, s->D};
+        unet::launch_rhs_dense(pb.nf, pb.fidx, real, pb.b, s->d_rhs_dense, s->st);
+        if (unet::forward_on(s->net, s->d_labels, s->d_rhs_dense, s->st))
+            return s->cuda_fail(cudaGetLastError(), "U-Net forward");
+        unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
+                                    unet::net_scal(s->net), s->d_x0c, s->st);
+        s->launches += 1 + 16 + 1;  // rhs scatter, network (2 scale/input, 10 conv, 2 pool, 2 concat), guess
+        cudaEventRecord(s->ev_net, s->st);
+        x0 = s->d_x0c;
+    }
+    // A learned MG solve that has not converged after kLearnedMaxit iterations
+    // counts as stalled and hands over to the plain PCG.
+    constexpr int kLearnedMaxit = 300;
+    int e = 0;
+    if (mg)
+        e = launch_pcg_mg(s->g, pb, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr, pb.b,
+                          tol, learned ? std::min(maxit, kLearnedMaxit) : maxit, s->st, x0,
+                          s->cfg.mg_sweeps > 0 ? s->cfg.mg_sweeps : 2,
+                          s->cfg.warm_start && p_out == s->d_p ? p_out : nullptr, p_out, s->wait_polls);
+    else if (mixed)
+        e = launch_pcg_mixed(s->g, pb, x0, tol, maxit, p_out, s->st, s->wait_polls);
+    else
+        e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st, s->wait_polls);
+    s->launches += 2;  // barrier reset, solver
+    cudaEventRecord(s->ev_pcg[1], s->st);
+    if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
+    cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);  // out, red and nf
+    if (defer && !learned) {
+        cudaEventRecord(s->ev[9], s->st);
+        s->solve_pending = true;
+        s->pending_guess = warm;
+        return FP_OK;
+    }
+    if (learned) cudaMemcpyAsync(s->h_bad, unet::net_status(s->net), sizeof(int), cudaMemcpyDeviceToHost, s->st);
+    cudaError_t ce = cudaStreamSynchronize(s->st);
+    if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
+    if (learned && *s->h_bad) return s->fail(FP_ERR_TIMEOUT, "U-Net forward: a bounded tensor-core wait gave up");
+    float pcg_ms = 0.0f, learned_ms = 0.0f;
+    cudaEventElapsedTime(&pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
+    if (learned) cudaEventElapsedTime(&learned_ms, s->ev_pcg[0], s->ev_net);
+    int iters = s->h_out->iters, outer = outer_of(s), dev_status = s->h_out->status, fallback = 0;
+    const float guess = learned || warm ? guess_of(s) : 1.0f;
+    if (learned) {
+        const double rel = s->h_red[1] > 0 ? std::sqrt(s->h_red[0] / s->h_red[1]) : 0.0;
+        if (*s->h_nf > 0 && dev_status != DEV_TIMEOUT && (dev_status != DEV_OK || !(rel <= tol))) {
+            // fallback: the plain FP64 PCG from x = 0
             fallback = 1;
             cudaEventRecord(s->ev_pcg[0], s->st);
-            const int e = launch_pcg(s->g, pb, pb.b, 1, tol, maxit, s->st, s->wait_polls);
+            e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st, s->wait_polls);
             cudaEventRecord(s->ev_pcg[1], s->st);
             if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
-            launch_scatter_p(pb, p_out, 1, s->g, s->st);
-            launch_true_residual(pb, 1, s->g, s->st);
-            launch_pcg_clear(pb, 1, 1, s->st);
-            s->launches += 1 + 1 + 1 + 3 + 1;
-            cudaMemcpyAsync(s->h_out, pb.out, sizeof(PcgOut), cudaMemcpyDeviceToHost, s->st);
-            cudaMemcpyAsync(s->h_red, pb.red, sizeof(double) * 2, cudaMemcpyDeviceToHost, s->st);
+            s->launches += 2;
+            cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);
             ce = cudaStreamSynchronize(s->st);
             if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve (fallback)");
-            inner_total += s->h_out->iters;
+            iters += s->h_out->iters;
             dev_status = s->h_out->status;
             ++outer;
             float ms = 0.0f;
@@ -636,7 +539,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             pcg_ms += ms;
         }
     }
-    return solve_tail(s, inner_total, outer, dev_status, pcg_ms, learned_ms, guess_relres, fallback);
+    return solve_tail(s, iters, outer, dev_status, pcg_ms, learned_ms, guess, fallback);
 }
 
 // Waits for a deferred solve and fills its statistics and status.
@@ -647,9 +550,8 @@ int solve_finalize(fp_solver* s) {
     if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
     float pcg_ms = 0.0f;
     cudaEventElapsedTime(&pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
-    const float guess = !s->pending_guess ? 1.0f
-                        : (s->h_out->bb > 0 ? float(std::sqrt(s->h_out->rr0 / s->h_out->bb)) : 0.0f);
-    return solve_tail(s, s->h_out->iters, 1, s->h_out->status, pcg_ms, 0.0f, guess, 0);
+    return solve_tail(s, s->h_out->iters, outer_of(s), s->h_out->status, pcg_ms, 0.0f,
+                      s->pending_guess ? guess_of(s) : 1.0f, 0);
 }
 
 // The statistics and status of a finished solve (host copies of its results).
@@ -669,17 +571,21 @@ int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float p
     else if (dev_status == DEV_TIMEOUT) status = FP_ERR_TIMEOUT;
     else if (dev_status != DEV_OK) status = FP_ERR_SOLVER;
     s->stats.solve_status = status;
-    if (status == FP_ERR_TIMEOUT && s->mgL > 0) {
-        // a solve that gave up mid-way leaves the MG work grids and level-0
-        // codes non-zero; restore the zero state the next solve relies on
+    if (status == FP_ERR_TIMEOUT) {
+        // a solve that gave up mid-way leaves its work grids (MG: the level-0
+        // codes too) non-zero; restore the zero state the next solve relies on
+        const size_t pbytes = sizeof(double) * size_t(s->padded);
+        for (void* a : {s->pb.R[0], s->pb.R[1], s->pb.Wv[0], s->pb.Wv[1], s->pb.S[0], s->pb.S[1], s->pb.invd,
+                        static_cast<void*>(s->pb.xd)})
+            cudaMemsetAsync(a, 0, pbytes, s->st);
         for (int l = 0; l < s->mgL; ++l) {
             const size_t np_ = size_t(s->mg[l].W + 2) * (s->mg[l].H + 2) * (s->mg[l].D + 2);
             cudaMemsetAsync(s->mg[l].x, 0, np_ * sizeof(float), s->st);
             cudaMemsetAsync(s->mg[l].b, 0, np_ * sizeof(float), s->st);
             cudaMemsetAsync(s->mg[l].code, 0, np_, s->st);
         }
-        for (double* a : {s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr})
-            cudaMemsetAsync(a, 0, sizeof(double) * size_t(s->padded), s->st);
+        if (s->mgL > 0)
+            for (double* a : {s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr}) cudaMemsetAsync(a, 0, pbytes, s->st);
     }
     if (status == FP_ERR_TIMEOUT) return s->fail(status, "PCG grid barrier timed out");
     if (dev_status == DEV_NAN) return s->fail(status, "PCG produced NaN");

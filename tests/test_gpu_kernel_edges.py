@@ -68,3 +68,67 @@ def test_csr_solve_leaves_x_alone_when_malformed():
         with pytest.raises(capi.FluidError) as e:
             capi.solve_csr_upper_noalloc(n, o.data_ptr(), c.data_ptr(), one.data_ptr(), one.data_ptr(), x.data_ptr())
         assert e.value.code == capi.FP_ERR_ARG and (x == 7.0).all()
+
+
+def _cg64(fl, diag, b, tol=1e-13):
+    """FP64 CG by torch of the unit operator over the FLUID mask fl (zero-padded by one cell)."""
+    import torch
+
+    def apply(v):
+        s = diag * v
+        for d in range(3):
+            s = s - torch.roll(v, 1, d) - torch.roll(v, -1, d)
+        return s * fl
+
+    x, r = torch.zeros_like(b), b.clone()
+    inv = torch.where(diag > 0, 1.0 / diag.clamp(min=1.0), torch.zeros_like(diag))
+    z = r * inv
+    p, rz, bb = z.clone(), (r * z).sum(), (b * b).sum()
+    for it in range(20000):
+        q = apply(p)
+        a = rz / (p * q).sum()
+        x, r = x + a * p, r - a * q
+        z = r * inv
+        new = (r * z).sum()
+        p, rz = z + (new / rz) * p, new
+        if it % 16 == 0 and float((r * r).sum()) <= tol * tol * float(bb):
+            break
+    return x
+
+
+# One CTA with one cell per thread and with more (2D, 870 cells); several CTAs; 148 CTAs just below and above one
+# cell per thread (71,944 and 78,336 cells); a share above the FP64 and one above the FP32 vectors' shared memory
+@pytest.mark.parametrize("solver", ["pcg", "pcg_mixed"])
+@pytest.mark.parametrize("shape", [(8, 8, 8), (32, 32, 1), (9, 31, 14), (48, 48, 36), (50, 50, 36), (112, 80, 96),
+                                   (128, 96, 114)])
+def test_pcg_sizes(solver, shape):
+    """A box of water under one layer of air.  The solver stops at ||b - A x|| <= tol ||b|| with tol = 1e-9, so its
+    relative error is at most cond(A) tol; the condition number of the operator on h layers of water under a free
+    surface is at most 12 / (2 - 2 cos(pi / (2 h + 1))), below 1.3e5 at h = 127, and FP32 storage adds 6e-8."""
+    import torch
+    from fluidprjct_b200 import capi
+    W, H, D = shape
+    lab = np.full((D, H, W), 1, np.uint8)
+    lab[:, 0], lab[:, -1], lab[:, :, 0], lab[:, :, -1] = 0, 0, 0, 0
+    if D > 1:
+        lab[0], lab[-1] = 0, 0
+    lab[:, -2][lab[:, -2] == 1] = 2
+    rng = np.random.default_rng(W * H + D)
+    rhs = (rng.standard_normal(lab.shape) * (lab == 1)).astype(np.float32)
+    s = capi.Solver(dim=3 if D > 1 else 2, dx=1.0 / W, dt=0.01, solver=solver, tol=1e-9, output_format=capi.OUT_NONE)
+    s.set_labels(lab if D > 1 else lab[0])
+    t = torch.nn.functional.pad(torch.from_numpy(lab).cuda().int(), (1, 1, 1, 1, 1, 1))
+    wet = ((t == 1) | (t == 2)).double()
+    fl = (t == 1).double()
+    diag = sum(torch.roll(wet, o, d) for d in range(3) for o in (1, -1)) * fl
+    want = _cg64(fl, diag, torch.nn.functional.pad(torch.from_numpy(rhs).cuda().double(), (1, 1, 1, 1, 1, 1)))
+    want = want[1:-1, 1:-1, 1:-1]
+    h = H - 3
+    bound = 1e-9 * 12 / (2 - 2 * np.cos(np.pi / (2 * h + 1))) + 1e-7
+    for _ in range(2):  # the second solve finds the work grids as the first left them
+        x, it, rr, rc = s.pressure_solve(rhs)
+        assert rc == 0 and rr <= 1e-9
+        err = torch.from_numpy(x).cuda().double() - want
+        assert float(err.norm() / want.norm()) <= bound
+        assert not x[lab != 1].any()
+    s.close()
