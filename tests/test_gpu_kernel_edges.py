@@ -132,3 +132,97 @@ def test_pcg_sizes(solver, shape):
         assert float(err.norm() / want.norm()) <= bound
         assert not x[lab != 1].any()
     s.close()
+
+
+def _faces_force(lab, p, dx, phi, com):
+    """The face-fraction force and torque over every face of the grid, in FP64 (phi: SDF at given points)."""
+    D, H, W = lab.shape
+    P = np.pad(p.astype(np.float64), 1)
+    L = np.pad(lab, 1)
+    fa = (L == 1) | (L == 2)
+    s, n = np.zeros_like(P), np.zeros_like(P)
+    for d in range(3):
+        for o in (1, -1):
+            s += np.roll(np.where(fa, P, 0.0), o, d)
+            n += np.roll(fa.astype(float), o, d)
+    ext = np.where(L == 3, np.divide(s, n, out=np.zeros_like(s), where=n > 0), P)
+    out = np.zeros(6)
+    ax = [np.arange(m + 1, dtype=np.float32) for m in (W, H, D)]
+    for a in range(3):
+        x = [(c if a == b else c[:-1] + np.float32(0.5)) * np.float32(dx) for b, c in enumerate(ax)]
+        X = np.stack(np.meshgrid(*x, indexing="ij")).astype(np.float32)  # 3, i, j, k
+        th = np.clip(0.5 - phi(X) / dx, 0, 1)
+        idx = np.stack(np.meshgrid(*[np.arange(len(c)) for c in x], indexing="ij"))
+        hi = tuple(idx[2 - b] + 1 for b in range(3))
+        lo = tuple(idx[2 - b] + (0 if 2 - b == a else 1) for b in range(3))
+        ok = (th > 0) & (L[lo] != 0) & (L[hi] != 0)
+        dF = np.where(ok, -th * (ext[hi] - ext[lo]) * dx * dx, 0.0)
+        r = X.astype(np.float64) - np.asarray(com, np.float64)[:, None, None, None]
+        f = np.zeros_like(r)
+        f[a] = dF
+        out[:3] += f.sum((1, 2, 3))
+        out[3:] += np.stack([r[1] * f[2] - r[2] * f[1], r[2] * f[0] - r[0] * f[2], r[0] * f[1] - r[1] * f[0]]).sum((1, 2, 3))
+    return out
+
+
+# a sphere inside; over a corner of the grid; wholly outside it; larger than it; paddles inside and past both ends
+@pytest.mark.parametrize("body", [("s", (0.5, 0.4, 0.5), 0.2), ("s", (0.02, 0.05, 0.9), 0.15), ("s", (2.0, 0.4, 0.5), 0.3),
+                                  ("s", (0.5, 0.4, 0.5), 3.0), ("p", 0.31, 0), ("p", -0.4, 0), ("p", 1.7, 0)])
+def test_body_force_box(body):
+    """The force sums only the faces of the body's box.  Against every face of the grid in FP64: the kernel's theta is
+    FP32 (rounding of phi / dx, about n 2^-24 for the n faces across the body), so 1e-5 of the sum of magnitudes."""
+    from fluidprjct_b200 import capi, scenes
+    n, dx = 24, np.float32(1 / 24)
+    lab = scenes.box_3d(n, n + 5, n - 3, float(dx), 2.0, 0.8, 2.0)
+    kw = dict(dx=float(dx), dt=0.002, solver="pcg_mg", output_format=capi.OUT_NONE, active_body=1)
+    s = capi.Solver(**kw, **(dict(body_radius=body[2], body_pos=body[1], body_density=0.0, body_mass=0.0)
+                             if body[0] == "s" else {}))
+    s.set_labels(lab)
+    if body[0] == "s":
+        s.load_sdf(None)
+        com = np.float32(body[1])
+        phi = lambda X: np.sqrt(((X - com[:, None, None, None]) ** 2).sum(0)) - np.float32(body[2])
+    else:
+        s.set_paddle(body[1], 0.0, 1.0)
+        com = np.float32([body[1], np.float32(0.5 * (n + 5) * float(dx)), np.float32(0.5 * (n - 3) * float(dx))])
+        phi = lambda X: X[0] - com[0]
+    lab = s.labels()
+    p = np.random.default_rng(5).standard_normal(lab.shape).astype(np.float32)
+    s.set_grid(capi.GRID_P, p)
+    s.phase(capi.PHASE_BODY)
+    st = s.stats()
+    got = np.array(list(st["body_force"]) + list(st["body_torque"]))
+    want = _faces_force(lab, p, float(dx), phi, com)
+    scale = np.abs(p).sum() * float(dx) ** 2 * 6 if (lab == 3).any() else 1e-12
+    assert np.abs(got - want).max() <= 1e-5 * scale
+    if body in (("s", (2.0, 0.4, 0.5), 0.3), ("p", -0.4, 0)):
+        assert not got.any()
+    s.close()
+
+
+@pytest.mark.parametrize("cells", [(120, 110), (128, 124), (330, 200)])
+def test_ref2d_scan_sizes(cells):
+    """The 2D step's scans below, at and above one pass of a block (16,384 bins or particles): P2G of one particle per
+    cell at its centre gives each face its own cell's velocity, and no particle is lost or reordered."""
+    from fluidprjct_b200 import capi
+    W, H = cells
+    lab = np.full((H, W), 2, np.uint8)
+    lab[0], lab[-1], lab[:, 0], lab[:, -1] = 0, 0, 0, 0
+    dx = 1.0 / 512
+    s = capi.Solver(dim=2, dx=dx, dt=1e-4, pic_weight=0.0, solver="pcg_mg", scheme="ref2d", output_format=capi.OUT_NONE)
+    s.set_labels(lab)
+    jj, ii = np.meshgrid(np.arange(1, H - 1), np.arange(1, W - 1), indexing="ij")
+    pos = np.stack([(ii.ravel() + 0.5) * dx, (jj.ravel() + 0.5) * dx, 0 * ii.ravel()], 1).astype(np.float32)
+    vel = np.random.default_rng(1).uniform(-1, 1, pos.shape).astype(np.float32)
+    vel[:, 2] = 0
+    s.set_particles(pos, vel)
+    s.phase(capi.PHASE_LABEL)
+    s.phase(capi.PHASE_P2G)
+    u, v = s.grid(capi.GRID_U)[0], s.grid(capi.GRID_V)[0]
+    # neighbours' weights are hat(1 +- 2^-24 W), so at most W 2^-23 of their speed leaks in
+    assert np.abs(u[1:-1, 1:-2] - vel[:, 0].reshape(H - 2, W - 2)).max() <= 8 * W * 2.0 ** -23
+    assert np.abs(v[1:-2, 1:-1] - vel[:, 1].reshape(H - 2, W - 2)).max() <= 8 * W * 2.0 ** -23
+    s.phase(capi.PHASE_CLEANUP)
+    p2, v2 = s.particles()
+    assert np.array_equal(p2, pos) and np.array_equal(v2, vel)
+    s.close()
