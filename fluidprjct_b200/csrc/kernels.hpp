@@ -108,6 +108,11 @@ void launch_label_scan(const uint8_t* base, const uint8_t* body_mark, const int*
 void launch_scatter(const float4* pos, const float4* vel, const int* key, const int* rank, const int* start, int64_t np,
                     float4* pos2, float4* vel2, cudaStream_t st);
 
+// In-place exclusive scan of n ints, the sum to *total; tile_sums has room for
+// scan_tiles(n) ints.  Returns the number of launches.
+int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st);
+int scan_tiles(int64_t n);
+
 // -------- P2G with the fused normalise / save / gravity epilogue (kernels_p2g.cu) --------
 // acc: [nu + nv + nw] (num, den) pairs, zero on entry and left zero (four launches).
 void launch_p2g(const float4* pos, const float4* vel, const int* start, Dims g, float dt, float3 gravity,
@@ -232,14 +237,14 @@ void launch_levelset_labels(const float* solid, const float* fluid, int64_t n, u
 // -------- the reference's own 2D step, scheme "ref2d" (kernels_ref2d.cu) --------
 // Scratch: start[(W+4)*(H+4)+1] (bins of cells -2..W+1 x -2..H+1), list, key,
 // rank [np], keep [np+1], misc[3] (non-finite u and v velocities, capped
-// substep loops).
+// substep loops), tiles (launch_scan over the bins or the keep flags).
 struct R2Scratch {
-    int *start, *list, *key, *rank, *keep, *misc;
+    int *start, *list, *key, *rank, *keep, *misc, *tiles;
 };
 void launch_r2_label(const uint8_t* base, uint8_t* labels, const float4* pos, int64_t np, Dims g, float dx,
                      cudaStream_t st);
-// mode 0: u, v = P2G; mode 1: u*, v* = P2G and u, v = P2G + gravity (5 launches)
-void launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, float dx, float dt, int mode,
+// mode 0: u, v = P2G; mode 1: u*, v* = P2G and u, v = P2G + gravity.  Returns the number of launches.
+int launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, float dx, float dt, int mode,
                    R2Scratch& sc, float* u, float* v, float* us, float* vs, cudaStream_t st);
 void launch_r2_forces(float* u, float* v, Dims g, float dt, cudaStream_t st);
 void launch_r2_project(float* u, float* v, const float* p, const uint8_t* labels, Dims g, float dx, float dt,
@@ -249,8 +254,8 @@ void launch_r2_particles(float4* pos, float4* vel, int64_t np, const float* u, c
                          const float* vs, const uint8_t* labels, Dims g, float dx, float dt, float alpha, int flags,
                          R2Scratch& sc, cudaStream_t st);
 // kept particles of sc.keep, in order, to pos2/vel2 (w = new index); the
-// count lands in sc.keep[np] (2 launches)
-void launch_r2_compact(const float4* pos, const float4* vel, int64_t np, R2Scratch& sc, float4* pos2, float4* vel2,
+// count lands in sc.keep[np].  Returns the number of launches.
+int launch_r2_compact(const float4* pos, const float4* vel, int64_t np, R2Scratch& sc, float4* pos2, float4* vel2,
                        cudaStream_t st);
 
 }  // namespace fp

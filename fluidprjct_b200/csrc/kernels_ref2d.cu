@@ -370,18 +370,19 @@ void launch_r2_label(const uint8_t* base, uint8_t* labels, const float4* pos, in
     if (np > 0) k_r2_label_mark<<<blocks_for(np), 256, 0, st>>>(pos, np, dx, g.W, g.H, labels);
 }
 
-void launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, float dx, float dt, int mode,
+int launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, float dx, float dt, int mode,
                    R2Scratch& sc, float* u, float* v, float* us, float* vs, cudaStream_t st) {
     const int nb = (g.W + 4) * (g.H + 4);
     cudaMemsetAsync(sc.start, 0, sizeof(int) * (nb + 1), st);
     cudaMemsetAsync(sc.misc, 0, sizeof(int) * 2, st);
     if (np > 0) k_r2_bin_count<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, dx, g.W, g.H, sc.start, sc.key, sc.rank,
                                                                 sc.misc);
-    k_scan_single_block<<<1, 1024, 0, st>>>(sc.start, nb, sc.start + nb);
+    const int scans = launch_scan(sc.start, nb, sc.start + nb, sc.tiles, st);
     if (np > 0) k_r2_bin_place<<<blocks_for(np), 256, 0, st>>>(sc.key, sc.rank, sc.start, np, sc.list);
     k_r2_bin_order<<<blocks_for(nb), 256, 0, st>>>(sc.start, nb, sc.list);
     k_r2_p2g<<<blocks_for(int64_t(g.W + 1) * (g.H + 1)), 256, 0, st>>>(pos, vel, sc.start, sc.list, sc.misc, g.W, g.H,
                                                                          dx, dt, mode, u, v, us, vs);
+    return scans + (np > 0 ? 4 : 2);
 }
 
 void launch_r2_forces(float* u, float* v, Dims g, float dt, cudaStream_t st) {
@@ -404,10 +405,11 @@ void launch_r2_particles(float4* pos, float4* vel, int64_t np, const float* u, c
     k_r2_particles<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, a, flags, sc.keep, sc.misc + 2);
 }
 
-void launch_r2_compact(const float4* pos, const float4* vel, int64_t np, R2Scratch& sc, float4* pos2, float4* vel2,
+int launch_r2_compact(const float4* pos, const float4* vel, int64_t np, R2Scratch& sc, float4* pos2, float4* vel2,
                        cudaStream_t st) {
-    k_scan_single_block<<<1, 1024, 0, st>>>(sc.keep, int(np), sc.keep + np);
+    const int scans = launch_scan(sc.keep, int(np), sc.keep + np, sc.tiles, st);
     if (np > 0) k_r2_compact<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, sc.keep, pos2, vel2);
+    return scans + (np > 0);
 }
 
 }  // namespace fp

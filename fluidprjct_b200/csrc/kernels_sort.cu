@@ -107,17 +107,89 @@ __global__ void k_scatter(const float4* __restrict__ pos, const float4* __restri
 }
 }  // namespace
 
-__global__ void k_scan_single_block(int* data, int n, int* total) {
+// 16 consecutive ints per thread and pass, as four vectors (data is 16-byte
+// aligned): one pass of a block covers 16,384.
+__global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, int* total) {
+    constexpr int ITEMS = 16;
     int carry = 0;
-    for (int base = 0; base < n; base += 1024) {
-        int i = base + threadIdx.x;
-        int v = i < n ? data[i] : 0;
+    for (int base = 0; base < n; base += 1024 * ITEMS) {
+        const int e0 = base + int(threadIdx.x) * ITEMS;
+        int v[ITEMS];
+#pragma unroll
+        for (int t = 0; t < ITEMS; t += 4) {
+            if (e0 + t + 3 < n) {
+                const int4 q = *reinterpret_cast<const int4*>(data + e0 + t);
+                v[t] = q.x; v[t + 1] = q.y; v[t + 2] = q.z; v[t + 3] = q.w;
+            } else {
+                for (int u = 0; u < 4; ++u) v[t + u] = e0 + t + u < n ? data[e0 + t + u] : 0;
+            }
+        }
+        int s = 0;
+#pragma unroll
+        for (int t = 0; t < ITEMS; ++t) s += v[t];
         int tot;
-        int pre = block_exclusive_scan<1024>(v, tot);
-        if (i < n) data[i] = carry + pre;
+        int pre = carry + block_exclusive_scan<1024>(s, tot);
+#pragma unroll
+        for (int t = 0; t < ITEMS; ++t) {
+            const int x = v[t];
+            v[t] = pre;
+            pre += x;
+        }
+#pragma unroll
+        for (int t = 0; t < ITEMS; t += 4) {
+            if (e0 + t + 3 < n) *reinterpret_cast<int4*>(data + e0 + t) = make_int4(v[t], v[t + 1], v[t + 2], v[t + 3]);
+            else
+                for (int u = 0; u < 4; ++u)
+                    if (e0 + t + u < n) data[e0 + t + u] = v[t + u];
+        }
         carry += tot;
     }
     if (threadIdx.x == 0 && total) *total = carry;
+}
+
+// The tile sums of data, and the scan of each tile from its offset.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tile_sums(const int* __restrict__ data, int n,
+                                                               int* __restrict__ tile_sums) {
+    const int e0 = (blockIdx.x * SCAN_BLOCK + threadIdx.x) * SCAN_ITEMS;
+    int s = 0;
+#pragma unroll
+    for (int t = 0; t < SCAN_ITEMS; ++t) s += e0 + t < n ? data[e0 + t] : 0;
+    int total;
+    block_exclusive_scan<SCAN_BLOCK>(s, total);
+    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(int* __restrict__ data, int n,
+                                                           const int* __restrict__ tile_offsets) {
+    const int e0 = (blockIdx.x * SCAN_BLOCK + threadIdx.x) * SCAN_ITEMS;
+    int v[SCAN_ITEMS];
+    int s = 0;
+#pragma unroll
+    for (int t = 0; t < SCAN_ITEMS; ++t) {
+        v[t] = e0 + t < n ? data[e0 + t] : 0;
+        s += v[t];
+    }
+    int total;
+    int pre = block_exclusive_scan<SCAN_BLOCK>(s, total) + tile_offsets[blockIdx.x];
+#pragma unroll
+    for (int t = 0; t < SCAN_ITEMS; ++t) {
+        if (e0 + t < n) data[e0 + t] = pre;
+        pre += v[t];
+    }
+}
+
+int scan_tiles(int64_t n) { return int((n + SCAN_TILE - 1) / SCAN_TILE); }
+
+int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st) {
+    // One pass of a single block, or the whole chip's three launches.
+    if (n <= 1024 * 16) {
+        k_scan_single_block<<<1, 1024, 0, st>>>(data, n, total);
+        return 1;
+    }
+    const int tiles = scan_tiles(n);
+    k_scan_tile_sums<<<tiles, SCAN_BLOCK, 0, st>>>(data, n, tile_sums);
+    k_scan_single_block<<<1, 1024, 0, st>>>(tile_sums, tiles, total);
+    k_scan_tiles<<<tiles, SCAN_BLOCK, 0, st>>>(data, n, tile_sums);
+    return 3;
 }
 
 void launch_bin(const float4* pos, int64_t np, Dims g, int* counts, int* key, int* rank, cudaStream_t st) {

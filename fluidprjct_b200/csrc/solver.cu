@@ -179,7 +179,7 @@ struct fp_solver {
     int* h_bad = nullptr;
     // scheme ref2d: bins over (W+4)*(H+4) cells, particle lists and keep flags
     R2Scratch r2{};
-    int r2_nb = 0;
+    int r2_nb = 0, r2_tiles = 0;
     int64_t r2_cap = 0;
     int* h_r2 = nullptr;    // pinned: [0] particles kept, [1] capped substep loops
     int* d_extmark = nullptr;  // wavefront markers of the velocity extrapolation (largest face grid)
@@ -206,8 +206,8 @@ struct fp_solver {
 namespace {
 
 void free_r2(fp_solver* s) {
-    dfree(s->r2.start); dfree(s->r2.misc);
-    s->r2_nb = 0;
+    dfree(s->r2.start); dfree(s->r2.misc); dfree(s->r2.tiles);
+    s->r2_nb = s->r2_tiles = 0;
 }
 
 void free_grid(fp_solver* s) {
@@ -763,6 +763,14 @@ int r2_alloc(fp_solver* s) {
         if (e != cudaSuccess) { free_r2(s); return s->cuda_fail(e, "device allocation of the 2D bins"); }
         s->r2_nb = nb;
     }
+    const int tiles = scan_tiles(std::max<int64_t>(nb, s->cap));
+    if (s->r2_tiles < tiles) {
+        dfree(s->r2.tiles);
+        s->r2_tiles = 0;
+        e = dalloc(&s->r2.tiles, size_t(tiles));
+        if (e != cudaSuccess) return s->cuda_fail(e, "device allocation of the 2D scan");
+        s->r2_tiles = tiles;
+    }
     if (s->r2_cap < s->cap || !s->r2.list) {
         dfree(s->r2.list); dfree(s->r2.keep);
         const int64_t n = std::max<int64_t>(s->cap, 1);
@@ -782,9 +790,8 @@ void r2_label(fp_solver* s) {
 }
 
 void r2_p2g(fp_solver* s, int mode) {
-    launch_r2_p2g(s->d_pos, s->d_vel, s->np, s->g, s->cfg.dx, s->cfg.dt, mode, s->r2, s->d_u, s->d_v, s->d_us, s->d_vs,
-                  s->st);
-    s->launches += s->np > 0 ? 5 : 3;
+    s->launches += launch_r2_p2g(s->d_pos, s->d_vel, s->np, s->g, s->cfg.dx, s->cfg.dt, mode, s->r2, s->d_u, s->d_v,
+                                 s->d_us, s->d_vs, s->st);
 }
 
 int r2_pressure(fp_solver* s) {
@@ -809,8 +816,7 @@ void r2_particles(fp_solver* s, int flags) {
 // kept), read the new count and the capped-loop count.
 int r2_compact(fp_solver* s, bool advected) {
     if (s->np == 0) return FP_OK;
-    launch_r2_compact(s->d_pos, s->d_vel, s->np, s->r2, s->d_pos2, s->d_vel2, s->st);
-    s->launches += 2;
+    s->launches += launch_r2_compact(s->d_pos, s->d_vel, s->np, s->r2, s->d_pos2, s->d_vel2, s->st);
     cudaMemcpyAsync(s->h_r2, s->r2.keep + s->np, sizeof(int), cudaMemcpyDeviceToHost, s->st);
     if (advected) cudaMemcpyAsync(s->h_r2 + 1, s->r2.misc + 2, sizeof(int), cudaMemcpyDeviceToHost, s->st);
     cudaError_t e = cudaStreamSynchronize(s->st);
