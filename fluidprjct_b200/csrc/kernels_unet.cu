@@ -1,20 +1,9 @@
 // kernels_unet.cu -- kernels of the learned pressure preconditioner (a 3D
 // U-Net; the layer table is in unet.hpp).
 //
-// The forward and backward-data convolutions run on tcgen05
-// (kernels_unet_tma.cu).  This file holds the rest, with the weight gradient
-// on the BF16 mma.sync path (m16n8k16, FP32 accumulation):
-//   k_corr3  weight gradients dw[t][co][ci] = sum_v g[v][co] x[v+off(t)][ci]
-//            (M = COUT, N = CIN, K = voxels), over bricks of 8x8x4 voxels
-//            whose zero-padded input halo (10x10x6, every input channel) is
-//            staged with cp.async.  The input may be the concatenation
-//            [up2(xa) | xb] of a 2x-upsampled coarse tensor and a same-level
-//            one: the upsampling is an index shift in the halo load.  Each
-//            CTA accumulates its tap group over its bricks in registers and
-//            writes one partial.  The partials are summed in a fixed order,
-//            so gradients are deterministic.
-// Smem rows are padded by 16 bytes, so each 8-row ldmatrix phase hits eight
-// distinct 16-byte bank groups.
+// The convolutions and their weight gradients run on tcgen05
+// (kernels_unet_tma.cu).  This file holds the rest: input and output, pooling,
+// the element-wise parts of the backward pass, the loss and Adam.
 #include <algorithm>
 #include <cstdio>
 
@@ -25,133 +14,7 @@ namespace fp {
 namespace unet {
 namespace {
 
-constexpr int BX = 8, BY = 8, BZ = 4;
-constexpr int HX = BX + 2, HY = BY + 2, HZ = BZ + 2, HALO = HX * HY * HZ;  // 600
 constexpr int THREADS = 256;
-constexpr int BRICK = BX * BY * BZ;  // 256 voxels = 16 M-tiles of 16
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool pred) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src),
-                 "r"(pred ? 16 : 0));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void ldsm_x4_t(unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3, unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2_t(unsigned& r0, unsigned& r1, unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-__device__ __forceinline__ void mma16816(float* c, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
-                                         unsigned b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Stage the zero-padded input halo of the brick at (x0, y0, z0) (its -1
-// corner) into sx, rows of RS bf16.  Channels [0, CA) come from the coarse
-// tensor at (x>>1, y>>1, z>>1), channels [CA, CA+CB) from the same level.
-template <int CA, int CB, int RS>
-__device__ __forceinline__ void load_halo(bf16* sx, const bf16* __restrict__ xa, const bf16* __restrict__ xb,
-                                          const Lvl& lv, const Lvl& lc, int x0, int y0, int z0) {
-    constexpr int CH = (CA + CB) / 8;
-    for (int i = threadIdx.x; i < HALO * CH; i += THREADS) {
-        const int ch = i % CH, hv = i / CH;
-        const int gx = x0 + hv % HX, gy = y0 + (hv / HX) % HY, gz = z0 + hv / (HX * HY);
-        const bool in = gx >= 0 && gx < lv.W && gy >= 0 && gy < lv.H && gz >= 0 && gz < lv.D;
-        const bf16* src;
-        if (CA > 0 && ch * 8 < CA)
-            src = in ? xa + blk8(lc.n(), (int64_t(gz >> 1) * lc.H + (gy >> 1)) * lc.W + (gx >> 1), ch) : xa;
-        else
-            src = in ? xb + blk8(lv.n(), (int64_t(gz) * lv.H + gy) * lv.W + gx, ch - CA / 8) : xb;
-        cp_async16(sx + hv * RS + ch * 8, src, in);
-    }
-}
-
-template <int CA, int CB, int COUT, int TPC>
-__global__ void __launch_bounds__(THREADS) k_corr3(CorrArgs a) {
-    constexpr int CIN = CA + CB;
-    constexpr int RS = CIN + 8;
-    constexpr int GS = COUT + 8;
-    constexpr int TILES = TPC * (COUT / 16) * (CIN / 8);
-    constexpr int NTW = (TILES + 7) / 8;
-    static_assert(27 % TPC == 0 && COUT % 16 == 0 && CIN % 16 == 0, "tiling");
-    extern __shared__ __align__(16) unsigned char smem[];
-    bf16* sx = reinterpret_cast<bf16*>(smem);
-    bf16* sg = sx + HALO * RS;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tap0 = blockIdx.y * TPC;
-    const int nbx = (a.lv.W + BX - 1) / BX, nby = (a.lv.H + BY - 1) / BY, nbz = (a.lv.D + BZ - 1) / BZ;
-    const int nbricks = nbx * nby * nbz;
-    // A (= g^T, 16 channels x 16 voxels) via ldmatrix.trans: voxel row, channel offset
-    const int akr = (lane & 7) + 8 * (lane >> 4), amoff = 8 * ((lane >> 3) & 1);
-    // B (= shifted x, 16 voxels x 8 channels) via ldmatrix.x2.trans
-    const int bkr = (lane & 7) + 8 * ((lane >> 3) & 1);
-    const unsigned sx_s = smem_addr(sx), sg_s = smem_addr(sg);
-
-    float acc[NTW][4];
-#pragma unroll
-    for (int i = 0; i < NTW; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-
-    for (int brick = blockIdx.x; brick < nbricks; brick += gridDim.x) {
-        const int bx = brick % nbx, by = (brick / nbx) % nby, bz = brick / (nbx * nby);
-        load_halo<CA, CB, RS>(sx, a.xa, a.xb, a.lv, a.lc, bx * BX - 1, by * BY - 1, bz * BZ - 1);
-        for (int i = tid; i < BRICK * (COUT / 8); i += THREADS) {
-            const int ch = i % (COUT / 8), v = i / (COUT / 8);
-            const int gx = bx * BX + (v & 7), gy = by * BY + ((v >> 3) & 7), gz = bz * BZ + (v >> 6);
-            const bool in = gx < a.lv.W && gy < a.lv.H && gz < a.lv.D;
-            const bf16* src = in ? a.g + blk8(a.lv.n(), (int64_t(gz) * a.lv.H + gy) * a.lv.W + gx, ch) : a.g;
-            cp_async16(sg + v * GS + ch * 8, src, in);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-#pragma unroll 1
-        for (int ks = 0; ks < 16; ++ks) {
-            const int z = ks >> 2, yy = (ks & 3) * 2;
-            const int av = (z * BY + yy + (akr >> 3)) * BX + (akr & 7);
-            const int bh = ((z + 1) * HY + (yy + (bkr >> 3) + 1)) * HX + ((bkr & 7) + 1);
-#pragma unroll
-            for (int i = 0; i < NTW; ++i) {
-                const int tile = warp + 8 * i;
-                if (TILES % 8 != 0 && tile >= TILES) continue;
-                const int tl = tile / ((COUT / 16) * (CIN / 8));
-                const int rem = tile % ((COUT / 16) * (CIN / 8));
-                const int cot = rem / (CIN / 8), cit = rem % (CIN / 8);
-                const int tap = tap0 + tl;
-                const int toff = ((tap / 9 - 1) * HY + ((tap / 3) % 3 - 1)) * HX + (tap % 3 - 1);
-                unsigned a0, a1, a2, a3, b0, b1;
-                ldsm_x4_t(a0, a1, a2, a3, sg_s + (av * GS + cot * 16 + amoff) * 2);
-                ldsm_x2_t(b0, b1, sx_s + ((bh + toff) * RS + cit * 8) * 2);
-                mma16816(acc[i], a0, a1, a2, a3, b0, b1);
-            }
-        }
-        __syncthreads();
-    }
-    const int g = lane >> 2, tq = lane & 3;
-    float* part = a.part + int64_t(blockIdx.x) * 27 * COUT * CIN;
-#pragma unroll
-    for (int i = 0; i < NTW; ++i) {
-        const int tile = warp + 8 * i;
-        if (tile >= TILES) continue;
-        const int tl = tile / ((COUT / 16) * (CIN / 8));
-        const int rem = tile % ((COUT / 16) * (CIN / 8));
-        const int cot = rem / (CIN / 8), cit = rem % (CIN / 8);
-        const int tap = tap0 + tl;
-        const int co = cot * 16 + g, ci = cit * 8 + 2 * tq;
-        float* p0 = part + (int64_t(tap) * COUT + co) * CIN + ci;
-        p0[0] = acc[i][0];
-        p0[1] = acc[i][1];
-        p0[8 * CIN] = acc[i][2];
-        p0[8 * CIN + 1] = acc[i][3];
-    }
-}
 
 __global__ void k_reduce_partials(const float* __restrict__ part, int nblk, int64_t n, float* __restrict__ out) {
     for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += int64_t(gridDim.x) * blockDim.x) {
@@ -489,46 +352,7 @@ int sm_count() {
     return n > 0 ? n : 148;
 }
 
-int nbricks_of(const Lvl& lv) {
-    return ((lv.W + BX - 1) / BX) * ((lv.H + BY - 1) / BY) * ((lv.D + BZ - 1) / BZ);
-}
-
-template <int CA, int CB, int COUT, int TPC>
-int run_corr(const CorrArgs& a, int nblk, cudaStream_t st) {
-    constexpr int CIN = CA + CB;
-    constexpr size_t smem = size_t(HALO * (CIN + 8) + BRICK * (COUT + 8)) * sizeof(bf16);
-    static DeviceMemo memo;
-    auto kern = k_corr3<CA, CB, COUT, TPC>;
-    memo.get([&](int) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        return 1;
-    });
-    kern<<<dim3(nblk, 27 / TPC), THREADS, smem, st>>>(a);
-    return int(cudaPeekAtLastError());
-}
-
-constexpr int kTpc[kLayers] = {27, 27, 9, 9, 3, 3, 3, 9, 9, 27};
-
 }  // namespace
-
-int corr_blocks(int layer, const Lvl& lv) {
-    const int groups = 27 / kTpc[layer];
-    return std::max(1, std::min(nbricks_of(lv), 2 * sm_count() / groups));
-}
-
-int corr_layer(int layer, const CorrArgs& a, int nblk, cudaStream_t st) {
-    switch (layer) {
-        case 0: case 1: case 9: return run_corr<0, 16, 16, 27>(a, nblk, st);
-        case 2: return run_corr<0, 16, 32, 9>(a, nblk, st);
-        case 3: case 7: return run_corr<0, 32, 32, 9>(a, nblk, st);
-        case 4: return run_corr<0, 32, 64, 3>(a, nblk, st);
-        case 5: return run_corr<0, 64, 64, 3>(a, nblk, st);
-        case 6: return run_corr<64, 32, 32, 3>(a, nblk, st);
-        case 8: return run_corr<32, 16, 16, 9>(a, nblk, st);
-    }
-    return int(cudaErrorInvalidValue);
-}
 
 void reduce_partials(const float* part, int nblk, int64_t n, float* out, cudaStream_t st) {
     const int blocks = int(std::min<int64_t>((n + 255) / 256, 4 * sm_count()));

@@ -143,16 +143,11 @@ int conv_bwd(fp_unet* u, int l, const bf16* g, const bf16* mask, bf16* y, cudaSt
     return conv_backward_layer_tma(l, g, a, st);
 }
 
-int wgrad(fp_unet* u, int l, const bf16* xa, const bf16* xb, const bf16* g, cudaStream_t st) {
-    CorrArgs a{};
-    a.xa = xa;
-    a.xb = xb;
-    a.g = g;
-    a.part = u->part;
-    a.lv = u->L[kSpec[l].level];
-    a.lc = kSpec[l].level < 2 ? u->L[kSpec[l].level + 1] : a.lv;
-    const int nblk = corr_blocks(l, a.lv);
-    int e = corr_layer(l, a, nblk, st);
+// x: the layer's whole input (a decoder layer's is the forward pass's concatenation)
+int wgrad(fp_unet* u, int l, const bf16* x, const bf16* g, cudaStream_t st) {
+    const Lvl& lv = u->L[kSpec[l].level];
+    const int nblk = corr_blocks(l, lv);
+    const int e = corr_layer(l, x, g, lv, u->part, nblk, u->d_status, st);
     reduce_partials(u->part, nblk, layer_size(l), u->grad + layer_offset(l), st);
     return e;
 }
@@ -165,29 +160,29 @@ int backward(fp_unet* u, const uint8_t* labels, const float* p, cudaStream_t st)
                          u->hpart, u->hblk, st);
     reduce_partials(u->hpart, u->hblk, kHead, u->grad + layer_offset(kLayers), st);
     int e = 0;
-    e |= wgrad(u, 9, nullptr, u->d0a, u->g9, st);
+    e |= wgrad(u, 9, u->d0a, u->g9, st);
     e |= conv_bwd(u, 9, u->g9, u->d0a, u->g8, st);
-    e |= wgrad(u, 8, u->d1, u->e0, u->g8, st);
+    e |= wgrad(u, 8, u->cat8, u->g8, st);
     e |= conv_bwd(u, 8, u->g8, nullptr, u->raw8, st);
     launch_sum_children_mask(u->raw8, L[0], 48, 32, u->d1, u->g7, st);
-    e |= wgrad(u, 7, nullptr, u->d1a, u->g7, st);
+    e |= wgrad(u, 7, u->d1a, u->g7, st);
     e |= conv_bwd(u, 7, u->g7, u->d1a, u->g6, st);
-    e |= wgrad(u, 6, u->e2, u->e1, u->g6, st);
+    e |= wgrad(u, 6, u->cat6, u->g6, st);
     e |= conv_bwd(u, 6, u->g6, nullptr, u->raw6, st);
     launch_sum_children_mask(u->raw6, L[1], 96, 64, u->e2, u->g5, st);
-    e |= wgrad(u, 5, nullptr, u->a2, u->g5, st);
+    e |= wgrad(u, 5, u->a2, u->g5, st);
     e |= conv_bwd(u, 5, u->g5, u->a2, u->g4, st);
-    e |= wgrad(u, 4, nullptr, u->q1, u->g4, st);
+    e |= wgrad(u, 4, u->q1, u->g4, st);
     e |= conv_bwd(u, 4, u->g4, nullptr, u->gq1, st);
     launch_skip_combine(u->raw6, L[1], 96, 64, 32, u->gq1, u->e1, u->g3, st);
-    e |= wgrad(u, 3, nullptr, u->a1, u->g3, st);
+    e |= wgrad(u, 3, u->a1, u->g3, st);
     e |= conv_bwd(u, 3, u->g3, u->a1, u->g2, st);
-    e |= wgrad(u, 2, nullptr, u->q0, u->g2, st);
+    e |= wgrad(u, 2, u->q0, u->g2, st);
     e |= conv_bwd(u, 2, u->g2, nullptr, u->gq0, st);
     launch_skip_combine(u->raw8, L[0], 48, 32, 16, u->gq0, u->e0, u->g1, st);
-    e |= wgrad(u, 1, nullptr, u->a0, u->g1, st);
+    e |= wgrad(u, 1, u->a0, u->g1, st);
     e |= conv_bwd(u, 1, u->g1, u->a0, u->g0, st);
-    e |= wgrad(u, 0, nullptr, u->X0, u->g0, st);
+    e |= wgrad(u, 0, u->X0, u->g0, st);
     return e;
 }
 

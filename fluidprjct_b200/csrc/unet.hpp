@@ -52,15 +52,6 @@ struct Lvl {
 // followed by B's.
 __host__ __device__ inline int64_t blk8(int64_t n, int64_t v, int cb) { return (int64_t(cb) * n + v) * 8; }
 
-// Arguments of the weight-gradient kernel: dw[t][co][ci] = sum_v g[v][co] x[v + off(t)][ci].
-struct CorrArgs {
-    const bf16* xa;
-    const bf16* xb;
-    const bf16* g;         // [V][COUT]
-    float* part;           // [gridDim.x][27][COUT][CIN] partial sums
-    Lvl lv, lc;
-};
-
 enum { EPI_RELU = 0, EPI_MASK = 1, EPI_RAW = 2, EPI_HEAD = 3 };
 
 // Arguments of the TMA-fed convolution (kernels_unet_tma.cu); its input is
@@ -79,9 +70,14 @@ int conv_backward_layer_tma(int layer, const bf16* in, const TmaConvArgs& a, cud
 // The first ca / 8 channel blocks of out = up2(coarse) on the fine level.
 void launch_upcat(const bf16* coarse, int ca, Lvl fine, bf16* out, cudaStream_t st);
 
-// Launchers (kernels_unet.cu).  Each returns 0 or a cudaError_t value.
-int corr_layer(int layer, const CorrArgs& a, int nblk, cudaStream_t st);
-int corr_blocks(int layer, const Lvl& lv);                               // gridDim.x for corr_layer
+// Weight gradient of a layer, dw[t][co][ci] = sum_v g[v][co] x[v + off(t)][ci],
+// as nblk = corr_blocks() partial sums [nblk][27][COUT][CIN] (to be added by
+// reduce_partials); x is the layer's whole input.  Returns 0 or a cudaError_t.
+int corr_blocks(int layer, const Lvl& lv);
+int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* part, int nblk, int* status,
+               cudaStream_t st);
+
+// Launchers (kernels_unet.cu).
 void reduce_partials(const float* part, int nblk, int64_t n, float* out, cudaStream_t st);
 
 void launch_rhs_scale(const uint8_t* labels, const float* rhs, Lvl real, double* red, float* scal, cudaStream_t st);

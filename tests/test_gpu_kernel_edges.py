@@ -226,3 +226,36 @@ def test_ref2d_scan_sizes(cells):
     p2, v2 = s.particles()
     assert np.array_equal(p2, pos) and np.array_equal(v2, vel)
     s.close()
+
+
+# one voxel on the coarsest level; whole 8 x 16 x 8 bricks; remainders in every axis; several bricks in z
+@pytest.mark.parametrize("shape", [(4, 4, 4), (8, 16, 32), (12, 20, 36), (28, 36, 20), (40, 12, 72)])
+def test_unet_gradient_tiles(shape):
+    """Every layer's weight gradient against the oracle, which rounds to BF16 where the kernels do: only the order of
+    FP32 sums and the BF16 flips it causes differ.  A flip is 2^-8 of one activation; 3e-2 and a cosine of 0.999 are
+    the bounds that the network's other gradient test uses for them."""
+    import torch
+    from fluidprjct_b200 import capi
+    from oracle import unet_oracle as U
+    D, H, W = shape
+    rng = np.random.default_rng(W + 10 * H + 100 * D)
+    lab = np.where(rng.random(shape) < 0.8, 1, rng.integers(0, 4, shape)).astype(np.uint8)
+    rhs, p = [np.where(lab == 1, rng.standard_normal(shape), 0).astype(np.float32) for _ in range(2)]
+    th = U.init_params(D + H)
+    net = capi.UNet(W, H, D, train=True)
+    net.set_params(th)
+    t = [torch.from_numpy(a).cuda() for a in (lab, rhs, p)]
+    torch.cuda.synchronize()
+    loss, g = net.loss_grad(*[a.data_ptr() for a in t])
+    loss_ref, g_ref = U.loss_grad(th, lab, rhs, p, bf=True)
+    assert abs(loss - loss_ref) <= 1e-3 * loss_ref
+    at = np.cumsum([0] + U.layer_sizes() + [U.HEAD])
+    for a, b in zip(at[:-1], at[1:]):
+        x, y = g[a:b].astype(np.float64), g_ref[a:b].astype(np.float64)
+        if not np.linalg.norm(y):
+            assert not x.any()
+            continue
+        assert np.linalg.norm(x - y) <= 3e-2 * np.linalg.norm(y)
+        assert x @ y >= 0.999 * np.linalg.norm(x) * np.linalg.norm(y)
+    loss2, g2 = net.loss_grad(*[a.data_ptr() for a in t])
+    assert loss2 == loss and np.array_equal(g2, g)
