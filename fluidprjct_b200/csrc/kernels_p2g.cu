@@ -8,22 +8,28 @@
 // (:700-761, gravity on every face with the x > (float)INT_MIN test).
 //
 // B200 design: particles are sorted by cell, and each CTA owns a brick of
-// BX x BY x BZ cells.  One thread per cell walks that cell's (contiguous)
-// particles once and sums their contributions to the 2 x 3 x 3 faces the cell
-// can reach in registers; it then adds them into shared-memory accumulators
-// covering the faces the brick's cells reach (one atomic per face and cell
-// instead of one per particle and corner).  Each brick adds its accumulated
-// (num, den) pairs into a global FP32 pair array with one vector reduction
-// per face, so every particle is walked once (a brick that instead re-walks
-// a one-cell halo to own its faces outright walks each particle 1.76 times
-// on average for 16 x 8 x 8 bricks); empty bricks return at once.  Small
-// bricks balance the SMs: the dam break's ~640 full 16 x 8 x 8 bricks filled
-// 1.4 waves of three CTAs per SM (0.232 ms for the phase at 128^3, 0.198 with
-// 8 x 8 x 8).  The default is 8 x 8 x 4 cells, one per thread of a 128-thread
-// CTA, eight CTAs per SM (0.180 ms; 8 x 8 x 8 with 256 threads at four per SM
-// 0.186, 8 x 4 x 4 0.182).  A second,
-// elementwise kernel divides, saves and adds gravity, and zeroes the pair
-// array for the next step.
+// BX x BY x BZ cells with one group of BX * BY threads per velocity component.
+// A thread walks a cell's (contiguous) particles once and sums its component's
+// contributions to the 2 x 3 x 3 faces the cell can reach in registers; the
+// group then adds them into shared-memory accumulators covering the faces the
+// brick's cells reach, one face offset at a time: distinct cells write
+// distinct faces at the same offset, so plain adds between group barriers do
+// (an FP32 shared-memory atomic is a compare-and-swap loop).  Each brick adds
+// its accumulated (num, den) pairs into a global FP32 pair array with one
+// vector reduction per face, so every particle is walked once per component (a
+// brick that instead re-walks a one-cell halo to own its faces outright walks
+// each particle 1.76 times on average for 16 x 8 x 8 bricks); empty bricks
+// return at once.  A second, elementwise kernel divides, saves and adds
+// gravity, and zeroes the pair array for the next step.
+//
+// Bound by the latency of the walk's particle loads, so by occupancy.  The
+// accumulate kernel takes 136 us for the 128^3 dam break (3.8 M particles),
+// 412 for the 160^3 pool (11 M, dx not a power of two), 508 for the
+// 256 x 128 x 256 tank (17.5 M) and 19 for a 50^3 box; one thread per cell for
+// all three components in turn, with shared-memory atomics, took 138, 420, 567
+// and 33 (a small grid's bricks then leave most of the chip idle).  8 x 8 x 4
+// bricks: 141, 430, 561 and 23 at five CTAs of 192 per SM, 165, 504 and 650 at
+// four.
 #include "kernels.hpp"
 
 namespace fp {
@@ -65,12 +71,12 @@ __device__ __forceinline__ void axis3(int s0, int base, float f, float (&w)[3]) 
     w[2] = lo ? 0.0f : f;
 }
 
-// Accumulates one velocity component of the particles [q0, q1) of cell
-// (ci, cj, ck) over the 2 x 3 x 3 faces that cell can reach (2 along the
-// component's own axis, whose base face is always the cell's), and adds them
-// into the brick's shared-memory accumulators, whose face (ex0, ey0, ez0) is
-// slot 0 (strides lsx, lsy).  COMP selects the component and its base-index
-// rules (AccumulateVelocities::operator(), FluidSolver3D.cu:469-574).  Weights are
+// Sums one velocity component of the particles [q0, q1) of cell (ci, cj, ck)
+// over the 2 x 3 x 3 faces that cell can reach (2 along the component's own
+// axis, whose base face is always the cell's): an and ad hold num and den,
+// pair = the component axis' two faces, index = the other two axes' slots.
+// COMP selects the component and its base-index rules
+// (AccumulateVelocities::operator(), FluidSolver3D.cu:469-574).  Weights are
 // (wx*wy)*wz as in the reference; the two faces along the component's axis
 // are one packed pair, so each particle costs 12 packed multiplies and 9
 // packed FMAs and adds per component.  num accumulates vel*wgt with one fused
@@ -81,14 +87,12 @@ template <int COMP>
 __device__ __forceinline__ float comp_of(const float4& v) { return COMP == 0 ? v.x : (COMP == 1 ? v.y : v.z); }
 
 template <int COMP, bool P2>
-__device__ __forceinline__ void splat_cell(const float4* __restrict__ pos, const float4* __restrict__ vel, int q0,
-                                           int q1, int ci, int cj, int ck, const Dims& g, float* s_num, float* s_den,
-                                           int ex0, int ey0, int ez0, int lsx, int lsy) {
+__device__ __forceinline__ void sum_cell(const float4* __restrict__ pos, const float4* __restrict__ vel, int q0, int q1,
+                                         int ci, int cj, int ck, const Dims& g, float2 (&an)[9], float2 (&ad)[9]) {
     const int W = g.W, H = g.H, D = g.D;
     // first face of each axis' slot range: the cell's own face on the
     // component's axis, the face below the cell on the other two
     const int sx0 = COMP == 0 ? ci : ci - 1, sy0 = COMP == 1 ? cj : cj - 1, sz0 = COMP == 2 ? ck : ck - 1;
-    float2 an[9], ad[9];  // pair = the component axis' two faces; index = the other two axes' slots
 #pragma unroll
     for (int m = 0; m < 9; ++m) { an[m] = make_float2(0.0f, 0.0f); ad[m] = make_float2(0.0f, 0.0f); }
     // (unrolling this walk by 2 or 4 measured slower: the larger code missed
@@ -163,110 +167,103 @@ __device__ __forceinline__ void splat_cell(const float4* __restrict__ pos, const
                 }
         }
     }
-    // into shared memory: slot m of the pair is face +0 / +1 along the
-    // component's axis; every slot lies inside the brick's reach region
-#pragma unroll
-    for (int m = 0; m < 9; ++m)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int o1 = m % 3, o2 = m / 3;
-            const float num = e ? an[m].y : an[m].x, den = e ? ad[m].y : ad[m].x;
-            if (den == 0.0f) continue;
-            const int fi = COMP == 0 ? sx0 + e : sx0 + o1;
-            const int fj = COMP == 1 ? sy0 + e : sy0 + (COMP == 0 ? o1 : o2);
-            const int fk = COMP == 2 ? sz0 + e : sz0 + o2;
-            const int sidx = (fi - ex0) + lsx * ((fj - ey0) + lsy * (fk - ez0));
-            atomicAdd(&s_num[sidx], num);
-            atomicAdd(&s_den[sidx], den);
-        }
 }
 
-// The faces the cells of a brick [i0, i0+BX) x [j0, j0+BY) x [k0, k0+BZ)
-// reach, per component: along the component's own axis the brick's faces
-// and the far one (N+1), along the other two one more on each side (N+2).
+// CTAs per SM that the register budget must allow (P2G_MIN_BLOCKS, a build
+// tunable): the walk over a cell's particles waits on their loads, so
+// occupancy decides.  At 64 registers, ten CTAs of 96 threads.
+#ifndef P2G_MIN_BLOCKS
+#define P2G_MIN_BLOCKS 10
+#endif
+
+// The faces around a brick: one more than its cells on each side of every axis
+// (one less is reached along a component's own axis).
 template <int BX, int BY, int BZ>
 struct Reach {
-    static constexpr int UX = BX + 1, UY = BY + 2, UZ = BZ + 2;
-    static constexpr int VX = BX + 2, VY = BY + 1, VZ = BZ + 2;
-    static constexpr int WX = BX + 2, WY = BY + 2, WZ = BZ + 1;
-    static constexpr int NU = UX * UY * UZ, NV = VX * VY * VZ, NW = WX * WY * WZ, N = NU + NV + NW;
+    static constexpr int X = BX + 2, Y = BY + 2, Z = BZ + 2, N = X * Y * Z;
 };
 
-// CTAs per SM that the register budget must allow (P2G_MIN_BLOCKS, a build
-// tunable): the walk over a cell's particles is latency-bound, so occupancy
-// and spills trade against each other.  With 256-thread 8 x 8 x 8 bricks at
-// 128^3, four per SM (64 registers, a 12-byte spill) took the phase to 0.186
-// ms; three (78 registers) gave 0.202, two 0.220, and five and six spilled
-// (0.30, 0.49 ms).  The default is 64 registers for the 128-thread CTAs.
-#ifndef P2G_MIN_BLOCKS
-#define P2G_MIN_BLOCKS 8
-#endif
+// One component of a brick, by the BX * BY threads of one group: thread t
+// takes cell (t % BX, t / BX) of every z slab in turn.
+template <int COMP, int BX, int BY, int BZ, bool P2>
+__device__ __forceinline__ void brick_component(const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                                const int* __restrict__ start, const Dims& g, int i0, int j0, int k0,
+                                                float2* s_acc) {
+    using R = Reach<BX, BY, BZ>;
+    const int t = int(threadIdx.x) % (BX * BY), lx = t % BX, ly = t / BX, ci = i0 + lx, cj = j0 + ly;
+    const bool in = ci < g.W && cj < g.H;
+#pragma unroll 1
+    for (int lz = 0; lz < BZ; ++lz) {
+        const int ck = k0 + lz, c = ci + cj * g.W + ck * g.W * g.H;
+        const bool ok = in && ck < g.D;
+        const int q0 = ok ? start[c] : 0, q1 = ok ? start[c + 1] : 0;
+        float2 an[9], ad[9];
+        sum_cell<COMP, P2>(pos, vel, q0, q1, ci, cj, ck, g, an, ad);
+        float2* s = s_acc + COMP * R::N + lx + ly * R::X + lz * R::X * R::Y;
+#pragma unroll
+        for (int m = 0; m < 9; ++m)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int o1 = m % 3, o2 = m / 3;
+                const int ox = COMP == 0 ? e : o1, oy = COMP == 1 ? e : (COMP == 0 ? o1 : o2), oz = COMP == 2 ? e : o2;
+                if (q1 > q0) {
+                    float2& f = s[ox + oy * R::X + oz * R::X * R::Y];
+                    const float2 v = f;
+                    f = make_float2(v.x + (e ? an[m].y : an[m].x), v.y + (e ? ad[m].y : ad[m].x));
+                }
+                asm volatile("bar.sync %0, %1;\n" ::"n"(COMP + 1), "n"(BX * BY) : "memory");
+            }
+    }
+}
 
 // Pass 1: one CTA per brick.  acc holds (num, den) pairs for the u, v and w
 // faces back to back ([nu | nv | nw]); it is zero on entry except for what
 // other bricks of this launch add.
-template <int BX, int BY, int BZ, int NT, bool P2>
-__global__ void __launch_bounds__(NT, P2G_MIN_BLOCKS) k_p2g_accum(const float4* __restrict__ pos,
-                                                                  const float4* __restrict__ vel,
-                                                                  const int* __restrict__ start, Dims g,
-                                                                  float2* __restrict__ acc) {
+template <int BX, int BY, int BZ, bool P2>
+__global__ void __launch_bounds__(3 * BX * BY, P2G_MIN_BLOCKS) k_p2g_accum(const float4* __restrict__ pos,
+                                                                           const float4* __restrict__ vel,
+                                                                           const int* __restrict__ start, Dims g,
+                                                                           float2* __restrict__ acc) {
     using R = Reach<BX, BY, BZ>;
-    __shared__ float s_num[R::N];
-    __shared__ float s_den[R::N];
+    constexpr int NT = 3 * BX * BY;
+    static_assert(BX * BY % 32 == 0, "a group is whole warps");
+    __shared__ float2 s_acc[3 * R::N];
 
     const int W = g.W, H = g.H, D = g.D;
     const int nbx = (W + BX - 1) / BX, nby = (H + BY - 1) / BY;
     const int bid = blockIdx.x;
     const int i0 = (bid % nbx) * BX, j0 = ((bid / nbx) % nby) * BY, k0 = (bid / (nbx * nby)) * BZ;
-    const int ni = min(BX, W - i0), nj = min(BY, H - j0), nk = min(BZ, D - k0);
 
     bool any = false;
-    for (int t = threadIdx.x; t < ni * nj * nk; t += NT) {
-        const int c = (i0 + t % ni) + (j0 + (t / ni) % nj) * W + (k0 + t / (ni * nj)) * W * H;
+    for (int t = threadIdx.x; t < BX * BY * BZ; t += NT) {
+        const int i = i0 + t % BX, j = j0 + (t / BX) % BY, k = k0 + t / (BX * BY);
+        if (i >= W || j >= H || k >= D) continue;
+        const int c = i + j * W + k * W * H;
         any |= start[c + 1] > start[c];
     }
     if (!__syncthreads_or(any)) return;  // no particle: nothing to add
-    for (int t = threadIdx.x; t < R::N; t += NT) { s_num[t] = 0.0f; s_den[t] = 0.0f; }
+    for (int t = threadIdx.x; t < 3 * R::N; t += NT) s_acc[t] = make_float2(0.0f, 0.0f);
     __syncthreads();
-
-    for (int t = threadIdx.x; t < ni * nj * nk; t += NT) {
-        const int ci = i0 + t % ni, cj = j0 + (t / ni) % nj, ck = k0 + t / (ni * nj);
-        const int c = ci + cj * W + ck * W * H;
-        const int q0 = start[c], q1 = start[c + 1];
-        if (q0 == q1) continue;
-        splat_cell<0, P2>(pos, vel, q0, q1, ci, cj, ck, g, s_num, s_den, i0, j0 - 1, k0 - 1, R::UX, R::UY);
-        splat_cell<1, P2>(pos, vel, q0, q1, ci, cj, ck, g, s_num + R::NU, s_den + R::NU, i0 - 1, j0, k0 - 1, R::VX,
-                      R::VY);
-        splat_cell<2, P2>(pos, vel, q0, q1, ci, cj, ck, g, s_num + R::NU + R::NV, s_den + R::NU + R::NV, i0 - 1, j0 - 1,
-                      k0, R::WX, R::WY);
-    }
+    const int grp = int(threadIdx.x) / (BX * BY);
+    if (grp == 0) brick_component<0, BX, BY, BZ, P2>(pos, vel, start, g, i0, j0, k0, s_acc);
+    else if (grp == 1) brick_component<1, BX, BY, BZ, P2>(pos, vel, start, g, i0, j0, k0, s_acc);
+    else brick_component<2, BX, BY, BZ, P2>(pos, vel, start, g, i0, j0, k0, s_acc);
     __syncthreads();
 
     // Add the reached faces inside the grid into acc (one 8-byte vector
     // reduction per face); faces outside the grid are dropped, as the
     // reference skips them.
     const int64_t nu = g.nu(), nv = g.nv();
-    for (int t = threadIdx.x; t < R::N; t += NT) {
-        const float den = s_den[t];
-        if (den == 0.0f) continue;
-        int fi, fj, fk;
-        int64_t idx;
-        if (t < R::NU) {
-            fi = i0 + t % R::UX; fj = j0 - 1 + (t / R::UX) % R::UY; fk = k0 - 1 + t / (R::UX * R::UY);
-            if (fi > W || fj < 0 || fj >= H || fk < 0 || fk >= D) continue;
-            idx = int64_t(fi) + int64_t(fj) * (W + 1) + int64_t(fk) * (W + 1) * H;
-        } else if (t < R::NU + R::NV) {
-            const int r = t - R::NU;
-            fi = i0 - 1 + r % R::VX; fj = j0 + (r / R::VX) % R::VY; fk = k0 - 1 + r / (R::VX * R::VY);
-            if (fi < 0 || fi >= W || fj > H || fk < 0 || fk >= D) continue;
-            idx = nu + int64_t(fi) + int64_t(fj) * W + int64_t(fk) * W * (H + 1);
-        } else {
-            const int r = t - R::NU - R::NV;
-            fi = i0 - 1 + r % R::WX; fj = j0 - 1 + (r / R::WX) % R::WY; fk = k0 + r / (R::WX * R::WY);
-            if (fi < 0 || fi >= W || fj < 0 || fj >= H || fk > D) continue;
-            idx = nu + nv + int64_t(fi) + int64_t(fj) * W + int64_t(fk) * W * H;
-        }
-        atomicAdd(&acc[idx], make_float2(s_num[t], den));
+    for (int t = threadIdx.x; t < 3 * R::N; t += NT) {
+        const float2 f = s_acc[t];
+        if (f.y == 0.0f) continue;
+        const int a = t / R::N, r = t - a * R::N;
+        const int fi = i0 + r % R::X - (a != 0), fj = j0 + (r / R::X) % R::Y - (a != 1),
+                  fk = k0 + r / (R::X * R::Y) - (a != 2);
+        const int nx = W + (a == 0), ny = H + (a == 1), nz = D + (a == 2);
+        if (fi < 0 || fi >= nx || fj < 0 || fj >= ny || fk < 0 || fk >= nz) continue;
+        const int64_t idx = (a == 0 ? 0 : a == 1 ? nu : nu + nv) + int64_t(fi) + int64_t(fj) * nx + int64_t(fk) * nx * ny;
+        atomicAdd(&acc[idx], f);
     }
 }
 
@@ -315,18 +312,17 @@ __global__ void k_copy(const float* __restrict__ s, float* __restrict__ d, int64
 // Brick shape and CTA size (build tunables).
 #ifndef P2G_BRICK_X
 #define P2G_BRICK_X 8
-#define P2G_BRICK_Y 8
+#define P2G_BRICK_Y 4
 #define P2G_BRICK_Z 4
-#define P2G_THREADS 128
 #endif
-constexpr int P2G_BX = P2G_BRICK_X, P2G_BY = P2G_BRICK_Y, P2G_BZ = P2G_BRICK_Z, P2G_NT = P2G_THREADS;
+constexpr int P2G_BX = P2G_BRICK_X, P2G_BY = P2G_BRICK_Y, P2G_BZ = P2G_BRICK_Z, P2G_NT = 3 * P2G_BX * P2G_BY;
 
 void launch_p2g(const float4* pos, const float4* vel, const int* start, Dims g, float dt, float3 gravity,
                 float2* acc, float* u, float* v, float* w, float* us, float* vs, float* ws, int fused_forces,
                 cudaStream_t st) {
     const int nb = ((g.W + P2G_BX - 1) / P2G_BX) * ((g.H + P2G_BY - 1) / P2G_BY) * ((g.D + P2G_BZ - 1) / P2G_BZ);
-    if (g.idx != 0.0f) k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, P2G_NT, true><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
-    else k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, P2G_NT, false><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
+    if (g.idx != 0.0f) k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, true><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
+    else k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, false><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
     const int64_t n3[3] = {g.nu(), g.nv(), g.nw()};
     float* dst[3] = {u, v, w};
     float* sav[3] = {us, vs, ws};

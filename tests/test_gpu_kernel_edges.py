@@ -259,3 +259,52 @@ def test_unet_gradient_tiles(shape):
         assert x @ y >= 0.999 * np.linalg.norm(x) * np.linalg.norm(y)
     loss2, g2 = net.loss_grad(*[a.data_ptr() for a in t])
     assert loss2 == loss and np.array_equal(g2, g)
+
+
+# grids smaller than a brick of 8 x 4 x 4, of whole bricks, with remainders in every axis, and flat
+@pytest.mark.parametrize("shape", [(5, 3, 2), (8, 4, 4), (16, 8, 8), (17, 9, 5), (23, 6, 13), (33, 17, 1)])
+def test_p2g_brick_edges(shape):
+    """P2G against numpy in FP64, with empty cells, crowded ones (up to 40 particles) and particles on the far edges.
+    Weights are products of three FP32 fractions (3 ulps each) and num and den sum at most 27 cells of at most 40
+    particles: relative error of a face below (3 + 27 * 40) 2^-24 of its terms' magnitude, 7e-5; faces whose weights
+    sum to less than 1e-3 are left out, since the fractions' absolute error (W 2^-24) is not small against them."""
+    from fluidprjct_b200 import capi
+    W, H, D = shape
+    dx = np.float32(0.125)
+    s = capi.Solver(dim=3 if D > 1 else 2, dx=float(dx), dt=0.01, output_format=capi.OUT_NONE)
+    lab = np.full((D, H, W), 2, np.uint8)
+    s.set_labels(lab if D > 1 else lab[0])
+    rng = np.random.default_rng(W)
+    n = W * H * D * 3
+    pos = (rng.random((n, 3)) * np.array([W, H, D]) * dx).astype(np.float32)
+    pos[: n // 6] = (rng.random((n // 6, 3)) * dx * 1.2).astype(np.float32)[:, :3]
+    pos[-3:] = [[W * dx, 0, 0], [0, H * dx, 0], [0, 0, D * dx]]
+    pos = np.minimum(pos, np.array([W, H, D], np.float32) * dx)
+    if D == 1:
+        pos[:, 2] = 0
+    vel = rng.uniform(-1, 1, pos.shape).astype(np.float32)
+    s.set_particles(pos, vel)
+    for _ in range(2):  # the second transfer finds the pair array as the first left it
+        s.phase(capi.PHASE_LABEL)
+        s.phase(capi.PHASE_P2G)
+    N = (W, H, D)
+    r = pos.astype(np.float64) / float(dx)
+    for a, which in enumerate((capi.GRID_U, capi.GRID_V, capi.GRID_W)):
+        sh = tuple(N[d] + (d == a) for d in range(3))
+        num, den = np.zeros(sh), np.zeros(sh)
+        b, f = [], []
+        for d in range(3):
+            t = r[:, d] - (0.0 if d == a else 0.5)
+            i = np.clip(np.floor(t), 0, N[d] if d == a else N[d] - 1)
+            b.append(i.astype(int)), f.append(np.clip(t - i, 0, 1))
+        for o in np.ndindex(2, 2, 2):
+            w = np.prod([f[d] if o[d] else 1 - f[d] for d in range(3)], axis=0)
+            q = [b[d] + o[d] for d in range(3)]
+            ok = np.all([q[d] < sh[d] for d in range(3)], axis=0)
+            np.add.at(num, tuple(c[ok] for c in q), (w * vel[:, a])[ok])
+            np.add.at(den, tuple(c[ok] for c in q), w[ok])
+        got = s.grid(which).transpose(2, 1, 0)
+        far = den > 1e-3
+        assert np.abs(got[far] - num[far] / den[far]).max() <= 1e-4
+        assert not got[den == 0].any()
+    s.close()
