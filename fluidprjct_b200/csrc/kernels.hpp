@@ -58,45 +58,66 @@ struct PressureBufs {
 // -------- multigrid-preconditioned PCG (kernels_mg.cu) --------
 constexpr int MG_MAX_LEVELS = 8;
 constexpr int MG_BLOCK_CELLS = 4096;           // levels at most this big are solved by one block ...
-constexpr int MG_SMEM_BUDGET = 180 * 1024;     // ... in shared memory, when their copies fit in this
-// One multigrid level: padded dense grids with a SOLID / zero halo.
+constexpr int MG_SMEM_BUDGET = 188 * 1024;     // ... in shared memory, when their copies fit in this
+constexpr int MG_OX = 4;                       // cells before a padded row's first one
+// One multigrid level: padded dense grids with a SOLID / zero halo; cell
+// (i, j, k) at (i + MG_OX) + (j + 1) sy + (k + 1) sz.
 struct MgLevel {
     int W, H, D;    // interior cells
-    int sy, sz;     // padded strides: W+2 and (W+2)*(H+2)
+    int sy, sz;     // padded strides: W up to a multiple of 4, + MG_OX; sy (H + 2)
     uint8_t* lab;   // labels (BODY folded into SOLID)
     float* x;       // correction (level 0: the preconditioned residual z)
     float* b;       // right-hand side (level 0: the residual r)
     uint8_t* code;  // per solve: FLUID cells 1 + diagonal, every other cell 0
 };
+// A quad -- four aligned cells of a row, at least one of them FLUID -- in a
+// level's list, as an int4: x the first cell's padded index; y the four codes
+// (level 0 only) and the bits below; z the padded index, on the next level, of
+// the first two cells' parent; w level 0: the first cell's dense index in
+// W x H x D, other levels: the padded index, on the finer level, of the first
+// cell's first child.
+constexpr uint32_t QUAD_CODES = 0x07070707u;
+constexpr uint32_t QUAD_ODD = 0x80u;            // j + k is odd: the first cell is black
+constexpr uint32_t QUAD_PARENT_ODD = 0x8000u;   // the parent row's J + K is odd
+constexpr uint32_t QUAD_Z = 0x800000u;          // the children's second z plane lies in the finer level
+constexpr uint32_t QUAD_PAR = QUAD_ODD | QUAD_PARENT_ODD;
+// The hierarchy and its buffers.
+struct MgBufs {
+    int L = 0;
+    MgLevel lv[MG_MAX_LEVELS]{};
+    int4* q[MG_MAX_LEVELS]{};   // quad lists of the grid-wide levels (level 0: from launch_pressure_setup)
+    int* nq = nullptr;          // [MG_MAX_LEVELS] their lengths
+    float4* rhs = nullptr;      // right-hand side by level-0 quad
+    // FP64 Krylov vectors by quad, 2 * cap pairs each
+    double2 *p = nullptr, *s = nullptr, *xs = nullptr, *r = nullptr, *w = nullptr;
+    int cap = 0;                // quads of level 0's grid
+    double* xd = nullptr;       // level-0 padded grid, zero between solves
+};
 // Fills lv[].W/H/D/sy/sz of the level hierarchy for a W x H x D grid (down to
 // at most 2 cells per axis, or MG_MAX_LEVELS levels); returns L.
 int mg_levels_for(int W, int H, int D, MgLevel* lv);
+int mg_npad(const MgLevel& L);  // cells of a level's padded grid, up to a multiple of 16
 int mg_max_blocks();
 // First block-solved level G of the hierarchy and the shared memory its
 // copies take (0: the block levels stay in global memory).
 int mg_split(const MgLevel* lv, int L, int* smem_bytes);
-// Level labels from the cell labels (per solve): the grid-wide coarse levels;
-// the solver kernel coarsens the shared-memory levels itself.  With l1list
-// (room for level 1's W*H*D cells) it also lists level 1's FLUID cells there
-// and their number in *l1n.  Returns the number of launches.
-int launch_mg_setup(const uint8_t* labels, Dims g, MgLevel* lv, int L, int* l1list, int* l1n, cudaStream_t st);
+// Level labels and quad lists of the grid-wide coarse levels from the cell
+// labels (per solve; nq[1..] zero before, as launch_pressure_setup leaves
+// them); the solver kernel coarsens the shared-memory levels itself.  Returns
+// the number of launches.
+int launch_mg_setup(const uint8_t* labels, const MgBufs& m, cudaStream_t st);
 // MG-preconditioned PCG (FP32 V-cycle, FP64 Krylov vectors and reductions) for
-// A x = rhs (compact) to ||r||/||rhs|| <= tol; solution in pb.X (FP64
-// compact).  p, q, xs, r are level-0 padded dense FP64 work grids, zero at
-// entry and on exit.
-// x0: compact initial guess (scaled on the device by its energy-optimal
-// factor), or null to start from x = 0.
+// the system of launch_pressure_setup to ||r||/||rhs|| <= tol; dense pressure
+// to pout (its non-FLUID cells must be zero), the true residual's
+// ||rhs - A x||^2 and ||rhs||^2 (FP64) to pb.red.
+// guess: a dense W x H x D guess (scaled on the device by its energy-optimal
+// factor; pout itself may be passed), or null to start from x = 0.  guess_dir:
+// it becomes the first search direction (a network's guess); otherwise
+// non-finite values in it read as 0.
 // nu0: red-black sweep pairs before and after the coarse correction on the
-// finest level (coarser levels take one pair; the cycle stays symmetric).
-// pprev: without x0, a dense W x H x D guess (the previous step's pressure),
-// gathered at the FLUID cells and scaled like x0; null to start from zero.
-// pout: the dense W x H x D pressure out (its non-FLUID cells must be zero),
-// or null.  The kernel also writes the true residual's ||rhs - A x||^2 and
-// ||rhs||^2 (FP64) to pb.red.  l1list / l1n: level 1's FLUID cells from
-// launch_mg_setup (or null), whose x and b the kernel leaves zero again.
-int launch_pcg_mg(Dims g, PressureBufs& pb, MgLevel* lv, int L, const int* l1list, const int* l1n, double* p,
-                  double* q, double* xs, double* r, const float* rhs, double tol, int maxit, cudaStream_t st, const float* x0 = nullptr, int nu0 = 2,
-                  const float* pprev = nullptr, float* pout = nullptr, unsigned wait_polls = kDefaultWaitPolls);
+// finest level.
+int launch_pcg_mg(Dims g, PressureBufs& pb, const MgBufs& m, double tol, int maxit, const float* guess, int guess_dir,
+                  int nu0, float* pout, cudaStream_t st);
 
 // -------- labelling and the particle sort (kernels_sort.cu) --------
 // counts[nc] must be zero on entry.  Writes key/rank per particle.
@@ -123,10 +144,15 @@ void launch_copy(const float* src, float* dst, int64_t n, cudaStream_t st);
 
 // -------- pressure (kernels_pressure.cu) --------
 // Compacts FLUID cells, builds rhs (FluidSolver3D.cu:1360-1474) and diagonals,
-// zeroes p and dd off the fluid.  If rhs_dense is non-null it replaces the
-// computed rhs (caller-provided system).
+// zeroes p off the fluid, and readies the solvers' barrier and status (poll
+// limit wait_polls).  If rhs_dense is non-null it replaces the computed rhs
+// (caller-provided system).  With a multigrid hierarchy (mg->L > 0) it also
+// lists level 0's quads with their right-hand sides and zeroes the lengths of
+// the other levels' lists.  pb.tile_sums: pressure_tiles(g) ints.
 void launch_pressure_setup(const uint8_t* labels, const float* u, const float* v, const float* w, Dims g, float dt,
-                           BodyKin body, const float* rhs_dense, float* p, PressureBufs& pb, cudaStream_t st);
+                           BodyKin body, const float* rhs_dense, float* p, PressureBufs& pb, const MgBufs* mg,
+                           unsigned wait_polls, cudaStream_t st);
+int pressure_tiles(Dims g);
 
 // -------- plain and mixed-precision PCG (kernels_pcg.cu) --------
 // Jacobi PCG with FP64 vectors from x0 = 0 for A x = b (the system of
@@ -134,15 +160,14 @@ void launch_pressure_setup(const uint8_t* labels, const float* u, const float* v
 // non-FLUID cells must be zero), the true residual's ||b - A x||^2 and ||b||^2
 // to pb.red, diagnostics to pb.out.  The padded work grids must be zero on
 // entry and are zero again on exit, unless a wait gave up.
-int launch_pcg(Dims g, PressureBufs& pb, double tol, int maxit, float* pout, cudaStream_t st,
-               unsigned wait_polls = kDefaultWaitPolls);
+int launch_pcg(Dims g, PressureBufs& pb, double tol, int maxit, float* pout, cudaStream_t st);
 // The same by FP64 iterative refinement around FP32-vector PCG solves, from
 // x = 0 or from the compact guess x0 scaled by its energy-optimal factor
 // (x0, b) / (x0, A x0).
-int launch_pcg_mixed(Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout, cudaStream_t st,
-                     unsigned wait_polls = kDefaultWaitPolls);
-// Barrier word to zero with its poll limit, status word to DEV_OK (before
-// every persistent-solver launch).
+int launch_pcg_mixed(Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout, cudaStream_t st);
+// Barrier word to zero with its poll limit, status word to DEV_OK: before a
+// second persistent solver on the same system (launch_pressure_setup does it
+// for the first).
 void launch_reset_barrier(GridBar* bar, int* status, unsigned wait_polls, cudaStream_t st);
 int pcg_max_blocks();
 

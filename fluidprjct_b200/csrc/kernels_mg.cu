@@ -1,8 +1,8 @@
 // kernels_mg.cu -- multigrid-preconditioned conjugate gradients for the
 // pressure Poisson system (FP_SOLVER_PCG_MG).
 //
-// Same system as the reference's cuDSS solve (FluidSolver3D.cu:1815-2062):
-// unit 7-point operator over FLUID cells, AIR = Dirichlet 0, SOLID/BODY and
+// Same system as the reference's cuDSS solve (FluidSolver3D.cu:1815-2062): unit
+// 7-point operator over FLUID cells, AIR = Dirichlet 0, SOLID/BODY and
 // out-of-domain = Neumann.  Preconditioner: one geometric multigrid V-cycle.
 //   * Levels coarsen by 2 per axis; a coarse cell is AIR if any child is AIR,
 //     else FLUID if any child is FLUID, else SOLID (Dirichlet priority), and
@@ -14,10 +14,25 @@
 //   * Smoother: red-black Gauss-Seidel over-relaxed by MG_SOR, red then black
 //     going down, black then red coming up (two pairs on the finest level by
 //     default, one on the other grid-wide levels, two on the block levels);
-//     the coarsest level does the same symmetric sweeps.  The V-cycle is therefore a symmetric positive definite
-//     preconditioner.  After the black sweep only red cells carry a residual,
-//     so restriction sums the red children.  The coarse correction is scaled
-//     by omega.  Level 0 works on the compact FLUID list.
+//     the coarsest level does the same symmetric sweeps.  The V-cycle is
+//     therefore a symmetric positive definite preconditioner.  After the black
+//     sweep only red cells carry a residual, so restriction sums the red
+//     children.  The coarse correction is scaled by omega.
+// Layout: every level is a padded grid whose rows are a multiple of four cells
+// apart and start four cells in (MG_OX), so that four cells of a row -- a quad
+// -- are one aligned 16-byte vector and both halos of a row are the zero gap
+// before the next one.  Grid-wide levels are walked as lists of the quads that
+// hold a FLUID cell: a sweep of a quad is eight loads (its row of x, b, the four
+// neighbouring rows, one cell at each end), where cell by cell it took 36, and
+// the issue of those loads is what a phase waited for: with one cell per
+// thread a level-0 sweep took 3.2 us at 485,000 FLUID cells and 9.8 at 2.2 M,
+// against 2.6 and 7.2.  A thread's first quads stay in shared memory (slot_of).
+// Code length counts as much as loads: a phase runs once between two grid
+// barriers, so its instructions are fetched as it goes, and the phases are short
+// functions, one quad a trip, rather than unrolled and inlined.
+// Per solve, before (a cell per thread and trip) and now: dam break 64 x 64 187
+// and 132 us, 128^3 849 and 730, pool 160^3 2350 and 1700, 256 x 128 x 256 2047
+// and 1460, at the same iterations.
 // Levels with more than MG_BLOCK_CELLS cells are swept by the whole grid with a
 // grid barrier between sweeps; every block then does the remaining coarse
 // levels on its own shared-memory copy with __syncthreads only (labels
@@ -30,12 +45,12 @@
 // levels as well reached 8.9 iterations, but their extra grid barriers made
 // the solve slower (1.067 ms).  The whole PCG (flexible, in the Chronopoulos-Gear
 // form, optionally started from a guess) runs in one persistent cooperative
-// launch with the bounded grid barrier.  Precision split: the V-cycle works in FP32; the
-// Krylov vectors (x, r, p, s) and all dot products are FP64, so the
-// recurrence residual tracks the true residual down to the 1e-6 target
-// without restarts.  Loops over the FLUID list take several cells per thread
-// per trip with all loads issued before use, the first four cached in shared
-// memory (the solve is latency bound: the 128^3 working set lives in L2).
+// launch with the bounded grid barrier.  Precision split: the V-cycle works in
+// FP32; the Krylov vectors (x, r, p, s; stored by quads) and all dot products
+// are FP64, so the recurrence residual tracks the true residual down to the
+// 1e-6 target without restarts.
+#include <algorithm>
+
 #include "device_memo.hpp"
 #include "kernels.hpp"
 #include "pcg_common.cuh"
@@ -44,7 +59,10 @@ namespace fp {
 
 namespace {
 
-constexpr int MG_THREADS = 1024;
+// One CTA per SM, 128 registers a thread.  Per solve of the four scenes above:
+// 384 threads 133, 791, 1852 and 1582 us, 512 132, 730, 1700 and 1457, 640 138,
+// 783, 1672 and 1388 (with 96 registers, some spilled): 512 is the best or near it.
+constexpr int MG_THREADS = 512;
 // Red-black sweep pairs before and after the coarse correction on the
 // grid-wide levels below the finest (MG_NU_GRID) and on the block levels
 // above the coarsest (MG_NU_BLOCK); build tunables.
@@ -73,13 +91,11 @@ constexpr int MG_THREADS = 1024;
 #define MG_SOR_VALUE 1.2f
 #endif
 constexpr float MG_SOR = MG_SOR_VALUE;
-__device__ __forceinline__ float sor(float x, float y) { return MG_SOR == 1.0f ? y : x + MG_SOR * (y - x); }
 // The same on the coarser levels (build tunable MG_SOR_COARSE_VALUE).
 #ifndef MG_SOR_COARSE_VALUE
 #define MG_SOR_COARSE_VALUE MG_SOR_VALUE
 #endif
 constexpr float MG_SORC = MG_SOR_COARSE_VALUE;
-__device__ __forceinline__ float sorc(float x, float y) { return MG_SORC == 1.0f ? y : x + MG_SORC * (y - x); }
 
 struct MgArgs {
     int L, G;                    // levels; levels [0, G) are grid-wide
@@ -91,20 +107,16 @@ struct MgArgs {
     int nu_grid;                 // ... on the other grid-wide levels
     int nu_block;                // ... on the block levels above the coarsest
     MgLevel lv[MG_MAX_LEVELS];
-    double* p;                   // level-0 padded dense Krylov vectors (FP64)
-    double* q;
-    double* xs;
-    double* r;
-    const float* rhs;            // compact right-hand side
-    const float* x0;             // compact initial guess, or null
-    const float* pprev;          // dense W x H x D guess (the previous pressure) when x0 is null, or null
-    const int* fidx;             // compact FLUID list (level-0 padded index)
-    const uint8_t* diag;         // compact diagonal, bit 7 = red/black colour
-    const int* nf;
-    const int* l1list;           // level 1's FLUID cells (padded indices, any order), or null
-    const int* l1n;              // their number
-    double* X;                   // compact solution out (FP64)
-    float* pout;                 // dense W x H x D pressure out (zero off the fluid already), or null
+    const int4* q[MG_MAX_LEVELS];  // quad lists of levels [0, max(G, 1)): MgQuad entries
+    const int* nq;               // their lengths
+    const float4* rhs;           // right-hand side by level-0 quad (zero off the fluid)
+    // FP64 Krylov vectors by quad: the first two cells of quad n at [n], the last two at [cap + n]
+    double2 *p, *s, *xs, *r, *w;
+    int cap;
+    double* xd;                  // level-0 grid for the FP64 solution, zero between solves
+    const float* guess;          // dense W x H x D guess, or null
+    int guess_dir;               // the guess is the first search direction (the network's)
+    float* pout;                 // dense W x H x D pressure out (zero off the fluid already)
     double* red;                 // [2] out: ||rhs - A x||^2 and ||rhs||^2 of the solution, in FP64
     double* part;
     GridBar* bar;
@@ -114,6 +126,11 @@ struct MgArgs {
     int maxit;
 };
 
+__host__ __device__ __forceinline__ int lv_index(const MgLevel& L, int i, int j, int k) {
+    return (i + MG_OX) + (j + 1) * L.sy + (k + 1) * L.sz;
+}
+// Cells of a level's padded grid (vector loads at its end stay inside).
+__host__ __device__ __forceinline__ int npad(const MgLevel& L) { return L.sz * (L.D + 2) + 2 * MG_OX; }
 __device__ __forceinline__ int lv_diag(const MgLevel& L, int c) {
     const uint8_t* l = L.lab;
     const int o[6] = {1, -1, L.sy, -L.sy, L.sz, -L.sz};
@@ -128,93 +145,191 @@ __device__ __forceinline__ float lv_nbsum(const MgLevel& L, int c) {
 }
 __device__ __forceinline__ int lv_cell(const MgLevel& L, int t, int& i, int& j, int& k) {
     i = t % L.W; j = (t / L.W) % L.H; k = t / (L.W * L.H);
-    return (i + 1) + (j + 1) * L.sy + (k + 1) * L.sz;
+    return lv_index(L, i, j, k);
 }
 
-// ---- level-0 operations over the compact FLUID list (colour and diagonal
-// precomputed in the diag byte), four cells per thread per trip ----
-constexpr int UNR = 4;
-template <int N = UNR>
-struct Cells {
-    int c[N];
-    uint8_t db[N];
-    bool ok[N];
+// 1 / d of the diagonals d = 1..6 by code 1 + d; 0 for codes 0 and 1 (a FLUID
+// cell with no FLUID or AIR neighbour takes x = 0).
+__shared__ float s_rcp[8];
+// Over-relaxed Gauss-Seidel value y = (b + nb) / d of a FLUID cell.  The
+// division is a multiplication by the rounded reciprocal: one more rounding, in
+// the FP32 preconditioner only.
+__device__ __forceinline__ float gs_value(float xo, float b, float nb, int dc, float w) {
+    const float y = (b + nb) * s_rcp[dc];
+    return dc > 1 ? xo + w * (y - xo) : (dc == 1 ? 0.0f : xo);
+}
+// ---- operations over quad lists ----
+// A thread's quads are n = t0 + q * stride for trips q = 0, 1, ..., one at a
+// time: a grid-wide phase's code is cold when it starts, and at 512 threads its
+// length costs more than a second quad's loads in flight gain (two quads a
+// trip: 0.83 against 0.72 ms for a warm-started 128^3 solve, 1.83 against 1.56
+// for 256 x 128 x 256).
+struct Quad {
+    int c;       // index of the first cell
+    uint32_t k;  // four codes (1 + diagonal, 0: not FLUID) and parity bits
+    int pc;      // index of its first cells' parent on the next level
 };
-// A thread's cells are n = t0 + q * stride for trips q = 0, 1, ...  Its first
-// UNR cells (q < UNR) are cached for the whole solve in shared memory, in its
-// own column (only the thread itself reads them): padded index and diag byte,
-// or `safe` and 0 past the end of the list.  `safe` is the padded index of
-// interior cell (0,0,0): it and its six stencil neighbours lie inside every
-// level-0 grid, so the unconditional loads of an idle lane stay in bounds (its
-// result is dropped).
-__shared__ int s_fc[UNR * MG_THREADS];
-__shared__ uint8_t s_fd[UNR * MG_THREADS];
-__device__ __forceinline__ void cache_cells(const int* fidx, const uint8_t* dg, int nf, int t0, int stride, int safe) {
-#pragma unroll
-    for (int q = 0; q < UNR; ++q) {
-        const int n = t0 + q * stride;
-        s_fc[q * MG_THREADS + threadIdx.x] = n < nf ? fidx[n] : safe;
-        s_fd[q * MG_THREADS + threadIdx.x] = n < nf ? dg[n] : 0;
+// The first trips' quads of the grid-wide levels, kept in shared memory for the
+// whole solve: two on levels 0 and 1, one on levels 2 and 3 (in each thread's
+// own column; only the thread itself reads them).
+constexpr int SLOTS = 6;
+__shared__ int s_qc[SLOTS * MG_THREADS], s_qp[SLOTS * MG_THREADS];
+__shared__ uint32_t s_qk[SLOTS * MG_THREADS];
+__shared__ int s_nq[MG_MAX_LEVELS];  // the lists' lengths
+__device__ __forceinline__ int slot_of(int l) { return l < 2 ? 2 * l : l + 2; }  // first slot of level l
+__device__ __forceinline__ int slots_of(int l) { return l < 2 ? 2 : (l <= 3 ? 1 : 0); }
+// Codes and parity bits of a list entry (level 0's carries its codes).
+__device__ __forceinline__ uint32_t codes_of(const MgLevel& L, int l, const int4& e) {
+    return l == 0 ? uint32_t(e.y) : *reinterpret_cast<const uint32_t*>(L.code + e.x) | (uint32_t(e.y) & QUAD_PAR);
+}
+// Fills the slots of levels [l0, l1) (the codes must be complete).
+__device__ __forceinline__ void fill_slots(const MgArgs& a, int l0, int l1, int t0, int st) {
+    for (int l = l0; l < min(l1, 4); ++l)
+        for (int u = 0; u < slots_of(l); ++u) {
+            const int n = t0 + u * st, at = (slot_of(l) + u) * MG_THREADS + threadIdx.x;
+            if (n >= s_nq[l]) continue;
+            const int4 e = a.q[l][n];
+            s_qc[at] = e.x;
+            s_qk[at] = codes_of(a.lv[l], l, e);
+            s_qp[at] = e.z;
+        }
+}
+// Calls f(quad, n) for each of the thread's quads of level l; the entry of the
+// next one is on its way meanwhile.
+template <class Fn>
+__device__ __forceinline__ void for_quads(const MgArgs& a, int l, Fn f) {
+    const int st = gridDim.x * MG_THREADS, nq = s_nq[l], slots = slots_of(l);
+    const int4* list = a.q[l];
+    int n = blockIdx.x * MG_THREADS + threadIdx.x, at = slot_of(l) * MG_THREADS + threadIdx.x, q = 0;
+    int4 next = make_int4(0, 0, 0, 0);
+    if (slots == 0 && n < nq) next = list[n];
+#pragma unroll 1
+    for (; n < nq; n += st, ++q, at += MG_THREADS) {
+        Quad Q;
+        if (q < slots) Q = Quad{s_qc[at], s_qk[at], s_qp[at]};
+        else Q = Quad{next.x, codes_of(a.lv[l], l, next), next.z};
+        if (q + 1 >= slots && n + st < nq) next = list[n + st];
+        f(Q, n);
     }
 }
-// Cells of trips q0 .. q0 + N - 1 (base = t0 + q0 * stride).
-template <int N>
-__device__ __forceinline__ void load_cells(Cells<N>& k, const int* fidx, const uint8_t* dg, int nf, int base, int q0,
-                                           int stride, int safe) {
-#pragma unroll
-    for (int u = 0; u < N; ++u) {
-        const int n = base + u * stride, q = q0 + u;
-        k.ok[u] = n < nf;
-        if (q < UNR) {
-            k.c[u] = s_fc[q * MG_THREADS + threadIdx.x];
-            k.db[u] = s_fd[q * MG_THREADS + threadIdx.x];
-        } else {
-            k.c[u] = k.ok[u] ? fidx[n] : safe;
-            k.db[u] = k.ok[u] ? dg[n] : 0;
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ int code_at(uint32_t k, int e) { return int((k >> (8 * e)) & 7u); }
+
+// Gauss-Seidel update of the FLUID cells of one colour (0 red: even i + j + k)
+// of a quad: cells 0, 2 or 1, 3.
+__device__ __forceinline__ void sweep_quad(const MgLevel& L, const Quad& Q, int color, float w) {
+    float* X = L.x + Q.c;
+    const float4 x = ld4(X), yp = ld4(X + L.sy), ym = ld4(X - L.sy), zp = ld4(X + L.sz), zm = ld4(X - L.sz);
+    const float xl = X[-1], xr = X[4];
+    const float4 b = ld4(L.b + Q.c);
+    const bool odd = (((Q.k >> 7) & 1u) ^ uint32_t(color)) != 0u;
+    const float nba = ((odd ? x.z : x.y) + (odd ? x.x : xl)) + ((odd ? yp.y : yp.x) + (odd ? ym.y : ym.x)) +
+                      ((odd ? zp.y : zp.x) + (odd ? zm.y : zm.x));
+    const float nbb = ((odd ? xr : x.w) + (odd ? x.z : x.y)) + ((odd ? yp.w : yp.z) + (odd ? ym.w : ym.z)) +
+                      ((odd ? zp.w : zp.z) + (odd ? zm.w : zm.z));
+    const float va = gs_value(odd ? x.y : x.x, odd ? b.y : b.x, nba, code_at(Q.k, odd ? 1 : 0), w);
+    const float vb = gs_value(odd ? x.w : x.z, odd ? b.w : b.z, nbb, code_at(Q.k, odd ? 3 : 2), w);
+    // the other colour's cells keep their values: this thread alone owns the quad
+    *reinterpret_cast<float4*>(X) = odd ? make_float4(x.x, va, x.z, vb) : make_float4(va, x.y, vb, x.w);
+}
+// Restriction into the listed cells of level Cl fused with that level's first
+// sweep: b_coarse = scale * sum over the red FLUID children of (b - A x), then
+// x_coarse = b/d on red FLUID cells, 0 on black ones.  After the black sweep
+// the black residuals vanish, so only the red children (offsets with an even
+// coordinate sum) are summed, in k, j, i order.  One thread per coarse cell;
+// its 2 x 2 x 2 children are four aligned pairs.  Children beyond an odd-sized
+// level are halo cells with code 0; those in z would have neighbours beyond
+// the grid, so they are not read.
+__device__ __forceinline__ void restrict_quads(const MgLevel& F, const MgLevel& Cl, float scale, const int4* list,
+                                               int nq, int t0, int st) {
+    for (int t = t0; t < 4 * nq; t += st) {
+        const int4 E = list[t >> 2];
+        const int e = t & 3, cc = E.x + e, r0 = E.w + 2 * e, r1 = r0 + F.sy, r2 = r0 + F.sz, r3 = r1 + F.sz;
+        const bool kk = (uint32_t(E.y) & QUAD_Z) != 0u;
+        const int dc = Cl.code[cc];
+        const float* X = F.x;
+        const float2 x0 = ld2(X + r0), x1 = ld2(X + r1);
+        const float a0 = X[r0 - 1], a1 = X[r0 - F.sy], a2 = X[r0 - F.sz];
+        const float b0 = X[r1 + 2], b1 = X[r1 + 1 + F.sy], b2 = X[r1 + 1 - F.sz];
+        const int d0 = F.code[r0], d1 = F.code[r1 + 1];
+        const float f0 = F.b[r0], f1 = F.b[r1 + 1];
+        float2 x2 = make_float2(0.0f, 0.0f), x3 = x2;
+        float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, f2 = 0.0f, f3 = 0.0f;
+        int d2 = 0, d3 = 0;
+        if (kk) {
+            x2 = ld2(X + r2); x3 = ld2(X + r3);
+            c0 = X[r2 + 2]; c1 = X[r2 + 1 - F.sy]; c2 = X[r2 + 1 + F.sz];
+            g0 = X[r3 - 1]; g1 = X[r3 + F.sy]; g2 = X[r3 + F.sz];
+            d2 = F.code[r2 + 1]; d3 = F.code[r3];
+            f2 = F.b[r2 + 1]; f3 = F.b[r3];
         }
+        if (dc == 0) continue;
+        auto res = [](int d, float bv, float xv, float nb) { return d > 0 ? bv - (float(d - 1) * xv - nb) : 0.0f; };
+        float s = res(d0, f0, x0.x, (x0.y + a0) + (x1.x + a1) + (x2.x + a2));
+        s += res(d1, f1, x1.y, (b0 + x1.x) + (b1 + x0.y) + (x3.y + b2));
+        s += res(d2, f2, x2.y, (c0 + x2.x) + (x3.y + c1) + (c2 + x0.y));
+        s += res(d3, f3, x3.x, (x3.y + g0) + (g1 + x2.x) + (g2 + x1.x));
+        s *= scale;
+        const bool red = ((uint32_t(E.y) >> 7) & 1u) == uint32_t(e & 1);
+        Cl.b[cc] = s;
+        Cl.x[cc] = red ? gs_value(0.0f, s, 0.0f, dc, MG_SORC) : 0.0f;
     }
 }
-__device__ void op0_sweep(const MgLevel& L, const int* fidx, const uint8_t* dg, int nf, int color, int t0, int stride) {
-    for (int base = t0, q0 = 0; base < nf; base += UNR * stride, q0 += UNR) {
-        Cells<> k;
-        load_cells(k, fidx, dg, nf, base, q0, stride, 1 + L.sy + L.sz);
-        float b[UNR], nb[UNR], xo[UNR];
+// The last (red) sweep of a coarse level fused with the prolongation of its
+// result: every FLUID fine cell with a FLUID parent adds omega * (parent's
+// value), where a red parent's value is its Gauss-Seidel update (recomputed
+// by each of its children from the final black neighbours, with the same
+// arithmetic, so all eight see the same bits) and a black parent's is final.
+// The coarse x is not needed after this, so it is not written back.  A quad's
+// four cells have two parents, an aligned pair.
+__device__ __forceinline__ void prolong_quad(const MgLevel& F, const MgLevel& Cl, float omega, const Quad& Q) {
+    const float* X = Cl.x + Q.pc;
+    float4 f = ld4(F.x + Q.c);
+    const int d = *reinterpret_cast<const uint16_t*>(Cl.code + Q.pc), d0 = d & 0xFF, d1 = d >> 8;
+    const float2 x = ld2(X), yp = ld2(X + Cl.sy), ym = ld2(X - Cl.sy), zp = ld2(X + Cl.sz), zm = ld2(X - Cl.sz);
+    const float xl = X[-1], xr = X[2];
+    const float2 b = ld2(Cl.b + Q.pc);
+    const bool odd = (Q.k & QUAD_PARENT_ODD) != 0u;  // the first parent is black
+    // the one parent that is red
+    const float nb = odd ? (xr + x.x) + (yp.y + ym.y) + (zp.y + zm.y) : (x.y + xl) + (yp.x + ym.x) + (zp.x + zm.x);
+    const float v = gs_value(odd ? x.y : x.x, odd ? b.y : b.x, nb, odd ? d1 : d0, MG_SORC);
+    const float v0 = odd ? x.x : v, v1 = odd ? v : x.y;
+    if (d0 > 0) {
+        if (code_at(Q.k, 0)) f.x = f.x + omega * v0;
+        if (code_at(Q.k, 1)) f.y = f.y + omega * v0;
+    }
+    if (d1 > 0) {
+        if (code_at(Q.k, 2)) f.z = f.z + omega * v1;
+        if (code_at(Q.k, 3)) f.w = f.w + omega * v1;
+    }
+    *reinterpret_cast<float4*>(F.x + Q.c) = f;
+}
+// Codes of the listed quads of a level from its labels (zero elsewhere).
+__device__ __forceinline__ void codes_quads(const MgLevel& L, const int4* list, int nq, int t0, int st) {
+    for (int n = t0; n < nq; n += st) {
+        const int c = list[n].x;
+        uint32_t k = 0;
 #pragma unroll
-        for (int u = 0; u < UNR; ++u) {
-            b[u] = L.b[k.c[u]];
-            nb[u] = lv_nbsum(L, k.c[u]);
-            xo[u] = MG_SOR == 1.0f ? 0.0f : L.x[k.c[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < UNR; ++u) {
-            const int d = k.db[u] & 0x7F;
-            if (k.ok[u] && (k.db[u] >> 7) == color) L.x[k.c[u]] = d > 0 ? sor(xo[u], (b[u] + nb[u]) / float(d)) : 0.0f;
-        }
+        for (int e = 0; e < 4; ++e)
+            if (L.lab[c + e] == FLUID) k |= uint32_t(1 + lv_diag(L, c + e)) << (8 * e);
+        *reinterpret_cast<uint32_t*>(L.code + c) = k;
     }
 }
-// ---- level operations over a (t0, stride) share of the work ----
+
+// ---- dense operations over a (t0, stride) share of a level: the block levels
+// in global memory, and the restriction into the first block level ----
 // They read the level's code (FLUID: 1 + diagonal, else 0) instead of labels,
 // and issue a cell's loads together, masked by the code afterwards: every
 // load is of an interior cell or its halo, so it stays in bounds.
 // Gauss-Seidel update of one FLUID cell (code dc > 0).
 __device__ __forceinline__ void gs_update(const MgLevel& L, int c) {
     const int dc = L.code[c];
-    const float bv = L.b[c], nb = lv_nbsum(L, c), xo = MG_SORC == 1.0f ? 0.0f : L.x[c];
-    if (dc > 0) L.x[c] = dc > 1 ? sorc(xo, (bv + nb) / float(dc - 1)) : 0.0f;
+    const float bv = L.b[c], nb = lv_nbsum(L, c), xo = L.x[c];
+    if (dc > 0) L.x[c] = gs_value(xo, bv, nb, dc, MG_SORC);
 }
-// Gauss-Seidel update of the FLUID cells of one colour.  With an even width
-// the work items are the cells of that colour only: cell i2 of a row is
-// i = 2 i2 + ((j + k + colour) & 1).
+// Gauss-Seidel update of the FLUID cells of one colour.
 __device__ void op_sweep(const MgLevel& L, int color, int t0, int stride) {
-    if ((L.W & 1) == 0) {
-        const int hw = L.W >> 1, n = hw * L.H * L.D;
-        for (int t = t0; t < n; t += stride) {
-            const int i2 = t % hw, r = t / hw, j = r % L.H, k = r / L.H;
-            const int i = 2 * i2 + ((j + k + color) & 1);
-            gs_update(L, (i + 1) + (j + 1) * L.sy + (k + 1) * L.sz);
-        }
-        return;
-    }
     const int n = L.W * L.H * L.D;
     for (int t = t0; t < n; t += stride) {
         int i, j, k;
@@ -228,13 +343,9 @@ __device__ __forceinline__ float fine_residual(const MgLevel& F, int c) {
     const float bv = F.b[c], xv = F.x[c], nb = lv_nbsum(F, c);
     return dc > 0 ? bv - (float(dc - 1) * xv - nb) : 0.0f;
 }
-// Restriction to the next level fused with that level's first sweep:
-// b_coarse = scale * sum over the red FLUID children of (b - A x), then
-// x_coarse = b/d on red FLUID cells, 0 elsewhere.  After the black sweep the
-// black residuals vanish, so only the red children (offsets with an even
-// coordinate sum) are read, in k, j, i order.  A child beyond
-// an odd-sized fine level (every 2D level in z) is skipped: its stencil would
-// leave the padded grid.
+// restrict_quads' operation over every cell of Cl (x and b zero off the fluid).
+// A child beyond an odd-sized fine level (every 2D level in z) is skipped: its
+// stencil would leave the padded grid.
 __device__ void op_restrict_first(const MgLevel& F, const MgLevel& Cl, float scale, int t0, int stride) {
     const int n = Cl.W * Cl.H * Cl.D;
     for (int t = t0; t < n; t += stride) {
@@ -244,35 +355,29 @@ __device__ void op_restrict_first(const MgLevel& F, const MgLevel& Cl, float sca
         float s = 0.0f, xv = 0.0f;
         if (dc > 0) {
             const bool ii = 2 * I + 1 < F.W, jj = 2 * J + 1 < F.H, kk = 2 * K + 1 < F.D;
-            const int c0 = (2 * I + 1) + (2 * J + 1) * F.sy + (2 * K + 1) * F.sz;
+            const int c0 = lv_index(F, 2 * I, 2 * J, 2 * K);
             s += fine_residual(F, c0);
             if (ii && jj) s += fine_residual(F, c0 + 1 + F.sy);
             if (ii && kk) s += fine_residual(F, c0 + 1 + F.sz);
             if (jj && kk) s += fine_residual(F, c0 + F.sy + F.sz);
             s *= scale;
-            if (((I + J + K) & 1) == 0) xv = dc > 1 ? sorc(0.0f, s / float(dc - 1)) : 0.0f;
+            if (((I + J + K) & 1) == 0) xv = gs_value(0.0f, s, 0.0f, dc, MG_SORC);
         }
         Cl.b[cc] = s;
         Cl.x[cc] = xv;
     }
 }
-// The last (red) sweep of a coarse level fused with the prolongation of its
-// result: every FLUID fine cell with a FLUID parent adds omega * (parent's
-// value), where a red parent's value is its Gauss-Seidel update (recomputed
-// by each of its children from the final black neighbours, with the same
-// arithmetic, so all eight see the same bits) and a black parent's is final.
-// The coarse x is not needed after this, so it is not written back.
+// prolong_quads' operation on one cell, and over every FLUID cell of F.
 __device__ __forceinline__ void prolong_one(const MgLevel& F, int c, const MgLevel& Cl, float omega, int i, int j,
                                             int k) {
     const int I = i >> 1, J = j >> 1, K = k >> 1;
-    const int cc = (I + 1) + (J + 1) * Cl.sy + (K + 1) * Cl.sz;
+    const int cc = lv_index(Cl, I, J, K);
     const int dc = Cl.code[cc];
     const float xc = Cl.x[cc], bc = Cl.b[cc], nb = lv_nbsum(Cl, cc), xf = F.x[c];
     if (dc == 0) return;
-    const float v = ((I + J + K) & 1) != 0 ? xc : (dc > 1 ? sorc(xc, (bc + nb) / float(dc - 1)) : 0.0f);
+    const float v = ((I + J + K) & 1) != 0 ? xc : gs_value(xc, bc, nb, dc, MG_SORC);
     F.x[c] = xf + omega * v;
 }
-// ... over every cell of the fine level F (dense levels)
 __device__ void op_prolong_red(const MgLevel& F, const MgLevel& Cl, float omega, int t0, int stride) {
     const int n = F.W * F.H * F.D;
     for (int t = t0; t < n; t += stride) {
@@ -281,47 +386,7 @@ __device__ void op_prolong_red(const MgLevel& F, const MgLevel& Cl, float omega,
         if (F.code[c] != 0) prolong_one(F, c, Cl, omega, i, j, k);
     }
 }
-// The same two operations over a list of the coarse (restriction) or fine
-// (prolongation) level's FLUID cells: the cells whose results the dense forms
-// compute, with the same arithmetic.  A thread's loads do not wait on the
-// cell's code, and one trip covers a level whose FLUID cells are fewer than
-// the grid's threads (at 128^3, level 1 has about 60 K of 262 K).  The other
-// cells' x and b stay zero: only FLUID cells are written, and the solve
-// clears them at its end.
-__device__ void op_restrict_first_list(const MgLevel& F, const MgLevel& Cl, float scale, const int* list, int n,
-                                       int t0, int stride) {
-    for (int t = t0; t < n; t += stride) {
-        const int cc = list[t];
-        const int I = cc % Cl.sy - 1, J = (cc / Cl.sy) % (Cl.H + 2) - 1, K = cc / Cl.sz - 1;
-        const int dc = Cl.code[cc];
-        const bool ii = 2 * I + 1 < F.W, jj = 2 * J + 1 < F.H, kk = 2 * K + 1 < F.D;
-        const int c0 = (2 * I + 1) + (2 * J + 1) * F.sy + (2 * K + 1) * F.sz;
-        float s = fine_residual(F, c0);
-        if (ii && jj) s += fine_residual(F, c0 + 1 + F.sy);
-        if (ii && kk) s += fine_residual(F, c0 + 1 + F.sz);
-        if (jj && kk) s += fine_residual(F, c0 + F.sy + F.sz);
-        s *= scale;
-        Cl.b[cc] = s;
-        Cl.x[cc] = ((I + J + K) & 1) == 0 && dc > 1 ? sorc(0.0f, s / float(dc - 1)) : 0.0f;
-    }
-}
-__device__ void op_prolong_red_list(const MgLevel& F, const MgLevel& Cl, float omega, const int* list, int n, int t0,
-                                    int stride) {
-    for (int t = t0; t < n; t += stride) {
-        const int c = list[t];
-        const int i = c % F.sy - 1, j = (c / F.sy) % (F.H + 2) - 1, k = c / F.sz - 1;
-        prolong_one(F, c, Cl, omega, i, j, k);
-    }
-}
-// ... over the level-0 FLUID list
-__device__ void op0_prolong_red(const MgLevel& F, const MgLevel& Cl, float omega, const int* fidx, int nf, int t0,
-                                int stride) {
-    for (int n = t0, q = 0; n < nf; n += stride, ++q) {
-        const int c = q < UNR ? s_fc[q * MG_THREADS + threadIdx.x] : fidx[n];
-        const int i = c % F.sy - 1, j = (c / F.sy) % (F.H + 2) - 1, k = c / F.sz - 1;
-        prolong_one(F, c, Cl, omega, i, j, k);
-    }
-}
+
 // Codes of the interior cells of a dense level from its labels.
 __device__ void op_codes(const MgLevel& L, int t0, int stride) {
     const int n = L.W * L.H * L.D;
@@ -343,7 +408,7 @@ __device__ __forceinline__ void coarsen_cell(const MgLevel& F, const MgLevel& Cl
             for (int a3 = 0; a3 < 2; ++a3) {
                 const int i = 2 * I + a3, j = 2 * J + b3, k = 2 * K + c3;
                 if (i >= F.W || j >= F.H || k >= F.D) continue;
-                const uint8_t l = F.lab[(i + 1) + (j + 1) * F.sy + (k + 1) * F.sz];
+                const uint8_t l = F.lab[lv_index(F, i, j, k)];
                 air |= l == AIR;
                 fluid |= l == FLUID;
             }
@@ -369,7 +434,6 @@ struct BlkLevel {
     int nred, nblack;     // FLUID cells of each colour
 };
 
-__host__ __device__ __forceinline__ int mg_npad(const MgLevel& L) { return (L.W + 2) * (L.H + 2) * (L.D + 2); }
 __host__ __device__ __forceinline__ int mg_cells(const MgLevel& L) { return L.W * L.H * L.D; }
 // Bytes of the block levels [G, L): every level's three FP32 grids (padded
 // cells rounded up to 4), then the two entry arrays (cells rounded up to 4),
@@ -378,9 +442,9 @@ __host__ __device__ __forceinline__ int mg_cells(const MgLevel& L) { return L.W 
 __host__ __device__ __forceinline__ int mg_smem_bytes(const MgLevel* lv, int G, int L) {
     int f = 0, e = 0, by = 0;
     for (int l = G; l < L; ++l) {
-        f += 3 * ((mg_npad(lv[l]) + 3) & ~3);
+        f += 3 * ((npad(lv[l]) + 3) & ~3);
         e += 2 * ((mg_cells(lv[l]) + 3) & ~3);
-        by += 2 * ((mg_npad(lv[l]) + 15) & ~15);
+        by += 2 * ((npad(lv[l]) + 15) & ~15);
     }
     return 4 * f + 4 * e + by;
 }
@@ -395,7 +459,7 @@ __device__ int block_levels_init(const MgArgs& a, BlkLevel* S) {
     if (t0 == 0) {
         float* f = reinterpret_cast<float*>(mg_smem);
         for (int l = G; l < L; ++l) {
-            const int n4 = (mg_npad(a.lv[l]) + 3) & ~3;
+            const int n4 = (npad(a.lv[l]) + 3) & ~3;
             S[l].m = a.lv[l];
             S[l].m.x = f; f += n4;
             S[l].m.b = f; f += n4;
@@ -409,9 +473,9 @@ __device__ int block_levels_init(const MgArgs& a, BlkLevel* S) {
         }
         uint8_t* by = reinterpret_cast<uint8_t*>(e);
         for (int l = G; l < L; ++l) {
-            const int n16 = (mg_npad(a.lv[l]) + 15) & ~15;
+            const int n16 = (npad(a.lv[l]) + 15) & ~15;
             S[l].m.lab = by; by += n16;
-            S[l].code = by; by += n16;
+            S[l].code = S[l].m.code = by; by += n16;
             S[l].cells = mg_cells(a.lv[l]);
             S[l].nred = S[l].nblack = 0;
         }
@@ -419,7 +483,12 @@ __device__ int block_levels_init(const MgArgs& a, BlkLevel* S) {
     uint4* z = reinterpret_cast<uint4*>(mg_smem);
     for (int i = t0; i < a.smem / 16; i += st) z[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    for (int c = t0; c < mg_npad(a.lv[G]); c += st) S[G].m.lab[c] = a.lv[G].lab[c];
+    {
+        // whole vectors (the grid and its copy are allocated up to a multiple of 16 bytes)
+        const uint4* src = reinterpret_cast<const uint4*>(a.lv[G].lab);
+        uint4* dst = reinterpret_cast<uint4*>(S[G].m.lab);
+        for (int c = t0; c < (npad(a.lv[G]) + 15) / 16; c += st) dst[c] = src[c];
+    }
     __syncthreads();
     for (int l = G + 1; l < L; ++l) {
         for (int t = t0; t < S[l].cells; t += st) coarsen_cell(S[l - 1].m, S[l].m, t);
@@ -427,15 +496,25 @@ __device__ int block_levels_init(const MgArgs& a, BlkLevel* S) {
     }
     for (int l = G; l < L; ++l) {
         BlkLevel& B = S[l];
-        for (int t = t0; t < B.cells; t += st) {
-            int i, j, k;
-            const int c = lv_cell(B.m, t, i, j, k);
-            if (B.m.lab[c] != FLUID) continue;
+        // (every lane of a warp takes part: one atomic per warp and colour)
+        for (int base = 0; base < B.cells; base += st) {
+            const int t = base + t0;
+            int i = 0, j = 0, k = 0;
+            const int c = lv_cell(B.m, min(t, B.cells - 1), i, j, k);
+            const bool fl = t < B.cells && B.m.lab[c] == FLUID, black = ((i + j + k) & 1) != 0;
+            const unsigned mr = __ballot_sync(0xffffffffu, fl && !black), mb = __ballot_sync(0xffffffffu, fl && black);
+            const int lane = t0 & 31;
+            int at = 0;
+            if (lane == 0 && mr) at = atomicAdd(&B.nred, __popc(mr));
+            if (lane == 1 && mb) at = atomicAdd(&B.nblack, __popc(mb));
+            const int r0 = __shfl_sync(0xffffffffu, at, 0), b0 = __shfl_sync(0xffffffffu, at, 1);
+            if (!fl) continue;
             B.code[c] = uint8_t(1 + lv_diag(B.m, c));
-            const int slot = ((i + j + k) & 1) == 0 ? atomicAdd(&B.nred, 1) : B.cells - 1 - atomicAdd(&B.nblack, 1);
-            const int pc = l + 1 < L ? ((i >> 1) + 1) + ((j >> 1) + 1) * S[l + 1].m.sy + ((k >> 1) + 1) * S[l + 1].m.sz : 0;
+            const unsigned below = (1u << lane) - 1u;
+            const int slot = black ? B.cells - 1 - (b0 + __popc(mb & below)) : r0 + __popc(mr & below);
+            const int pc = l + 1 < L ? lv_index(S[l + 1].m, i >> 1, j >> 1, k >> 1) : 0;
             B.ent[slot] = uint32_t(c) | (uint32_t(pc) << 16);
-            if (l > G) B.kid[slot] = uint32_t((2 * i + 1) + (2 * j + 1) * S[l - 1].m.sy + (2 * k + 1) * S[l - 1].m.sz);
+            if (l > G) B.kid[slot] = uint32_t(lv_index(S[l - 1].m, 2 * i, 2 * j, 2 * k));
         }
     }
     __syncthreads();
@@ -459,8 +538,7 @@ __device__ void bl_sweep(const BlkLevel& B, int color, int t0, int st) {
     const uint32_t* e = color == 0 ? B.ent : B.ent + (B.cells - B.nblack);
     for (int t = t0; t < n; t += st) {
         const int c = int(e[t] & 0xFFFFu);
-        const int d = B.code[c] - 1;
-        B.m.x[c] = d > 0 ? sorc(B.m.x[c], (B.m.b[c] + lv_nbsum(B.m, c)) / float(d)) : 0.0f;
+        B.m.x[c] = gs_value(B.m.x[c], B.m.b[c], lv_nbsum(B.m, c), B.code[c], MG_SORC);
     }
 }
 // rs = b - A x on the red FLUID cells (after a black sweep the black ones vanish).
@@ -484,8 +562,7 @@ __device__ void bl_restrict(const BlkLevel& F, const BlkLevel& C, float scale, i
         s += r[sz]; s += r[sz + 1]; s += r[sz + sy]; s += r[sz + sy + 1];
         s *= scale;
         C.m.b[cc] = s;
-        const int d = C.code[cc] - 1;
-        C.m.x[cc] = (t < C.nred && d > 0) ? sorc(0.0f, s / float(d)) : 0.0f;
+        C.m.x[cc] = t < C.nred ? gs_value(0.0f, s, 0.0f, C.code[cc], MG_SORC) : 0.0f;
     }
 }
 // Prolongation: every FLUID cell of F adds omega * its parent's x when the
@@ -505,7 +582,7 @@ __device__ void bl_prolong(const BlkLevel& F, const BlkLevel& C, float omega, in
 // level l0's last black sweep: the final red sweep of level l0 is the
 // grid-wide prolongation into level l0 - 1, which recomputes it from this
 // block's copy.
-__device__ void block_vcycle_smem(const MgArgs& a, int l0, int nl, const BlkLevel* S) {
+__device__ __noinline__ void block_vcycle_smem(const MgArgs& a, int l0, int nl, const BlkLevel* S) {
     const int t0 = threadIdx.x, st = blockDim.x;
     const BlkLevel& B0 = S[l0];
     const MgLevel& G0 = a.lv[l0];
@@ -560,7 +637,7 @@ __device__ void block_vcycle_smem(const MgArgs& a, int l0, int nl, const BlkLeve
 // right-hand side).  With l0 > 0 the stage stops after level l0's last black
 // sweep: the final red sweep of level l0 is the grid-wide prolongation into
 // level l0 - 1, which recomputes it.  With l0 == 0 it finishes level 0 itself.
-__device__ void block_vcycle_global(const MgArgs& a, int l0) {
+__device__ __noinline__ void block_vcycle_global(const MgArgs& a, int l0) {
     const int t0 = threadIdx.x, st = blockDim.x;
     for (int l = l0; l < a.L - 1; ++l) {
         op_sweep(a.lv[l], 1, t0, st); __syncthreads();
@@ -599,6 +676,25 @@ __device__ void block_vcycle_global(const MgArgs& a, int l0) {
     }
 }
 
+// The grid-wide operations of the cycle.  Functions of their own, not inlined
+// at each of their places in it: the cycle's code then stays in the instruction
+// cache.
+__device__ __noinline__ void grid_sweep(const MgArgs& a, int l, int color) {
+    const float w = l == 0 ? MG_SOR : MG_SORC;
+    const MgLevel& L = a.lv[l];
+    for_quads(a, l, [&](const Quad& Q, int) { sweep_quad(L, Q, color, w); });
+}
+__device__ __noinline__ void grid_restrict(const MgArgs& a, int l, int G) {
+    const int t0 = blockIdx.x * MG_THREADS + threadIdx.x, st = gridDim.x * MG_THREADS;
+    if (l + 1 < G) restrict_quads(a.lv[l], a.lv[l + 1], a.rscale, a.q[l + 1], s_nq[l + 1], t0, st);
+    else op_restrict_first(a.lv[l], a.lv[l + 1], a.rscale, t0, st);
+}
+__device__ __noinline__ void grid_prolong(const MgArgs& a, int lf, const MgLevel* Cp) {
+    const MgLevel& F = a.lv[lf];
+    const MgLevel C = *Cp;
+    for_quads(a, lf, [&](const Quad& Q, int) { prolong_quad(F, C, a.omega, Q); });
+}
+
 // z = V-cycle(r) with r = lv[0].b, z = lv[0].x.  The caller has already done
 // the first (red) sweep of level 0 (z = w b/d on red FLUID cells, 0 on black
 // ones) and a grid barrier since.  Ends with a grid barrier; returns false if
@@ -606,35 +702,22 @@ __device__ void block_vcycle_global(const MgArgs& a, int l0) {
 // sweep pair (level 0 two more per extra pair): black sweep, restriction (with
 // the next level's first sweep), black sweep, red sweep (with the
 // prolongation into the finer level).  nl: the levels that hold FLUID cells.
-// n1: the number of level 1's listed FLUID cells (a.l1list), or -1 for none.
-__device__ bool vcycle(const MgArgs& a, const BlkLevel* S, int nl, int n1) {
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+__device__ bool vcycle(const MgArgs& a, const BlkLevel* S, int nl) {
     const unsigned nb = gridDim.x;
     const int G = min(a.G, a.L - 1);
-    const int nf = *a.nf;
-    // restriction from level l and prolongation into level lf >= 1, level 1
-    // over its FLUID list when there is one
-    auto restrict_first = [&](int l) {
-        if (l == 0 && n1 >= 0) op_restrict_first_list(a.lv[0], a.lv[1], a.rscale, a.l1list, n1, t0, st);
-        else op_restrict_first(a.lv[l], a.lv[l + 1], a.rscale, t0, st);
-    };
-    auto prolong_into = [&](int lf, const MgLevel& Cl) {
-        if (lf == 1 && n1 >= 0) op_prolong_red_list(a.lv[1], Cl, a.omega, a.l1list, n1, t0, st);
-        else op_prolong_red(a.lv[lf], Cl, a.omega, t0, st);
-    };
-    // one grid-wide sweep of level l (colour 0 red, 1 black) and a barrier
     auto sweep = [&](int l, int color) {
-        if (l == 0) op0_sweep(a.lv[0], a.fidx, a.diag, nf, color, t0, st);
-        else op_sweep(a.lv[l], color, t0, st);
+        grid_sweep(a, l, color);
         return grid_barrier(a.bar, nb, a.status);
     };
+#pragma unroll 1
     for (int l = 0; l < G; ++l) {
         // pre-smoothing (red, black)^nu (nu = nu0 on level 0, else nu_grid); the
         // first red sweep is fused upstream
-        if (!sweep(l, 1)) return false;
-        for (int e = 1; e < (l == 0 ? a.nu0 : a.nu_grid); ++e)
-            if (!sweep(l, 0) || !sweep(l, 1)) return false;
-        restrict_first(l);
+        const int n = 2 * (l == 0 ? a.nu0 : a.nu_grid) - 1;
+#pragma unroll 1
+        for (int e = 0; e < n; ++e)
+            if (!sweep(l, (e & 1) ^ 1)) return false;
+        grid_restrict(a, l, G);
         if (!grid_barrier(a.bar, nb, a.status)) return false;
     }
     if (a.smem) {
@@ -642,126 +725,121 @@ __device__ bool vcycle(const MgArgs& a, const BlkLevel* S, int nl, int n1) {
         // same arithmetic, so the same bits) and prolongs from that copy: no
         // grid barrier and no copy-out between the stage and the prolongation.
         block_vcycle_smem(a, G, nl, S);
-        MgLevel cg = S[G].m;  // level G in this block's shared memory
-        cg.code = S[G].code;
-        if (G == 1) op0_prolong_red(a.lv[0], cg, a.omega, a.fidx, nf, t0, st);
-        else prolong_into(G - 1, cg);
+        grid_prolong(a, G - 1, &S[G].m);
         if (!grid_barrier(a.bar, nb, a.status)) return false;
     } else {
         if (blockIdx.x == 0) block_vcycle_global(a, G);
         if (!grid_barrier(a.bar, nb, a.status)) return false;
         if (G > 0) {  // level G's last red sweep, fused with its prolongation into level G - 1
-            if (G == 1) op0_prolong_red(a.lv[0], a.lv[1], a.omega, a.fidx, nf, t0, st);
-            else prolong_into(G - 1, a.lv[G]);
+            grid_prolong(a, G - 1, &a.lv[G]);
             if (!grid_barrier(a.bar, nb, a.status)) return false;
         }
     }
+#pragma unroll 1
     for (int l = G - 1; l >= 0; --l) {
         // post-smoothing (black, red)^nu, the reverse of the pre-smoothing; the
         // first red sweep was fused with the prolongation, the last red sweep
         // with the next prolongation
-        if (!sweep(l, 1)) return false;
-        for (int e = 1; e < (l == 0 ? a.nu0 : a.nu_grid); ++e)
-            if (!sweep(l, 0) || !sweep(l, 1)) return false;
-        if (l == 0) op0_sweep(a.lv[0], a.fidx, a.diag, nf, 0, t0, st);
-        else if (l == 1) op0_prolong_red(a.lv[0], a.lv[1], a.omega, a.fidx, nf, t0, st);
-        else prolong_into(l - 1, a.lv[l]);
+        const int n = 2 * (l == 0 ? a.nu0 : a.nu_grid) - 1;
+#pragma unroll 1
+        for (int e = 0; e < n; ++e)
+            if (!sweep(l, (e & 1) ^ 1)) return false;
+        if (l == 0) grid_sweep(a, 0, 0);
+        else grid_prolong(a, l - 1, &a.lv[l]);
         if (!grid_barrier(a.bar, nb, a.status)) return false;
     }
     return true;
 }
 
-// Level-0 first sweep value of one FLUID cell: b/d on red cells, 0 on black.
-__device__ __forceinline__ float first_red0(float b, uint8_t db) {
-    const int d = db & 0x7F;
-    return ((db >> 7) == 0 && d > 0) ? sor(0.0f, b / float(d)) : 0.0f;
+// Level-0 first sweep value of one cell with code dc: b/d on red FLUID cells, else 0.
+__device__ __forceinline__ float first_red0(float b, int dc, bool red) {
+    return red ? gs_value(0.0f, b, 0.0f, dc, MG_SOR) : 0.0f;
+}
+// b0 and the first sweep's z of one quad from its residual.
+__device__ __forceinline__ void start_cycle(const MgLevel& F, int c, uint32_t k, float4 b) {
+    const bool odd = ((k >> 7) & 1u) != 0u;
+    *reinterpret_cast<float4*>(F.b + c) = b;
+    *reinterpret_cast<float4*>(F.x + c) =
+        make_float4(first_red0(b.x, code_at(k, 0), !odd), first_red0(b.y, code_at(k, 1), odd),
+                    first_red0(b.z, code_at(k, 2), !odd), first_red0(b.w, code_at(k, 3), odd));
 }
 
-__global__ void __launch_bounds__(MG_THREADS) k_pcg_mg(MgArgs a) {
-    const int nf = *a.nf;
-    const int nb = int(gridDim.x);
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, st = nb * blockDim.x;
-    const MgLevel& F = a.lv[0];
-    const int n1 = a.l1list && a.L > 1 ? *a.l1n : -1;  // level 1's listed FLUID cells
-    float* b0 = F.b;  // FP32 copy of r: the V-cycle's right-hand side
-    float* z = F.x;   // FP32 preconditioned residual
-    double* r = a.r;
-    int red = 0;      // reduction counter (partial buffers double-buffered by parity)
-    auto partial = [&](double v0, double v1, double v2) {
-        double3 bs = block_sum3(v0, v1, v2);
-        double* pp = a.part + (red & 1) * 3 * nb;
-        if (threadIdx.x == 0) { pp[blockIdx.x] = bs.x; pp[nb + blockIdx.x] = bs.y; pp[2 * nb + blockIdx.x] = bs.z; }
+struct D4 {
+    double v[4];
+};
+__device__ __forceinline__ D4 ldq(const double2* p, int cap, int n) {
+    const double2 a = p[n], b = p[cap + n];
+    return D4{{a.x, a.y, b.x, b.y}};
+}
+__device__ __forceinline__ void stq(double2* p, int cap, int n, const D4& d) {
+    p[n] = make_double2(d.v[0], d.v[1]);
+    p[cap + n] = make_double2(d.v[2], d.v[3]);
+}
+// A z at the four cells of a quad exactly (FP32 values summed in FP64), 0 off the fluid; zc: z itself.
+__device__ __forceinline__ D4 apply_quad(const MgLevel& F, int c, uint32_t k, float4& zc) {
+    const float* z = F.x + c;
+    zc = ld4(z);
+    const float4 yp = ld4(z + F.sy), ym = ld4(z - F.sy), zp = ld4(z + F.sz), zm = ld4(z - F.sz);
+    const float xl = z[-1], xr = z[4];
+    auto at = [&](int e, float v, float r, float l, float a, float b, float f, float g) {
+        const int dc = code_at(k, e);
+        const double s = (double(r) + double(l)) + (double(a) + double(b)) + (double(f) + double(g));
+        return dc > 0 ? double(dc - 1) * double(v) - s : 0.0;
     };
-    auto total = [&]() { double3 t = grid_sum3(a.part + (red & 1) * 3 * nb, nb); ++red; return t; };
-    const int sy = F.sy, sz = F.sz;
+    return D4{{at(0, zc.x, zc.y, xl, yp.x, ym.x, zp.x, zm.x), at(1, zc.y, zc.z, zc.x, yp.y, ym.y, zp.y, zm.y),
+               at(2, zc.z, zc.w, zc.y, yp.z, ym.z, zp.z, zm.z), at(3, zc.w, xr, zc.z, yp.w, ym.w, zp.w, zm.w)}};
+}
+
+__global__ void __launch_bounds__(MG_THREADS, 1) k_pcg_mg(const __grid_constant__ MgArgs a) {
+    const int nb = int(gridDim.x);
+    const int t0 = blockIdx.x * MG_THREADS + threadIdx.x, st = nb * MG_THREADS;
+    const MgLevel& F = a.lv[0];
+    if (threadIdx.x < MG_MAX_LEVELS) s_nq[threadIdx.x] = a.nq[threadIdx.x];
+    if (threadIdx.x < 8) s_rcp[threadIdx.x] = threadIdx.x > 1 ? 1.0f / float(threadIdx.x - 1) : 0.0f;
+    __syncthreads();
+    const int nq = s_nq[0], cap = a.cap, G = min(a.G, a.L - 1);
+    const int4* list = a.q[0];
+    int red = 0;  // reductions so far (the partial buffers alternate)
+    auto sum = [&](double (&v)[3]) {
+        return grid_reduce(v, a.part + (red++ & 1) * 3 * nb, a.bar, nb, a.status);
+    };
     __shared__ BlkLevel s_lv[MG_MAX_LEVELS];  // the shared-memory block levels
     const int nl = a.smem ? block_levels_init(a, s_lv) : a.L;  // every block: its own copy
 
-    // level codes: level 0 on its FLUID cells (zero elsewhere, restored at the
-    // end), the dense grid-wide levels (and, without shared-memory copies, the
-    // block levels) over all their cells
-    for (int l = 1; l <= (a.smem ? a.G : a.L - 1); ++l) op_codes(a.lv[l], t0, st);
-    cache_cells(a.fidx, a.diag, nf, t0, st, 1 + sy + sz);
-    // r = rhs, the V-cycle's right-hand side and first sweep, the level-0
-    // codes and the guess.  A dense guess (the previous pressure, zero off the
-    // current fluid and outside the grid) also gets its stencil A g and the
-    // dot products here: it was complete before the launch, so its
-    // neighbours need no grid barrier.  A compact guess needs one.
-    const bool dense_guess = a.pprev != nullptr;
-    double rrl = 0.0, xb = 0.0, xq = 0.0;
-    constexpr int UI = 2;
-    for (int base = t0, q0 = 0; base < nf; base += UI * st, q0 += UI) {
-        Cells<UI> k;
-        load_cells(k, a.fidx, a.diag, nf, base, q0, st, 1 + sy + sz);
-        float bvf[UI], g[UI];
-        double qv[UI];
+    // level codes: the listed quads of the grid-wide levels (zero elsewhere,
+    // restored at the end), the other levels over all their cells
+    for (int l = 1; l < G; ++l) codes_quads(a.lv[l], a.q[l], s_nq[l], t0, st);
+    for (int l = max(G, 1); l <= (a.smem ? G : a.L - 1); ++l) op_codes(a.lv[l], t0, st);
+    fill_slots(a, 0, 1, t0, st);
+    // r = rhs, the level-0 codes, and the guess (kept as the FP32 values z) or
+    // the V-cycle's right-hand side and first sweep
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int n = t0; n < nq; n += st) {
+        const int4 e = list[n];
+        const uint32_t k = uint32_t(e.y);
+        const float4 bf = a.rhs[n];
+        const D4 r{{double(bf.x), double(bf.y), double(bf.z), double(bf.w)}};
+        *reinterpret_cast<uint32_t*>(F.code + e.x) = k & QUAD_CODES;
+        stq(a.r, cap, n, r);
 #pragma unroll
-        for (int u = 0; u < UI; ++u) {
-            const int n = base + u * st;
-            bvf[u] = k.ok[u] ? a.rhs[n] : 0.0f;
-            g[u] = 0.0f;
-            qv[u] = 0.0;
-            if (!k.ok[u]) continue;
-            if (a.x0) {
-                g[u] = a.x0[n];
-            } else if (dense_guess) {
-                const int c = k.c[u];
-                const int i = c % sy - 1, j = (c / sy) % (F.H + 2) - 1, kk = c / sz - 1;
-                const int64_t e = (int64_t(kk) * F.H + j) * F.W + i, sY = F.W, sZ = int64_t(F.W) * F.H;
-                auto gv = [&](bool in, int64_t off) {
-                    const float v = in ? a.pprev[e + off] : 0.0f;
-                    return isfinite(v) ? double(v) : 0.0;
-                };
-                const double gc = gv(true, 0);
-                g[u] = float(gc);
-                qv[u] = double(k.db[u] & 0x7F) * gc - ((gv(i + 1 < F.W, 1) + gv(i > 0, -1)) +
-                                                        (gv(j + 1 < F.H, sY) + gv(j > 0, -sY)) +
-                                                        (gv(kk + 1 < F.D, sZ) + gv(kk > 0, -sZ)));
-            }
-        }
+        for (int m = 0; m < 4; ++m) v[0] += r.v[m] * r.v[m];
+        if (a.guess) {
+            float g[4];
 #pragma unroll
-        for (int u = 0; u < UI; ++u) {
-            if (!k.ok[u]) continue;
-            const int c = k.c[u];
-            const double rv = double(bvf[u]);
-            F.code[c] = uint8_t(1 + (k.db[u] & 0x7F));
-            r[c] = rv;
-            b0[c] = float(rv);
-            z[c] = first_red0(float(rv), k.db[u]);  // the V-cycle's first sweep
-            a.xs[c] = double(g[u]);
-            if (dense_guess) {
-                a.q[c] = qv[u];
-                xb += double(g[u]) * rv;
-                xq += double(g[u]) * qv[u];
+            for (int m = 0; m < 4; ++m) {
+                g[m] = code_at(k, m) ? a.guess[e.w + m] : 0.0f;
+                if (!a.guess_dir && !isfinite(g[m])) g[m] = 0.0f;
             }
-            rrl += rv * rv;
+            *reinterpret_cast<float4*>(F.x + e.x) = make_float4(g[0], g[1], g[2], g[3]);
+        } else {
+            stq(a.xs, cap, n, D4{{0.0, 0.0, 0.0, 0.0}});
+            start_cycle(F, e.x, k, bf);
         }
     }
-    const bool guess = a.x0 || a.pprev;
-    double bb_warm = 0.0;  // ||b||^2 when started from a guess
     // With a guess g the solve's first flexible-CG step uses g as its
     // preconditioned residual: z0 = g, p0 = z0, alpha0 = (r0, z0) / (p0, A p0)
-    // -- the energy-optimal scaling -- and x1 = alpha0 g.  For the network's
+    // -- the energy-optimal scaling: the A-norm error of alpha0 g is never
+    // above that of x = 0 -- and x1 = alpha0 g.  For the network's
     // guess N(b) (the learned preconditioner), p0, A p0, gamma0 = (r0, z0) and
     // (p0, A p0) stay in the recurrence, so the next direction (from the
     // V-cycle) is made A-conjugate to p0 by the Polak-Ribiere beta.  The
@@ -769,57 +847,50 @@ __global__ void __launch_bounds__(MG_THREADS) k_pcg_mg(MgArgs a) {
     // cost iterations (11.2 against 10.8 per warm-started solve at 128^3).
     bool dir0 = false;
     double gam0 = 0.0, alpha0 = 0.0, den0 = 0.0;
-    if (guess) {
-        // Scale the guess by its energy-optimal factor alpha = (x0, b) / (x0, A x0):
-        // the A-norm error of alpha x0 is never above that of x = 0.  Then r = b - A x.
-        if (a.x0) {
-            if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-            for (int n = t0; n < nf; n += st) {
-                const int c = a.fidx[n];
-                const double* xp = a.xs + c;
-                const double qc = double(a.diag[n] & 0x7F) * xp[0] -
-                                  ((xp[1] + xp[-1]) + (xp[sy] + xp[-sy]) + (xp[sz] + xp[-sz]));
-                a.q[c] = qc;
-                xb += xp[0] * r[c];
-                xq += xp[0] * qc;
-            }
-        }
-        partial(xb, xq, rrl);
-        if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-        const double3 t = total();
-        const double alpha = (t.y > 0.0 && isfinite(t.x / t.y)) ? t.x / t.y : 0.0;
-        dir0 = alpha != 0.0 && a.x0 != nullptr;  // the learned guess only (see above)
-        gam0 = t.x; alpha0 = alpha; den0 = t.y;
-        bb_warm = t.z;  // all reads of x ended before the barrier above
-        rrl = 0.0;
-        for (int base = t0, q0 = 0; base < nf; base += UI * st, q0 += UI) {
-            Cells<UI> k;
-            load_cells(k, a.fidx, a.diag, nf, base, q0, st, 1 + sy + sz);
-            double xv[UI], rv0[UI], qc[UI];
+    if (!sum(v)) return;
+    fill_slots(a, 1, G, t0, st);
+    const double bb = v[0];
+    double rr = bb;
+    if (a.guess) {
+        v[0] = v[1] = v[2] = 0.0;
+        for_quads(a, 0, [&](const Quad& Q, int n) {
+            const int c = Q.c;
+            const uint32_t k = Q.k;
+            float4 g;
+            const D4 s = apply_quad(F, c, k, g), r = ldq(a.r, cap, n);
+            const double gd[4] = {double(g.x), double(g.y), double(g.z), double(g.w)};
+            stq(a.s, cap, n, s);
 #pragma unroll
-            for (int u = 0; u < UI; ++u) {
-                xv[u] = a.xs[k.c[u]];
-                rv0[u] = r[k.c[u]];
-                qc[u] = a.q[k.c[u]];
+            for (int m = 0; m < 4; ++m) {
+                v[0] += gd[m] * r.v[m];
+                v[1] += gd[m] * s.v[m];
             }
+        });
+        if (!sum(v)) return;
+        const double alpha = (v[1] > 0.0 && isfinite(v[0] / v[1])) ? v[0] / v[1] : 0.0;
+        dir0 = alpha != 0.0 && a.guess_dir;
+        gam0 = v[0]; alpha0 = alpha; den0 = v[1];
+        v[0] = v[1] = v[2] = 0.0;
+        for_quads(a, 0, [&](const Quad& Q, int n) {
+            const int c = Q.c;
+            const uint32_t k = Q.k;
+            const float4 g = ld4(F.x + c);
+            const D4 s = ldq(a.s, cap, n);
+            D4 r = ldq(a.r, cap, n), x{{double(g.x), double(g.y), double(g.z), double(g.w)}};
+            if (a.guess_dir) stq(a.p, cap, n, x);  // p0 = g; s holds A p0
 #pragma unroll
-            for (int u = 0; u < UI; ++u) {
-                if (!k.ok[u]) continue;
-                const int c = k.c[u];
-                a.xs[c] = xv[u] * alpha;
-                if (a.x0) a.p[c] = xv[u];  // the learned guess: p0 = g; q holds A p0
-                const double rv = rv0[u] - alpha * qc[u];
-                r[c] = rv;
-                b0[c] = float(rv);
-                z[c] = first_red0(float(rv), k.db[u]);
-                rrl += rv * rv;
+            for (int m = 0; m < 4; ++m) {
+                x.v[m] *= alpha;
+                r.v[m] = r.v[m] - alpha * s.v[m];
+                v[0] += r.v[m] * r.v[m];
             }
-        }
+            stq(a.xs, cap, n, x);
+            stq(a.r, cap, n, r);
+            start_cycle(F, c, k, make_float4(float(r.v[0]), float(r.v[1]), float(r.v[2]), float(r.v[3])));
+        });
+        if (!sum(v)) return;
+        rr = v[0];
     }
-    partial(rrl, 0.0, 0.0);
-    if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-    double rr = total().x;
-    const double bb = guess ? bb_warm : rr;
     const double rr0 = rr;
     const double thr = a.tol * a.tol * bb;
     // Flexible preconditioned CG in the Chronopoulos-Gear form: after the
@@ -830,88 +901,68 @@ __global__ void __launch_bounds__(MG_THREADS) k_pcg_mg(MgArgs a) {
     // gamma_old, and (p, A p) = delta + 2 beta zeta + beta^2 (p, A p)_old holds
     // for any beta, so alpha = gamma / (p, A p) needs no symmetry of the
     // V-cycle (over-relaxed smoothing makes it slightly non-symmetric).  Two
-    // grid-wide passes per iteration besides the cycle.  w is kept in the
-    // compact X buffer (the solution is written there only at the end); s
-    // lives in q.
-    double* w = a.X;
+    // grid-wide passes per iteration besides the cycle.
     double gam = 0.0, gam_old = gam0, alpha_old = dir0 ? alpha0 : 1.0, den_old = dir0 ? den0 : 1.0;
     int it = 0, stt = DEV_OK;
     while (rr > thr && bb > 0.0) {
         if (it >= a.maxit) { stt = DEV_MAXIT; break; }
-        if (!vcycle(a, s_lv, nl, n1)) return;  // z = M^-1 r
-        double gl = 0.0, dl = 0.0, sl = 0.0;
-        constexpr int U3 = 3;  // three cells in flight fit the register budget with FP64 sums
-        for (int base = t0, q0 = 0; base < nf; base += U3 * st, q0 += U3) {
-            Cells<U3> k;
-            load_cells(k, a.fidx, a.diag, nf, base, q0, st, 1 + sy + sz);
-            float zc[U3];
-            double zn[U3], rc[U3], sc[U3];  // A z exactly: FP32 values summed in FP64
-#pragma unroll
-            for (int u = 0; u < U3; ++u) {
-                const float* zp = z + k.c[u];
-                zc[u] = zp[0];
-                zn[u] = (double(zp[1]) + double(zp[-1])) + (double(zp[sy]) + double(zp[-sy])) +
-                        (double(zp[sz]) + double(zp[-sz]));
-                rc[u] = r[k.c[u]];
-                sc[u] = a.q[k.c[u]];
-            }
-#pragma unroll
-            for (int u = 0; u < U3; ++u) {
-                if (!k.ok[u]) continue;
-                const double zv = double(zc[u]);
-                const double wv = double(k.db[u] & 0x7F) * zv - zn[u];
-                w[base + u * st] = wv;
-                gl += rc[u] * zv;
-                dl += zv * wv;
-                sl += zv * sc[u];
-            }
-        }
-        partial(gl, dl, sl);
-        if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-        const double3 t = total();
-        gam = t.x;
-        if (isnan(t.x) || isnan(t.y) || isnan(t.z)) { stt = DEV_NAN; break; }
+        if (!vcycle(a, s_lv, nl)) return;  // z = M^-1 r
         const bool coupled = it > 0 || dir0;  // a previous direction to conjugate against
-        const double beta = coupled ? -alpha_old * t.z / gam_old : 0.0;
-        const double den = coupled ? t.y + beta * (2.0 * t.z + beta * den_old) : t.y;
+        v[0] = v[1] = v[2] = 0.0;
+        for_quads(a, 0, [&](const Quad& Q, int n) {
+            const int c = Q.c;
+            const uint32_t k = Q.k;
+            float4 zf;
+            const D4 r = ldq(a.r, cap, n);
+            D4 s{{0.0, 0.0, 0.0, 0.0}};
+            if (coupled) s = ldq(a.s, cap, n);
+            const D4 w = apply_quad(F, c, k, zf);
+            const double z[4] = {double(zf.x), double(zf.y), double(zf.z), double(zf.w)};
+            stq(a.w, cap, n, w);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                v[0] += r.v[m] * z[m];
+                v[1] += z[m] * w.v[m];
+                v[2] += z[m] * s.v[m];
+            }
+        });
+        if (!sum(v)) return;
+        gam = v[0];
+        if (isnan(v[0]) || isnan(v[1]) || isnan(v[2])) { stt = DEV_NAN; break; }
+        const double beta = coupled ? -alpha_old * v[2] / gam_old : 0.0;
+        const double den = coupled ? v[1] + beta * (2.0 * v[2] + beta * den_old) : v[1];
         if (!(den > 0.0)) { stt = DEV_BREAKDOWN; break; }
         const double alpha = gam / den;
-        rrl = 0.0;
-        constexpr int U2 = 2;  // FP64: two cells in flight fit the register budget
-        for (int base = t0, q0 = 0; base < nf; base += U2 * st, q0 += U2) {
-            Cells<U2> k;
-            load_cells(k, a.fidx, a.diag, nf, base, q0, st, 1 + sy + sz);
-            double pv[U2], sv[U2], xv[U2], rv[U2], wv[U2];
-            float zc[U2];
+        v[0] = v[1] = v[2] = 0.0;
+        for_quads(a, 0, [&](const Quad& Q, int n) {
+            const int c = Q.c;
+            const uint32_t k = Q.k;
+            const float4 zf = ld4(F.x + c);
+            const D4 w = ldq(a.w, cap, n);
+            D4 x = ldq(a.xs, cap, n), r = ldq(a.r, cap, n);
+            D4 p{{double(zf.x), double(zf.y), double(zf.z), double(zf.w)}}, s = w;
+            if (coupled) {
+                const D4 po = ldq(a.p, cap, n), so = ldq(a.s, cap, n);
 #pragma unroll
-            for (int u = 0; u < U2; ++u) {
-                const int c = k.c[u];
-                zc[u] = z[c];
-                pv[u] = a.p[c];
-                sv[u] = a.q[c];
-                xv[u] = a.xs[c];
-                rv[u] = r[c];
-                wv[u] = k.ok[u] ? w[base + u * st] : 0.0;
+                for (int m = 0; m < 4; ++m) {
+                    p.v[m] = p.v[m] + beta * po.v[m];
+                    s.v[m] = w.v[m] + beta * so.v[m];
+                }
             }
 #pragma unroll
-            for (int u = 0; u < U2; ++u) {
-                if (!k.ok[u]) continue;
-                const int c = k.c[u];
-                const double pn = coupled ? double(zc[u]) + beta * pv[u] : double(zc[u]);
-                const double sn = coupled ? wv[u] + beta * sv[u] : wv[u];
-                a.p[c] = pn;
-                a.q[c] = sn;
-                a.xs[c] = xv[u] + alpha * pn;
-                const double rn = rv[u] - alpha * sn;
-                r[c] = rn;
-                b0[c] = float(rn);
-                z[c] = first_red0(float(rn), k.db[u]);
-                rrl += rn * rn;
+            for (int m = 0; m < 4; ++m) {
+                x.v[m] = x.v[m] + alpha * p.v[m];
+                r.v[m] = r.v[m] - alpha * s.v[m];
+                v[0] += r.v[m] * r.v[m];
             }
-        }
-        partial(rrl, 0.0, 0.0);
-        if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-        rr = total().x;
+            stq(a.p, cap, n, p);
+            stq(a.s, cap, n, s);
+            stq(a.xs, cap, n, x);
+            stq(a.r, cap, n, r);
+            start_cycle(F, c, k, make_float4(float(r.v[0]), float(r.v[1]), float(r.v[2]), float(r.v[3])));
+        });
+        if (!sum(v)) return;
+        rr = v[0];
         ++it;
         if (isnan(rr)) { stt = DEV_NAN; break; }
         gam_old = gam;
@@ -919,43 +970,55 @@ __global__ void __launch_bounds__(MG_THREADS) k_pcg_mg(MgArgs a) {
         den_old = den;
     }
     // The true residual of the FP64 solution, ||rhs - A x||^2 and ||rhs||^2,
-    // then the compact and dense solution; zero the level-0 work grids at the
-    // FLUID cells so the next solve starts from zero whatever cells are fluid.
+    // then the dense solution; zero the work grids at the listed quads so the
+    // next solve starts from zero whatever cells are fluid.
+    for_quads(a, 0, [&](const Quad& Q, int n) {
+        const int c = Q.c;
+        const uint32_t k = Q.k;
+        const D4 x = ldq(a.xs, cap, n);
+        double2* X = reinterpret_cast<double2*>(a.xd + c);
+        X[0] = make_double2(x.v[0], x.v[1]);
+        X[1] = make_double2(x.v[2], x.v[3]);
+    });
     if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-    {
-        double e2 = 0.0, b2 = 0.0;
-        for (int n = t0; n < nf; n += st) {
-            const int c = a.fidx[n];
-            const double* xp = a.xs + c;
-            const double ax = double(a.diag[n] & 0x7F) * xp[0] -
-                              ((xp[1] + xp[-1]) + (xp[sy] + xp[-sy]) + (xp[sz] + xp[-sz]));
-            const double bv = double(a.rhs[n]), e = bv - ax;
-            e2 += e * e;
-            b2 += bv * bv;
+    v[0] = v[1] = v[2] = 0.0;
+    for_quads(a, 0, [&](const Quad& Q, int n) {
+        const int c = Q.c;
+        const uint32_t k = Q.k;
+        const float4 bf = a.rhs[n];
+        const float b[4] = {bf.x, bf.y, bf.z, bf.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int dc = code_at(k, m);
+            if (dc == 0) continue;
+            const double* x = a.xd + c + m;
+            const double ax = double(dc - 1) * x[0] -
+                              ((x[1] + x[-1]) + (x[F.sy] + x[-F.sy]) + (x[F.sz] + x[-F.sz]));
+            const double bv = double(b[m]), e = bv - ax;
+            v[0] += e * e;
+            v[1] += bv * bv;
         }
-        partial(e2, b2, 0.0);
+    });
+    if (!sum(v)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.red[0] = v[0]; a.red[1] = v[1]; }
+    for (int n = t0; n < nq; n += st) {
+        const int4 e = list[n];
+        const uint32_t k = uint32_t(e.y);
+        const D4 x = ldq(a.xs, cap, n);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (code_at(k, m)) a.pout[e.w + m] = float(x.v[m]);
+        double2* X = reinterpret_cast<double2*>(a.xd + e.x);
+        X[0] = X[1] = make_double2(0.0, 0.0);
+        *reinterpret_cast<float4*>(F.x + e.x) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        *reinterpret_cast<uint32_t*>(F.code + e.x) = 0u;
     }
-    if (!grid_barrier(a.bar, unsigned(nb), a.status)) return;
-    {
-        const double3 t = total();
-        if (blockIdx.x == 0 && threadIdx.x == 0) { a.red[0] = t.x; a.red[1] = t.y; }
-    }
-    for (int n = t0; n < nf; n += st) {
-        const int c = a.fidx[n];
-        const double xv = a.xs[c];
-        a.X[n] = xv;
-        if (a.pout) {
-            const int i = c % sy - 1, j = (c / sy) % (F.H + 2) - 1, k = c / sz - 1;
-            a.pout[(int64_t(k) * F.H + j) * F.W + i] = float(xv);
+    for (int l = 1; l < G; ++l)
+        for (int n = t0; n < s_nq[l]; n += st) {
+            const int c = a.q[l][n].x;
+            *reinterpret_cast<float4*>(a.lv[l].x + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            *reinterpret_cast<uint32_t*>(a.lv[l].code + c) = 0u;
         }
-        a.xs[c] = fmin(fabs(xv), 0.0);  // +0 computed from the load (a constant store would wait on it)
-        a.p[c] = 0.0; a.q[c] = 0.0; r[c] = 0.0; b0[c] = 0.0f; z[c] = 0.0f; F.code[c] = 0;
-    }
-    for (int t = t0; t < n1; t += st) {  // level 1's FLUID cells: x and b back to zero
-        const int c = a.l1list[t];
-        a.lv[1].x[c] = 0.0f;
-        a.lv[1].b[c] = 0.0f;
-    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.out->iters = it;
         atomicCAS(a.status, DEV_OK, stt);
@@ -966,42 +1029,57 @@ __global__ void __launch_bounds__(MG_THREADS) k_pcg_mg(MgArgs a) {
     }
 }
 
-// Coarse labels with Dirichlet priority: AIR if any child AIR, else FLUID if
-// any child FLUID, else SOLID.
-__global__ void k_coarsen(MgLevel F, MgLevel Cl) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < Cl.W * Cl.H * Cl.D) coarsen_cell(F, Cl, t);
-}
-
-// Level 1 straight from the cell labels, by the same rule (BODY, like SOLID,
-// is neither AIR nor FLUID); level 0 itself needs no padded label copy, as
-// its operations read the FLUID list's diagonal bytes and codes.
-// It also appends level 1's FLUID cells (padded indices) to list, one atomic
-// per block, in no fixed order: every use of the list treats its cells
-// independently.  *nlist must be zero before the launch; at most cap entries
-// are written.
+// Labels of level Cl from the finer level's, with Dirichlet priority (AIR if
+// any child AIR, else FLUID if any child FLUID, else SOLID; BODY, like SOLID,
+// is neither), one thread per quad, and the list of the quads that hold a
+// FLUID cell (one atomic per block, in no fixed order: every use of the list
+// treats its quads independently).  raw: the finer level is the cell labels
+// themselves (W x H x D, no padding).  *nlist must be zero before the launch.
 constexpr int COARSEN_THREADS = 256;
-__global__ void __launch_bounds__(COARSEN_THREADS) k_coarsen_cells(const uint8_t* __restrict__ lab, Dims g, MgLevel Cl,
-                                                                   int* __restrict__ list, int* __restrict__ nlist,
-                                                                   int cap) {
+template <bool RAW>
+__global__ void __launch_bounds__(COARSEN_THREADS) k_coarsen(const uint8_t* __restrict__ raw, MgLevel F, MgLevel Cl,
+                                                             MgLevel next, int4* __restrict__ list,
+                                                             int* __restrict__ nlist) {
+    const int nqr = (Cl.W + 3) >> 2;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = t < nqr * Cl.H * Cl.D;
     bool listed = false;
-    int cc = 0;
-    if (t < Cl.W * Cl.H * Cl.D) {
-        int I, J, K;
-        cc = lv_cell(Cl, t, I, J, K);
-        bool air = false, fluid = false;
+    int4 entry = make_int4(0, 0, 0, 0);
+    if (in) {
+        const int r = t / nqr, Q = t - r * nqr, K = r / Cl.H, J = r - K * Cl.H;
+        uint32_t air = 0, fluid = 0;  // a byte per coarse cell
+#pragma unroll
         for (int c3 = 0; c3 < 2; ++c3)
-            for (int b3 = 0; b3 < 2; ++b3)
-                for (int a3 = 0; a3 < 2; ++a3) {
-                    const int i = 2 * I + a3, j = 2 * J + b3, k = 2 * K + c3;
-                    if (i >= g.W || j >= g.H || k >= g.D) continue;
-                    const uint8_t l = lab[int64_t(i) + int64_t(j) * g.W + int64_t(k) * g.W * g.H];
-                    air |= l == AIR;
-                    fluid |= l == FLUID;
+#pragma unroll
+            for (int b3 = 0; b3 < 2; ++b3) {
+                const int j = 2 * J + b3, k = 2 * K + c3;
+                if (j >= F.H || k >= F.D) continue;
+                const uint8_t* row = RAW ? raw + int64_t(8 * Q) + int64_t(j) * F.W + int64_t(k) * F.W * F.H
+                                         : F.lab + lv_index(F, 8 * Q, j, k);
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    // (a padded row reads its zero gap, SOLID, beyond the last cell)
+                    if (8 * Q + m >= F.W) break;
+                    const uint8_t l = row[m];
+                    if (l == AIR) air |= 1u << (8 * (m >> 1));
+                    if (l == FLUID) fluid |= 1u << (8 * (m >> 1));
                 }
-        Cl.lab[cc] = air ? AIR : (fluid ? FLUID : SOLID);
-        listed = fluid && !air;
+            }
+        uint32_t lab = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t m = 1u << (8 * e);
+            const uint32_t v = (air & m) ? uint32_t(AIR) : (fluid & m) ? uint32_t(FLUID) : uint32_t(SOLID);
+            lab |= v << (8 * e);
+            listed |= v == uint32_t(FLUID);
+        }
+        const int cc = lv_index(Cl, 4 * Q, J, K);
+        *reinterpret_cast<uint32_t*>(Cl.lab + cc) = lab;
+        uint32_t par = ((J + K) & 1) ? QUAD_ODD : 0u;
+        if (((J >> 1) + (K >> 1)) & 1) par |= QUAD_PARENT_ODD;
+        if (2 * K + 1 < F.D) par |= QUAD_Z;
+        entry = make_int4(cc, int(par), next.W ? lv_index(next, 2 * Q, J >> 1, K >> 1) : 0,
+                          lv_index(F, 8 * Q, 2 * J, 2 * K));
     }
     if (!list) return;  // uniform across the block
     __shared__ int s_off[COARSEN_THREADS / 32];
@@ -1016,18 +1094,20 @@ __global__ void __launch_bounds__(COARSEN_THREADS) k_coarsen_cells(const uint8_t
         s_base = tot > 0 ? atomicAdd(nlist, tot) : 0;
     }
     __syncthreads();
-    const int slot = s_base + s_off[wid] + __popc(m & ((1u << lane) - 1u));
-    if (listed && slot < cap) list[slot] = cc;
+    if (listed) list[s_base + s_off[wid] + __popc(m & ((1u << lane) - 1u))] = entry;
 }
 
 }  // namespace
+
+int mg_npad(const MgLevel& L) { return (npad(L) + 15) & ~15; }
 
 int mg_levels_for(int W, int H, int D, MgLevel* lv) {
     int L = 0;
     int w = W, h = H, d = D;
     while (L < MG_MAX_LEVELS) {
         lv[L].W = w; lv[L].H = h; lv[L].D = d;
-        lv[L].sy = w + 2; lv[L].sz = (w + 2) * (h + 2);
+        lv[L].sy = ((w + 3) & ~3) + MG_OX;
+        lv[L].sz = lv[L].sy * (h + 2);
         ++L;
         if (w <= 2 && h <= 2 && d <= 2) break;
         w = (w + 1) / 2; h = (h + 1) / 2; d = (d + 1) / 2;
@@ -1038,57 +1118,53 @@ int mg_levels_for(int W, int H, int D, MgLevel* lv) {
 int mg_max_blocks() {
     static DeviceMemo memo;
     return memo.get([](int dev) {
-        int sms = 0, per = 0;
+        int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(k_pcg_mg, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM_BUDGET);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg_mg, MG_THREADS, MG_SMEM_BUDGET);
-        return sms * std::max(1, per);
+        return sms;
     });
 }
 
 int mg_split(const MgLevel* lv, int L, int* smem_bytes) {
     *smem_bytes = 0;
     if (L <= 1) return 0;
-    int G = 1;  // level 0 is always swept grid-wide on its FLUID list
+    int G = 1;  // level 0 is always swept grid-wide on its list
     for (int l = 0; l < L; ++l)
         if (int64_t(lv[l].W) * lv[l].H * lv[l].D > MG_BLOCK_CELLS) G = std::max(G, l + 1);
     for (G = std::min(G, L - 1); G < L; ++G) {
         const int b = mg_smem_bytes(lv, G, L);
         // the FLUID lists hold padded indices in 16 bits
-        if (b <= MG_SMEM_BUDGET && mg_npad(lv[G]) <= 65535) { *smem_bytes = b; return G; }
+        if (b <= MG_SMEM_BUDGET && npad(lv[G]) <= 65535) { *smem_bytes = b; return G; }
     }
     return L - 1;  // not even the coarsest level fits: the block levels stay in global memory
 }
 
-int launch_mg_setup(const uint8_t* labels, Dims g, MgLevel* lv, int L, int* l1list, int* l1n, cudaStream_t st) {
+int launch_mg_setup(const uint8_t* labels, const MgBufs& m, cudaStream_t st) {
     int smem = 0;
-    const int G = mg_split(lv, L, &smem);
-    const int last = smem ? G : L - 1;  // deeper shared-memory levels: coarsened by the solver kernel
+    const int G = mg_split(m.lv, m.L, &smem);
+    const int last = smem ? G : m.L - 1;  // deeper shared-memory levels: coarsened by the solver kernel
     for (int l = 1; l <= last; ++l) {
-        const int n = lv[l].W * lv[l].H * lv[l].D;
-        if (l == 1) {
-            if (l1list) cudaMemsetAsync(l1n, 0, sizeof(int), st);
-            k_coarsen_cells<<<(n + COARSEN_THREADS - 1) / COARSEN_THREADS, COARSEN_THREADS, 0, st>>>(labels, g, lv[1],
-                                                                                                   l1list, l1n, n);
-        }
-        else k_coarsen<<<(n + 255) / 256, 256, 0, st>>>(lv[l - 1], lv[l]);
+        const MgLevel& C = m.lv[l];
+        const int n = ((C.W + 3) >> 2) * C.H * C.D, nb = (n + COARSEN_THREADS - 1) / COARSEN_THREADS;
+        const MgLevel next = l + 1 < m.L ? m.lv[l + 1] : MgLevel{};
+        int4* list = l < G ? m.q[l] : nullptr;
+        if (l == 1) k_coarsen<true><<<nb, COARSEN_THREADS, 0, st>>>(labels, m.lv[0], C, next, list, m.nq + l);
+        else k_coarsen<false><<<nb, COARSEN_THREADS, 0, st>>>(nullptr, m.lv[l - 1], C, next, list, m.nq + l);
     }
     return last;
 }
 
-int launch_pcg_mg(Dims g, PressureBufs& pb, MgLevel* lv, int L, const int* l1list, const int* l1n, double* p,
-                  double* q, double* xs, double* r, const float* rhs, double tol, int maxit, cudaStream_t st,
-                  const float* x0, int nu0, const float* pprev, float* pout, unsigned wait_polls) {
-    // One block per 4096 cells (each thread's UNR cells per trip), at most one
-    // per SM: a small grid waits at cheaper barriers (one block: __syncthreads).
-    const int64_t want = (g.nc() + int64_t(MG_THREADS) * UNR - 1) / (int64_t(MG_THREADS) * UNR);
+int launch_pcg_mg(Dims g, PressureBufs& pb, const MgBufs& m, double tol, int maxit, const float* guess, int guess_dir,
+                  int nu0, float* pout, cudaStream_t st) {
+    // One block per 4096 cells, at most one per SM: a small grid waits at
+    // cheaper barriers (one block: __syncthreads).
+    const int64_t want = (g.nc() + 4095) / 4096;
     const int nb = int(std::max<int64_t>(1, std::min<int64_t>(mg_max_blocks(), want)));
-    int* status = &pb.out->status;
-    launch_reset_barrier(pb.bar, status, wait_polls, st);
-    MgArgs a;
-    a.L = L;
-    a.G = mg_split(lv, L, &a.smem);
-    for (int l = 0; l < L; ++l) a.lv[l] = lv[l];
+    MgArgs a{};
+    a.L = m.L;
+    a.G = mg_split(m.lv, m.L, &a.smem);
+    for (int l = 0; l < m.L; ++l) { a.lv[l] = m.lv[l]; a.q[l] = m.q[l]; }
+    a.nq = m.nq;
     a.rscale = g.D > 1 ? 0.25f : 0.5f;
     // The piecewise-constant prolongation underestimates the coarse correction;
     // scaling it by 1.7 roughly halves the PCG iterations (29 -> 15 at 128^3,
@@ -1104,13 +1180,14 @@ int launch_pcg_mg(Dims g, PressureBufs& pb, MgLevel* lv, int L, const int* l1lis
     a.nu0 = std::max(1, nu0);
     a.nu_grid = MG_NU_GRID;
     a.nu_block = MG_NU_BLOCK;
-    a.p = p; a.q = q; a.xs = xs; a.r = r; a.rhs = rhs; a.x0 = x0; a.pprev = x0 ? nullptr : pprev;
-    a.fidx = pb.fidx; a.diag = pb.diag; a.nf = pb.nf;
-    a.l1list = l1list; a.l1n = l1n;
-    a.X = static_cast<double*>(pb.X);
+    a.rhs = m.rhs;
+    a.p = m.p; a.s = m.s; a.xs = m.xs; a.r = m.r; a.w = m.w;
+    a.cap = m.cap;
+    a.xd = m.xd;
+    a.guess = guess; a.guess_dir = guess_dir;
     a.pout = pout;
     a.red = pb.red;
-    a.part = pb.part; a.bar = pb.bar; a.status = status; a.out = pb.out;
+    a.part = pb.part; a.bar = pb.bar; a.status = &pb.out->status; a.out = pb.out;
     a.tol = tol; a.maxit = maxit;
     void* args[] = {&a};
     cudaError_t e =

@@ -470,7 +470,7 @@ __global__ void k_reset_pcg(GridBar* bar, int* status, unsigned limit) {
 
 template <class K>
 int launch(K kern, int bytes_per_cell, Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout,
-           cudaStream_t st, unsigned wait_polls) {
+           cudaStream_t st) {
     // One CTA per 1024 cells of the grid, at most one per SM: with up to half
     // of the cells FLUID a small system has one cell per thread, and a
     // one-CTA grid's barrier is a block barrier.
@@ -488,7 +488,6 @@ int launch(K kern, int bytes_per_cell, Dims g, PressureBufs& pb, const float* x0
     const int64_t most = (nc + nb - 1) / nb;
     a.cap = most <= PCG_THREADS ? 0 : int(std::min<int64_t>(PCG_SMEM / bytes_per_cell, most + 15)) & ~15;
     void* args[] = {&a};
-    launch_reset_barrier(pb.bar, a.status, wait_polls, st);
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)kern, dim3(nb), dim3(PCG_THREADS), args,
                                                       size_t(a.cap) * bytes_per_cell, st);
     return e == cudaSuccess ? 0 : int(e);
@@ -511,13 +510,12 @@ void launch_reset_barrier(GridBar* bar, int* status, unsigned wait_polls, cudaSt
     k_reset_pcg<<<1, 1, 0, st>>>(bar, status, wait_polls);
 }
 
-int launch_pcg(Dims g, PressureBufs& pb, double tol, int maxit, float* pout, cudaStream_t st, unsigned wait_polls) {
-    return launch(k_pcg64, cell_bytes<double>(), g, pb, nullptr, tol, maxit, pout, st, wait_polls);
+int launch_pcg(Dims g, PressureBufs& pb, double tol, int maxit, float* pout, cudaStream_t st) {
+    return launch(k_pcg64, cell_bytes<double>(), g, pb, nullptr, tol, maxit, pout, st);
 }
 
-int launch_pcg_mixed(Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout, cudaStream_t st,
-                     unsigned wait_polls) {
-    return launch(k_pcg_mixed, cell_bytes<float>(), g, pb, x0, tol, maxit, pout, st, wait_polls);
+int launch_pcg_mixed(Dims g, PressureBufs& pb, const float* x0, double tol, int maxit, float* pout, cudaStream_t st) {
+    return launch(k_pcg_mixed, cell_bytes<float>(), g, pb, x0, tol, maxit, pout, st);
 }
 
 }  // namespace fp

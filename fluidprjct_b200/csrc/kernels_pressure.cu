@@ -28,75 +28,86 @@ namespace fp {
 namespace {
 
 constexpr int SCAN_BLOCK = 1024;
-constexpr int SCAN_ITEMS = 4;
-constexpr int SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
-
-__device__ __forceinline__ int64_t padded_index(int i, int j, int k, const Dims& g) {
-    return int64_t(i + 1) + int64_t(j + 1) * (g.W + 2) + int64_t(k + 1) * (g.W + 2) * (g.H + 2);
-}
 
 __device__ __forceinline__ bool solidish(uint8_t l) { return l == SOLID || l == BODY; }
 
-// Pass 1 of the fluid compaction: tile counts of FLUID cells; zero p off the
-// fluid (the solve writes every FLUID cell; until then they keep the previous
-// pressure, which a warm-started MG solve reads as its guess).
-__global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __restrict__ labels, int64_t nc,
-                                                            float* __restrict__ p, int* __restrict__ tile_sums) {
-    int64_t e0 = int64_t(blockIdx.x) * SCAN_TILE + int64_t(threadIdx.x) * SCAN_ITEMS;
+// The compaction works on quads, four aligned cells of a row (fewer at the end
+// of a row whose width is no multiple of four), one per thread, in row order:
+// the FLUID cells come out in i-fastest order, and so do the quads that hold
+// any.  A tile is one block's quads; its counts of both are packed in one int.
+__device__ __forceinline__ int quads_of_row(const Dims& g) { return (g.W + 3) >> 2; }
+
+// Pass 1: the tiles' counts; zero p off the fluid (the solve writes every FLUID
+// cell; until then they keep the previous pressure, which a warm-started MG
+// solve reads as its guess); ready the solvers' barrier, status and list
+// lengths.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __restrict__ labels, Dims g,
+                                                            float* __restrict__ p, int* __restrict__ tile_sums,
+                                                            int stride, GridBar* bar, int* status, unsigned limit,
+                                                            int* __restrict__ nq) {
+    const int nqr = quads_of_row(g), q = blockIdx.x * SCAN_BLOCK + threadIdx.x;
     int s = 0;
-#pragma unroll
-    for (int t = 0; t < SCAN_ITEMS; ++t) {
-        int64_t e = e0 + t;
-        if (e < nc) {
-            const bool f = labels[e] == FLUID;
+    if (q < nqr * g.H * g.D) {
+        const int row = q / nqr, Q = q - row * nqr;
+        const int64_t e0 = int64_t(row) * g.W + 4 * Q;
+        const int m = min(4, g.W - 4 * Q);
+        for (int t = 0; t < m; ++t) {
+            const bool f = labels[e0 + t] == FLUID;
             s += f;
-            if (!f) p[e] = 0.0f;
+            if (!f) p[e0 + t] = 0.0f;
         }
+        s |= int(s > 0) << 16;
     }
     int total;
     block_exclusive_scan<SCAN_BLOCK>(s, total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+    if (threadIdx.x == 0) {
+        tile_sums[blockIdx.x] = total & 0xFFFF;
+        tile_sums[stride + blockIdx.x] = total >> 16;
+        if (blockIdx.x == 0) {
+            bar->count = 0;
+            bar->limit = limit;
+            *status = DEV_OK;
+            if (nq)
+                for (int l = 0; l < MG_MAX_LEVELS; ++l) nq[l] = 0;
+        }
+    }
 }
 
-// RHSCalculator3D::operator() (FluidSolver3D.cu:1371-1456) at FLUID cell (i,j,k).
-__device__ __forceinline__ float rhs_at(const uint8_t* __restrict__ lab, const float* __restrict__ u,
-                                        const float* __restrict__ v, const float* __restrict__ w, const Dims& g,
-                                        int i, int j, int k, float scale, const BodyKin& body) {
-    const int W = g.W, H = g.H;
-    const float dx = g.dx;
-    const int64_t ui = int64_t(i) + int64_t(j) * (W + 1) + int64_t(k) * (W + 1) * H;
-    const int64_t vi = int64_t(i) + int64_t(j) * W + int64_t(k) * W * (H + 1);
-    const int64_t wi = int64_t(i) + int64_t(j) * W + int64_t(k) * W * H;
-    const float u0 = u[ui], u1 = u[ui + 1], v0 = v[vi], v1 = v[vi + W], w0 = w[wi], w1 = w[wi + int64_t(W) * H];
+// RHSCalculator3D::operator() (FluidSolver3D.cu:1371-1456) at FLUID cell
+// (i,j,k) from its faces' velocities and its neighbours' labels (-x, +x, -y,
+// +y, -z, +z).
+__device__ __forceinline__ float rhs_at(float u0, float u1, float v0, float v1, float w0, float w1,
+                                        const uint8_t (&nl)[6], float dx, int i, int j, int k, float scale,
+                                        const BodyKin& body) {
     float div = u1 - u0 + v1 - v0 + w1 - w0;
     float rhs = -scale * div;
     uint8_t l;
-    l = label_at(lab, g, i - 1, j, k);
+    l = nl[0];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3(float(i) * dx, (float(j) + 0.5f) * dx, (float(k) + 0.5f) * dx)).x : 0.0f;
         rhs -= scale * (u0 - s);
     }
-    l = label_at(lab, g, i + 1, j, k);
+    l = nl[1];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3(float(i + 1) * dx, (float(j) + 0.5f) * dx, (float(k) + 0.5f) * dx)).x : 0.0f;
         rhs += scale * (u1 - s);
     }
-    l = label_at(lab, g, i, j - 1, k);
+    l = nl[2];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3((float(i) + 0.5f) * dx, float(j) * dx, (float(k) + 0.5f) * dx)).y : 0.0f;
         rhs -= scale * (v0 - s);
     }
-    l = label_at(lab, g, i, j + 1, k);
+    l = nl[3];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3((float(i) + 0.5f) * dx, float(j + 1) * dx, (float(k) + 0.5f) * dx)).y : 0.0f;
         rhs += scale * (v1 - s);
     }
-    l = label_at(lab, g, i, j, k - 1);
+    l = nl[4];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3((float(i) + 0.5f) * dx, (float(j) + 0.5f) * dx, float(k) * dx)).z : 0.0f;
         rhs -= scale * (w0 - s);
     }
-    l = label_at(lab, g, i, j, k + 1);
+    l = nl[5];
     if (solidish(l)) {
         float s = l == BODY ? body_vel_at(body, make_float3((float(i) + 0.5f) * dx, (float(j) + 0.5f) * dx, float(k + 1) * dx)).z : 0.0f;
         rhs += scale * (w1 - s);
@@ -104,45 +115,95 @@ __device__ __forceinline__ float rhs_at(const uint8_t* __restrict__ lab, const f
     return rhs;
 }
 
-// Pass 3: write the compact system (fidx, diag, b) of every FLUID cell.
+// Level 0's quad list for the multigrid solver (null pointers: not wanted).
+struct QuadOut {
+    int4* q;
+    float4* rhs;
+    int sy0, sz0, sy1, sz1;  // padded strides of levels 0 and 1 (sy1 = 0: there is no level 1)
+};
+
+// Pass 3: the compact system (fidx, diag, b) of every FLUID cell, and the quad
+// list.  A thread loads all labels and velocities of its quad before it uses
+// any: cell by cell, each cell's loads waited for the one before (27 us at
+// 128^3, 34 at 160^3, against 18 and 30; 256 x 128 x 256, where the writes bound
+// it, 51 either way).
 __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_build(const uint8_t* __restrict__ labels,
                                                             const float* __restrict__ u, const float* __restrict__ v,
                                                             const float* __restrict__ w, Dims g, float scale,
                                                             BodyKin body, const float* __restrict__ rhs_dense,
-                                                            const int* __restrict__ tile_off, int* __restrict__ fidx,
-                                                            uint8_t* __restrict__ diag, float* __restrict__ b) {
-    const int64_t nc = g.nc();
-    int64_t e0 = int64_t(blockIdx.x) * SCAN_TILE + int64_t(threadIdx.x) * SCAN_ITEMS;
-    uint8_t lab[SCAN_ITEMS];
+                                                            const int* __restrict__ tile_off, int stride,
+                                                            int* __restrict__ fidx, uint8_t* __restrict__ diag,
+                                                            float* __restrict__ b, QuadOut qo) {
+    const int W = g.W, H = g.H, D = g.D;
+    const int nqr = quads_of_row(g), q = blockIdx.x * SCAN_BLOCK + threadIdx.x;
+    const int row = q / nqr, Q = q - row * nqr, k = row / H, j = row - k * H, i0 = 4 * Q;
+    const bool in = q < nqr * H * D;
+    const int64_t e0 = int64_t(row) * W + i0, wh = int64_t(W) * H;
+    // labels i0 - 1 .. i0 + 4 of the row; cells beyond the grid are SOLID
+    uint8_t lx[6];
     int s = 0;
 #pragma unroll
-    for (int t = 0; t < SCAN_ITEMS; ++t) {
-        int64_t e = e0 + t;
-        lab[t] = e < nc ? labels[e] : SOLID;
-        s += lab[t] == FLUID;
-    }
+    for (int t = 0; t < 6; ++t) lx[t] = in && i0 + t >= 1 && i0 + t <= W ? labels[e0 + t - 1] : SOLID;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) s += lx[t + 1] == FLUID;
+    s |= int(s > 0) << 16;
     int total;
-    int n = block_exclusive_scan<SCAN_BLOCK>(s, total) + tile_off[blockIdx.x];
+    const int pre = block_exclusive_scan<SCAN_BLOCK>(s, total);
+    if ((s & 0xFFFF) == 0) return;
+    int n = (pre & 0xFFFF) + tile_off[blockIdx.x];
+    const int nq = (pre >> 16) + tile_off[stride + blockIdx.x];
+
+    uint8_t ly[2][4], lz[2][4];
+    float uf[5], vf[2][4], wf[2][4], rd[4];
+    const int64_t ui = int64_t(i0) + int64_t(row) * (W + 1);
+    const int64_t vi = int64_t(i0) + int64_t(j) * W + int64_t(k) * W * (H + 1);
 #pragma unroll
-    for (int t = 0; t < SCAN_ITEMS; ++t) {
-        if (lab[t] != FLUID) continue;
-        int64_t e = e0 + t;
-        // 32-bit decode: cell indices fit in an int (the padded index does too)
-        const uint32_t eu = uint32_t(e), W = uint32_t(g.W), H = uint32_t(g.H);
-        const uint32_t ej = eu / W;
-        const int i = int(eu - ej * W), j = int(ej % H), k = int(ej / H);
-        fidx[n] = int(padded_index(i, j, k, g));
-        int d = 0;
-        const int off[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-#pragma unroll
-        for (int o = 0; o < 6; ++o) {
-            uint8_t l = label_at(labels, g, i + off[o][0], j + off[o][1], k + off[o][2]);
-            d += (l == FLUID || l == AIR);
+    for (int t = 0; t < 4; ++t) {
+        const bool c = i0 + t < W;
+        ly[0][t] = c && j > 0 ? labels[e0 + t - W] : SOLID;
+        ly[1][t] = c && j + 1 < H ? labels[e0 + t + W] : SOLID;
+        lz[0][t] = c && k > 0 ? labels[e0 + t - wh] : SOLID;
+        lz[1][t] = c && k + 1 < D ? labels[e0 + t + wh] : SOLID;
+        if (rhs_dense) {
+            rd[t] = c ? rhs_dense[e0 + t] : 0.0f;
+        } else {
+            vf[0][t] = c ? v[vi + t] : 0.0f;
+            vf[1][t] = c ? v[vi + t + W] : 0.0f;
+            wf[0][t] = c ? w[e0 + t] : 0.0f;
+            wf[1][t] = c ? w[e0 + t + wh] : 0.0f;
         }
-        diag[n] = uint8_t(d | (((i + j + k) & 1) << 7));  // bit 7: red/black colour
-        b[n] = rhs_dense ? rhs_dense[e] : rhs_at(labels, u, v, w, g, i, j, k, scale, body);
+    }
+    if (!rhs_dense)
+#pragma unroll
+        for (int t = 0; t < 5; ++t) uf[t] = i0 + t <= W ? u[ui + t] : 0.0f;
+
+    const int pidx = (i0 + 1) + (j + 1) * (W + 2) + (k + 1) * (W + 2) * (H + 2);
+    uint32_t codes = 0;
+    float rq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (lx[t + 1] != FLUID) continue;
+        const uint8_t nl[6] = {lx[t], lx[t + 2], ly[0][t], ly[1][t], lz[0][t], lz[1][t]};
+        int d = 0;
+#pragma unroll
+        for (int o = 0; o < 6; ++o) d += (nl[o] == FLUID || nl[o] == AIR);
+        const float r = rhs_dense ? rd[t]
+                                  : rhs_at(uf[t], uf[t + 1], vf[0][t], vf[1][t], wf[0][t], wf[1][t], nl, g.dx, i0 + t,
+                                           j, k, scale, body);
+        fidx[n] = pidx + t;
+        diag[n] = uint8_t(d);
+        b[n] = r;
+        rq[t] = r;
+        codes |= uint32_t(1 + d) << (8 * t);
         ++n;
     }
+    if (!qo.q) return;
+    if ((j + k) & 1) codes |= QUAD_ODD;
+    if (((j >> 1) + (k >> 1)) & 1) codes |= QUAD_PARENT_ODD;
+    const int c = (i0 + MG_OX) + (j + 1) * qo.sy0 + (k + 1) * qo.sz0;
+    const int pc = qo.sy1 ? (2 * Q + MG_OX) + ((j >> 1) + 1) * qo.sy1 + ((k >> 1) + 1) * qo.sz1 : 0;
+    qo.q[nq] = make_int4(c, int(codes), pc, int(e0));
+    qo.rhs[nq] = make_float4(rq[0], rq[1], rq[2], rq[3]);
 }
 
 // ---------------------------------------------------------------- projection
@@ -376,15 +437,31 @@ __global__ void k_csr_reset(CsrCtl* ctl, unsigned limit) {
 
 // ---------------------------------------------------------------- launchers
 
+static int quad_tiles(Dims g) {
+    const int64_t nq = int64_t((g.W + 3) / 4) * g.H * g.D;
+    return int((nq + SCAN_BLOCK - 1) / SCAN_BLOCK);
+}
+// Two rows of tile counts, each from a multiple of four (k_scan_rows reads vectors).
+int pressure_tiles(Dims g) { return 2 * ((quad_tiles(g) + 3) & ~3); }
+
 void launch_pressure_setup(const uint8_t* labels, const float* u, const float* v, const float* w, Dims g, float dt,
-                           BodyKin body, const float* rhs_dense, float* p, PressureBufs& pb, cudaStream_t st) {
-    const int64_t nc = g.nc();
-    const int ntiles = int((nc + SCAN_TILE - 1) / SCAN_TILE);
+                           BodyKin body, const float* rhs_dense, float* p, PressureBufs& pb, const MgBufs* mg,
+                           unsigned wait_polls, cudaStream_t st) {
+    const int ntiles = quad_tiles(g), stride = pressure_tiles(g) / 2;
     const float scale = (1000.0f * g.dx) / dt;  // rho*dx/dt, FluidSolver3D.cu:1520
-    k_fluid_tiles<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, nc, p, pb.tile_sums);
-    k_scan_single_block<<<1, 1024, 0, st>>>(pb.tile_sums, ntiles, pb.nf);
-    k_fluid_build<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, u, v, w, g, scale, body, rhs_dense, pb.tile_sums, pb.fidx,
-                                                 pb.diag, pb.b);
+    QuadOut qo{};
+    if (mg && mg->L > 0) {
+        qo.q = mg->q[0];
+        qo.rhs = mg->rhs;
+        qo.sy0 = mg->lv[0].sy; qo.sz0 = mg->lv[0].sz;
+        if (mg->L > 1) { qo.sy1 = mg->lv[1].sy; qo.sz1 = mg->lv[1].sz; }
+    }
+    int* nq = qo.q ? mg->nq : nullptr;
+    k_fluid_tiles<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, g, p, pb.tile_sums, stride, pb.bar, &pb.out->status,
+                                                 wait_polls, nq);
+    k_scan_rows<<<2, 1024, 0, st>>>(pb.tile_sums, ntiles, stride, pb.nf, nq);
+    k_fluid_build<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, u, v, w, g, scale, body, rhs_dense, pb.tile_sums, stride,
+                                                 pb.fidx, pb.diag, pb.b, qo);
 }
 
 void launch_project(float* u, float* v, float* w, const float* p, const uint8_t* labels, Dims g, float dt, BodyKin b,

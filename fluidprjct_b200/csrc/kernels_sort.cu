@@ -105,11 +105,10 @@ __global__ void k_scatter(const float4* __restrict__ pos, const float4* __restri
     pos2[slot] = pos[q];
     vel2[slot] = vel[q];
 }
-}  // namespace
 
 // 16 consecutive ints per thread and pass, as four vectors (data is 16-byte
 // aligned): one pass of a block covers 16,384.
-__global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, int* total) {
+__device__ __forceinline__ void scan_block(int* data, int n, int* total) {
     constexpr int ITEMS = 16;
     int carry = 0;
     for (int base = 0; base < n; base += 1024 * ITEMS) {
@@ -145,6 +144,12 @@ __global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, in
         carry += tot;
     }
     if (threadIdx.x == 0 && total) *total = carry;
+}
+}  // namespace
+
+__global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, int* total) { scan_block(data, n, total); }
+__global__ void __launch_bounds__(1024) k_scan_rows(int* data, int n, int stride, int* total0, int* total1) {
+    scan_block(data + blockIdx.x * stride, n, blockIdx.x ? total1 : total0);
 }
 
 // The tile sums of data, and the scan of each tile from its offset.

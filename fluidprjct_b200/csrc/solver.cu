@@ -157,16 +157,12 @@ struct fp_solver {
     // pressure
     PressureBufs pb{};
     int64_t padded = 0;
-    // multigrid hierarchy (level 0 shares the padded layout of pb)
-    MgLevel mg[MG_MAX_LEVELS]{};
-    int mgL = 0;
-    double *d_mgp = nullptr, *d_mgq = nullptr, *d_mgx = nullptr, *d_mgr = nullptr;
-    int *d_l1list = nullptr, *d_l1n = nullptr;  // level 1's FLUID cells (multigrid)
+    MgBufs mg{};  // multigrid hierarchy
     // learned initial guess
     fp_unet* net = nullptr;
     std::string learned_path;
     float* d_rhs_dense = nullptr;  // dense right-hand side (network input, FP_GRID_RHS)
-    float* d_x0c = nullptr;        // compact initial guess
+    float* d_x0c = nullptr;        // initial guess: compact (mixed) or dense (multigrid)
     cudaEvent_t ev_net = nullptr;
     // a PCG / MG solve whose read-back one_step has deferred (ev[9] marks it)
     bool solve_pending = false;
@@ -222,12 +218,12 @@ void free_grid(fp_solver* s) {
     for (int i = 0; i < 2; ++i) { dfree(pb.R[i]); dfree(pb.Wv[i]); dfree(pb.S[i]); }
     dfree(pb.invd); dfree(pb.P); dfree(pb.X);
     dfree(pb.x64); dfree(pb.xd); dfree(pb.part); dfree(pb.bar); dfree(pb.out);
-    for (int l = 0; l < s->mgL; ++l) {
-        dfree(s->mg[l].lab); dfree(s->mg[l].x); dfree(s->mg[l].b); dfree(s->mg[l].code);
+    MgBufs& m = s->mg;
+    for (int l = 0; l < m.L; ++l) {
+        dfree(m.lv[l].lab); dfree(m.lv[l].x); dfree(m.lv[l].b); dfree(m.lv[l].code); dfree(m.q[l]);
     }
-    s->mgL = 0;
-    dfree(s->d_mgp); dfree(s->d_mgq); dfree(s->d_mgx); dfree(s->d_mgr);
-    dfree(s->d_l1list); dfree(s->d_l1n);
+    dfree(m.nq); dfree(m.rhs); dfree(m.p); dfree(m.s); dfree(m.xs); dfree(m.r); dfree(m.w); dfree(m.xd);
+    m = MgBufs{};
     dfree(s->d_rhs_dense); dfree(s->d_x0c);
     if (s->net) { fp_unet_destroy(s->net); s->net = nullptr; }
     free_r2(s);
@@ -265,6 +261,20 @@ int load_net(fp_solver* s) {
     return FP_OK;
 }
 
+// The zero state of the multigrid work grids between solves.
+cudaError_t mg_zero(const MgBufs& m, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    auto ck = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    for (int l = 0; l < m.L; ++l) {
+        const size_t n = size_t(mg_npad(m.lv[l]));
+        ck(cudaMemsetAsync(m.lv[l].x, 0, n * sizeof(float), st));
+        ck(cudaMemsetAsync(m.lv[l].b, 0, n * sizeof(float), st));
+        ck(cudaMemsetAsync(m.lv[l].code, 0, n, st));
+    }
+    if (m.L > 0) ck(cudaMemsetAsync(m.xd, 0, sizeof(double) * size_t(mg_npad(m.lv[0])), st));
+    return e;
+}
+
 int alloc_grid(fp_solver* s, int W, int H, int D) {
     free_grid(s);
     s->W = W; s->H = H; s->D = D;
@@ -276,7 +286,7 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
     }
     const int64_t nc = s->g.nc();
     s->padded = int64_t(W + 2) * (H + 2) * (D + 2);
-    const int ntiles = int((nc + 4095) / 4096) + 1;
+    const int ntiles = std::max(int((nc + 4095) / 4096) + 1, pressure_tiles(s->g));
     const int maxb = pcg_max_blocks();
     cudaError_t e = cudaSuccess;
     auto ck = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
@@ -308,26 +318,23 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
     if (s->cfg.solver == FP_SOLVER_PCG_LEARNED || s->cfg.solver == FP_SOLVER_PCG_LEARNED_MIXED)
         ck(dalloc(&s->d_x0c, nc));
     if (s->cfg.solver == FP_SOLVER_PCG_MG || s->cfg.solver == FP_SOLVER_PCG_LEARNED) {
-        s->mgL = mg_levels_for(W, H, D, s->mg);
-        for (int l = 0; l < s->mgL && e == cudaSuccess; ++l) {
-            MgLevel& L = s->mg[l];
-            const size_t np_ = size_t(L.W + 2) * (L.H + 2) * (L.D + 2);
+        MgBufs& m = s->mg;
+        m.L = mg_levels_for(W, H, D, m.lv);
+        int smem = 0;
+        const int G = mg_split(m.lv, m.L, &smem);
+        auto quads = [](const MgLevel& L) { return size_t((L.W + 3) / 4) * L.H * L.D; };
+        for (int l = 0; l < m.L && e == cudaSuccess; ++l) {
+            MgLevel& L = m.lv[l];
+            const size_t np_ = size_t(mg_npad(L));
             ck(dalloc(&L.lab, np_)); ck(dalloc(&L.x, np_)); ck(dalloc(&L.b, np_)); ck(dalloc(&L.code, np_));
-            if (e == cudaSuccess) {
-                ck(cudaMemsetAsync(L.lab, 0, np_, s->st));  // SOLID halo
-                ck(cudaMemsetAsync(L.code, 0, np_, s->st));
-                ck(cudaMemsetAsync(L.x, 0, np_ * sizeof(float), s->st));
-                ck(cudaMemsetAsync(L.b, 0, np_ * sizeof(float), s->st));
-            }
+            if (l < std::max(G, 1)) ck(dalloc(&m.q[l], quads(L)));
+            if (e == cudaSuccess) ck(cudaMemsetAsync(L.lab, 0, np_, s->st));  // SOLID halo
         }
-        if (s->mgL > 1) {
-            ck(dalloc(&s->d_l1list, size_t(s->mg[1].W) * s->mg[1].H * s->mg[1].D));
-            ck(dalloc(&s->d_l1n, 1));
-        }
-        ck(dalloc(&s->d_mgp, size_t(s->padded))); ck(dalloc(&s->d_mgq, size_t(s->padded)));
-        ck(dalloc(&s->d_mgx, size_t(s->padded))); ck(dalloc(&s->d_mgr, size_t(s->padded)));
-        for (double* a : {s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr})
-            if (e == cudaSuccess) ck(cudaMemsetAsync(a, 0, sizeof(double) * size_t(s->padded), s->st));
+        m.cap = int(quads(m.lv[0]));
+        ck(dalloc(&m.nq, size_t(MG_MAX_LEVELS))); ck(dalloc(&m.rhs, size_t(m.cap)));
+        for (double2** a : {&m.p, &m.s, &m.xs, &m.r, &m.w}) ck(dalloc(a, size_t(2) * m.cap));
+        ck(dalloc(&m.xd, size_t(mg_npad(m.lv[0]))));
+        if (e == cudaSuccess) ck(mg_zero(m, s->st));
     }
     if (e != cudaSuccess) { free_grid(s); return s->cuda_fail(e, "device allocation of the grid"); }
     for (float* a : {s->d_u, s->d_us}) ck(cudaMemsetAsync(a, 0, sizeof(float) * s->g.nu(), s->st));
@@ -472,7 +479,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     const bool learned = learned_solver(s), mg = mg_solver(s), mixed = mixed_solver(s);
     const bool warm = s->cfg.solver == FP_SOLVER_PCG_MG && s->cfg.warm_start && p_out == s->d_p;
     if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
-    if (mg) s->launches += launch_mg_setup(s->d_labels, s->g, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->st);
+    if (mg) s->launches += launch_mg_setup(s->d_labels, s->mg, s->st);
     cudaEventRecord(s->ev_pcg[0], s->st);
     const float* x0 = nullptr;
     if (learned) {
@@ -480,8 +487,12 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
         unet::launch_rhs_dense(pb.nf, pb.fidx, real, pb.b, s->d_rhs_dense, s->st);
         if (unet::forward_on(s->net, s->d_labels, s->d_rhs_dense, s->st))
             return s->cuda_fail(cudaGetLastError(), "U-Net forward");
-        unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
-                                    unet::net_scal(s->net), s->d_x0c, s->st);
+        if (mg)
+            unet::launch_output_dense(s->d_labels, real, unet::net_level0(s->net), unet::net_out(s->net),
+                                      unet::net_scal(s->net), s->d_x0c, s->st);
+        else
+            unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
+                                        unet::net_scal(s->net), s->d_x0c, s->st);
         s->launches += 1 + 16 + 1;  // rhs scatter, network (2 scale/input, 10 conv, 2 pool, 2 concat), guess
         cudaEventRecord(s->ev_net, s->st);
         x0 = s->d_x0c;
@@ -491,15 +502,14 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     constexpr int kLearnedMaxit = 300;
     int e = 0;
     if (mg)
-        e = launch_pcg_mg(s->g, pb, s->mg, s->mgL, s->d_l1list, s->d_l1n, s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr, pb.b,
-                          tol, learned ? std::min(maxit, kLearnedMaxit) : maxit, s->st, x0,
-                          s->cfg.mg_sweeps > 0 ? s->cfg.mg_sweeps : 2,
-                          s->cfg.warm_start && p_out == s->d_p ? p_out : nullptr, p_out, s->wait_polls);
+        e = launch_pcg_mg(s->g, pb, s->mg, tol, learned ? std::min(maxit, kLearnedMaxit) : maxit,
+                          learned ? x0 : (warm ? p_out : nullptr), learned, s->cfg.mg_sweeps > 0 ? s->cfg.mg_sweeps : 2,
+                          p_out, s->st);
     else if (mixed)
-        e = launch_pcg_mixed(s->g, pb, x0, tol, maxit, p_out, s->st, s->wait_polls);
+        e = launch_pcg_mixed(s->g, pb, x0, tol, maxit, p_out, s->st);
     else
-        e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st, s->wait_polls);
-    s->launches += 2;  // barrier reset, solver
+        e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
+    s->launches += 1;
     cudaEventRecord(s->ev_pcg[1], s->st);
     if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
     cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);  // out, red and nf
@@ -524,7 +534,8 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             // fallback: the plain FP64 PCG from x = 0
             fallback = 1;
             cudaEventRecord(s->ev_pcg[0], s->st);
-            e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st, s->wait_polls);
+            launch_reset_barrier(pb.bar, &pb.out->status, s->wait_polls, s->st);
+            e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
             cudaEventRecord(s->ev_pcg[1], s->st);
             if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
             s->launches += 2;
@@ -578,14 +589,7 @@ int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float p
         for (void* a : {s->pb.R[0], s->pb.R[1], s->pb.Wv[0], s->pb.Wv[1], s->pb.S[0], s->pb.S[1], s->pb.invd,
                         static_cast<void*>(s->pb.xd)})
             cudaMemsetAsync(a, 0, pbytes, s->st);
-        for (int l = 0; l < s->mgL; ++l) {
-            const size_t np_ = size_t(s->mg[l].W + 2) * (s->mg[l].H + 2) * (s->mg[l].D + 2);
-            cudaMemsetAsync(s->mg[l].x, 0, np_ * sizeof(float), s->st);
-            cudaMemsetAsync(s->mg[l].b, 0, np_ * sizeof(float), s->st);
-            cudaMemsetAsync(s->mg[l].code, 0, np_, s->st);
-        }
-        if (s->mgL > 0)
-            for (double* a : {s->d_mgp, s->d_mgq, s->d_mgx, s->d_mgr}) cudaMemsetAsync(a, 0, pbytes, s->st);
+        mg_zero(s->mg, s->st);
     }
     if (status == FP_ERR_TIMEOUT) return s->fail(status, "PCG grid barrier timed out");
     if (dev_status == DEV_NAN) return s->fail(status, "PCG produced NaN");
@@ -595,7 +599,8 @@ int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float p
 int phase_pressure(fp_solver* s, bool defer = false) {
     s->launches += 3;  // fluid tiles, tile scan, fluid build
     BodyKin b = body_kin(s);
-    launch_pressure_setup(s->d_labels, s->d_u, s->d_v, s->d_w, s->g, s->cfg.dt, b, nullptr, s->d_p, s->pb, s->st);
+    launch_pressure_setup(s->d_labels, s->d_u, s->d_v, s->d_w, s->g, s->cfg.dt, b, nullptr, s->d_p, s->pb, &s->mg,
+                          s->wait_polls, s->st);
     return solve_system(s, s->d_p, defer);
 }
 
@@ -1881,7 +1886,8 @@ int fp_pressure_solve(fp_solver* s, const float* rhs, float* x, int64_t n, int* 
     // rhs in d_scratch; the dense solution goes to d_scratch2 (zeroed by the
     // setup), leaving the solver's own pressure grid untouched.
     float* xdense = s->d_scratch2;
-    launch_pressure_setup(s->d_labels, s->d_u, s->d_v, s->d_w, s->g, s->cfg.dt, b, s->d_scratch, xdense, s->pb, s->st);
+    launch_pressure_setup(s->d_labels, s->d_u, s->d_v, s->d_w, s->g, s->cfg.dt, b, s->d_scratch, xdense, s->pb,
+                          &s->mg, s->wait_polls, s->st);
     int rc = solve_system(s, xdense);
     if (rc) return rc;
     if (e == cudaSuccess) e = cudaMemcpyAsync(x, xdense, sizeof(float) * n, cudaMemcpyDeviceToHost, s->st);

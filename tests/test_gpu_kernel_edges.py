@@ -134,6 +134,48 @@ def test_pcg_sizes(solver, shape):
     s.close()
 
 
+def _ragged(shape, seed):
+    """Labels: water with 3 % AIR and 8 % SOLID cells strewn in, SOLID where a piece of water touches no AIR."""
+    from scipy.ndimage import binary_dilation, label
+    rng = np.random.default_rng(seed)
+    lab = rng.choice([0, 1, 2], size=shape, p=[0.08, 0.89, 0.03]).astype(np.uint8)
+    part, n = label(lab == 1)
+    open_ = np.unique(part[binary_dilation(lab == 2) & (lab == 1)])
+    lab[(lab == 1) & ~np.isin(part, open_)] = 0
+    if not (lab == 1).any():
+        lab.flat[:2] = 1, 2
+    return lab
+
+
+# rows of one cell, of a quad with 1, 2 and 3 cells over, and of whole quads; one level only; the last grid-wide and the
+# first block level; 2D; lists of up to one, two and more quads a thread
+@pytest.mark.parametrize("shape", [(1, 5, 4), (4, 3, 2), (5, 5, 5), (6, 70, 1), (7, 33, 18), (31, 30, 29), (64, 64, 1),
+                                   (129, 131, 1), (34, 61, 47), (66, 64, 70), (128, 128, 40), (157, 96, 83)])
+def test_mg_quad_rows(shape):
+    """The solve ends with ||b - A x|| <= 1e-9 ||b|| in FP64; rounding x to FP32 adds at most ||A|| 2^-24 ||x||, and
+    ||A|| <= 12.  Twice the first term leaves room for the recurrence's drift."""
+    import torch
+    from fluidprjct_b200 import capi
+    W, H, D = shape
+    lab = _ragged((D, H, W), W * H + D)
+    rng = np.random.default_rng(7)
+    t = torch.nn.functional.pad(torch.from_numpy(lab).cuda().int(), (1, 1, 1, 1, 1, 1))
+    fl = (t == 1).double()
+    wet = ((t == 1) | (t == 2)).double()
+    diag = sum(torch.roll(wet, o, d) for d in range(3) for o in (1, -1)) * fl
+    s = capi.Solver(dim=3 if D > 1 else 2, dx=1.0 / 64, dt=0.01, solver="pcg_mg", tol=1e-9, output_format=capi.OUT_NONE)
+    s.set_labels(lab if D > 1 else lab[0])
+    for _ in range(2):  # the second solve finds the work grids as the first left them
+        rhs = (rng.standard_normal(lab.shape) * (lab == 1)).astype(np.float32)
+        x, it, rr, rc = s.pressure_solve(rhs)
+        b = torch.nn.functional.pad(torch.from_numpy(rhs).cuda().double(), (1, 1, 1, 1, 1, 1))
+        y = torch.nn.functional.pad(torch.from_numpy(x).cuda().double(), (1, 1, 1, 1, 1, 1))
+        res = b - (diag * y - sum(torch.roll(y, o, d) for d in range(3) for o in (1, -1)) * fl)
+        assert rc == 0 and not x[lab != 1].any()
+        assert float(res.norm()) <= 2e-9 * float(b.norm()) + 12 * 2.0 ** -24 * float(y.norm())
+    s.close()
+
+
 def _faces_force(lab, p, dx, phi, com):
     """The face-fraction force and torque over every face of the grid, in FP64 (phi: SDF at given points)."""
     D, H, W = lab.shape
