@@ -24,8 +24,8 @@
 //
 // Bound by the latency of the walk's particle loads, so by occupancy.  The
 // accumulate kernel takes 136 us for the 128^3 dam break (3.8 M particles),
-// 412 for the 160^3 pool (11 M, dx not a power of two), 508 for the
-// 256 x 128 x 256 tank (17.5 M) and 19 for a 50^3 box; one thread per cell for
+// 412 for the 160^3 pool (11 M, dx not a power of two and divided by; 325
+// since), 508 for the 256 x 128 x 256 tank (17.5 M) and 19 for a 50^3 box; one thread per cell for
 // all three components in turn, with shared-memory atomics, took 138, 420, 567
 // and 33 (a small grid's bricks then leave most of the chip idle).  8 x 8 x 4
 // bricks: 141, 430, 561 and 23 at five CTAs of 192 per SM, 165, 504 and 650 at

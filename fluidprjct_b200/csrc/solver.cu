@@ -282,7 +282,10 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
     {
         // dx a power of two: its reciprocal is exact, and x * (1/dx) == x / dx
         int ex = 0;
-        if (std::frexp(double(s->cfg.dx), &ex) == 0.5) s->g.idx = float(1.0 / double(s->cfg.dx));
+        const double r = 1.0 / double(s->cfg.dx);
+        if (std::frexp(double(s->cfg.dx), &ex) == 0.5) s->g.idx = float(r);
+        s->g.rhi = float(r);
+        s->g.rlo = float(r - double(s->g.rhi));
     }
     const int64_t nc = s->g.nc();
     s->padded = int64_t(W + 2) * (H + 2) * (D + 2);

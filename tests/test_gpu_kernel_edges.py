@@ -350,3 +350,25 @@ def test_p2g_brick_edges(shape):
         assert np.abs(got[far] - num[far] / den[far]).max() <= 1e-4
         assert not got[den == 0].any()
     s.close()
+
+
+@pytest.mark.parametrize("dx", [1 / 160, 0.1, 0.02, 1 / 3, 0.0123, 1.9999999, 1.0000001, 0.99999994, 7.7, 0.25])
+def test_cell_of_a_boundary_particle(dx):
+    """Cells are floor(p / dx) of the FP32 quotient, exactly: one particle per row of cells, on a cell boundary or within
+    three ulps of it, marks its cell FLUID and no other."""
+    from fluidprjct_b200 import capi
+    W, H, D = 64, 30, 30
+    d = np.float32(dx)
+    s = capi.Solver(dim=3, dx=float(d), dt=0.01, output_format=capi.OUT_NONE)
+    s.set_labels(np.full((D, H, W), 2, np.uint8))
+    rng = np.random.default_rng(3)
+    j, k = np.meshgrid(np.arange(H), np.arange(D), indexing="ij")
+    j, k = j.ravel(), k.ravel()
+    x = (rng.integers(1, W, j.size).astype(np.float32) * d).view(np.int32) + rng.integers(-3, 4, j.size, dtype=np.int32)
+    pos = np.stack([x.view(np.float32), (j + np.float32(0.5)) * d, (k + np.float32(0.5)) * d], 1).astype(np.float32)
+    s.set_particles(pos)
+    s.phase(capi.PHASE_LABEL)
+    want = np.full((D, H, W), 2, np.uint8)
+    want[k, j, np.floor(pos[:, 0] / d).astype(int)] = 1
+    assert np.array_equal(s.labels(), want)
+    s.close()
