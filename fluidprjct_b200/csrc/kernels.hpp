@@ -135,7 +135,7 @@ int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st);
 int scan_tiles(int64_t n);
 
 // -------- P2G with the fused normalise / save / gravity epilogue (kernels_p2g.cu) --------
-// acc: [nu + nv + nw] (num, den) pairs, zero on entry and left zero (four launches).
+// acc: [nu + nv + nw] (num, den) pairs, zero on entry and left zero (two launches).
 void launch_p2g(const float4* pos, const float4* vel, const int* start, Dims g, float dt, float3 gravity,
                 float2* acc, float* u, float* v, float* w, float* us, float* vs, float* ws, int fused_forces,
                 cudaStream_t st);

@@ -22,7 +22,10 @@
 // return at once.  A second, elementwise kernel divides, saves and adds
 // gravity, and zeroes the pair array for the next step.
 //
-// Bound by the latency of the walk's particle loads, so by occupancy.  The
+// Bound by the L1 data pipe (three quarters busy: a lane's 16-byte loads lie a
+// cell's particles apart) and by the latency of those loads, so by occupancy.
+// Staging a slab's particles in shared memory for all three components halved
+// the pipe's work but took a third more instructions (152 us at 128^3).  The
 // accumulate kernel takes 136 us for the 128^3 dam break (3.8 M particles),
 // 412 for the 160^3 pool (11 M, dx not a power of two and divided by; 325
 // since), 508 for the 256 x 128 x 256 tank (17.5 M) and 19 for a 50^3 box; one thread per cell for
@@ -61,27 +64,19 @@ __device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
     return *reinterpret_cast<float2*>(&d);
 }
 
-// Weights of the three face slots s0, s0+1, s0+2 along a non-staggered axis:
-// the particle's corners are faces base (1 - f) and base + 1 (f), with base
-// s0 or s0 + 1.
-__device__ __forceinline__ void axis3(int s0, int base, float f, float (&w)[3]) {
-    const bool lo = base == s0;
-    w[0] = lo ? 1.0f - f : 0.0f;
-    w[1] = lo ? f : 1.0f - f;
-    w[2] = lo ? 0.0f : f;
-}
-
 // Sums one velocity component of the particles [q0, q1) of cell (ci, cj, ck)
 // over the 2 x 3 x 3 faces that cell can reach (2 along the component's own
-// axis, whose base face is always the cell's): an and ad hold num and den,
-// pair = the component axis' two faces, index = the other two axes' slots.
-// COMP selects the component and its base-index rules
-// (AccumulateVelocities::operator(), FluidSolver3D.cu:469-574).  Weights are
-// (wx*wy)*wz as in the reference; the two faces along the component's axis
-// are one packed pair, so each particle costs 12 packed multiplies and 9
-// packed FMAs and adds per component.  num accumulates vel*wgt with one fused
-// multiply-add (the reference rounds the product first; its float atomics
-// already leave the last bits of the sums order-dependent).
+// axis): an and ad hold num and den, pair = the component axis' two faces,
+// index = p slot + 3 q slot of the other two axes.  COMP selects the component.
+// The reference's base indices (AccumulateVelocities::operator(),
+// FluidSolver3D.cu:469-574) follow from the cell, which is floor(r) clamped to
+// the grid: along the own axis the base face is the cell's own, or the next one
+// beyond the grid's far edge; along the others it is the face below the cell or
+// the cell's own.  Weights are (wx*wy)*wz as in the reference; the two faces
+// along the component's axis are one packed pair, so each particle costs 12
+// packed multiplies and 9 packed FMAs and adds per component.  num accumulates
+// vel*wgt with one fused multiply-add (the reference rounds the product first;
+// its float atomics already leave the last bits of the sums order-dependent).
 // The particle's velocity component COMP.
 template <int COMP>
 __device__ __forceinline__ float comp_of(const float4& v) { return COMP == 0 ? v.x : (COMP == 1 ? v.y : v.z); }
@@ -89,10 +84,9 @@ __device__ __forceinline__ float comp_of(const float4& v) { return COMP == 0 ? v
 template <int COMP, bool P2>
 __device__ __forceinline__ void sum_cell(const float4* __restrict__ pos, const float4* __restrict__ vel, int q0, int q1,
                                          int ci, int cj, int ck, const Dims& g, float2 (&an)[9], float2 (&ad)[9]) {
-    const int W = g.W, H = g.H, D = g.D;
-    // first face of each axis' slot range: the cell's own face on the
-    // component's axis, the face below the cell on the other two
-    const int sx0 = COMP == 0 ? ci : ci - 1, sy0 = COMP == 1 ? cj : cj - 1, sz0 = COMP == 2 ? ck : ck - 1;
+    const int co = COMP == 0 ? ci : (COMP == 1 ? cj : ck), cp = COMP == 0 ? cj : ci, cq = COMP == 2 ? cj : ck;
+    const float fo = float(co), fe = float(COMP == 0 ? g.W : (COMP == 1 ? g.H : g.D)), fp = float(cp), fq = float(cq);
+    const float tp = cp > 0 ? fp : -INFINITY, tq = cq > 0 ? fq : -INFINITY;
 #pragma unroll
     for (int m = 0; m < 9; ++m) { an[m] = make_float2(0.0f, 0.0f); ad[m] = make_float2(0.0f, 0.0f); }
     // (unrolling this walk by 2 or 4 measured slower: the larger code missed
@@ -101,71 +95,26 @@ __device__ __forceinline__ void sum_cell(const float4* __restrict__ pos, const f
         const float4 P = pos[q];
         const float vc = comp_of<COMP>(vel[q]);
         const float rx = to_grid<P2>(P.x, g), ry = to_grid<P2>(P.y, g), rz = to_grid<P2>(P.z, g);
-        int bi, bj, bk;
-        float fx, fy, fz;
-        if (COMP == 0) {
-            bi = clampi(int(floorf(rx)), 0, W); bj = clampi(int(floorf(ry - 0.5f)), 0, H - 1);
-            bk = clampi(int(floorf(rz - 0.5f)), 0, D - 1);
-            fx = clamp01(rx - float(bi)); fy = clamp01((ry - 0.5f) - float(bj)); fz = clamp01((rz - 0.5f) - float(bk));
-        } else if (COMP == 1) {
-            bi = clampi(int(floorf(rx - 0.5f)), 0, W - 1); bj = clampi(int(floorf(ry)), 0, H);
-            bk = clampi(int(floorf(rz - 0.5f)), 0, D - 1);
-            fx = clamp01((rx - 0.5f) - float(bi)); fy = clamp01(ry - float(bj)); fz = clamp01((rz - 0.5f) - float(bk));
-        } else {
-            bi = clampi(int(floorf(rx - 0.5f)), 0, W - 1); bj = clampi(int(floorf(ry - 0.5f)), 0, H - 1);
-            bk = clampi(int(floorf(rz)), 0, D);
-            fx = clamp01((rx - 0.5f) - float(bi)); fy = clamp01((ry - 0.5f) - float(bj)); fz = clamp01(rz - float(bk));
-        }
+        const float ro = COMP == 0 ? rx : (COMP == 1 ? ry : rz), rp = (COMP == 0 ? ry : rx) - 0.5f,
+                    rq = (COMP == 2 ? ry : rz) - 0.5f;
+        const bool past = ro >= fe, lp = rp < tp, lq = rq < tq;
+        const float wo = __saturatef(ro - (past ? fe : fo)), wp = __saturatef(rp - (lp ? fp - 1.0f : fp)),
+                    wq = __saturatef(rq - (lq ? fq - 1.0f : fq));
+        const float2 w2 = past ? make_float2(0.0f, 1.0f - wo) : make_float2(1.0f - wo, wo);
+        const float p3[3] = {lp ? 1.0f - wp : 0.0f, lp ? wp : 1.0f - wp, lp ? 0.0f : wp};
+        const float q3[3] = {lq ? 1.0f - wq : 0.0f, lq ? wq : 1.0f - wq, lq ? 0.0f : wq};
         const float2 vv = make_float2(vc, vc);
-        if (COMP == 0) {
-            // faces along the component's axis: the base is the cell's own face,
-            // or the next one for a particle beyond the grid's far edge (whose
-            // cell key is clamped); the other two axes' bases are always the
-            // face below the cell or the cell's own (axis3)
-            const float2 wa = bi == sx0 ? make_float2(1.0f - fx, fx) : make_float2(0.0f, 1.0f - fx);
-            float wy[3], wz[3];
-            axis3(sy0, bj, fy, wy);
-            axis3(sz0, bk, fz, wz);
+        // (wx * wy) * wz, as in the reference
 #pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const float2 wab = f2_mul(wa, make_float2(wy[b], wy[b]));
+        for (int b = 0; b < 3; ++b)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float2 wgt = f2_mul(wab, make_float2(wz[c], wz[c]));
-                    an[b + 3 * c] = f2_fma(vv, wgt, an[b + 3 * c]);
-                    ad[b + 3 * c] = f2_add(ad[b + 3 * c], wgt);
-                }
+            for (int c = 0; c < 3; ++c) {
+                float2 w;
+                if (COMP == 2) w = f2_mul(make_float2(p3[b] * q3[c], p3[b] * q3[c]), w2);
+                else w = f2_mul(f2_mul(w2, make_float2(p3[b], p3[b])), make_float2(q3[c], q3[c]));
+                an[b + 3 * c] = f2_fma(vv, w, an[b + 3 * c]);
+                ad[b + 3 * c] = f2_add(ad[b + 3 * c], w);
             }
-        } else if (COMP == 1) {
-            const float2 wb = bj == sy0 ? make_float2(1.0f - fy, fy) : make_float2(0.0f, 1.0f - fy);
-            float wx[3], wz[3];
-            axis3(sx0, bi, fx, wx);
-            axis3(sz0, bk, fz, wz);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float2 wab = f2_mul(make_float2(wx[a], wx[a]), wb);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float2 wgt = f2_mul(wab, make_float2(wz[c], wz[c]));
-                    an[a + 3 * c] = f2_fma(vv, wgt, an[a + 3 * c]);
-                    ad[a + 3 * c] = f2_add(ad[a + 3 * c], wgt);
-                }
-            }
-        } else {
-            const float2 wc = bk == sz0 ? make_float2(1.0f - fz, fz) : make_float2(0.0f, 1.0f - fz);
-            float wx[3], wy[3];
-            axis3(sx0, bi, fx, wx);
-            axis3(sy0, bj, fy, wy);
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    const float wab = wx[a] * wy[b];
-                    const float2 wgt = f2_mul(make_float2(wab, wab), wc);
-                    an[a + 3 * b] = f2_fma(vv, wgt, an[a + 3 * b]);
-                    ad[a + 3 * b] = f2_add(ad[a + 3 * b], wgt);
-                }
-        }
     }
 }
 
@@ -267,30 +216,46 @@ __global__ void __launch_bounds__(3 * BX * BY, P2G_MIN_BLOCKS) k_p2g_accum(const
     }
 }
 
-// +0 computed from x (min(|x|, 0) is +0 for every x, NaN and infinities
-// included).  A store of a constant to an address whose load is still in
-// flight in the same thread waits on that load in the memory pipeline (on B200
-// a read-then-clear pass over 50 MB ran at 0.2 ms against 0.03 ms); a value
-// computed from the load is stored only after the load has returned.
-__device__ __forceinline__ float dep_zero(float x) { return fminf(fabsf(x), 0.0f); }
-
-// Pass 2, over every face of one component: num/den (ComputeVelocityFunc
-// :598-605), u* <- u, u += dt*g (the x > (float)INT_MIN test of applyForces),
-// and acc <- 0.
+// Pass 2, over every face: num/den (ComputeVelocityFunc :598-605), u* <- u, u +=
+// dt*g (the x > (float)INT_MIN test of applyForces), and acc <- 0 where it is
+// not 0 already: most faces of a scene are away from its particles, and their
+// pair needs no store.  Bound by memory, so a thread loads all its pairs before
+// it uses any: 22.9 us at 128^3, 41 at 160^3 and 84 for 256 x 128 x 256 (500 MB),
+// against 29, 55 and 114 face by face, and 31, 57 and 114 as a launch per
+// component that stored every pair.
+struct FinishArgs {
+    int64_t end[3];  // faces of u; of u and v; of all
+    float g[3];
+    float *dst[3], *sav[3];
+};
+constexpr int FINISH_THREADS = 256, FINISH_FACES = 4;
 template <bool FUSED>
-__global__ void k_p2g_finish(float2* __restrict__ acc, int64_t n, float dt, float gc, float* __restrict__ dst,
-                             float* __restrict__ sav) {
-    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const float2 a = acc[t];
-    acc[t] = make_float2(dep_zero(a.x), dep_zero(a.y));
-    float val = 0.0f;
-    if (a.y > 1e-8f) val = a.x / a.y;
-    if (FUSED) {
-        sav[t] = val;
-        dst[t] = (val > -2147483648.0f) ? val + dt * gc : val;
-    } else {
-        dst[t] = val;
+__global__ void __launch_bounds__(FINISH_THREADS) k_p2g_finish(float2* __restrict__ acc, float dt, FinishArgs f) {
+    const int64_t t0 = int64_t(blockIdx.x) * (FINISH_THREADS * FINISH_FACES) + threadIdx.x;
+    float2 a[FINISH_FACES];
+#pragma unroll
+    for (int m = 0; m < FINISH_FACES; ++m) {
+        const int64_t t = t0 + m * FINISH_THREADS;
+        a[m] = t < f.end[2] ? acc[t] : make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int m = 0; m < FINISH_FACES; ++m) {
+        const int64_t t = t0 + m * FINISH_THREADS;
+        if (t >= f.end[2]) return;
+        const int c = t < f.end[0] ? 0 : (t < f.end[1] ? 1 : 2);
+        const int64_t i = c == 0 ? t : t - (c == 1 ? f.end[0] : f.end[1]);
+        float* dst = c == 0 ? f.dst[0] : (c == 1 ? f.dst[1] : f.dst[2]);
+        if (a[m].x != 0.0f || a[m].y != 0.0f) acc[t] = make_float2(0.0f, 0.0f);
+        float val = 0.0f;
+        if (a[m].y > 1e-8f) val = a[m].x / a[m].y;
+        if (FUSED) {
+            float* sav = c == 0 ? f.sav[0] : (c == 1 ? f.sav[1] : f.sav[2]);
+            const float gc = c == 0 ? f.g[0] : (c == 1 ? f.g[1] : f.g[2]);
+            sav[i] = val;
+            dst[i] = (val > -2147483648.0f) ? val + dt * gc : val;
+        } else {
+            dst[i] = val;
+        }
     }
 }
 
@@ -323,17 +288,12 @@ void launch_p2g(const float4* pos, const float4* vel, const int* start, Dims g, 
     const int nb = ((g.W + P2G_BX - 1) / P2G_BX) * ((g.H + P2G_BY - 1) / P2G_BY) * ((g.D + P2G_BZ - 1) / P2G_BZ);
     if (g.idx != 0.0f) k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, true><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
     else k_p2g_accum<P2G_BX, P2G_BY, P2G_BZ, false><<<nb, P2G_NT, 0, st>>>(pos, vel, start, g, acc);
-    const int64_t n3[3] = {g.nu(), g.nv(), g.nw()};
-    float* dst[3] = {u, v, w};
-    float* sav[3] = {us, vs, ws};
-    const float gc[3] = {gravity.x, gravity.y, gravity.z};
-    float2* a = acc;
-    for (int c = 0; c < 3; ++c) {
-        const unsigned nb2 = unsigned((n3[c] + 255) / 256);
-        if (fused_forces) k_p2g_finish<true><<<nb2, 256, 0, st>>>(a, n3[c], dt, gc[c], dst[c], sav[c]);
-        else k_p2g_finish<false><<<nb2, 256, 0, st>>>(a, n3[c], dt, gc[c], dst[c], sav[c]);
-        a += n3[c];
-    }
+    const FinishArgs f{{g.nu(), g.nu() + g.nv(), g.nu() + g.nv() + g.nw()},
+                       {gravity.x, gravity.y, gravity.z}, {u, v, w}, {us, vs, ws}};
+    constexpr int per = FINISH_THREADS * FINISH_FACES;
+    const unsigned nb2 = unsigned((f.end[2] + per - 1) / per);
+    if (fused_forces) k_p2g_finish<true><<<nb2, FINISH_THREADS, 0, st>>>(acc, dt, f);
+    else k_p2g_finish<false><<<nb2, FINISH_THREADS, 0, st>>>(acc, dt, f);
 }
 
 void launch_forces(float* u, float* v, float* w, Dims g, float dt, float3 gravity, cudaStream_t st) {

@@ -435,7 +435,7 @@ void phase_label(fp_solver* s) {
 
 void phase_p2g(fp_solver* s, int fused) {
     if (!s->sorted) phase_label(s);
-    s->launches += 4;
+    s->launches += 2;
     launch_p2g(s->d_pos, s->d_vel, s->d_start, s->g, s->cfg.dt, gravity3(), s->d_acc, s->d_u, s->d_v, s->d_w,
                s->d_us, s->d_vs, s->d_ws, fused, s->st);
 }
