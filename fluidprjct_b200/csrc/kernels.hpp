@@ -120,11 +120,11 @@ int launch_pcg_mg(Dims g, PressureBufs& pb, const MgBufs& m, double tol, int max
                   int nu0, float* pout, cudaStream_t st);
 
 // -------- labelling and the particle sort (kernels_sort.cu) --------
-// counts[nc] must be zero on entry.  Writes key/rank per particle.
+// counts must be zero on entry.  Writes key/rank per particle.
 void launch_bin(const float4* pos, int64_t np, Dims g, int* counts, int* key, int* rank, cudaStream_t st);
 // Labels from the SOLID map, the body mark and counts; exclusive scan of counts
-// into start[nc+1]; start[nc] = np.
-void launch_label_scan(const uint8_t* base, const uint8_t* body_mark, const int* counts, uint8_t* labels, int* start,
+// into start[nc+1]; start[nc] = np; counts left zero.
+void launch_label_scan(const uint8_t* base, const uint8_t* body_mark, int* counts, uint8_t* labels, int* start,
                        int* tile_sums, Dims g, cudaStream_t st);
 void launch_scatter(const float4* pos, const float4* vel, const int* key, const int* rank, const int* start, int64_t np,
                     float4* pos2, float4* vel2, cudaStream_t st);

@@ -37,10 +37,28 @@ __device__ __forceinline__ bool solidish(uint8_t l) { return l == SOLID || l == 
 // any.  A tile is one block's quads; its counts of both are packed in one int.
 __device__ __forceinline__ int quads_of_row(const Dims& g) { return (g.W + 3) >> 2; }
 
+// The labels of a quad's m cells (SOLID beyond them), at a row's address that is
+// a multiple of four if the width W is one.
+__device__ __forceinline__ uchar4 quad_labels(const uint8_t* __restrict__ l, int m, int W) {
+    if ((W & 3) == 0) return *reinterpret_cast<const uchar4*>(l);
+    return make_uchar4(l[0], m > 1 ? l[1] : SOLID, m > 2 ? l[2] : SOLID, m > 3 ? l[3] : SOLID);
+}
+__device__ __forceinline__ void quad_floats(const float* __restrict__ a, int m, int W, float (&v)[4]) {
+    if ((W & 3) == 0) {
+        const float4 q = *reinterpret_cast<const float4*>(a);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v[t] = t < m ? a[t] : 0.0f;
+    }
+}
+
 // Pass 1: the tiles' counts; zero p off the fluid (the solve writes every FLUID
 // cell; until then they keep the previous pressure, which a warm-started MG
 // solve reads as its guess); ready the solvers' barrier, status and list
-// lengths.
+// lengths.  Bound by memory; with a quad's labels and zeros as vectors, where the
+// width is a multiple of four, 5.6 us at 128^3, 8.9 at 160^3 and 16 for 256 x 128
+// x 256, against 7.7, 12.2 and 22.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __restrict__ labels, Dims g,
                                                             float* __restrict__ p, int* __restrict__ tile_sums,
                                                             int stride, GridBar* bar, int* status, unsigned limit,
@@ -50,11 +68,15 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __res
     if (q < nqr * g.H * g.D) {
         const int row = q / nqr, Q = q - row * nqr;
         const int64_t e0 = int64_t(row) * g.W + 4 * Q;
-        const int m = min(4, g.W - 4 * Q);
-        for (int t = 0; t < m; ++t) {
-            const bool f = labels[e0 + t] == FLUID;
-            s += f;
-            if (!f) p[e0 + t] = 0.0f;
+        const uchar4 l = quad_labels(labels + e0, g.W - 4 * Q, g.W);
+        const bool f[4] = {l.x == FLUID, l.y == FLUID, l.z == FLUID, l.w == FLUID};
+        s = f[0] + f[1] + f[2] + f[3];
+        if (s == 0 && (g.W & 3) == 0) {
+            *reinterpret_cast<float4*>(p + e0) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (!f[t] && 4 * Q + t < g.W) p[e0 + t] = 0.0f;
         }
         s |= int(s > 0) << 16;
     }
@@ -125,8 +147,8 @@ struct QuadOut {
 // Pass 3: the compact system (fidx, diag, b) of every FLUID cell, and the quad
 // list.  A thread loads all labels and velocities of its quad before it uses
 // any: cell by cell, each cell's loads waited for the one before (27 us at
-// 128^3, 34 at 160^3, against 18 and 30; 256 x 128 x 256, where the writes bound
-// it, 51 either way).
+// 128^3, 34 at 160^3, 51 for 256 x 128 x 256, where the writes bound it, against
+// 18, 30 and 51, and 18, 29 and 48 with vector loads).
 __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_build(const uint8_t* __restrict__ labels,
                                                             const float* __restrict__ u, const float* __restrict__ v,
                                                             const float* __restrict__ w, Dims g, float scale,
@@ -140,10 +162,10 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_build(const uint8_t* __res
     const bool in = q < nqr * H * D;
     const int64_t e0 = int64_t(row) * W + i0, wh = int64_t(W) * H;
     // labels i0 - 1 .. i0 + 4 of the row; cells beyond the grid are SOLID
-    uint8_t lx[6];
+    const uchar4 none = make_uchar4(SOLID, SOLID, SOLID, SOLID), lq = in ? quad_labels(labels + e0, W - i0, W) : none;
+    const uint8_t lx[6] = {in && i0 > 0 ? labels[e0 - 1] : SOLID, lq.x, lq.y, lq.z, lq.w,
+                           in && i0 + 4 < W ? labels[e0 + 4] : SOLID};
     int s = 0;
-#pragma unroll
-    for (int t = 0; t < 6; ++t) lx[t] = in && i0 + t >= 1 && i0 + t <= W ? labels[e0 + t - 1] : SOLID;
 #pragma unroll
     for (int t = 0; t < 4; ++t) s += lx[t + 1] == FLUID;
     s |= int(s > 0) << 16;
@@ -153,25 +175,23 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_build(const uint8_t* __res
     int n = (pre & 0xFFFF) + tile_off[blockIdx.x];
     const int nq = (pre >> 16) + tile_off[stride + blockIdx.x];
 
-    uint8_t ly[2][4], lz[2][4];
     float uf[5], vf[2][4], wf[2][4], rd[4];
     const int64_t ui = int64_t(i0) + int64_t(row) * (W + 1);
     const int64_t vi = int64_t(i0) + int64_t(j) * W + int64_t(k) * W * (H + 1);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        const bool c = i0 + t < W;
-        ly[0][t] = c && j > 0 ? labels[e0 + t - W] : SOLID;
-        ly[1][t] = c && j + 1 < H ? labels[e0 + t + W] : SOLID;
-        lz[0][t] = c && k > 0 ? labels[e0 + t - wh] : SOLID;
-        lz[1][t] = c && k + 1 < D ? labels[e0 + t + wh] : SOLID;
-        if (rhs_dense) {
-            rd[t] = c ? rhs_dense[e0 + t] : 0.0f;
-        } else {
-            vf[0][t] = c ? v[vi + t] : 0.0f;
-            vf[1][t] = c ? v[vi + t + W] : 0.0f;
-            wf[0][t] = c ? w[e0 + t] : 0.0f;
-            wf[1][t] = c ? w[e0 + t + wh] : 0.0f;
-        }
+    const int m = W - i0;
+    const uchar4 y0 = j > 0 ? quad_labels(labels + e0 - W, m, W) : none,
+                 y1 = j + 1 < H ? quad_labels(labels + e0 + W, m, W) : none,
+                 z0 = k > 0 ? quad_labels(labels + e0 - wh, m, W) : none,
+                 z1 = k + 1 < D ? quad_labels(labels + e0 + wh, m, W) : none;
+    const uint8_t ly[2][4] = {{y0.x, y0.y, y0.z, y0.w}, {y1.x, y1.y, y1.z, y1.w}};
+    const uint8_t lz[2][4] = {{z0.x, z0.y, z0.z, z0.w}, {z1.x, z1.y, z1.z, z1.w}};
+    if (rhs_dense) {
+        quad_floats(rhs_dense + e0, m, W, rd);
+    } else {
+        quad_floats(v + vi, m, W, vf[0]);
+        quad_floats(v + vi + W, m, W, vf[1]);
+        quad_floats(w + e0, m, W, wf[0]);
+        quad_floats(w + e0 + wh, m, W, wf[1]);
     }
     if (!rhs_dense)
 #pragma unroll

@@ -346,6 +346,7 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
     ck(cudaMemsetAsync(s->d_acc, 0, sizeof(float2) * (s->g.nu() + s->g.nv() + s->g.nw()), s->st));
     ck(cudaMemsetAsync(s->d_p, 0, sizeof(float) * nc, s->st));
     ck(cudaMemsetAsync(s->d_bodymark, 0, nc, s->st));
+    ck(cudaMemsetAsync(s->d_counts, 0, sizeof(int) * (nc + 1), s->st));
     for (int i = 0; i < 2; ++i) {
         ck(cudaMemsetAsync(pb.R[i], 0, pbytes, s->st)); ck(cudaMemsetAsync(pb.Wv[i], 0, pbytes, s->st));
         ck(cudaMemsetAsync(pb.S[i], 0, pbytes, s->st));
@@ -419,7 +420,6 @@ void fill_body_stats(fp_solver* s) {
 // ---------------------------------------------------------------- phases
 void phase_label(fp_solver* s) {
     s->launches += 5;  // bin, label tiles, tile scan, start tiles, scatter
-    cudaMemsetAsync(s->d_counts, 0, sizeof(int) * (s->g.nc() + 1), s->st);
     if (body_on(s)) {
         launch_mark_body(s->d_bodymark, s->g, body_shape(s), s->st);  // MarkBodyCellsFunctor at the body's pose
         s->launches += 1;
