@@ -166,6 +166,7 @@ struct fp_solver {
     cudaEvent_t ev_net = nullptr;
     // a PCG / MG solve whose read-back one_step has deferred (ev[9] marks it)
     bool solve_pending = false;
+    bool timed = true;  // record timer events (mark)
     bool pending_guess = false;
     // pinned result mirrors
     PcgOut* h_out = nullptr;
@@ -417,6 +418,16 @@ void fill_body_stats(fp_solver* s) {
     s->stats.body_angles[0] = h.theta; s->stats.body_angles[1] = h.psi; s->stats.body_angles[2] = h.phi;
 }
 
+// Timer events, left out of the steps whose timers nobody can read (all but the
+// last of an fp_step call): an event between two kernels keeps the second one
+// from starting for 2 to 4 us, 25 us of a 64 x 64 step's 250.
+void mark(fp_solver* s, cudaEvent_t ev) {
+    if (s->timed) cudaEventRecord(ev, s->st);
+}
+void elapsed(fp_solver* s, float* ms, cudaEvent_t from, cudaEvent_t to) {
+    if (s->timed) cudaEventElapsedTime(ms, from, to);
+}
+
 // ---------------------------------------------------------------- phases
 void phase_label(fp_solver* s) {
     s->launches += 5;  // bin, label tiles, tile scan, start tiles, scatter
@@ -483,7 +494,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     const bool warm = s->cfg.solver == FP_SOLVER_PCG_MG && s->cfg.warm_start && p_out == s->d_p;
     if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
     if (mg) s->launches += launch_mg_setup(s->d_labels, s->mg, s->st);
-    cudaEventRecord(s->ev_pcg[0], s->st);
+    mark(s, s->ev_pcg[0]);
     const float* x0 = nullptr;
     if (learned) {
         const unet::Lvl real{s->W, s->H, s->D};
@@ -497,7 +508,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
                                         unet::net_scal(s->net), s->d_x0c, s->st);
         s->launches += 1 + 16 + 1;  // rhs scatter, network (2 scale/input, 10 conv, 2 pool, 2 concat), guess
-        cudaEventRecord(s->ev_net, s->st);
+        mark(s, s->ev_net);
         x0 = s->d_x0c;
     }
     // A learned MG solve that has not converged after kLearnedMaxit iterations
@@ -513,7 +524,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     else
         e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
     s->launches += 1;
-    cudaEventRecord(s->ev_pcg[1], s->st);
+    mark(s, s->ev_pcg[1]);
     if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
     cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);  // out, red and nf
     if (defer && !learned) {
@@ -527,8 +538,8 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
     if (learned && *s->h_bad) return s->fail(FP_ERR_TIMEOUT, "U-Net forward: a bounded tensor-core wait gave up");
     float pcg_ms = 0.0f, learned_ms = 0.0f;
-    cudaEventElapsedTime(&pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
-    if (learned) cudaEventElapsedTime(&learned_ms, s->ev_pcg[0], s->ev_net);
+    elapsed(s, &pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
+    if (learned) elapsed(s, &learned_ms, s->ev_pcg[0], s->ev_net);
     int iters = s->h_out->iters, outer = outer_of(s), dev_status = s->h_out->status, fallback = 0;
     const float guess = learned || warm ? guess_of(s) : 1.0f;
     if (learned) {
@@ -536,10 +547,10 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
         if (*s->h_nf > 0 && dev_status != DEV_TIMEOUT && (dev_status != DEV_OK || !(rel <= tol))) {
             // fallback: the plain FP64 PCG from x = 0
             fallback = 1;
-            cudaEventRecord(s->ev_pcg[0], s->st);
+            mark(s, s->ev_pcg[0]);
             launch_reset_barrier(pb.bar, &pb.out->status, s->wait_polls, s->st);
             e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
-            cudaEventRecord(s->ev_pcg[1], s->st);
+            mark(s, s->ev_pcg[1]);
             if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
             s->launches += 2;
             cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);
@@ -549,7 +560,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             dev_status = s->h_out->status;
             ++outer;
             float ms = 0.0f;
-            cudaEventElapsedTime(&ms, s->ev_pcg[0], s->ev_pcg[1]);
+            elapsed(s, &ms, s->ev_pcg[0], s->ev_pcg[1]);
             pcg_ms += ms;
         }
     }
@@ -563,7 +574,7 @@ int solve_finalize(fp_solver* s) {
     const cudaError_t ce = cudaEventSynchronize(s->ev[9]);
     if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
     float pcg_ms = 0.0f;
-    cudaEventElapsedTime(&pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
+    elapsed(s, &pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
     return solve_tail(s, s->h_out->iters, outer_of(s), s->h_out->status, pcg_ms, 0.0f,
                       s->pending_guess ? guess_of(s) : 1.0f, 0);
 }
@@ -841,9 +852,9 @@ int r2_compact(fp_solver* s, bool advected) {
 int one_step_ref2d(fp_solver* s) {
     int rc = r2_alloc(s);
     if (rc) return rc;
-    cudaEventRecord(s->ev[0], s->st);
+    mark(s, s->ev[0]);
     r2_label(s);
-    cudaEventRecord(s->ev[1], s->st);
+    mark(s, s->ev[1]);
     const bool ext = s->cfg.extrapolate != 0;
     if (ext) {  // P2G, extrapolation, save, forces
         r2_p2g(s, 0);
@@ -855,12 +866,12 @@ int one_step_ref2d(fp_solver* s) {
     } else {
         r2_p2g(s, 1);  // P2G + save + forces
     }
-    cudaEventRecord(s->ev[2], s->st);
+    mark(s, s->ev[2]);
     rc = r2_pressure(s);
-    cudaEventRecord(s->ev[3], s->st);
+    mark(s, s->ev[3]);
     if (rc != FP_OK) return rc;
     r2_project(s);
-    cudaEventRecord(s->ev[4], s->st);
+    mark(s, s->ev[4]);
     if (ext) {  // G2P, extrapolation, then advection and clean-up
         r2_particles(s, 1);
         rc = r2_extrapolate(s, true);
@@ -869,9 +880,14 @@ int one_step_ref2d(fp_solver* s) {
     } else {
         r2_particles(s, 7);  // G2P, advection, clean-up
     }
-    cudaEventRecord(s->ev[5], s->st);
+    mark(s, s->ev[5]);
     rc = r2_compact(s, true);
     if (rc != FP_OK) return rc;
+    ++s->steps;
+    s->stats.step = s->steps;
+    s->stats.num_particles = s->np;
+    s->stats.kernel_launches = s->launches;
+    if (!s->timed) return FP_OK;
     float t[5];
     for (int i = 0; i < 5; ++i) cudaEventElapsedTime(&t[i], s->ev[i], s->ev[i + 1]);
     s->stats.t_label = t[0];
@@ -883,10 +899,6 @@ int one_step_ref2d(fp_solver* s) {
     s->stats.t_g2p = 0.0f;
     s->stats.t_advect = t[4];
     cudaEventElapsedTime(&s->stats.t_total, s->ev[0], s->ev[5]);
-    ++s->steps;
-    s->stats.step = s->steps;
-    s->stats.num_particles = s->np;
-    s->stats.kernel_launches = s->launches;
     return FP_OK;
 }
 
@@ -904,13 +916,18 @@ int check_ready(fp_solver* s) {
 // while the GPU completes this one (the solve's own read-back still waits).
 int one_step(fp_solver* s, bool finish = true) {
     NvtxRange step_range("fp_step");
+    struct Untimed {  // timers are on outside of a step
+        fp_solver* s;
+        ~Untimed() { s->timed = true; }
+    } untimed{s};
+    s->timed = finish;
     if (ref2d(s)) return one_step_ref2d(s);
-    cudaEventRecord(s->ev[0], s->st);
+    mark(s, s->ev[0]);
     { NvtxRange r("label"); phase_label(s); }
-    cudaEventRecord(s->ev[1], s->st);
+    mark(s, s->ev[1]);
     { NvtxRange r("p2g+save+forces"); phase_p2g(s, 1); }  // P2G + save + forces
-    cudaEventRecord(s->ev[2], s->st);
-    cudaEventRecord(s->ev[3], s->st);
+    mark(s, s->ev[2]);
+    mark(s, s->ev[3]);
     // The solve's statistics are read back only after the projection and
     // advection are issued (solve_finalize), so the GPU does not idle while
     // the host reads them; a failed solve is still reported by this call.
@@ -919,11 +936,11 @@ int one_step(fp_solver* s, bool finish = true) {
     // the particles as they were; a body is integrated only after a good solve.
     int rc;
     { NvtxRange r("pressure"); rc = phase_pressure(s, true); }
-    cudaEventRecord(s->ev[4], s->st);
+    mark(s, s->ev[4]);
     auto fail_after = [&](int rc0) { const int r = solve_finalize(s); return rc0 != FP_OK ? rc0 : r; };
     if (rc != FP_OK) return fail_after(rc);
     { NvtxRange r("project"); phase_project(s, true); }
-    cudaEventRecord(s->ev[5], s->st);
+    mark(s, s->ev[5]);
     if (body_on(s)) {
         // the body phase waits for its own force anyway; finish the solve first
         rc = solve_finalize(s);
@@ -931,8 +948,8 @@ int one_step(fp_solver* s, bool finish = true) {
     }
     { NvtxRange r("body"); rc = phase_body(s); }
     if (rc != FP_OK) return fail_after(rc);
-    cudaEventRecord(s->ev[6], s->st);
-    cudaEventRecord(s->ev[7], s->st);
+    mark(s, s->ev[6]);
+    mark(s, s->ev[7]);
     NvtxRange adv_range("g2p+advect");
     if (s->cfg.extrapolate > 0) {
         phase_g2p_advect(s, 1, 0, true);
@@ -942,7 +959,7 @@ int one_step(fp_solver* s, bool finish = true) {
     } else {
         phase_g2p_advect(s, 1, 1, true);
     }
-    cudaEventRecord(s->ev[8], s->st);
+    mark(s, s->ev[8]);
     rc = solve_finalize(s);
     if (rc != FP_OK) return rc;
     ++s->steps;
