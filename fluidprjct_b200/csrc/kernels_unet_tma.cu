@@ -393,24 +393,29 @@ __global__ void __launch_bounds__(THREADS) k_conv3_tma(const __grid_constant__ C
 // taps (24 of 80 blocks), and shifting x's address by one voxel gives the x
 // taps.  Both operands are read as the channel-blocked tensors lie (MN-major,
 // no swizzle: 16-byte groups of 8 channels, one plane apart; 8 voxels of a row
-// are one core matrix, the next row the next), so a TMA box needs no
+// are one core matrix, a row of 16 the K of one MMA), so a TMA box needs no
 // rearranging.  A CTA takes one (y tap, 16 output channels, 16 input channels)
 // for a share of the bricks and keeps the three x taps' accumulators (480 TMEM
 // columns) over all of them; at its end the four epilogue warps add the eight
 // planes' diagonal blocks in a fixed order and write one partial sum.
-// Bound by the MMAs and their operand reads: 2,048 bricks x 72 MMAs of M128
-// N160 K16 per 16 x 16 channels at 128^3.  Of the kernels of a 128^3 training
-// step, warp-level MMAs with the accumulators of all taps in registers took
-// 3.07 of 4.76 ms (a brick's operands pass through ldmatrix 27 times), this
-// kernel takes 1.08 of 2.73.
+// Bound by the MMAs: 4,096 bricks x 36 MMAs of M128 N160 K16 per 16 x 16
+// channels at 128^3, at 160 cycles each (16 x 4, 32 x 2 and 64 x 1 bricks take
+// the same time).  Bricks of 8 x 16 voxels in two stages, so rows of 128 and 160
+// bytes and one brick on its way, took 1.08 ms per 128^3 training step, these
+// with rows of 256 and 288 bytes and four on their way 0.76; warp-level MMAs with
+// the accumulators of all taps in registers (a brick's operands pass through
+// ldmatrix 27 times) 3.07.
+constexpr int CTX = 16, CTY = 4, CHX = CTX + 2;        // a brick's rows, of g and (with the x taps' halo) of x
 constexpr int CZ = 8, CPZ = CZ + 2;                    // planes of g and of x
-constexpr int CG_PLANE = TX * TY * 16;                 // one 8-channel plane of g: 2,048 bytes
-constexpr int CX_PLANE = HX * TY * 16;                 // one of x (for one y tap): 2,560 bytes
+constexpr int CG_PLANE = CTX * CTY * 16;               // one 8-channel plane of g: 1,024 bytes
+constexpr int CX_PLANE = CHX * CTY * 16;               // one of x (for one y tap): 1,152 bytes
 constexpr int CG_BYTES = 2 * CZ * CG_PLANE, CX_BYTES = 2 * CPZ * CX_PLANE;
-constexpr int CSTAGE = CG_BYTES + CX_BYTES;            // 83,968 bytes; two stages
+constexpr int CSTAGE = CG_BYTES + CX_BYTES, CNST = 5;  // 39,424 bytes a stage
 constexpr int CN = CPZ * 16;                           // N of an MMA, TMEM columns of an x tap
-constexpr size_t CORR_SMEM = 2 * size_t(CSTAGE) + 8 * 6 + 16 + 128;
+constexpr int CBARS = 2 * CNST + 2;                    // full and empty per stage, done, spare
+constexpr size_t CORR_SMEM = CNST * size_t(CSTAGE) + 8 * CBARS + 16 + 128;
 static_assert(3 * CN <= 512, "TMEM columns");
+static_assert(CSTAGE % 128 == 0 && CG_BYTES % 128 == 0, "TMA destinations");
 static_assert(size_t(CZ) * 3 * 16 * 16 * 4 <= size_t(CSTAGE), "the planes' blocks reuse a stage");
 
 __host__ __device__ constexpr uint32_t corr_idesc() {  // both operands MN-major (bits 15 and 16)
@@ -438,9 +443,9 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 127u) & ~127u;
     unsigned char* sbase = smem_raw + (base - raw);
-    // barriers, 8 bytes each: full[2], empty[2], done, spare; then the TMEM slot
-    const uint32_t full0 = base + 2 * CSTAGE, empty0 = full0 + 16, done = empty0 + 16, spare = done + 8;
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sbase + 2 * CSTAGE + 48);
+    // barriers, 8 bytes each: full and empty of each stage, done, spare; then the TMEM slot
+    const uint32_t full0 = base + CNST * CSTAGE, empty0 = full0 + 8 * CNST, done = empty0 + 8 * CNST, spare = done + 8;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sbase + CNST * CSTAGE + 8 * CBARS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cig = a.cin / 16, cog = a.cout / 16;
     const int ci0 = int(blockIdx.y) % cig, co0 = (int(blockIdx.y) / cig) % cog, dy = int(blockIdx.y) / (cig * cog) - 1;
@@ -451,7 +456,7 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
     if (tid == 0) {
-        for (int q = 0; q < 6; ++q) mbar_init(full0 + 8u * q, 1);
+        for (int q = 0; q < CBARS; ++q) mbar_init(full0 + 8u * q, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
 
-    const int nbx = (a.lv.W + TX - 1) / TX, nby = (a.lv.H + TY - 1) / TY, nbz = (a.lv.D + CZ - 1) / CZ;
+    const int nbx = (a.lv.W + CTX - 1) / CTX, nby = (a.lv.H + CTY - 1) / CTY, nbz = (a.lv.D + CZ - 1) / CZ;
     const int nbricks = nbx * nby * nbz;
     const int mine = int(blockIdx.x) < nbricks ? (nbricks - 1 - int(blockIdx.x)) / int(gridDim.x) + 1 : 0;
 
@@ -468,36 +473,39 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
             auto load = [&](int i) {
                 const int brick = int(blockIdx.x) + i * int(gridDim.x);
                 const int bx = brick % nbx, by = (brick / nbx) % nby, bz = brick / (nbx * nby);
-                const uint32_t stage = base + uint32_t((i & 1) * CSTAGE), full = full0 + 8u * (i & 1);
+                const uint32_t stage = base + uint32_t((i % CNST) * CSTAGE), full = full0 + 8u * (i % CNST);
                 mbar_expect_tx(full, CSTAGE);
                 // x coordinates are 8 times a voxel index: multiples of 8 elements (16 bytes)
-                tma_load_4d(stage, &tg, full, 8 * bx * TX, by * TY, bz * CZ, 2 * co0);
-                tma_load_4d(stage + CG_BYTES, &tx, full, 8 * (bx * TX - 1), by * TY + dy, bz * CZ - 1, 2 * ci0);
+                tma_load_4d(stage, &tg, full, 8 * bx * CTX, by * CTY, bz * CZ, 2 * co0);
+                tma_load_4d(stage + CG_BYTES, &tx, full, 8 * (bx * CTX - 1), by * CTY + dy, bz * CZ - 1, 2 * ci0);
             };
             bool ok = true;
-            if (mine > 0) load(0);
-            for (int i = 0; i < mine && ok; ++i) {
-                if (!mbar_wait_bounded(full0 + 8u * (i & 1), uint32_t((i >> 1) & 1))) { ok = false; break; }
+            int i = 0, issued = 0;  // bricks consumed, and loaded or on their way
+            while (issued < min(mine, CNST - 1)) load(issued++);
+            for (; i < mine; ++i) {
+                const int st = i % CNST;
+                if (!mbar_wait_bounded(full0 + 8u * st, uint32_t((i / CNST) & 1))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t sg = base + uint32_t((i & 1) * CSTAGE), sx = sg + CG_BYTES;
+                const uint32_t sg = base + uint32_t(st * CSTAGE), sx = sg + CG_BYTES;
                 // rows outer, x taps inner: three accumulation chains interleave
-#pragma unroll 1
-                for (int y = 0; y < TY; y += 2) {
-                    const uint64_t ad = umma_desc(sg + uint32_t(y * TX * 16), TX * 16, CG_PLANE);
+#pragma unroll
+                for (int y = 0; y < CTY; ++y) {
+                    const uint64_t ad = umma_desc(sg + uint32_t(y * CTX * 16), 128, CG_PLANE);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
-                        const uint64_t bd = umma_desc(sx + uint32_t((y * HX + d) * 16), HX * 16, CX_PLANE);
+                        const uint64_t bd = umma_desc(sx + uint32_t((y * CHX + d) * 16), 128, CX_PLANE);
                         umma_bf16(tmem + uint32_t(d * CN), ad, bd, corr_idesc(), (i | y) != 0 ? 1u : 0u);
                     }
                 }
-                umma_commit(i + 1 < mine ? empty0 + 8u * (i & 1) : done);
-                // the next brick's load into the other stage, once the MMAs that read it are done
-                if (i + 1 < mine) {
-                    if (i >= 1 && !mbar_wait_bounded(empty0 + 8u * ((i - 1) & 1), uint32_t(((i - 1) >> 1) & 1))) {
+                umma_commit(i + 1 < mine ? empty0 + 8u * st : done);
+                // the load of the brick four further on, into the stage of the brick before, once the MMAs that
+                // read it are done
+                if (i + CNST - 1 < mine) {
+                    if (i >= 1 && !mbar_wait_bounded(empty0 + 8u * ((i - 1) % CNST), uint32_t(((i - 1) / CNST) & 1))) {
                         ok = false;
                         break;
                     }
-                    load(i + 1);
+                    load(issued++);
                 }
             }
             if (!ok) {
@@ -505,6 +513,8 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
                 // completes once every MMA issued so far has; the epilogue's wait gives up by itself
                 umma_commit(spare);
                 mbar_wait_bounded(spare, 0u);
+                for (; i < issued; ++i)  // the loads under way
+                    if (!mbar_wait_bounded(full0 + 8u * (i % CNST), uint32_t((i / CNST) & 1))) break;
             }
         }
     } else if (mine > 0) {
@@ -687,7 +697,7 @@ int corr_sms() {
 
 // CTAs per (y tap, channel groups): together one per SM.
 int corr_blocks(int layer, const Lvl& lv) {
-    const int nb = ((lv.W + TX - 1) / TX) * ((lv.H + TY - 1) / TY) * ((lv.D + CZ - 1) / CZ);
+    const int nb = ((lv.W + CTX - 1) / CTX) * ((lv.H + CTY - 1) / CTY) * ((lv.D + CZ - 1) / CZ);
     return std::max(1, std::min(nb, corr_sms() / corr_groups(layer)));
 }
 
@@ -697,7 +707,7 @@ int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* pa
     CUtensorMap tg, tx;
     std::memset(&tg, 0, sizeof tg);
     std::memset(&tx, 0, sizeof tx);
-    if (!make_map(&tg, g, cout, lv, TX, TY, CZ, 2) || !make_map(&tx, x, cin, lv, HX, TY, CPZ, 2))
+    if (!make_map(&tg, g, cout, lv, CTX, CTY, CZ, 2) || !make_map(&tx, x, cin, lv, CHX, CTY, CPZ, 2))
         return int(cudaErrorNotSupported);
     corr_sms();  // the kernel's shared-memory opt-in on this device
     k_corr_tma<<<dim3(nblk, corr_groups(layer)), THREADS, CORR_SMEM, st>>>(tg, tx, CorrArgs{part, lv, cout, cin, status});
