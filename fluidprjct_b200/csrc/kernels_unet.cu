@@ -50,35 +50,76 @@ __device__ __forceinline__ void block_sum_d(double (&v)[N], double* sh) {
     __syncthreads();
 }
 
+// Coordinates of voxel t of a level.  A level has fewer than 2^32 voxels (its
+// activations take over 100 bytes each), and 64-bit divisions would take most of
+// the time of these kernels.
+__device__ __forceinline__ void voxel(int64_t t, const Lvl& l, int& i, int& j, int& k) {
+    const unsigned u = unsigned(t), r = u / unsigned(l.W);
+    i = int(u - r * unsigned(l.W));
+    k = int(r / unsigned(l.H));
+    j = int(r - unsigned(k) * unsigned(l.H));
+}
+// The same of item t of C / 8 channel blocks, voxels fastest.
+__device__ __forceinline__ void block_voxel(int64_t t, const Lvl& l, int64_t& v, int& ch) {
+    ch = 0;
+    const int64_t n = l.n();
+    while (t >= n) { t -= n; ++ch; }  // at most 12 blocks
+    v = t;
+}
+// Sum of n <= THREADS values in their order, by a block of THREADS threads; in
+// thread 0.  Loaded together: one thread that loaded as it added took 12 us for
+// two sums of 256, this 4.5.
+__device__ __forceinline__ double ordered_sum(const double* __restrict__ a, int n) {
+    __shared__ double sh[THREADS];
+    __syncthreads();
+    if (int(threadIdx.x) < n) sh[threadIdx.x] = a[threadIdx.x];
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int b = 0; b < n; ++b) s += sh[b];
+    return s;
+}
+
 __device__ __forceinline__ uint8_t label_net(const uint8_t* __restrict__ lab, const Lvl& real, int i, int j, int k) {
     if (i >= real.W || j >= real.H || k >= real.D) return 0;  // padding counts as SOLID
     return lab[(int64_t(k) * real.H + j) * real.W + i];
 }
 
+// A thread's terms are added in their order, but loaded in batches: one after the
+// other, each waited for a memory round trip (10 us at 128^3, k_loss_part 36;
+// in batches 6 and 25).
+constexpr int RED_BATCH = 8;
 __global__ void __launch_bounds__(THREADS) k_rhs_scale_part(const uint8_t* __restrict__ lab,
                                                              const float* __restrict__ rhs, Lvl real,
                                                              double* __restrict__ red) {
     __shared__ double sh[2 * THREADS / 32];
     double v[2] = {0.0, 0.0};
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < real.n(); t += int64_t(gridDim.x) * blockDim.x)
-        if (lab[t] == 1) {
-            const double r = rhs[t];
-            v[0] += r * r;
-            v[1] += 1.0;
+    const int64_t n = real.n(), st = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t0 < n; t0 += RED_BATCH * st) {
+        uint8_t l[RED_BATCH];
+        float r[RED_BATCH];
+#pragma unroll
+        for (int m = 0; m < RED_BATCH; ++m) {
+            const int64_t t = t0 + m * st;
+            l[m] = t < n ? lab[t] : 0;
+            r[m] = t < n ? rhs[t] : 0.0f;
         }
+#pragma unroll
+        for (int m = 0; m < RED_BATCH; ++m)
+            if (l[m] == 1) {
+                v[0] += double(r[m]) * double(r[m]);
+                v[1] += 1.0;
+            }
+    }
     block_sum_d<2>(v, sh);
     if (threadIdx.x == 0) {
         red[blockIdx.x] = v[0];
         red[RED_BLOCKS + blockIdx.x] = v[1];
     }
 }
-__global__ void k_rhs_scale_final(const double* __restrict__ red, float* __restrict__ scal) {
+__global__ void __launch_bounds__(THREADS) k_rhs_scale_final(const double* __restrict__ red, float* __restrict__ scal) {
+    const double ss = ordered_sum(red, RED_BLOCKS), n = ordered_sum(red + RED_BLOCKS, RED_BLOCKS);
     if (threadIdx.x != 0) return;
-    double ss = 0.0, n = 0.0;
-    for (int b = 0; b < RED_BLOCKS; ++b) {
-        ss += red[b];
-        n += red[RED_BLOCKS + b];
-    }
     const double s = (n > 0.0 && ss > 0.0) ? sqrt(ss / n) : 1.0;
     scal[0] = float(s);
     scal[1] = float(1.0 / s);
@@ -88,7 +129,8 @@ __global__ void k_input(const uint8_t* __restrict__ lab, const float* __restrict
                         const float* __restrict__ scal, bf16* __restrict__ x0) {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= net.n()) return;
-    const int i = int(t % net.W), j = int((t / net.W) % net.H), k = int(t / (int64_t(net.W) * net.H));
+    int i, j, k;
+    voxel(t, net, i, j, k);
     const uint8_t l = label_net(lab, real, i, j, k);
     const float c0 = l == 1 ? __fmul_rn(rhs[(int64_t(k) * real.H + j) * real.W + i], scal[1]) : 0.0f;
     __align__(16) bf16 v[16];
@@ -126,9 +168,10 @@ __global__ void k_pool(const bf16* __restrict__ e, Lvl fine, int C, bf16* __rest
     const Lvl cl{fine.W / 2, fine.H / 2, fine.D / 2};
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= cl.n() * CH) return;
-    const int64_t V = t % cl.n();
-    const int ch = int(t / cl.n());
-    const int I = int(V % cl.W), J = int((V / cl.W) % cl.H), K = int(V / (int64_t(cl.W) * cl.H));
+    int64_t V;
+    int ch, I, J, K;
+    block_voxel(t, cl, V, ch);
+    voxel(V, cl, I, J, K);
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int dz = 0; dz < 2; ++dz)
         for (int dy = 0; dy < 2; ++dy)
@@ -150,9 +193,10 @@ __global__ void k_sum_children_mask(const bf16* __restrict__ raw, Lvl fine, int 
     const Lvl cl{fine.W / 2, fine.H / 2, fine.D / 2};
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= cl.n() * CH) return;
-    const int64_t V = t % cl.n();
-    const int ch = int(t / cl.n());
-    const int I = int(V % cl.W), J = int((V / cl.W) % cl.H), K = int(V / (int64_t(cl.W) * cl.H));
+    int64_t V;
+    int ch, I, J, K;
+    block_voxel(t, cl, V, ch);
+    voxel(V, cl, I, J, K);
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int dz = 0; dz < 2; ++dz)
         for (int dy = 0; dy < 2; ++dy)
@@ -175,9 +219,10 @@ __global__ void k_skip_combine(const bf16* __restrict__ raw, Lvl fine, int ctot,
     const int CH = C / 8;
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= fine.n() * CH) return;
-    const int64_t v = t % fine.n();
-    const int ch = int(t / fine.n());
-    const int i = int(v % fine.W), j = int((v / fine.W) % fine.H), k = int(v / (int64_t(fine.W) * fine.H));
+    int64_t v;
+    int ch, i, j, k;
+    block_voxel(t, fine, v, ch);
+    voxel(v, fine, i, j, k);
     const Lvl cl{fine.W / 2, fine.H / 2, fine.D / 2};
     float r[8], q[8], m[8];
     load8(raw + blk8(fine.n(), v, ca / 8 + ch), r);
@@ -194,14 +239,29 @@ __global__ void __launch_bounds__(THREADS) k_loss_part(const uint8_t* __restrict
     __shared__ double sh[2 * THREADS / 32];
     double v[2] = {0.0, 0.0};
     const float inv_s = scal[1];
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < real.n();
-         t += int64_t(gridDim.x) * blockDim.x) {
-        if (lab[t] != 1) continue;
-        const int i = int(t % real.W), j = int((t / real.W) % real.H), k = int(t / (int64_t(real.W) * real.H));
-        const float tv = __fmul_rn(p[t], inv_s);
-        const double e = double(out[(int64_t(k) * net.H + j) * net.W + i]) - double(tv);
-        v[0] += e * e;
-        v[1] += double(tv) * double(tv);
+    const int64_t n = real.n(), st = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t0 < n; t0 += RED_BATCH * st) {
+        uint8_t l[RED_BATCH];
+        float pv[RED_BATCH], ov[RED_BATCH];
+#pragma unroll
+        for (int m = 0; m < RED_BATCH; ++m) {
+            const int64_t t = t0 + m * st;
+            l[m] = 0;
+            if (t >= n) continue;
+            int i, j, k;
+            voxel(t, real, i, j, k);
+            l[m] = lab[t];
+            pv[m] = p[t];
+            ov[m] = out[(int64_t(k) * net.H + j) * net.W + i];
+        }
+#pragma unroll
+        for (int m = 0; m < RED_BATCH; ++m) {
+            if (l[m] != 1) continue;
+            const float tv = __fmul_rn(pv[m], inv_s);
+            const double e = double(ov[m]) - double(tv);
+            v[0] += e * e;
+            v[1] += double(tv) * double(tv);
+        }
     }
     block_sum_d<2>(v, sh);
     if (threadIdx.x == 0) {
@@ -209,18 +269,18 @@ __global__ void __launch_bounds__(THREADS) k_loss_part(const uint8_t* __restrict
         red[RED_BLOCKS + blockIdx.x] = v[1];
     }
 }
-__global__ void k_loss_final(double* __restrict__ red, float* __restrict__ scal) {
+__global__ void __launch_bounds__(THREADS) k_loss_final(double* __restrict__ red, float* __restrict__ scal) {
+    const double ee = ordered_sum(red, RED_BLOCKS);
+    double tt = ordered_sum(red + RED_BLOCKS, RED_BLOCKS);
     if (threadIdx.x != 0) return;
-    double ee = 0.0, tt = 0.0;
-    for (int b = 0; b < RED_BLOCKS; ++b) {
-        ee += red[b];
-        tt += red[RED_BLOCKS + b];
-    }
     if (!(tt > 0.0)) tt = 1.0;
     red[2 * RED_BLOCKS] = ee / tt;  // loss
     scal[2] = float(2.0 / tt);
 }
 
+// As in k_rhs_scale_part, HEAD_BATCH voxels' loads together (70 us at 128^3 one
+// by one, 49 by two; 22 at memory speed, the rest is the FP64 sums).
+constexpr int HEAD_BATCH = 2;
 __global__ void __launch_bounds__(THREADS) k_head_bwd(const uint8_t* __restrict__ lab, const float* __restrict__ p,
                                                        Lvl real, Lvl net, const float* __restrict__ out,
                                                        const bf16* __restrict__ d0, const float* __restrict__ hw,
@@ -231,24 +291,39 @@ __global__ void __launch_bounds__(THREADS) k_head_bwd(const uint8_t* __restrict_
 #pragma unroll
     for (int c = 0; c < 16; ++c) hp[c] = 0.0;
     const float inv_s = scal[1], k2 = scal[2];
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < net.n(); t += int64_t(gridDim.x) * blockDim.x) {
-        const int i = int(t % net.W), j = int((t / net.W) % net.H), k = int(t / (int64_t(net.W) * net.H));
-        const uint8_t l = label_net(lab, real, i, j, k);
-        float go = 0.0f;
-        if (l == 1) {
-            const float tv = __fmul_rn(p[(int64_t(k) * real.H + j) * real.W + i], inv_s);
-            go = (out[t] - tv) * k2;
-        }
-        float f[16], o[16];
-        load8(d0 + blk8(net.n(), t, 0), f);
-        load8(d0 + blk8(net.n(), t, 1), f + 8);
+    const int64_t n = net.n(), st = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t0 < n; t0 += HEAD_BATCH * st) {
+        uint4 lo[HEAD_BATCH], hi[HEAD_BATCH];
+        float go[HEAD_BATCH];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            o[c] = f[c] > 0.0f ? go * hw[c] : 0.0f;
-            hp[c] += double(go) * double(f[c]);
+        for (int m = 0; m < HEAD_BATCH; ++m) {
+            const int64_t t = t0 + m * st;
+            go[m] = 0.0f;
+            if (t >= n) continue;
+            int i, j, k;
+            voxel(t, net, i, j, k);
+            lo[m] = *reinterpret_cast<const uint4*>(d0 + blk8(n, t, 0));
+            hi[m] = *reinterpret_cast<const uint4*>(d0 + blk8(n, t, 1));
+            if (i >= real.W || j >= real.H || k >= real.D) continue;
+            const int64_t r = (int64_t(k) * real.H + j) * real.W + i;
+            const float pv = p[r], ov = out[t];
+            if (lab[r] == 1) go[m] = (ov - __fmul_rn(pv, inv_s)) * k2;
         }
-        store8(g9 + blk8(net.n(), t, 0), o);
-        store8(g9 + blk8(net.n(), t, 1), o + 8);
+#pragma unroll
+        for (int m = 0; m < HEAD_BATCH; ++m) {
+            const int64_t t = t0 + m * st;
+            if (t >= n) break;
+            float f[16], o[16];
+            load8(reinterpret_cast<const bf16*>(&lo[m]), f);
+            load8(reinterpret_cast<const bf16*>(&hi[m]), f + 8);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                o[c] = f[c] > 0.0f ? go[m] * hw[c] : 0.0f;
+                hp[c] += double(go[m]) * double(f[c]);
+            }
+            store8(g9 + blk8(n, t, 0), o);
+            store8(g9 + blk8(n, t, 1), o + 8);
+        }
     }
     block_sum_d<16>(hp, sh);
     if (threadIdx.x == 0)
@@ -260,7 +335,8 @@ __global__ void k_output_dense(const uint8_t* __restrict__ lab, Lvl real, Lvl ne
                                const float* __restrict__ scal, float* __restrict__ x) {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= real.n()) return;
-    const int i = int(t % real.W), j = int((t / real.W) % real.H), k = int(t / (int64_t(real.W) * real.H));
+    int i, j, k;
+    voxel(t, real, i, j, k);
     x[t] = lab[t] == 1 ? out[(int64_t(k) * net.H + j) * net.W + i] * scal[0] : 0.0f;
 }
 
@@ -299,10 +375,10 @@ __global__ void __launch_bounds__(THREADS) k_gnorm_part(const float* __restrict_
     block_sum_d<1>(v, sh);
     if (threadIdx.x == 0) red[blockIdx.x] = v[0];
 }
-__global__ void k_gnorm_final(double* __restrict__ red, float clip, float* __restrict__ scal) {
+__global__ void __launch_bounds__(THREADS) k_gnorm_final(double* __restrict__ red, float clip,
+                                                         float* __restrict__ scal) {
+    const double ss = ordered_sum(red, RED_BLOCKS);
     if (threadIdx.x != 0) return;
-    double ss = 0.0;
-    for (int b = 0; b < RED_BLOCKS; ++b) ss += red[b];
     const double nrm = sqrt(ss);
     red[2 * RED_BLOCKS + 1] = nrm;
     scal[3] = (nrm > double(clip) && isfinite(nrm)) ? float(double(clip) / nrm) : (isfinite(nrm) ? 1.0f : 0.0f);
@@ -361,7 +437,7 @@ void reduce_partials(const float* part, int nblk, int64_t n, float* out, cudaStr
 
 void launch_rhs_scale(const uint8_t* labels, const float* rhs, Lvl real, double* red, float* scal, cudaStream_t st) {
     k_rhs_scale_part<<<RED_BLOCKS, THREADS, 0, st>>>(labels, rhs, real, red);
-    k_rhs_scale_final<<<1, 32, 0, st>>>(red, scal);
+    k_rhs_scale_final<<<1, THREADS, 0, st>>>(red, scal);
 }
 
 void launch_input(const uint8_t* labels, const float* rhs, Lvl real, Lvl net, const float* scal, bf16* x0,
@@ -388,7 +464,7 @@ void launch_skip_combine(const bf16* raw, Lvl fine, int ctot, int ca, int C, con
 void launch_loss(const uint8_t* labels, const float* p, Lvl real, Lvl net, const float* out, double* red, float* scal,
                  cudaStream_t st) {
     k_loss_part<<<RED_BLOCKS, THREADS, 0, st>>>(labels, p, real, net, out, scal, red);
-    k_loss_final<<<1, 32, 0, st>>>(red, scal);
+    k_loss_final<<<1, THREADS, 0, st>>>(red, scal);
 }
 
 int head_blocks(Lvl net) { return int(std::min<int64_t>((net.n() + THREADS - 1) / THREADS, 2 * sm_count())); }
@@ -417,7 +493,7 @@ void launch_rhs_dense(const int* nf, const int* fidx, Lvl real, const float* b, 
 void launch_adam(float* w, float* m, float* v, const float* g, int64_t n, float lr, float b1, float b2, float eps,
                  float bc1, float bc2, float clip, double* red, float* scal, cudaStream_t st) {
     k_gnorm_part<<<RED_BLOCKS, THREADS, 0, st>>>(g, n, red);
-    k_gnorm_final<<<1, 32, 0, st>>>(red, clip, scal);
+    k_gnorm_final<<<1, THREADS, 0, st>>>(red, clip, scal);
     k_adam<<<unsigned((n + 255) / 256), 256, 0, st>>>(w, m, v, g, scal, n, lr, b1, b2, eps, bc1, bc2);
 }
 

@@ -570,11 +570,10 @@ __global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CU
 // [up2(coarse) | skip]; the skip tensor already lives in the blocks after
 // them.  One thread per (fine voxel, 8 channels), voxels fastest.
 __global__ void k_upcat(const bf16* __restrict__ coarse, int ca, Lvl fine, bf16* __restrict__ out) {
-    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= fine.n() * (ca / 8)) return;
-    const int64_t v = t % fine.n();
-    const int c = int(t / fine.n());
-    const int i = int(v % fine.W), j = int((v / fine.W) % fine.H), k = int(v / (int64_t(fine.W) * fine.H));
+    const unsigned v = blockIdx.x * blockDim.x + threadIdx.x;  // (a level has fewer than 2^32 voxels)
+    if (v >= fine.n()) return;
+    const int c = int(blockIdx.y);
+    const unsigned r = v / unsigned(fine.W), k = r / unsigned(fine.H), i = v - r * unsigned(fine.W), j = r - k * unsigned(fine.H);
     const Lvl cl{fine.W / 2, fine.H / 2, fine.D / 2};
     *reinterpret_cast<uint4*>(out + blk8(fine.n(), v, c)) = *reinterpret_cast<const uint4*>(
         coarse + blk8(cl.n(), (int64_t(k >> 1) * cl.H + (j >> 1)) * cl.W + (i >> 1), c));
@@ -715,8 +714,7 @@ int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* pa
 }
 
 void launch_upcat(const bf16* coarse, int ca, Lvl fine, bf16* out, cudaStream_t st) {
-    const int64_t n = fine.n() * (ca / 8);
-    k_upcat<<<unsigned((n + 255) / 256), 256, 0, st>>>(coarse, ca, fine, out);
+    k_upcat<<<dim3(unsigned((fine.n() + 255) / 256), ca / 8), 256, 0, st>>>(coarse, ca, fine, out);
 }
 
 }  // namespace unet
