@@ -1,9 +1,9 @@
 // kernels_unet.cu -- kernels of the learned pressure preconditioner (a 3D
 // U-Net; the layer table is in unet.hpp).
 //
-// The convolutions and their weight gradients run on tcgen05
-// (kernels_unet_tma.cu).  This file holds the rest: input and output, pooling,
-// the element-wise parts of the backward pass, the loss and Adam.
+// The convolutions run on tcgen05 (kernels_unet_tma.cu).  This file holds the
+// rest: the weight gradients, input and output, pooling, the element-wise parts
+// of the backward pass, the loss and Adam.
 #include <algorithm>
 #include <cstdio>
 
@@ -15,6 +15,162 @@ namespace unet {
 namespace {
 
 constexpr int THREADS = 256;
+
+// ---------------------------------------------------------------- weight gradients
+// k_corr3: dw[t][co][ci] = sum_v g[v][co] x[v + off(t)][ci] on the BF16 mma.sync
+// path (m16n8k16, FP32 accumulation; M = COUT, N = CIN, K = voxels), over bricks
+// of 8 x 8 x 4 voxels whose operands, x's with a zero-padded halo, are staged
+// with cp.async.  A CTA keeps the sums of its TPC taps over its bricks in
+// registers and writes one partial; the partials are added in a fixed order.
+//
+// Bound by ldmatrix: a brick's operands pass through it once per tap.  A warp's
+// unit is a tap, 16 input and 16 COG output channels: one x4 load of x serves 2
+// COG MMAs, and g's are loaded once per 16 voxels for all the warp's units, where
+// a warp that took 16 x 8 tiles one by one loaded both for each (x4 and x2 per
+// MMA).  Two buffers, where two CTAs of them fit an SM, let a brick's loads run
+// during the one before.  1.31 ms per 128^3 training step, against 3.07.
+//
+// Each sum keeps its order, brick by brick and 16 voxels at a time, one MMA after
+// the other: FP32 accumulation of the tensor cores is not exact, and a training
+// step's weights (Adam divides by the gradient's size) show another order's
+// rounding where a gradient nearly cancels.  tcgen05 sums over stacked planes took
+// 0.76 ms for the same layers, but moved single weights by 1e-3 of the weights'
+// size after one step.
+constexpr int BX = 8, BY = 8, BZ = 4, BRICK = BX * BY * BZ;
+constexpr int HX = BX + 2, HY = BY + 2, HZ = BZ + 2, HALO = HX * HY * HZ;  // 600
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src, bool pred) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(pred ? 16 : 0));
+}
+__device__ __forceinline__ void ldsm_x4_t(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+struct CorrArgs {
+    const bf16 *x, *g;
+    float* part;  // [gridDim.x][27][COUT][CIN] partial sums
+    Lvl lv;
+};
+
+// A CTA's TPC taps and 16 NCI input channels go to NW warps of U units each, unit
+// u = warp + NW i: output channels group u % NCG, then input channels, then taps
+// (NW is a multiple of NCG: a warp has one group).
+template <int CIN, int COUT, int TPC, int NCI, int NW, int COG, int NBUF>
+__global__ void __launch_bounds__(32 * NW) k_corr3(CorrArgs a) {
+    constexpr int NT = 32 * NW, RS = 16 * NCI + 8, GS = COUT + 8;  // (rows padded by 16 bytes: ldmatrix without conflicts)
+    constexpr int NCG = COUT / 16 / COG, UNITS = TPC * NCI * NCG, U = UNITS / NW, CIGS = CIN / 16 / NCI;
+    static_assert(27 % TPC == 0 && COUT % (16 * COG) == 0 && CIN % (16 * NCI) == 0, "tiling");
+    static_assert(UNITS % NW == 0 && NW % NCG == 0, "units");
+    constexpr int XB = HALO * RS * 2, BUF = XB + BRICK * GS * 2;  // bytes
+    extern __shared__ __align__(16) unsigned char smem[];
+    const unsigned base = smem_addr(smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tap0 = int(blockIdx.y) / CIGS * TPC, ci0 = int(blockIdx.y) % CIGS * (16 * NCI), cg = warp % NCG;
+    const Lvl lv = a.lv;
+    const int nbx = (lv.W + BX - 1) / BX, nby = (lv.H + BY - 1) / BY, nbz = (lv.D + BZ - 1) / BZ;
+    const int nbricks = nbx * nby * nbz;
+
+    auto load = [&](int brick, unsigned buf) {
+        const int x0 = brick % nbx * BX, y0 = brick / nbx % nby * BY, z0 = brick / (nbx * nby) * BZ;
+        const int64_t n = lv.n();
+        for (int hv = tid; hv < HALO; hv += NT) {
+            const int gx = x0 - 1 + hv % HX, gy = y0 - 1 + hv / HX % HY, gz = z0 - 1 + hv / (HX * HY);
+            const bool in = gx >= 0 && gx < lv.W && gy >= 0 && gy < lv.H && gz >= 0 && gz < lv.D;
+            const bf16* src = in ? a.x + blk8(n, (int64_t(gz) * lv.H + gy) * lv.W + gx, ci0 / 8) : a.x;
+            const int64_t step = in ? 8 * n : 0;
+#pragma unroll
+            for (int ch = 0; ch < 2 * NCI; ++ch) cp_async16(buf + unsigned((hv * RS + ch * 8) * 2), src + ch * step, in);
+        }
+        for (int v = tid; v < BRICK; v += NT) {
+            const int gx = x0 + (v & 7), gy = y0 + ((v >> 3) & 7), gz = z0 + (v >> 6);
+            const bool in = gx < lv.W && gy < lv.H && gz < lv.D;
+            const bf16* src = in ? a.g + blk8(n, (int64_t(gz) * lv.H + gy) * lv.W + gx, 0) : a.g;
+            const int64_t step = in ? 8 * n : 0;
+#pragma unroll
+            for (int ch = 0; ch < COUT / 8; ++ch)
+                cp_async16(buf + unsigned(XB + (v * GS + ch * 8) * 2), src + ch * step, in);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // g^T (16 channels x 16 voxels): voxel row, channel offset; x (16 voxels x 16 channels): the same the other way
+    const int akr = (lane & 7) + 8 * (lane >> 4), amoff = 8 * ((lane >> 3) & 1);
+    const int bkr = (lane & 7) + 8 * ((lane >> 3) & 1), bmoff = 8 * (lane >> 4);
+    int boff[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        const int u = (warp + NW * i) / NCG, cip = u % NCI, tap = tap0 + u / NCI;
+        const int toff = ((tap / 9 - 1) * HY + ((tap / 3) % 3 - 1)) * HX + (tap % 3 - 1);
+        boff[i] = (toff * RS + cip * 16) * 2;
+    }
+    float acc[U][COG][2][4];
+#pragma unroll
+    for (int i = 0; i < U * COG * 8; ++i) (&acc[0][0][0][0])[i] = 0.0f;
+
+    int it = 0;
+    if (int(blockIdx.x) < nbricks) load(blockIdx.x, base);
+    for (int brick = blockIdx.x; brick < nbricks; brick += gridDim.x, ++it) {
+        const unsigned buf = base + unsigned(NBUF == 2 ? (it & 1) * BUF : 0);
+        if (NBUF == 2 && brick + int(gridDim.x) < nbricks) {
+            load(brick + gridDim.x, base + unsigned(((it + 1) & 1) * BUF));
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int ks = 0; ks < 16; ++ks) {
+            const int z = ks >> 2, yy = (ks & 3) * 2;
+            const int av = (z * BY + yy + (akr >> 3)) * BX + (akr & 7);
+            const int bh = ((z + 1) * HY + (yy + (bkr >> 3) + 1)) * HX + ((bkr & 7) + 1);
+            unsigned ar[COG][4];
+#pragma unroll
+            for (int c = 0; c < COG; ++c)
+                ldsm_x4_t(ar[c], buf + unsigned(XB + (av * GS + (cg * COG + c) * 16 + amoff) * 2));
+            const unsigned bx = buf + unsigned((bh * RS + bmoff) * 2);
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                unsigned br[4];
+                ldsm_x4_t(br, bx + unsigned(boff[i]));
+#pragma unroll
+                for (int c = 0; c < COG; ++c) {
+                    mma16816(acc[i][c][0], ar[c], br[0], br[1]);
+                    mma16816(acc[i][c][1], ar[c], br[2], br[3]);
+                }
+            }
+        }
+        __syncthreads();
+        if (NBUF == 1 && brick + int(gridDim.x) < nbricks) load(brick + gridDim.x, base);
+    }
+    const int gr = lane >> 2, tq = lane & 3;
+    float* part = a.part + int64_t(blockIdx.x) * 27 * COUT * CIN;
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        const int u = (warp + NW * i) / NCG, cip = u % NCI, tap = tap0 + u / NCI;
+#pragma unroll
+        for (int c = 0; c < COG; ++c)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int co = (cg * COG + c) * 16 + gr, ci = ci0 + cip * 16 + h * 8 + 2 * tq;
+                float* p0 = part + (int64_t(tap) * COUT + co) * CIN + ci;
+                p0[0] = acc[i][c][h][0];
+                p0[1] = acc[i][c][h][1];
+                p0[8 * CIN] = acc[i][c][h][2];
+                p0[8 * CIN + 1] = acc[i][c][h][3];
+            }
+    }
+}
 
 __global__ void k_reduce_partials(const float* __restrict__ part, int nblk, int64_t n, float* __restrict__ out) {
     for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += int64_t(gridDim.x) * blockDim.x) {
@@ -428,7 +584,56 @@ int sm_count() {
     return n > 0 ? n : 148;
 }
 
+int nbricks_of(const Lvl& lv) {
+    return ((lv.W + BX - 1) / BX) * ((lv.H + BY - 1) / BY) * ((lv.D + BZ - 1) / BZ);
+}
+
+template <int CIN, int COUT, int TPC, int NCI, int NW, int COG>
+int run_corr(const CorrArgs& a, int nblk, cudaStream_t st) {
+    constexpr size_t one = size_t(HALO * (16 * NCI + 8) + BRICK * (COUT + 8)) * sizeof(bf16);
+    constexpr int NBUF = 4 * (one + 1024) <= 228 * 1024 ? 2 : 1;  // two CTAs per SM of two buffers
+    constexpr size_t smem = NBUF * one;
+    static DeviceMemo memo;
+    auto kern = k_corr3<CIN, COUT, TPC, NCI, NW, COG, NBUF>;
+    memo.get([&](int) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        return 1;
+    });
+    kern<<<dim3(nblk, 27 / TPC * (CIN / 16 / NCI)), 32 * NW, smem, st>>>(a);
+    return int(cudaPeekAtLastError());
+}
+
+// The number of brick shares of a layer, and so the order of its sums, goes by
+// these; how a share's taps and channels are spread over CTAs (corr_layer) does
+// not change a sum.
+constexpr int kTpc[kLayers] = {27, 27, 9, 9, 3, 3, 3, 9, 9, 27};
+
 }  // namespace
+
+int corr_blocks(int layer, const Lvl& lv) {
+    const int groups = 27 / kTpc[layer];
+    return std::max(1, std::min(nbricks_of(lv), 2 * sm_count() / groups));
+}
+
+int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* part, int nblk, cudaStream_t st) {
+    const CorrArgs a{x, g, part, lv};
+    // A CTA of few input channels and all taps stages little for much work and has
+    // room for two buffers, but there are fewer of them.  us at 128^3 (64^3 for
+    // layers 2, 3, 6 and 7, 32^3 for 4 and 5), all channels and few taps against
+    // this: 48 -> 16 622 and 401, 96 -> 32 466 and 245 (255 with 27 taps of 16
+    // channels), 64 -> 64 55 and 38; for 32 -> 32 83 and 87, so not there.
+    switch (layer) {
+        case 0: case 1: case 9: return run_corr<16, 16, 27, 1, 9, 1>(a, nblk, st);
+        case 2: return run_corr<16, 32, 9, 1, 9, 2>(a, nblk, st);
+        case 3: case 7: return run_corr<32, 32, 9, 2, 9, 2>(a, nblk, st);
+        case 4: return run_corr<32, 64, 3, 2, 12, 2>(a, nblk, st);
+        case 5: return run_corr<64, 64, 27, 1, 18, 2>(a, nblk, st);
+        case 6: return run_corr<96, 32, 9, 2, 9, 2>(a, nblk, st);
+        case 8: return run_corr<48, 16, 27, 1, 9, 1>(a, nblk, st);
+    }
+    return int(cudaErrorInvalidValue);
+}
 
 void reduce_partials(const float* part, int nblk, int64_t n, float* out, cudaStream_t st) {
     const int blocks = int(std::min<int64_t>((n + 255) / 256, 4 * sm_count()));

@@ -384,188 +384,6 @@ __global__ void __launch_bounds__(THREADS) k_conv3_tma(const __grid_constant__ C
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(NCOLS));
 }
 
-// ---- weight gradients: dw[t][co][ci] = sum_v g[v][co] x[v + off(t)][ci]
-// A contraction over voxels of 16 x 16 channels per tap, which alone would
-// fill an eighth of an MMA's 128 rows.  Stacking the z planes of a brick fills
-// it: M = 8 planes of g x 16 output channels, N = 10 planes of x x 16 input
-// channels, K = the voxels of a plane, so that one MMA multiplies every plane
-// of g with every plane of x; the blocks p - zo - 1 = -1, 0, 1 are the three z
-// taps (24 of 80 blocks), and shifting x's address by one voxel gives the x
-// taps.  Both operands are read as the channel-blocked tensors lie (MN-major,
-// no swizzle: 16-byte groups of 8 channels, one plane apart; 8 voxels of a row
-// are one core matrix, a row of 16 the K of one MMA), so a TMA box needs no
-// rearranging.  A CTA takes one (y tap, 16 output channels, 16 input channels)
-// for a share of the bricks and keeps the three x taps' accumulators (480 TMEM
-// columns) over all of them; at its end the four epilogue warps add the eight
-// planes' diagonal blocks in a fixed order and write one partial sum.
-// Bound by the MMAs: 4,096 bricks x 36 MMAs of M128 N160 K16 per 16 x 16
-// channels at 128^3, at 160 cycles each (16 x 4, 32 x 2 and 64 x 1 bricks take
-// the same time).  Bricks of 8 x 16 voxels in two stages, so rows of 128 and 160
-// bytes and one brick on its way, took 1.08 ms per 128^3 training step, these
-// with rows of 256 and 288 bytes and four on their way 0.76; warp-level MMAs with
-// the accumulators of all taps in registers (a brick's operands pass through
-// ldmatrix 27 times) 3.07.
-constexpr int CTX = 16, CTY = 4, CHX = CTX + 2;        // a brick's rows, of g and (with the x taps' halo) of x
-constexpr int CZ = 8, CPZ = CZ + 2;                    // planes of g and of x
-constexpr int CG_PLANE = CTX * CTY * 16;               // one 8-channel plane of g: 1,024 bytes
-constexpr int CX_PLANE = CHX * CTY * 16;               // one of x (for one y tap): 1,152 bytes
-constexpr int CG_BYTES = 2 * CZ * CG_PLANE, CX_BYTES = 2 * CPZ * CX_PLANE;
-constexpr int CSTAGE = CG_BYTES + CX_BYTES, CNST = 5;  // 39,424 bytes a stage
-constexpr int CN = CPZ * 16;                           // N of an MMA, TMEM columns of an x tap
-constexpr int CBARS = 2 * CNST + 2;                    // full and empty per stage, done, spare
-constexpr size_t CORR_SMEM = CNST * size_t(CSTAGE) + 8 * CBARS + 16 + 128;
-static_assert(3 * CN <= 512, "TMEM columns");
-static_assert(CSTAGE % 128 == 0 && CG_BYTES % 128 == 0, "TMA destinations");
-static_assert(size_t(CZ) * 3 * 16 * 16 * 4 <= size_t(CSTAGE), "the planes' blocks reuse a stage");
-
-__host__ __device__ constexpr uint32_t corr_idesc() {  // both operands MN-major (bits 15 and 16)
-    return umma_idesc_bf16(CN) | (1u << 15) | (1u << 16);
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-struct CorrArgs {
-    float* part;  // [gridDim.x][27][cout][cin]
-    Lvl lv;
-    int cout, cin;
-    int* status;
-};
-
-__global__ void __launch_bounds__(THREADS) k_corr_tma(const __grid_constant__ CUtensorMap tg,
-                                                      const __grid_constant__ CUtensorMap tx, CorrArgs a) {
-    extern __shared__ unsigned char smem_raw[];
-    const uint32_t raw = smem_u32(smem_raw);
-    const uint32_t base = (raw + 127u) & ~127u;
-    unsigned char* sbase = smem_raw + (base - raw);
-    // barriers, 8 bytes each: full and empty of each stage, done, spare; then the TMEM slot
-    const uint32_t full0 = base + CNST * CSTAGE, empty0 = full0 + 8 * CNST, done = empty0 + 8 * CNST, spare = done + 8;
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sbase + CNST * CSTAGE + 8 * CBARS);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cig = a.cin / 16, cog = a.cout / 16;
-    const int ci0 = int(blockIdx.y) % cig, co0 = (int(blockIdx.y) / cig) % cog, dy = int(blockIdx.y) / (cig * cog) - 1;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
-                     "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-    }
-    if (tid == 0) {
-        for (int q = 0; q < CBARS; ++q) mbar_init(full0 + 8u * q, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
-
-    const int nbx = (a.lv.W + CTX - 1) / CTX, nby = (a.lv.H + CTY - 1) / CTY, nbz = (a.lv.D + CZ - 1) / CZ;
-    const int nbricks = nbx * nby * nbz;
-    const int mine = int(blockIdx.x) < nbricks ? (nbricks - 1 - int(blockIdx.x)) / int(gridDim.x) + 1 : 0;
-
-    if (warp == 4) {
-        if (lane == 0) {
-            auto load = [&](int i) {
-                const int brick = int(blockIdx.x) + i * int(gridDim.x);
-                const int bx = brick % nbx, by = (brick / nbx) % nby, bz = brick / (nbx * nby);
-                const uint32_t stage = base + uint32_t((i % CNST) * CSTAGE), full = full0 + 8u * (i % CNST);
-                mbar_expect_tx(full, CSTAGE);
-                // x coordinates are 8 times a voxel index: multiples of 8 elements (16 bytes)
-                tma_load_4d(stage, &tg, full, 8 * bx * CTX, by * CTY, bz * CZ, 2 * co0);
-                tma_load_4d(stage + CG_BYTES, &tx, full, 8 * (bx * CTX - 1), by * CTY + dy, bz * CZ - 1, 2 * ci0);
-            };
-            bool ok = true;
-            int i = 0, issued = 0;  // bricks consumed, and loaded or on their way
-            while (issued < min(mine, CNST - 1)) load(issued++);
-            for (; i < mine; ++i) {
-                const int st = i % CNST;
-                if (!mbar_wait_bounded(full0 + 8u * st, uint32_t((i / CNST) & 1))) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t sg = base + uint32_t(st * CSTAGE), sx = sg + CG_BYTES;
-                // rows outer, x taps inner: three accumulation chains interleave
-#pragma unroll
-                for (int y = 0; y < CTY; ++y) {
-                    const uint64_t ad = umma_desc(sg + uint32_t(y * CTX * 16), 128, CG_PLANE);
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const uint64_t bd = umma_desc(sx + uint32_t((y * CHX + d) * 16), 128, CX_PLANE);
-                        umma_bf16(tmem + uint32_t(d * CN), ad, bd, corr_idesc(), (i | y) != 0 ? 1u : 0u);
-                    }
-                }
-                umma_commit(i + 1 < mine ? empty0 + 8u * st : done);
-                // the load of the brick four further on, into the stage of the brick before, once the MMAs that
-                // read it are done
-                if (i + CNST - 1 < mine) {
-                    if (i >= 1 && !mbar_wait_bounded(empty0 + 8u * ((i - 1) % CNST), uint32_t(((i - 1) / CNST) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    load(issued++);
-                }
-            }
-            if (!ok) {
-                if (a.status) atomicExch(a.status, DEV_TIMEOUT_CODE);
-                // completes once every MMA issued so far has; the epilogue's wait gives up by itself
-                umma_commit(spare);
-                mbar_wait_bounded(spare, 0u);
-                for (; i < issued; ++i)  // the loads under way
-                    if (!mbar_wait_bounded(full0 + 8u * (i % CNST), uint32_t((i / CNST) & 1))) break;
-            }
-        }
-    } else if (mine > 0) {
-        bool got = true;
-        if (lane == 0) got = mbar_wait_bounded(done, 0u);
-        got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
-        if (!got && lane == 0 && a.status) atomicExch(a.status, DEV_TIMEOUT_CODE);
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        // row m = (channel half, plane zo, channel): this lane's
-        const int m = warp * 32 + lane, zo = (m >> 3) & 7, co = (m >> 6) * 8 + (m & 7);
-        float* S = reinterpret_cast<float*>(sbase);  // [zo][dz][co][ci], over the consumed stage 0
-        const uint32_t lanes = tmem + (uint32_t(warp * 32) << 16);
-#pragma unroll 1
-        for (int d = 0; d < 3; ++d) {
-            float acc[3][16];
-#pragma unroll
-            for (int p = 0; p < CPZ; ++p) {
-                float v[16];
-                tmem_ld8(lanes + uint32_t(d * CN + p * 8), v);
-                tmem_ld8(lanes + uint32_t(d * CN + CPZ * 8 + p * 8), v + 8);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-                for (int z = 0; z < 3; ++z)
-                    if (p == zo + z)
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) acc[z][q] = v[q];
-            }
-#pragma unroll
-            for (int z = 0; z < 3; ++z)
-#pragma unroll
-                for (int q = 0; q < 16; q += 4)
-                    *reinterpret_cast<float4*>(S + ((zo * 3 + z) * 16 + co) * 16 + q) =
-                        make_float4(acc[z][q], acc[z][q + 1], acc[z][q + 2], acc[z][q + 3]);
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
-            for (int t = tid; t < 3 * 16 * 16; t += EPI_THREADS) {
-                float sum = 0.0f;
-#pragma unroll
-                for (int z = 0; z < CZ; ++z) sum += S[z * 768 + t];
-                const int dz = t >> 8, c = (t >> 4) & 15, ci = t & 15;
-                const int tap = dz * 9 + (dy + 1) * 3 + d;
-                a.part[((int64_t(blockIdx.x) * 27 + tap) * a.cout + co0 * 16 + c) * a.cin + ci0 * 16 + ci] = sum;
-            }
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
-}
-
 // up2(coarse) into the first ca / 8 channel blocks of a decoder layer's input
 // [up2(coarse) | skip]; the skip tensor already lives in the blocks after
 // them.  One thread per (fine voxel, 8 channels), voxels fastest.
@@ -595,16 +413,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 }
 
 // Tensor map of a channel-blocked [C/8][D][H][W][8] bf16 tensor seen as
-// (8 W, H, D, C / 8), with boxes of bx x by x bz voxels and bc 8-channel
-// planes (rows of 16 bx contiguous bytes).
-bool make_map(CUtensorMap* map, const bf16* ptr, int C, const Lvl& lv, int bx = HX, int by = HY, int bz = HZ,
-              int bc = 1) {
+// (8 W, H, D, C / 8): one box is an 8-channel halo plane of HX x HY x HZ
+// voxels, HY * HZ rows of 160 contiguous bytes.
+bool make_map(CUtensorMap* map, const bf16* ptr, int C, const Lvl& lv) {
     auto enc = encoder();
     if (!enc) return false;
     const cuuint64_t dims[4] = {cuuint64_t(lv.W) * 8, cuuint64_t(lv.H), cuuint64_t(lv.D), cuuint64_t(C / 8)};
     const cuuint64_t strides[3] = {cuuint64_t(lv.W) * 16, cuuint64_t(lv.H) * lv.W * 16,
                                    cuuint64_t(lv.D) * lv.H * lv.W * 16};
-    const cuuint32_t box[4] = {cuuint32_t(8 * bx), cuuint32_t(by), cuuint32_t(bz), cuuint32_t(bc)};
+    const cuuint32_t box[4] = {8 * HX, HY, HZ, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(ptr), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -678,39 +495,6 @@ int conv_backward_layer_tma(int layer, const bf16* in, const TmaConvArgs& a, cud
         case 2: return run_tma<32, 16, 16, EPI_RAW>(in, a, st);
     }
     return int(cudaErrorInvalidValue);
-}
-
-namespace {
-int corr_groups(int layer) { return 3 * (kSpec[layer].cout / 16) * ((kSpec[layer].ca + kSpec[layer].cb) / 16); }
-int corr_sms() {
-    static DeviceMemo memo;
-    const int n = memo.get([](int dev) {
-        int sms = 0;
-        cudaFuncSetAttribute(k_corr_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, int(CORR_SMEM));
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        return std::max(sms, 0);
-    });
-    return n > 0 ? n : 148;
-}
-}  // namespace
-
-// CTAs per (y tap, channel groups): together one per SM.
-int corr_blocks(int layer, const Lvl& lv) {
-    const int nb = ((lv.W + CTX - 1) / CTX) * ((lv.H + CTY - 1) / CTY) * ((lv.D + CZ - 1) / CZ);
-    return std::max(1, std::min(nb, corr_sms() / corr_groups(layer)));
-}
-
-int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* part, int nblk, int* status,
-               cudaStream_t st) {
-    const int cin = kSpec[layer].ca + kSpec[layer].cb, cout = kSpec[layer].cout;
-    CUtensorMap tg, tx;
-    std::memset(&tg, 0, sizeof tg);
-    std::memset(&tx, 0, sizeof tx);
-    if (!make_map(&tg, g, cout, lv, CTX, CTY, CZ, 2) || !make_map(&tx, x, cin, lv, CHX, CTY, CPZ, 2))
-        return int(cudaErrorNotSupported);
-    corr_sms();  // the kernel's shared-memory opt-in on this device
-    k_corr_tma<<<dim3(nblk, corr_groups(layer)), THREADS, CORR_SMEM, st>>>(tg, tx, CorrArgs{part, lv, cout, cin, status});
-    return int(cudaPeekAtLastError());
 }
 
 void launch_upcat(const bf16* coarse, int ca, Lvl fine, bf16* out, cudaStream_t st) {

@@ -147,7 +147,7 @@ int conv_bwd(fp_unet* u, int l, const bf16* g, const bf16* mask, bf16* y, cudaSt
 int wgrad(fp_unet* u, int l, const bf16* x, const bf16* g, cudaStream_t st) {
     const Lvl& lv = u->L[kSpec[l].level];
     const int nblk = corr_blocks(l, lv);
-    const int e = corr_layer(l, x, g, lv, u->part, nblk, u->d_status, st);
+    const int e = corr_layer(l, x, g, lv, u->part, nblk, st);
     reduce_partials(u->part, nblk, layer_size(l), u->grad + layer_offset(l), st);
     return e;
 }

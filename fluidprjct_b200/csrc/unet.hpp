@@ -74,8 +74,7 @@ void launch_upcat(const bf16* coarse, int ca, Lvl fine, bf16* out, cudaStream_t 
 // as nblk = corr_blocks() partial sums [nblk][27][COUT][CIN] (to be added by
 // reduce_partials); x is the layer's whole input.  Returns 0 or a cudaError_t.
 int corr_blocks(int layer, const Lvl& lv);
-int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* part, int nblk, int* status,
-               cudaStream_t st);
+int corr_layer(int layer, const bf16* x, const bf16* g, const Lvl& lv, float* part, int nblk, cudaStream_t st);
 
 // Launchers (kernels_unet.cu).
 void reduce_partials(const float* part, int nblk, int64_t n, float* out, cudaStream_t st);
