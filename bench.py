@@ -261,7 +261,7 @@ def run_ours(args, rank, local, world):
         note = ("189 B per fluid cell + 5 B per cell per MG-PCG iteration; the kernel is bound by its "
                 "~20 grid barriers per iteration and L2 latency (the working set stays in L2), not by HBM")
     else:
-        kernel = "k_pcg_cg"
+        kernel = "k_pcg_mixed" if "mixed" in args.solver else "k_pcg64"
         solve_bytes = [41.0 * p["num_fluid_cells"] * p["pcg_iters"] + 17.0 * p["num_fluid_cells"] * p["outer_iters"]
                        for p in per]
         note = "41 B per fluid cell per iteration + 17 B per fluid cell; working set is L2-resident at 128^3"
