@@ -155,10 +155,13 @@ __device__ __forceinline__ void brick_component(const float4* __restrict__ pos, 
             for (int e = 0; e < 2; ++e) {
                 const int o1 = m % 3, o2 = m / 3;
                 const int ox = COMP == 0 ? e : o1, oy = COMP == 1 ? e : (COMP == 0 ? o1 : o2), oz = COMP == 2 ? e : o2;
-                if (q1 > q0) {
+                // a face that none of the cell's particles reaches has weight 0 here, and a num of 0 times
+                // their velocities: NaN for one that is not finite, so it is left out
+                const float den = e ? ad[m].y : ad[m].x;
+                if (den != 0.0f) {
                     float2& f = s[ox + oy * R::X + oz * R::X * R::Y];
                     const float2 v = f;
-                    f = make_float2(v.x + (e ? an[m].y : an[m].x), v.y + (e ? ad[m].y : ad[m].x));
+                    f = make_float2(v.x + (e ? an[m].y : an[m].x), v.y + den);
                 }
                 asm volatile("bar.sync %0, %1;\n" ::"n"(COMP + 1), "n"(BX * BY) : "memory");
             }

@@ -372,3 +372,49 @@ def test_cell_of_a_boundary_particle(dx):
     want[k, j, np.floor(pos[:, 0] / d).astype(int)] = 1
     assert np.array_equal(s.labels(), want)
     s.close()
+
+
+def test_p2g_of_a_velocity_that_is_not_finite():
+    """A particle whose velocity has become infinite or NaN (here from faces set so) spoils the eight faces per component
+    that it reaches and no other, not even those that other particles of its cell could reach.  The weights are exact
+    (products of quarters), so the other faces are those of the finite particles, to the rounding of at most 18 terms,
+    their sum and a quotient."""
+    from fluidprjct_b200 import capi
+    W, H, D, dx = 20, 14, 13, 0.125
+    s = capi.Solver(dim=3, dx=dx, dt=0.01, output_format=capi.OUT_NONE)
+    s.set_labels(np.full((D, H, W), 2, np.uint8))
+    k, j, i = np.meshgrid(*[np.arange(m) for m in (D, H, W)], indexing="ij")
+    cell = np.stack([i.ravel(), j.ravel(), k.ravel()], 1)
+    rng = np.random.default_rng(4)
+    s.set_particles(((cell + rng.choice([0.25, 0.75], cell.shape)) * dx).astype(np.float32))
+    grids = (capi.GRID_U, capi.GRID_V, capi.GRID_W)
+    for which in grids:
+        g = rng.uniform(-1, 1, s.grid(which).shape).astype(np.float32)
+        g[0, 0, 0], g[4, 3, 8], g[6, 8, 13] = np.inf, np.nan, -np.inf  # a corner, an edge of a brick, inside one
+        s.set_grid(which, g)
+    s.phase(capi.PHASE_G2P)
+    s.phase(capi.PHASE_LABEL)
+    s.phase(capi.PHASE_P2G)
+    pos, vel = s.particles()
+    r, vel = pos.astype(np.float64) / dx, vel.astype(np.float64)
+    N = (W, H, D)
+    for a, which in enumerate(grids):
+        good = np.isfinite(vel[:, a])
+        sh = tuple(N[d] + (d == a) for d in range(3))
+        num, den, hit = np.zeros(sh), np.zeros(sh), np.zeros(sh, bool)
+        t = r - 0.5 * (np.arange(3) != a)
+        b = np.maximum(np.floor(t), 0).astype(int)
+        f = np.clip(t - b, 0, 1)
+        for o in np.ndindex(2, 2, 2):
+            w = np.prod(np.where(o, f, 1 - f), axis=1)
+            q = b + np.array(o)
+            ok = (q < sh).all(1) & (w > 0)
+            hit[tuple(q[ok & ~good].T)] = True
+            np.add.at(num, tuple(q[ok & good].T), (w * np.where(good, vel[:, a], 0))[ok & good])
+            np.add.at(den, tuple(q[ok & good].T), w[ok & good])
+        got = s.grid(which).transpose(2, 1, 0)
+        assert hit.any() and not np.isfinite(got[hit]).any()
+        rest = ~hit & (den > 0)
+        assert np.isfinite(got[rest]).all()
+        assert np.abs(got[rest] - num[rest] / den[rest]).max() <= 24 * 2.0 ** -24
+    s.close()
