@@ -26,12 +26,14 @@
 // cell's particles apart) and by the latency of those loads, so by occupancy.
 // Staging a slab's particles in shared memory for all three components halved
 // the pipe's work but took a third more instructions (152 us at 128^3).  The
-// accumulate kernel takes 136 us for the 128^3 dam break (3.8 M particles),
-// 412 for the 160^3 pool (11 M, dx not a power of two and divided by; 325
-// since), 508 for the 256 x 128 x 256 tank (17.5 M) and 19 for a 50^3 box; one thread per cell for
-// all three components in turn, with shared-memory atomics, took 138, 420, 567
-// and 33 (a small grid's bricks then leave most of the chip idle).  8 x 8 x 4
-// bricks: 141, 430, 561 and 23 at five CTAs of 192 per SM, 165, 504 and 650 at
+// accumulate kernel takes 131 us for the 128^3 dam break (3.8 M particles), 319
+// for the 160^3 pool (11 M, dx not a power of two), 488 for the 256 x 128 x 256
+// tank (17.5 M) and 14.4 for a 50^3 box; with a hardware barrier in place of the
+// one-warp groups' __syncwarp 135, 323, 510 and 15.  With hardware barriers, and
+// x / dx still a division: this split 136, 412, 508 and 19; one thread per cell
+// for all three components in turn, with shared-memory atomics, 138, 420, 567
+// and 33 (a small grid's bricks then leave most of the chip idle); 8 x 8 x 4
+// bricks 141, 430, 561 and 23 at five CTAs of 192 per SM, 165, 504 and 650 at
 // four.
 #include "kernels.hpp"
 
@@ -132,6 +134,15 @@ struct Reach {
     static constexpr int X = BX + 2, Y = BY + 2, Z = BZ + 2, N = X * Y * Z;
 };
 
+// Barrier of one component's group of N threads.  The lanes come out of walks of
+// different lengths: a group of one warp synchronises as a warp, a larger one by
+// the form of the barrier that does not need its warps converged.
+template <int COMP, int N>
+__device__ __forceinline__ void group_sync() {
+    if constexpr (N == 32) __syncwarp();
+    else asm volatile("barrier.sync %0, %1;\n" ::"n"(COMP + 1), "n"(N) : "memory");
+}
+
 // One component of a brick, by the BX * BY threads of one group: thread t
 // takes cell (t % BX, t / BX) of every z slab in turn.
 template <int COMP, int BX, int BY, int BZ, bool P2>
@@ -163,7 +174,7 @@ __device__ __forceinline__ void brick_component(const float4* __restrict__ pos, 
                     const float2 v = f;
                     f = make_float2(v.x + (e ? an[m].y : an[m].x), v.y + den);
                 }
-                asm volatile("bar.sync %0, %1;\n" ::"n"(COMP + 1), "n"(BX * BY) : "memory");
+                group_sync<COMP, BX * BY>();
             }
     }
 }
