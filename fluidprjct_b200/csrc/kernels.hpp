@@ -240,10 +240,12 @@ constexpr int kCsrPartials = 4 * kCsrMaxBlocks;  // doubles in part
 // and columns first (x is written only if they pass).  Returns 0 or a
 // cudaError_t value.
 int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, const double* b, double* x, double* work,
-                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st);
-// The same from host arrays, complete on return.
+                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st,
+                  unsigned wait_polls = kDefaultWaitPolls);
+// The same from host arrays, complete on return, as an FP_* status; x, *iters
+// and *relres are written only with FP_OK.
 int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x, double tol,
-                 int maxit, int* iters, double* relres, cudaStream_t st);
+                 int maxit, int* iters, double* relres, cudaStream_t st, unsigned wait_polls = kDefaultWaitPolls);
 
 // -------- velocity extrapolation (kernels_extrap.cu) --------
 // Values equal to VEL_UNKNOWN on an nx x ny face grid, depth waves; the first

@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdio>
 
+#include "../../include/fluidprjct.h"
 #include "device_memo.hpp"
 #include "kernels.hpp"
 #include "pcg_common.cuh"
@@ -494,7 +495,8 @@ void launch_project(float* u, float* v, float* w, const float* p, const uint8_t*
 }
 
 int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, const double* b, double* x, double* work,
-                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st) {
+                  int64_t stride, double* part, CsrCtl* ctl, int check, double tol, int maxit, cudaStream_t st,
+                  unsigned wait_polls) {
     static DeviceMemo memo;
     const int resident = memo.get([](int dev) {
         int sms = 0;
@@ -503,7 +505,7 @@ int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, co
     });
     // One row per thread while that fits one CTA per SM (a one-CTA grid's barrier is a block barrier).
     const int nb = std::max(1, std::min(resident, (n - 1) / CSR_THREADS + 1));
-    k_csr_reset<<<1, 1, 0, st>>>(ctl, kDefaultWaitPolls);
+    k_csr_reset<<<1, 1, 0, st>>>(ctl, wait_polls);
     CsrCgArgs a{};
     a.n = n; a.check = check; a.maxit = maxit; a.tol = tol;
     a.off = off; a.cols = cols; a.vals = vals; a.b = b; a.x = x;
@@ -516,15 +518,14 @@ int launch_csr_cg(int n, const int* off, const int* cols, const double* vals, co
 }
 
 int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x, double tol,
-                 int maxit, int* iters, double* relres, cudaStream_t st) {
-    if (n <= 0) return -1;
+                 int maxit, int* iters, double* relres, cudaStream_t st, unsigned wait_polls) {
     const size_t nnz = size_t(offsets[n]), N = size_t(n);
     // one allocation: doubles (values, b, x, the work vectors), the partials and the control block, then the integers
     const size_t nd = nnz + (2 + kCsrVectors) * N;
     const size_t bytes = sizeof(double) * (nd + kCsrPartials) + sizeof(CsrCtl) + sizeof(int) * (N + 1 + nnz);
     unsigned char* base = nullptr;
     cudaError_t e = cudaMalloc(&base, bytes);
-    if (e != cudaSuccess) return int(e);
+    if (e != cudaSuccess) return FP_ERR_CUDA;
     double* d_vals = reinterpret_cast<double*>(base);
     double *d_b = d_vals + nnz, *d_x = d_b + N, *work = d_x + N;
     double* part = d_vals + nd;
@@ -537,16 +538,22 @@ int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals,
     ck(cudaMemcpyAsync(d_vals, vals, sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
     ck(cudaMemcpyAsync(d_b, b, sizeof(double) * N, cudaMemcpyHostToDevice, st));
     if (e == cudaSuccess)
-        ck(cudaError_t(launch_csr_cg(n, d_off, d_cols, d_vals, d_b, d_x, work, int64_t(N), part, ctl, 0, tol, maxit, st)));
+        ck(cudaError_t(launch_csr_cg(n, d_off, d_cols, d_vals, d_b, d_x, work, int64_t(N), part, ctl, 0, tol, maxit, st,
+                                     wait_polls)));
     CsrCtl h{};
     ck(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, st));
-    ck(cudaMemcpyAsync(x, d_x, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
     ck(cudaStreamSynchronize(st));
-    if (e == cudaSuccess && h.status != DEV_OK) e = cudaErrorUnknown;  // a bounded wait gave up
+    const bool gave_up = e == cudaSuccess && h.status != DEV_OK;
+    if (e == cudaSuccess && !gave_up) {
+        ck(cudaMemcpyAsync(x, d_x, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+        ck(cudaStreamSynchronize(st));
+    }
+    cudaFree(base);
+    if (gave_up) return FP_ERR_TIMEOUT;
+    if (e != cudaSuccess) return FP_ERR_CUDA;
     if (iters) *iters = h.iters;
     if (relres) *relres = h.bb > 0 ? sqrt(h.rr / h.bb) : 0.0;
-    cudaFree(base);
-    return e == cudaSuccess ? 0 : int(e);
+    return FP_OK;
 }
 
 }  // namespace fp

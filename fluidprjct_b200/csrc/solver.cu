@@ -1925,8 +1925,7 @@ int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double*
         if (offsets[i + 1] < offsets[i]) return FP_ERR_ARG;
     for (int e = 0; e < offsets[n]; ++e)
         if (cols[e] < 0 || cols[e] >= n) return FP_ERR_ARG;
-    int rc = csr_cg_solve(n, offsets, cols, vals, b, x, tol, max_iters, iters, relres, 0);
-    return rc ? FP_ERR_CUDA : FP_OK;
+    return csr_cg_solve(n, offsets, cols, vals, b, x, tol, max_iters, iters, relres, 0);
 }
 
 }  // extern "C"

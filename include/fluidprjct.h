@@ -325,7 +325,10 @@ int fp_pressure_solve(fp_solver* s, const float* rhs, float* x, int64_t n, int* 
 
 /* Stand-alone SPD solve of an upper-triangle CSR matrix (the storage passed to
  * cuDSS with CUDSS_MVIEW_UPPER, FluidSolver3D.cu:1932-1945) by GPU CG with
- * FP64 vectors: the known-answer path of test.cu:223-395.  Host arrays. */
+ * FP64 vectors: the known-answer path of test.cu:223-395.  Host arrays.
+ * FP_OK also when CG stops at max_iters or breaks down: check *relres against
+ * tol.  FP_ERR_TIMEOUT: a grid-barrier wait of the solver gave up (after about
+ * a minute).  x, *iters and *relres are written only with FP_OK. */
 int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x,
                        double tol, int max_iters, int* iters, double* relres);
 
@@ -340,6 +343,9 @@ int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double*
  *     must be 0, offsets must not decrease, columns must lie in [0, n);
  *   - like fp_solve_csr_upper it returns FP_OK when CG stops at max_iters or
  *     breaks down: check *relres against tol;
+ *   - FP_ERR_TIMEOUT: a grid-barrier wait of the solver gave up (after about a
+ *     minute); *iters and *relres are then unchanged, x is an unfinished
+ *     iterate;
  *   - the call is synchronous (it reads its result back and drains its
  *     stream before returning), so it must not be issued on a stream that is
  *     being captured;

@@ -85,3 +85,27 @@ def test_wait_limit_rejects_negative_values():
         s.set_wait_limit(-1)
     assert e.value.code == capi.FP_ERR_ARG
     s.close()
+
+
+def test_timed_out_csr_solve_is_no_answer():
+    """The stand-alone CSR solve with a poll limit of 1 on 148 blocks, through the internal entry that takes the limit
+    (fp_solve_csr_upper returns its status as it is): FP_ERR_TIMEOUT, with the caller's x, iteration count and residual
+    untouched.  The same call with the default limit then solves."""
+    import ctypes as C
+    from fluidprjct_b200 import capi
+    n = 148 * 512
+    off, cols = np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32)
+    vals, b = np.random.default_rng(2).uniform(1, 2, n), np.ones(n)
+    solve = capi.lib()._ZN2fp12csr_cg_solveEiPKiS1_PKdS3_PddiPiS4_P11CUstream_stj  # fp::csr_cg_solve
+    solve.restype = C.c_int
+    x, it, rr = np.full(n, 7.0), C.c_int(-3), C.c_double(-3.0)
+
+    def call(polls):
+        p = lambda a: C.c_void_p(a.ctypes.data)
+        return solve(C.c_int(n), p(off), p(cols), p(vals), p(b), p(x), C.c_double(1e-12), C.c_int(10), C.byref(it),
+                     C.byref(rr), C.c_void_p(None), C.c_uint(polls))
+
+    assert call(1) == capi.FP_ERR_TIMEOUT
+    assert (x == 7.0).all() and it.value == -3 and rr.value == -3.0
+    assert call(1 << 27) == capi.FP_OK
+    assert np.abs(x * vals - 1).max() <= 1e-12 and 0 < it.value <= 10 and 0 <= rr.value <= 1e-12
