@@ -58,6 +58,19 @@ __device__ __forceinline__ float to_grid(float x, const Dims& g) {
     return P2 ? x * g.idx : over_const(x, g.dx, g.rhi, g.rlo);
 }
 
+// Nanoseconds of the GPU's clock, the same for all SMs (32 ns steps on a B200).
+// A kernel that notes it costs nothing, where a timing event between two kernels
+// keeps the second one from starting for 2 to 5 us.
+__device__ __forceinline__ unsigned long long clock_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// ... noted at *at (if not null) by the grid's first thread.
+__device__ __forceinline__ void note_clock(unsigned long long* at) {
+    if (at && blockIdx.x == 0 && threadIdx.x == 0) *at = clock_ns();
+}
+
 __device__ __forceinline__ int clampi(int a, int lo, int hi) { return min(max(a, lo), hi); }
 __device__ __forceinline__ float clamp01(float f) { return fminf(fmaxf(f, 0.0f), 1.0f); }
 

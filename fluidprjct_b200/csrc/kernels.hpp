@@ -12,6 +12,7 @@ namespace fp {
 struct GridBar {
     unsigned count;
     unsigned limit;  // polls after which a wait gives up (set at launch)
+    unsigned long long* gave_up;  // where a wait that gives up notes the device clock, or null
 };
 
 // Polls after which a grid-barrier wait of the persistent solvers gives up
@@ -28,6 +29,9 @@ struct PcgOut {
     double rr0;     // ||b - A x0||^2 of the initial iterate (MG and mixed)
     int outer;      // refinement loops (plain PCG: 1; MG leaves it alone)
     int pad_;
+    // device clock (clock_ns) at the start of launch_pressure_setup, and at the
+    // solve kernel's start and end (or when a wait of it gave up)
+    unsigned long long t_setup, t_begin, t_end;
 };
 
 // Device buffers of the pressure system.  Compact arrays are indexed by the

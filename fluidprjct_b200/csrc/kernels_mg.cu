@@ -867,6 +867,7 @@ __device__ __forceinline__ D4 apply_quad(const MgLevel& F, int c, uint32_t k, fl
 }
 
 __global__ void __launch_bounds__(MG_THREADS, 1) k_pcg_mg(const __grid_constant__ MgArgs a) {
+    note_solve(&a.out->t_begin);
     const int nb = int(gridDim.x);
     const int t0 = blockIdx.x * MG_THREADS + threadIdx.x, st = nb * MG_THREADS;
     const MgLevel& F = a.lv[0];
@@ -1100,6 +1101,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_pcg_mg(const __grid_constant_
         a.out->bb = bb;
         a.out->rz = gam;
         a.out->rr0 = rr0;
+        note_solve(&a.out->t_end);
     }
 }
 

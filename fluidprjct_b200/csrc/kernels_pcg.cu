@@ -364,6 +364,7 @@ __device__ __forceinline__ void report(const PcgArgs& a, int iters, int outer, i
     a.out->rr0 = rr0;
     a.red[0] = res[0];
     a.red[1] = res[1];
+    note_solve(&a.out->t_end);
 }
 
 __device__ __forceinline__ Share share_of(const PcgArgs& a, bool& one) {
@@ -380,6 +381,7 @@ __device__ __forceinline__ Share share_of(const PcgArgs& a, bool& one) {
 
 // The FP64 solver: CG from x = 0, then the true residual of its solution.
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg64(PcgArgs a) {
+    note_solve(&a.out->t_begin);
     bool one;
     Share h = share_of(a, one);
     Cg cg;
@@ -396,6 +398,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg64(PcgArgs a) {
 // The mixed-precision solver: r = b - A x in FP64, A c = r by FP32 CG to a
 // loose tolerance, x += c, until ||r|| <= tol ||b||.
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg_mixed(PcgArgs a) {
+    note_solve(&a.out->t_begin);
     bool one;
     Share h = share_of(a, one);
     const int tid = threadIdx.x;

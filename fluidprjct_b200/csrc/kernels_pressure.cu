@@ -62,8 +62,9 @@ __device__ __forceinline__ void quad_floats(const float* __restrict__ a, int m, 
 // x 256, against 7.7, 12.2 and 22.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __restrict__ labels, Dims g,
                                                             float* __restrict__ p, int* __restrict__ tile_sums,
-                                                            int stride, GridBar* bar, int* status, unsigned limit,
+                                                            int stride, GridBar* bar, PcgOut* out, unsigned limit,
                                                             int* __restrict__ nq) {
+    note_clock(&out->t_setup);
     const int nqr = quads_of_row(g), q = blockIdx.x * SCAN_BLOCK + threadIdx.x;
     int s = 0;
     if (q < nqr * g.H * g.D) {
@@ -89,7 +90,8 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_fluid_tiles(const uint8_t* __res
         if (blockIdx.x == 0) {
             bar->count = 0;
             bar->limit = limit;
-            *status = DEV_OK;
+            bar->gave_up = &out->t_end;
+            out->status = DEV_OK;
             if (nq)
                 for (int l = 0; l < MG_MAX_LEVELS; ++l) nq[l] = 0;
         }
@@ -448,6 +450,7 @@ __global__ void __launch_bounds__(CSR_THREADS) k_csr_cg(CsrCgArgs a) {
 __global__ void k_csr_reset(CsrCtl* ctl, unsigned limit) {
     ctl->bar.count = 0;
     ctl->bar.limit = limit;
+    ctl->bar.gave_up = nullptr;
     ctl->status = DEV_OK;
     ctl->bad_off = ctl->bad_col = 0;
     ctl->iters = 0;
@@ -478,8 +481,7 @@ void launch_pressure_setup(const uint8_t* labels, const float* u, const float* v
         if (mg->L > 1) { qo.sy1 = mg->lv[1].sy; qo.sz1 = mg->lv[1].sz; }
     }
     int* nq = qo.q ? mg->nq : nullptr;
-    k_fluid_tiles<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, g, p, pb.tile_sums, stride, pb.bar, &pb.out->status,
-                                                 wait_polls, nq);
+    k_fluid_tiles<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, g, p, pb.tile_sums, stride, pb.bar, pb.out, wait_polls, nq);
     k_scan_rows<<<2, 1024, 0, st>>>(pb.tile_sums, ntiles, stride, pb.nf, nq);
     k_fluid_build<<<ntiles, SCAN_BLOCK, 0, st>>>(labels, u, v, w, g, scale, body, rhs_dense, pb.tile_sums, stride,
                                                  pb.fidx, pb.diag, pb.b, qo);

@@ -136,7 +136,6 @@ struct fp_solver {
     Dims g{};
     cudaStream_t st = nullptr;
     cudaEvent_t ev[10]{};
-    cudaEvent_t ev_pcg[2]{};
     int64_t launches = 0;   // kernels launched by this solver
     float pcg_ms = 0.0f;
     unsigned wait_polls = kDefaultWaitPolls;  // grid-barrier poll limit (fp_set_wait_limit)
@@ -163,7 +162,7 @@ struct fp_solver {
     std::string learned_path;
     float* d_rhs_dense = nullptr;  // dense right-hand side (network input, FP_GRID_RHS)
     float* d_x0c = nullptr;        // initial guess: compact (mixed) or dense (multigrid)
-    cudaEvent_t ev_net = nullptr;
+    cudaEvent_t ev_net[2]{};  // around the network
     // a PCG / MG solve whose read-back one_step has deferred (ev[9] marks it)
     bool solve_pending = false;
     bool timed = true;  // record timer events (mark)
@@ -424,9 +423,6 @@ void fill_body_stats(fp_solver* s) {
 void mark(fp_solver* s, cudaEvent_t ev) {
     if (s->timed) cudaEventRecord(ev, s->st);
 }
-void elapsed(fp_solver* s, float* ms, cudaEvent_t from, cudaEvent_t to) {
-    if (s->timed) cudaEventElapsedTime(ms, from, to);
-}
 
 // ---------------------------------------------------------------- phases
 void phase_label(fp_solver* s) {
@@ -473,6 +469,8 @@ float guess_of(const fp_solver* s) {
     return s->h_out->bb > 0 ? float(std::sqrt(s->h_out->rr0 / s->h_out->bb)) : 0.0f;
 }
 int outer_of(const fp_solver* s) { return mixed_solver(s) ? s->h_out->outer : 1; }
+// Device time of the solve kernel read back in h_out, in ms (also of one that gave up).
+float solve_ms(const fp_solver* s) { return float(double(s->h_out->t_end - s->h_out->t_begin) * 1e-6); }
 
 // Pressure solve of the system already set up in s->pb (fidx, diag, b); writes
 // the dense solution to p_out and the diagnostics to s->stats.
@@ -494,9 +492,9 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     const bool warm = s->cfg.solver == FP_SOLVER_PCG_MG && s->cfg.warm_start && p_out == s->d_p;
     if (learned && !s->net) return s->fail(FP_ERR_STATE, "learned solver: no weights loaded (fp_load_learned)");
     if (mg) s->launches += launch_mg_setup(s->d_labels, s->mg, s->st);
-    mark(s, s->ev_pcg[0]);
     const float* x0 = nullptr;
     if (learned) {
+        cudaEventRecord(s->ev_net[0], s->st);
         const unet::Lvl real{s->W, s->H, s->D};
         unet::launch_rhs_dense(pb.nf, pb.fidx, real, pb.b, s->d_rhs_dense, s->st);
         if (unet::forward_on(s->net, s->d_labels, s->d_rhs_dense, s->st))
@@ -508,7 +506,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             unet::launch_output_compact(pb.nf, pb.fidx, real, unet::net_level0(s->net), unet::net_out(s->net),
                                         unet::net_scal(s->net), s->d_x0c, s->st);
         s->launches += 1 + 16 + 1;  // rhs scatter, network (2 scale/input, 10 conv, 2 pool, 2 concat), guess
-        mark(s, s->ev_net);
+        cudaEventRecord(s->ev_net[1], s->st);
         x0 = s->d_x0c;
     }
     // A learned MG solve that has not converged after kLearnedMaxit iterations
@@ -524,7 +522,6 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     else
         e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
     s->launches += 1;
-    mark(s, s->ev_pcg[1]);
     if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
     cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);  // out, red and nf
     if (defer && !learned) {
@@ -537,9 +534,9 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
     cudaError_t ce = cudaStreamSynchronize(s->st);
     if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
     if (learned && *s->h_bad) return s->fail(FP_ERR_TIMEOUT, "U-Net forward: a bounded tensor-core wait gave up");
-    float pcg_ms = 0.0f, learned_ms = 0.0f;
-    elapsed(s, &pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
-    if (learned) elapsed(s, &learned_ms, s->ev_pcg[0], s->ev_net);
+    float learned_ms = 0.0f;
+    if (learned) cudaEventElapsedTime(&learned_ms, s->ev_net[0], s->ev_net[1]);
+    float pcg_ms = learned_ms + solve_ms(s);
     int iters = s->h_out->iters, outer = outer_of(s), dev_status = s->h_out->status, fallback = 0;
     const float guess = learned || warm ? guess_of(s) : 1.0f;
     if (learned) {
@@ -547,10 +544,8 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
         if (*s->h_nf > 0 && dev_status != DEV_TIMEOUT && (dev_status != DEV_OK || !(rel <= tol))) {
             // fallback: the plain FP64 PCG from x = 0
             fallback = 1;
-            mark(s, s->ev_pcg[0]);
             launch_reset_barrier(pb.bar, &pb.out->status, s->wait_polls, s->st);
             e = launch_pcg(s->g, pb, tol, maxit, p_out, s->st);
-            mark(s, s->ev_pcg[1]);
             if (e) return s->cuda_fail(cudaError_t(e), "cooperative PCG launch");
             s->launches += 2;
             cudaMemcpyAsync(s->h_out, pb.out, kRbBytes, cudaMemcpyDeviceToHost, s->st);
@@ -559,9 +554,7 @@ int solve_system(fp_solver* s, float* p_out, bool defer = false) {
             iters += s->h_out->iters;
             dev_status = s->h_out->status;
             ++outer;
-            float ms = 0.0f;
-            elapsed(s, &ms, s->ev_pcg[0], s->ev_pcg[1]);
-            pcg_ms += ms;
+            pcg_ms += solve_ms(s);
         }
     }
     return solve_tail(s, iters, outer, dev_status, pcg_ms, learned_ms, guess, fallback);
@@ -573,9 +566,7 @@ int solve_finalize(fp_solver* s) {
     s->solve_pending = false;
     const cudaError_t ce = cudaEventSynchronize(s->ev[9]);
     if (ce != cudaSuccess) return s->cuda_fail(ce, "pressure solve");
-    float pcg_ms = 0.0f;
-    elapsed(s, &pcg_ms, s->ev_pcg[0], s->ev_pcg[1]);
-    return solve_tail(s, s->h_out->iters, outer_of(s), s->h_out->status, pcg_ms, 0.0f,
+    return solve_tail(s, s->h_out->iters, outer_of(s), s->h_out->status, solve_ms(s), 0.0f,
                       s->pending_guess ? guess_of(s) : 1.0f, 0);
 }
 
@@ -1158,8 +1149,7 @@ int fp_create(const fp_config* cfg, fp_solver** out) {
     if (s->cfg.device >= 0) e = cudaSetDevice(s->cfg.device);  // the calling thread's device from here on
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
     for (auto& ev : s->ev) if (e == cudaSuccess) e = cudaEventCreate(&ev);
-    for (auto& ev : s->ev_pcg) if (e == cudaSuccess) e = cudaEventCreate(&ev);
-    if (e == cudaSuccess) e = cudaEventCreate(&s->ev_net);
+    for (auto& ev : s->ev_net) if (e == cudaSuccess) e = cudaEventCreate(&ev);
     if (e == cudaSuccess) {
         void* rb = nullptr;
         e = cudaMallocHost(&rb, kRbBytes);
@@ -1188,8 +1178,7 @@ int fp_destroy(fp_solver* s) {
     if (s->h_bforce) cudaFreeHost(s->h_bforce);
     if (s->h_r2) cudaFreeHost(s->h_r2);
     for (auto& ev : s->ev) if (ev) cudaEventDestroy(ev);
-    for (auto& ev : s->ev_pcg) if (ev) cudaEventDestroy(ev);
-    if (s->ev_net) cudaEventDestroy(s->ev_net);
+    for (auto& ev : s->ev_net) if (ev) cudaEventDestroy(ev);
     if (s->h_out) cudaFreeHost(s->h_out);  // h_red and h_nf lie inside it
     if (s->h_bad) cudaFreeHost(s->h_bad);
     if (s->d_bad) cudaFree(s->d_bad);

@@ -188,7 +188,8 @@ typedef struct fp_step_stats {
     double  body_pos[3], body_vel[3], body_omega[3], body_angles[3];
     double  body_force[3], body_torque[3];
     int64_t kernel_launches;   /* kernels this library launched, cumulative     */
-    float   t_pcg;             /* device time of the pressure solve, last step  */
+    float   t_pcg;             /* device time of the last pressure solve, also of
+                                  one that failed                               */
     float   t_learned;         /* of which the learned initial guess            */
     int64_t particles_removed; /* FP_SCHEME_REF2D: deleted by the last clean-up  */
     int32_t advect_capped;     /* FP_SCHEME_REF2D: particles whose substep loop

@@ -109,3 +109,27 @@ def test_timed_out_csr_solve_is_no_answer():
     assert (x == 7.0).all() and it.value == -3 and rr.value == -3.0
     assert call(1 << 27) == capi.FP_OK
     assert np.abs(x * vals - 1).max() <= 1e-12 and 0 < it.value <= 10 and 0 <= rr.value <= 1e-12
+
+
+@pytest.mark.parametrize("solver", ["pcg_mg", "pcg", "pcg_mixed", "pcg_learned", "pcg_learned_mixed"])
+def test_solve_times_of_a_call_that_fails_before_its_last_step(O, solver):
+    """t_pcg and t_learned are those of the last solve, also when it is the one that failed and the call's last step was
+    still to come.  A solve's time lies within its pressure phase."""
+    from fluidprjct_b200 import capi
+    from fluidprjct_b200.learned import DEFAULT_WEIGHTS
+    s = _pool_with_sphere(O, solver)[0]
+    learned = "learned" in solver
+    if learned:
+        s.load_learned(DEFAULT_WEIGHTS)
+    s.step(2)
+    st = s.stats()
+    assert 0 < st["t_pcg"] <= st["t_pressure"] and (0 < st["t_learned"] < st["t_pcg"] if learned else st["t_learned"] == 0)
+    s.set_wait_limit(1)
+    with pytest.raises(capi.FluidError) as e:
+        s.step(3)
+    assert e.value.code == capi.FP_ERR_TIMEOUT
+    st2 = s.stats()
+    # a solve that gives up at its first barriers takes less time than one that ends
+    assert 0 < st2["t_pcg"] - st2["t_learned"] < st["t_pcg"] - st["t_learned"]
+    assert st2["t_learned"] > 0 if learned else st2["t_learned"] == 0
+    s.close()
