@@ -134,8 +134,9 @@ void launch_scatter(const float4* pos, const float4* vel, const int* key, const 
                     float4* pos2, float4* vel2, cudaStream_t st);
 
 // In-place exclusive scan of n ints, the sum to *total; tile_sums has room for
-// scan_tiles(n) ints.  Returns the number of launches.
-int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st);
+// scan_tiles(n) ints; the start's device clock to *at if it is not null.
+// Returns the number of launches.
+int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st, unsigned long long* at = nullptr);
 int scan_tiles(int64_t n);
 
 // -------- P2G with the fused normalise / save / gravity epilogue (kernels_p2g.cu) --------
@@ -271,15 +272,19 @@ void launch_levelset_labels(const float* solid, const float* fluid, int64_t n, u
 // substep loops), tiles (launch_scan over the bins or the keep flags).
 struct R2Scratch {
     int *start, *list, *key, *rank, *keep, *misc, *tiles;
+    unsigned long long* clock;  // [R2_CLOCKS] device clock at the start of the phases' first kernels
 };
+enum { R2_AT_LABEL, R2_AT_P2G, R2_AT_PROJECT, R2_AT_PARTICLES, R2_AT_END, R2_CLOCKS };
+// Without particles the kernels that note P2G, particles and the end do not run.
+void launch_r2_note(R2Scratch& sc, int which, cudaStream_t st);
 void launch_r2_label(const uint8_t* base, uint8_t* labels, const float4* pos, int64_t np, Dims g, float dx,
-                     cudaStream_t st);
+                     R2Scratch& sc, cudaStream_t st);
 // mode 0: u, v = P2G; mode 1: u*, v* = P2G and u, v = P2G + gravity.  Returns the number of launches.
 int launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, float dx, float dt, int mode,
                    R2Scratch& sc, float* u, float* v, float* us, float* vs, cudaStream_t st);
 void launch_r2_forces(float* u, float* v, Dims g, float dt, cudaStream_t st);
 void launch_r2_project(float* u, float* v, const float* p, const uint8_t* labels, Dims g, float dx, float dt,
-                       cudaStream_t st);
+                       R2Scratch& sc, cudaStream_t st);
 // flags: 1 G2P, 2 advection, 4 clean-up (sets sc.keep)
 void launch_r2_particles(float4* pos, float4* vel, int64_t np, const float* u, const float* v, const float* us,
                          const float* vs, const uint8_t* labels, Dims g, float dx, float dt, float alpha, int flags,

@@ -50,7 +50,9 @@ __device__ __forceinline__ int host_trunc(float t) {
     return __float2int_rz(t);
 }
 
-__global__ void k_r2_label_reset(const uint8_t* __restrict__ base, uint8_t* __restrict__ lab, int64_t n) {
+__global__ void k_r2_label_reset(const uint8_t* __restrict__ base, uint8_t* __restrict__ lab, int64_t n,
+                                 unsigned long long* at) {
+    note_clock(at);
     for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n; c += int64_t(gridDim.x) * blockDim.x)
         lab[c] = base[c] == L_SOLID ? L_SOLID : L_AIR;
 }
@@ -77,7 +79,8 @@ __device__ __forceinline__ int r2_bin(float q, float dx, int n) {
 
 __global__ void k_r2_bin_count(const float4* __restrict__ pos, const float4* __restrict__ vel, int64_t np, float dx,
                                int W, int H, int* __restrict__ counts, int* __restrict__ key, int* __restrict__ rank,
-                               int* __restrict__ nonfinite) {
+                               int* __restrict__ nonfinite, unsigned long long* at) {
+    note_clock(at);
     const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= np) return;
     const float4 p = pos[q], v = vel[q];
@@ -201,7 +204,8 @@ __global__ void k_r2_forces(float* __restrict__ u, float* __restrict__ v, int W,
 }
 
 __global__ void k_r2_project(float* __restrict__ u, float* __restrict__ v, const float* __restrict__ p,
-                             const uint8_t* __restrict__ lab, int W, int H, float scale) {
+                             const uint8_t* __restrict__ lab, int W, int H, float scale, unsigned long long* at) {
+    note_clock(at);
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= int64_t(W) * H) return;
     const int i = int(t % W), j = int(t / W);
@@ -289,7 +293,8 @@ __device__ bool r2_project_particle(const R2Grid& g, float& x, float& y) {
 // particle; they read only grids and labels, so one thread runs all three.
 // keep[q] = 1 unless the clean-up deletes the particle.
 __global__ void k_r2_particles(float4* __restrict__ pos, float4* __restrict__ vel, int64_t np, R2Grid g, int flags,
-                               int* __restrict__ keep, int* __restrict__ capped) {
+                               int* __restrict__ keep, int* __restrict__ capped, unsigned long long* at) {
+    note_clock(at);
     const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= np) return;
     float4 P = pos[q], V = vel[q];
@@ -359,14 +364,18 @@ __global__ void k_r2_compact(const float4* __restrict__ pos, const float4* __res
     vel2[d] = vel[q];
 }
 
+__global__ void k_r2_note(unsigned long long* at) { note_clock(at); }
+
 unsigned blocks_for(int64_t n, int t = 256) { return unsigned((n + t - 1) / t); }
 
 }  // namespace
 
+void launch_r2_note(R2Scratch& sc, int which, cudaStream_t st) { k_r2_note<<<1, 1, 0, st>>>(sc.clock + which); }
+
 void launch_r2_label(const uint8_t* base, uint8_t* labels, const float4* pos, int64_t np, Dims g, float dx,
-                     cudaStream_t st) {
+                     R2Scratch& sc, cudaStream_t st) {
     const int64_t nc = int64_t(g.W) * g.H;
-    k_r2_label_reset<<<blocks_for(nc), 256, 0, st>>>(base, labels, nc);
+    k_r2_label_reset<<<blocks_for(nc), 256, 0, st>>>(base, labels, nc, sc.clock + R2_AT_LABEL);
     if (np > 0) k_r2_label_mark<<<blocks_for(np), 256, 0, st>>>(pos, np, dx, g.W, g.H, labels);
 }
 
@@ -376,7 +385,7 @@ int launch_r2_p2g(const float4* pos, const float4* vel, int64_t np, Dims g, floa
     cudaMemsetAsync(sc.start, 0, sizeof(int) * (nb + 1), st);
     cudaMemsetAsync(sc.misc, 0, sizeof(int) * 2, st);
     if (np > 0) k_r2_bin_count<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, dx, g.W, g.H, sc.start, sc.key, sc.rank,
-                                                                sc.misc);
+                                                                sc.misc, sc.clock + R2_AT_P2G);
     const int scans = launch_scan(sc.start, nb, sc.start + nb, sc.tiles, st);
     if (np > 0) k_r2_bin_place<<<blocks_for(np), 256, 0, st>>>(sc.key, sc.rank, sc.start, np, sc.list);
     k_r2_bin_order<<<blocks_for(nb), 256, 0, st>>>(sc.start, nb, sc.list);
@@ -391,9 +400,10 @@ void launch_r2_forces(float* u, float* v, Dims g, float dt, cudaStream_t st) {
 }
 
 void launch_r2_project(float* u, float* v, const float* p, const uint8_t* labels, Dims g, float dx, float dt,
-                       cudaStream_t st) {
+                       R2Scratch& sc, cudaStream_t st) {
     const float scale = dt / (1000.0f * dx);  // host float arithmetic, as applyPressure :721
-    k_r2_project<<<blocks_for(int64_t(g.W) * g.H), 256, 0, st>>>(u, v, p, labels, g.W, g.H, scale);
+    k_r2_project<<<blocks_for(int64_t(g.W) * g.H), 256, 0, st>>>(u, v, p, labels, g.W, g.H, scale,
+                                                                   sc.clock + R2_AT_PROJECT);
 }
 
 void launch_r2_particles(float4* pos, float4* vel, int64_t np, const float* u, const float* v, const float* us,
@@ -402,12 +412,13 @@ void launch_r2_particles(float4* pos, float4* vel, int64_t np, const float* u, c
     if (np == 0) return;
     R2Grid a{u, v, us, vs, labels, g.W, g.H, dx, dt, alpha};
     if (flags & 2) cudaMemsetAsync(sc.misc + 2, 0, sizeof(int), st);
-    k_r2_particles<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, a, flags, sc.keep, sc.misc + 2);
+    k_r2_particles<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, a, flags, sc.keep, sc.misc + 2,
+                                                   flags & 1 ? sc.clock + R2_AT_PARTICLES : nullptr);
 }
 
 int launch_r2_compact(const float4* pos, const float4* vel, int64_t np, R2Scratch& sc, float4* pos2, float4* vel2,
                        cudaStream_t st) {
-    const int scans = launch_scan(sc.keep, int(np), sc.keep + np, sc.tiles, st);
+    const int scans = launch_scan(sc.keep, int(np), sc.keep + np, sc.tiles, st, sc.clock + R2_AT_END);
     if (np > 0) k_r2_compact<<<blocks_for(np), 256, 0, st>>>(pos, vel, np, sc.keep, pos2, vel2);
     return scans + (np > 0);
 }

@@ -185,14 +185,18 @@ __device__ __forceinline__ void scan_block(int* data, int n, int* total) {
 }
 }  // namespace
 
-__global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, int* total) { scan_block(data, n, total); }
+__global__ void __launch_bounds__(1024) k_scan_single_block(int* data, int n, int* total, unsigned long long* at) {
+    note_clock(at);
+    scan_block(data, n, total);
+}
 __global__ void __launch_bounds__(1024) k_scan_rows(int* data, int n, int stride, int* total0, int* total1) {
     scan_block(data + blockIdx.x * stride, n, blockIdx.x ? total1 : total0);
 }
 
 // The tile sums of data, and the scan of each tile from its offset.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tile_sums(const int* __restrict__ data, int n,
-                                                               int* __restrict__ tile_sums) {
+                                                               int* __restrict__ tile_sums, unsigned long long* at) {
+    note_clock(at);
     const int e0 = (blockIdx.x * SCAN_BLOCK + threadIdx.x) * SCAN_ITEMS;
     int s = 0;
 #pragma unroll
@@ -222,14 +226,14 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(int* __restrict__ dat
 
 int scan_tiles(int64_t n) { return int((n + SCAN_TILE - 1) / SCAN_TILE); }
 
-int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st) {
+int launch_scan(int* data, int n, int* total, int* tile_sums, cudaStream_t st, unsigned long long* at) {
     // One pass of a single block, or the whole chip's three launches.
     if (n <= 1024 * 16) {
-        k_scan_single_block<<<1, 1024, 0, st>>>(data, n, total);
+        k_scan_single_block<<<1, 1024, 0, st>>>(data, n, total, at);
         return 1;
     }
     const int tiles = scan_tiles(n);
-    k_scan_tile_sums<<<tiles, SCAN_BLOCK, 0, st>>>(data, n, tile_sums);
+    k_scan_tile_sums<<<tiles, SCAN_BLOCK, 0, st>>>(data, n, tile_sums, at);
     k_scan_single_block<<<1, 1024, 0, st>>>(tile_sums, tiles, total);
     k_scan_tiles<<<tiles, SCAN_BLOCK, 0, st>>>(data, n, tile_sums);
     return 3;

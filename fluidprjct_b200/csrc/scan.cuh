@@ -39,8 +39,9 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int& total) {
 }
 
 // In-place exclusive scan of n ints (16-byte aligned) by one block of 1024
-// threads; the grand total is written to *total (if non-null).
-__global__ void k_scan_single_block(int* data, int n, int* total);
+// threads; the grand total is written to *total and the start's device clock to
+// *at (each if non-null).
+__global__ void k_scan_single_block(int* data, int n, int* total, unsigned long long* at = nullptr);
 // The same of two rows, data and data + stride (a multiple of 4), by two blocks.
 __global__ void k_scan_rows(int* data, int n, int stride, int* total0, int* total1);
 

@@ -177,7 +177,8 @@ struct fp_solver {
     R2Scratch r2{};
     int r2_nb = 0, r2_tiles = 0;
     int64_t r2_cap = 0;
-    int* h_r2 = nullptr;    // pinned: [0] particles kept, [1] capped substep loops
+    // pinned: [0] particles kept, [2] capped substep loops, from [4] the phases' clocks (as from misc + 2 on)
+    int* h_r2 = nullptr;
     int* d_extmark = nullptr;  // wavefront markers of the velocity extrapolation (largest face grid)
     // body
     BodyKin body{};
@@ -769,7 +770,8 @@ int r2_alloc(fp_solver* s) {
     if (s->r2_nb != nb) {
         free_r2(s);
         e = dalloc(&s->r2.start, size_t(nb) + 1);
-        if (e == cudaSuccess) e = dalloc(&s->r2.misc, size_t(4));
+        if (e == cudaSuccess) e = dalloc(&s->r2.misc, size_t(4 + 2 * R2_CLOCKS));
+        if (e == cudaSuccess) s->r2.clock = reinterpret_cast<unsigned long long*>(s->r2.misc + 4);
         if (e != cudaSuccess) { free_r2(s); return s->cuda_fail(e, "device allocation of the 2D bins"); }
         s->r2_nb = nb;
     }
@@ -795,7 +797,7 @@ int r2_alloc(fp_solver* s) {
 }
 
 void r2_label(fp_solver* s) {
-    launch_r2_label(s->d_base, s->d_labels, s->d_pos, s->np, s->g, s->cfg.dx, s->st);
+    launch_r2_label(s->d_base, s->d_labels, s->d_pos, s->np, s->g, s->cfg.dx, s->r2, s->st);
     s->launches += s->np > 0 ? 2 : 1;
 }
 
@@ -811,7 +813,7 @@ int r2_pressure(fp_solver* s) {
 }
 
 void r2_project(fp_solver* s) {
-    launch_r2_project(s->d_u, s->d_v, s->d_p, s->d_labels, s->g, s->cfg.dx, s->cfg.dt, s->st);
+    launch_r2_project(s->d_u, s->d_v, s->d_p, s->d_labels, s->g, s->cfg.dx, s->cfg.dt, s->r2, s->st);
     s->launches += 1;
 }
 
@@ -822,19 +824,27 @@ void r2_particles(fp_solver* s, int flags) {
     s->launches += 1;
 }
 
+void r2_note(fp_solver* s, int which) {
+    launch_r2_note(s->r2, which, s->st);
+    s->launches += 1;
+}
+void r2_read_misc(fp_solver* s) {
+    cudaMemcpyAsync(s->h_r2 + 2, s->r2.misc + 2, sizeof(int) * (2 + 2 * R2_CLOCKS), cudaMemcpyDeviceToHost, s->st);
+}
+
 // After r2_particles with the clean-up flag: drop deleted particles (order
 // kept), read the new count and the capped-loop count.
 int r2_compact(fp_solver* s, bool advected) {
     if (s->np == 0) return FP_OK;
     s->launches += launch_r2_compact(s->d_pos, s->d_vel, s->np, s->r2, s->d_pos2, s->d_vel2, s->st);
     cudaMemcpyAsync(s->h_r2, s->r2.keep + s->np, sizeof(int), cudaMemcpyDeviceToHost, s->st);
-    if (advected) cudaMemcpyAsync(s->h_r2 + 1, s->r2.misc + 2, sizeof(int), cudaMemcpyDeviceToHost, s->st);
+    if (advected) r2_read_misc(s);
     cudaError_t e = cudaStreamSynchronize(s->st);
     if (e != cudaSuccess) return s->cuda_fail(e, "2D particle clean-up");
     std::swap(s->d_pos, s->d_pos2);
     std::swap(s->d_vel, s->d_vel2);
     s->stats.particles_removed = s->np - s->h_r2[0];
-    if (advected) s->stats.advect_capped = s->h_r2[1];
+    if (advected) s->stats.advect_capped = s->h_r2[2];
     s->np = s->h_r2[0];
     return FP_OK;
 }
@@ -843,9 +853,8 @@ int r2_compact(fp_solver* s, bool advected) {
 int one_step_ref2d(fp_solver* s) {
     int rc = r2_alloc(s);
     if (rc) return rc;
-    mark(s, s->ev[0]);
     r2_label(s);
-    mark(s, s->ev[1]);
+    if (s->np == 0) r2_note(s, R2_AT_P2G);
     const bool ext = s->cfg.extrapolate != 0;
     if (ext) {  // P2G, extrapolation, save, forces
         r2_p2g(s, 0);
@@ -857,12 +866,9 @@ int one_step_ref2d(fp_solver* s) {
     } else {
         r2_p2g(s, 1);  // P2G + save + forces
     }
-    mark(s, s->ev[2]);
     rc = r2_pressure(s);
-    mark(s, s->ev[3]);
     if (rc != FP_OK) return rc;
     r2_project(s);
-    mark(s, s->ev[4]);
     if (ext) {  // G2P, extrapolation, then advection and clean-up
         r2_particles(s, 1);
         rc = r2_extrapolate(s, true);
@@ -871,25 +877,31 @@ int one_step_ref2d(fp_solver* s) {
     } else {
         r2_particles(s, 7);  // G2P, advection, clean-up
     }
-    mark(s, s->ev[5]);
+    if (s->np == 0) {
+        r2_note(s, R2_AT_PARTICLES);
+        r2_note(s, R2_AT_END);
+        r2_read_misc(s);
+        const cudaError_t e = cudaStreamSynchronize(s->st);
+        if (e != cudaSuccess) return s->cuda_fail(e, "2D step");
+    }
     rc = r2_compact(s, true);
     if (rc != FP_OK) return rc;
     ++s->steps;
     s->stats.step = s->steps;
     s->stats.num_particles = s->np;
     s->stats.kernel_launches = s->launches;
-    if (!s->timed) return FP_OK;
-    float t[5];
-    for (int i = 0; i < 5; ++i) cudaEventElapsedTime(&t[i], s->ev[i], s->ev[i + 1]);
-    s->stats.t_label = t[0];
-    s->stats.t_p2g = t[1];
+    // the phase timers, of every step (a later one of the call may fail)
+    const auto* at = reinterpret_cast<const unsigned long long*>(s->h_r2 + 4);
+    auto ms = [](unsigned long long from, unsigned long long to) { return float(double(int64_t(to - from)) * 1e-6); };
+    s->stats.t_label = ms(at[R2_AT_LABEL], at[R2_AT_P2G]);
+    s->stats.t_p2g = ms(at[R2_AT_P2G], s->h_out->t_setup);
     s->stats.t_forces = 0.0f;
-    s->stats.t_pressure = t[2];
-    s->stats.t_project = t[3];
+    s->stats.t_pressure = ms(s->h_out->t_setup, at[R2_AT_PROJECT]);
+    s->stats.t_project = ms(at[R2_AT_PROJECT], at[R2_AT_PARTICLES]);
     s->stats.t_body = 0.0f;
     s->stats.t_g2p = 0.0f;
-    s->stats.t_advect = t[4];
-    cudaEventElapsedTime(&s->stats.t_total, s->ev[0], s->ev[5]);
+    s->stats.t_advect = ms(at[R2_AT_PARTICLES], at[R2_AT_END]);
+    s->stats.t_total = ms(at[R2_AT_LABEL], at[R2_AT_END]);
     return FP_OK;
 }
 
@@ -1158,7 +1170,7 @@ int fp_create(const fp_config* cfg, fp_solver** out) {
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_bad, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&s->d_bad, sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_bforce, sizeof(double) * 8);
-    if (e == cudaSuccess) e = cudaMallocHost(&s->h_r2, sizeof(int) * 2);
+    if (e == cudaSuccess) e = cudaMallocHost(&s->h_r2, sizeof(int) * (4 + 2 * R2_CLOCKS));
     if (e != cudaSuccess) {
         std::fprintf(stderr, "fp_create: %s\n", cudaGetErrorString(e));
         fp_destroy(s);
@@ -1601,14 +1613,14 @@ int fp_run_phase(fp_solver* s, int phase) {
                     if (rc) return rc;
                 }
                 r2_particles(s, 2);
-                if (s->np) cudaMemcpyAsync(s->h_r2 + 1, s->r2.misc + 2, sizeof(int), cudaMemcpyDeviceToHost, s->st);
+                if (s->np) r2_read_misc(s);
                 break;
             case FP_PHASE_CLEANUP: r2_particles(s, 4); rc = r2_compact(s, false); break;
             default: return s->fail(FP_ERR_ARG, "unknown phase");
         }
         cudaError_t e = cudaStreamSynchronize(s->st);
         if (e != cudaSuccess) return s->cuda_fail(e, "phase");
-        if (phase == FP_PHASE_ADVECT && s->np) s->stats.advect_capped = s->h_r2[1];
+        if (phase == FP_PHASE_ADVECT && s->np) s->stats.advect_capped = s->h_r2[2];
         return rc;
     }
     switch (phase) {

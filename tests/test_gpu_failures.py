@@ -133,3 +133,39 @@ def test_solve_times_of_a_call_that_fails_before_its_last_step(O, solver):
     assert 0 < st2["t_pcg"] - st2["t_learned"] < st["t_pcg"] - st["t_learned"]
     assert st2["t_learned"] > 0 if learned else st2["t_learned"] == 0
     s.close()
+
+
+def test_ref2d_timers_of_a_call_that_fails_in_its_second_step():
+    """The 2D scheme's phase timers are those of the last step that ended, also when a later step of the call fails.  A
+    block of water falls freely (no divergence, nothing to solve) and reaches the floor in its second step; the grid
+    spacing is so large that the right-hand side there is about 2e38 and the FP32 V-cycle overflows."""
+    from fluidprjct_b200 import capi
+    n, dx = 20, 1e34
+    dt = float(np.sqrt(0.6 * dx / 9.81))  # a fall of 0.6 cells in the first step
+    lab = np.full((n, n), capi.AIR, np.uint8)
+    lab[0], lab[-1], lab[:, 0], lab[:, -1] = [capi.SOLID] * 4
+    s = capi.Solver(dim=2, dx=dx, dt=dt, pic_weight=0.05, solver="pcg_mg", scheme="ref2d", output_format=capi.OUT_NONE)
+    s.set_labels(lab)
+    j, i = np.meshgrid(np.arange(2, 10), np.arange(4, 16), indexing="ij")
+    pos = np.stack([(i.ravel() + 0.5) * dx, (j.ravel() + 0.5) * dx, 0.0 * i.ravel()], 1).astype(np.float32)
+    names = ("t_label", "t_p2g", "t_pressure", "t_project", "t_advect", "t_total")
+
+    def timers():
+        st = s.stats()
+        assert all(st[k] > 0 for k in names)
+        assert abs(sum(st[k] for k in names[:-1]) - st["t_total"]) <= 1e-5 * st["t_total"]
+        return [st[k] for k in names]
+
+    s.set_particles(pos)
+    s.step(1)
+    first = timers()
+    s.set_particles(pos)
+    with pytest.raises(capi.FluidError) as e:
+        s.step(3)
+    assert e.value.code == capi.FP_ERR_SOLVER and s.stats()["step"] == 2
+    assert timers() != first
+    # no particles: no phase is left out
+    s.set_particles(np.zeros((0, 3), np.float32))
+    s.step(2)
+    assert s.stats()["step"] == 4 and timers() != first
+    s.close()
