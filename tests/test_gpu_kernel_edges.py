@@ -469,3 +469,149 @@ def test_p2g_brick_edges_at_any_spacing(shape, dx):
         assert np.abs(got[heavy] - num[heavy] / den[heavy]).max() <= 1.2e-4
         assert not got[den == 0].any()
     s.close()
+
+
+def _mg_residual(lab, seed, solves=2):
+    """Solves by pcg_mg to 1e-9 with random right-hand sides and the bound of test_mg_quad_rows."""
+    import torch
+    from fluidprjct_b200 import capi
+    D, H, W = lab.shape
+    rng = np.random.default_rng(seed)
+    t = torch.nn.functional.pad(torch.from_numpy(lab).cuda().int(), (1, 1, 1, 1, 1, 1))
+    fl = (t == 1).double()
+    wet = ((t == 1) | (t == 2)).double()
+    diag = sum(torch.roll(wet, o, d) for d in range(3) for o in (1, -1)) * fl
+    s = capi.Solver(dim=3 if D > 1 else 2, dx=1.0 / 64, dt=0.01, solver="pcg_mg", tol=1e-9, output_format=capi.OUT_NONE)
+    s.set_labels(lab if D > 1 else lab[0])
+    for _ in range(solves):  # the second solve finds the work grids as the first left them
+        rhs = (rng.standard_normal(lab.shape) * (lab == 1)).astype(np.float32)
+        x, it, rr, rc = s.pressure_solve(rhs)
+        b = torch.nn.functional.pad(torch.from_numpy(rhs).cuda().double(), (1, 1, 1, 1, 1, 1))
+        y = torch.nn.functional.pad(torch.from_numpy(x).cuda().double(), (1, 1, 1, 1, 1, 1))
+        res = b - (diag * y - sum(torch.roll(y, o, d) for d in range(3) for o in (1, -1)) * fl)
+        assert rc == 0 and it > 0 and not x[lab != 1].any()
+        assert float(res.norm()) <= 2e-9 * float(b.norm()) + 12 * 2.0 ** -24 * float(y.norm())
+    s.close()
+
+
+# grids that no coarser one follows: level 0 is the whole hierarchy, swept by one block in global memory
+@pytest.mark.parametrize("shape", [(2, 2, 2), (2, 1, 2), (2, 2, 1), (1, 2, 1)])
+@pytest.mark.parametrize("air", [0, 1, -1])
+def test_mg_one_level(shape, air):
+    """A hierarchy of one level, all FLUID but one AIR cell (a red or a black one)."""
+    lab = np.full(shape[::-1], 1, np.uint8)
+    lab.flat[air] = 2
+    _mg_residual(lab, 3)
+
+
+# 938 and 1016 cells are left on the last of eight levels, in rows of one cell, which with their padding do not fit
+@pytest.mark.parametrize("shape", [(3, 120000, 1), (4, 130000, 1), (2, 3, 120000)])
+def test_mg_block_level_in_global_memory(shape):
+    """Grids so long that not even the last level's copy fits in shared memory: block 0 solves it in global memory."""
+    _mg_residual(_ragged(shape[::-1], shape[0]), 5)
+
+
+def _face_terms(lab, p, dx, phi, com):
+    """The face-fraction force's terms over every face of the grid, in FP64: (6, n) force and torque contributions, and
+    each face's largest one (theta = 1).  phi gives the SDF at FP32 points and where it is in doubt."""
+    P, L = np.pad(p.astype(np.float64), 1), np.pad(lab, 1)
+    fa = (L == 1) | (L == 2)
+    s, n = np.zeros_like(P), np.zeros_like(P)
+    for d in range(3):
+        for o in (1, -1):
+            s += np.roll(np.where(fa, P, 0.0), o, d)
+            n += np.roll(fa.astype(float), o, d)
+    ext = np.where(L == 3, np.divide(s, n, out=np.zeros_like(s), where=n > 0), P)
+    terms, doubt = [], []
+    for a in range(3):
+        c = [np.arange(m + (b == a), dtype=np.float32) for b, m in enumerate(lab.shape[::-1])]
+        X = np.stack(np.meshgrid(*[(v if a == b else v + np.float32(0.5)) * np.float32(dx) for b, v in enumerate(c)],
+                                 indexing="ij")).astype(np.float32).reshape(3, -1)
+        i = np.stack(np.meshgrid(*[np.arange(len(v)) for v in c], indexing="ij")).reshape(3, -1)
+        hi = tuple(i[2 - b] + 1 for b in range(3))
+        lo = tuple(i[2 - b] + (2 - b != a) for b in range(3))
+        f, unsure = phi(X)
+        full = np.where((L[lo] != 0) & (L[hi] != 0), -(ext[hi] - ext[lo]) * dx * dx, 0.0)
+        r = X.astype(np.float64) - np.asarray(com, np.float64)[:, None]
+
+        def wrench(dF):
+            F = np.zeros_like(r)
+            F[a] = dF
+            return np.concatenate([F, np.cross(r, F, axis=0)])
+        terms.append(wrench(np.clip(0.5 - f / dx, 0, 1) * full))
+        doubt.append(wrench(np.where(unsure, full, 0.0)))
+    return np.concatenate(terms, 1), np.concatenate(doubt, 1)
+
+
+# spheres inside, over a corner, outside and around the grid; paddles inside and past both ends; a voxel SDF turned about
+# all axes: inside, over a corner, wholly outside
+@pytest.mark.parametrize("body", [("s", (0.5, 0.4, 0.5), 0.2), ("s", (0.02, 0.05, 0.9), 0.15), ("s", (2.0, 0.4, 0.5), 0.3),
+                                  ("s", (0.5, 0.4, 0.5), 3.0), ("p", 0.31, 0), ("p", -0.4, 0), ("p", 1.7, 0),
+                                  ("v", (0.55, 0.5, 0.45), 0), ("v", (0.05, 0.1, 0.8), 0), ("v", (-3.0, 0.5, 0.5), 0)])
+def test_body_force_of_every_face_in_the_box(body, tmp_path):
+    """The force and torque of the body's box against all faces of the grid, to 1e-5 of the sum of the terms' magnitudes
+    (FP32 theta: the rounding of phi / dx, about n 2^-24 for the n faces across).  A face at a voxel's side, where FP32
+    may read the next voxel, may count as any theta from 0 to 1."""
+    from fluidprjct_b200 import capi, scenes
+    n, dx = 24, np.float32(1 / 24)
+    lab = scenes.box_3d(n, n + 5, n - 3, float(dx), 2.0, 0.8, 2.0)
+    kw = dict(dx=float(dx), dt=0.5, solver="pcg_mg", output_format=capi.OUT_NONE, active_body=1, body_mass=1e-3)
+    if body[0] == "s":
+        kw.update(body_radius=body[2], body_pos=body[1], body_density=0.0)
+    elif body[0] == "v":
+        kw.update(body_pos=body[1])
+    s = capi.Solver(**kw)
+    s.set_labels(lab)
+    com = np.float32(body[1]) if body[0] != "p" else None
+    weight = 1e-3
+    if body[0] == "s":
+        s.load_sdf(None)
+        phi = lambda X: (np.sqrt(((X - com[:, None]) ** 2).sum(0)) - np.float32(body[2]), False)
+    elif body[0] == "p":
+        s.set_paddle(body[1], 0.0, 1.0)
+        com = np.float32([body[1], np.float32(0.5 * (n + 5) * float(dx)), np.float32(0.5 * (n - 3) * float(dx))])
+        phi = lambda X: (X[0] - com[0], False)
+        weight = 0.0
+    else:
+        nv, org, cell = np.array([17, 11, 23]), np.float32([-0.1, 0.2, 0.05]), np.float32(0.03)
+        val = np.random.default_rng(8).uniform(-1.0, 0.4, nv).astype(np.float32) * dx
+        with open(tmp_path / "body.sdf", "w") as f:
+            f.write(" ".join(map(str, nv)) + "\n" + " ".join("%.9g" % v for v in [*org, cell]) + "\n")
+            f.write("\n".join("%.9g" % v for v in val.transpose(2, 1, 0).ravel()))
+        s.load_sdf(tmp_path / "body.sdf")
+        s.set_body_state(omega=(0.8, 1.1, -0.7))  # turned by the first integration, in the rotation from the second on
+        for _ in range(2):
+            s.phase(capi.PHASE_BODY)
+            s.set_body_state(pos=body[1], vel=(0, 0, 0), omega=(0, 0, 0))
+        th, ps, ph = s.stats()["body_angles"]
+        ct, st, cp, sp, cf, sf = np.cos(th), np.sin(th), np.cos(ps), np.sin(ps), np.cos(ph), np.sin(ph)
+        R = np.array([[ct * cp, st * sf - ct * cf * sp, cf * st + ct * sf * sp], [sp, cf * cp, -cp * sf],
+                      [-cp * st, ct * sf + cf * st * sp, ct * cf - st * sf * sp]]).astype(np.float32)
+        assert np.abs(R - np.eye(3)).max() > 0.3
+        lc = org + (nv * cell).astype(np.float32) * np.float32(0.5)
+
+        def phi(X):
+            d = (X - com[:, None]).astype(np.float64)
+            q = (R.astype(np.float64).T @ d + lc[:, None] - org[:, None]) / cell
+            unsure = (np.abs(q - np.round(q)) < 2e-4).any(0) & ((q > -1) & (q < nv[:, None] + 1)).all(0)
+            i = np.floor(q).astype(int)
+            ins = ((i >= 0) & (i < nv[:, None])).all(0)
+            i = np.where(ins, i, 0)
+            return np.where(ins, val[tuple(i)], np.float32(1e30)), unsure
+        s.phase(capi.PHASE_LABEL)
+    lab = s.labels()
+    p = np.random.default_rng(5).standard_normal(lab.shape).astype(np.float32)
+    s.set_grid(capi.GRID_P, p)
+    s.phase(capi.PHASE_BODY)
+    st = s.stats()
+    got = np.array(list(st["body_force"]) + list(st["body_torque"]))
+    got[1] += float(np.float32(weight)) * float(np.float32(9.81))
+    terms, doubt = _face_terms(lab, p, float(dx), phi, com)
+    tol = 1e-5 * np.abs(terms).sum(1) + 1e-12
+    assert (np.abs(got - terms.sum(1)) <= tol + np.abs(doubt).sum(1)).all(), (got, terms.sum(1), tol)
+    # the bound sees a face: most of the body's carry more than it
+    if np.abs(terms).sum() > 0:
+        assert (np.median(np.abs(terms[:3][terms[:3] != 0])) > tol[:3]).all()
+    else:
+        assert not got[3:].any()
+    s.close()
