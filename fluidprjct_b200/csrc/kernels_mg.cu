@@ -110,7 +110,7 @@ struct MgArgs {
     int nu_grid;                 // ... on the other grid-wide levels
     int nu_block;                // ... on the block levels above the coarsest
     MgLevel lv[MG_MAX_LEVELS];
-    const int4* q[MG_MAX_LEVELS];  // quad lists of levels [0, max(G, 1)): MgQuad entries
+    const int4* q[MG_MAX_LEVELS];  // quad lists of levels [0, max(G, 1)) (QUAD_* entries)
     const int* nq;               // their lengths
     const float4* rhs;           // right-hand side by level-0 quad (zero off the fluid)
     // FP64 Krylov vectors by quad: the first two cells of quad n at [n], the last two at [cap + n]
@@ -370,7 +370,7 @@ __device__ void op_restrict_first(const MgLevel& F, const MgLevel& Cl, float sca
         Cl.x[cc] = xv;
     }
 }
-// prolong_quads' operation on one cell, and over every FLUID cell of F.
+// prolong_quad's operation on one cell, and over every FLUID cell of F.
 __device__ __forceinline__ void prolong_one(const MgLevel& F, int c, const MgLevel& Cl, float omega, int i, int j,
                                             int k) {
     const int I = i >> 1, J = j >> 1, K = k >> 1;

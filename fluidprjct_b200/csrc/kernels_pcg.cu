@@ -150,7 +150,7 @@ __device__ bool cg_one(const PcgArgs& a, Share& h, const float* rhs, double tol,
     const int n = h.n0 + int(threadIdx.x);
     // an idle thread reads around interior cell (0,0,0): in bounds, its result dropped
     const int c = ok ? a.fidx[n] : 1 + a.sy + a.sz;
-    const int dg = ok ? a.diag[n] & 0x7F : 0;
+    const int dg = ok ? a.diag[n] : 0;
     const int offs[6] = {1, -1, a.sy, -a.sy, a.sz, -a.sz};
     T* const R0 = static_cast<T*>(a.R[0]);
     T* const invd = static_cast<T*>(a.invd);
@@ -244,7 +244,7 @@ __device__ bool cg_many(const PcgArgs& a, Share& h, const float* rhs, double tol
     const int sy = a.sy, sz = a.sz;
     for (int l = tid; l < h.m; l += PCG_THREADS) {
         const int c = G.c[l];
-        const uint8_t d = G.d[l] & 0x7F;
+        const uint8_t d = G.d[l];
         const T r = T(rhs[h.n0 + l]);
         const Own<T>& o = l < ms ? S : G;
         if (l < ms) { S.c[l] = c; S.d[l] = d; }
@@ -264,7 +264,7 @@ __device__ bool cg_many(const PcgArgs& a, Share& h, const float* rhs, double tol
                 const int l = min(base + q * PCG_THREADS, l1 - 1);
                 const T* up = U + o.c[l];
                 r[q] = o.r[l];
-                d[q] = o.d[l] & 0x7F;
+                d[q] = o.d[l];
                 nbs[q] = up[1];
                 nbs[q] += up[-1];
                 nbs[q] += up[sy];
@@ -286,7 +286,7 @@ __device__ bool cg_many(const PcgArgs& a, Share& h, const float* rhs, double tol
     };
     auto update = [&](const Own<T>& o, int l0, int l1, T al, T be) {
         for (int l = l0 + tid; l < l1; l += PCG_THREADS) {
-            const T inv = inv_of(o.d[l] & 0x7F, T(0)), r = o.r[l];
+            const T inv = inv_of(o.d[l], T(0)), r = o.r[l];
             const T s = fmaT(be, o.s[l], o.w[l]);
             const T p = fmaT(be, o.p[l], r * inv);
             o.x[l] = fmaT(al, p, o.x[l]);
@@ -328,7 +328,7 @@ __device__ __forceinline__ bool residual64(const PcgArgs& a, Share& h, float* r,
     v[0] = v[1] = 0.0;
     for (int l = threadIdx.x; l < h.m; l += PCG_THREADS) {
         const int n = h.n0 + l;
-        const double b = double(a.b[n]), e = b - apply64(a, a.fidx[n], a.diag[n] & 0x7F);
+        const double b = double(a.b[n]), e = b - apply64(a, a.fidx[n], a.diag[n]);
         if (r) r[n] = float(e);
         v[0] += e * e;
         v[1] += b * b;
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg_mixed(PcgArgs a) {
             const int n = h.n0 + l;
             const double x = double(a.x0[n]);
             v[0] += x * double(a.b[n]);
-            v[1] += x * apply64(a, a.fidx[n], a.diag[n] & 0x7F);
+            v[1] += x * apply64(a, a.fidx[n], a.diag[n]);
         }
         if (!reduce(a, h, v)) return;
         const double alpha = (v[1] > 0.0 && isfinite(v[0] / v[1])) ? v[0] / v[1] : 0.0;

@@ -77,9 +77,9 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nblocks, int
 // -- loads that wait on the barrier but not on the sums, so that their round
 // trip overlaps the partials' -- and the total, one warp per sum with all its
 // loads issued together.  Returns false if the barrier gave up.  Fixed order
-// throughout.  (Against block_sum3 + grid_barrier + grid_sum3, whose total is
-// a two-level tree over the whole block: one block barrier and half of the
-// shuffle steps fewer per reduction.)
+// throughout.  (One block barrier and half of the shuffle steps fewer per
+// reduction than sums over the whole block before the barrier and a two-level
+// tree over the whole block after it.)
 template <int N, class Mid>
 __device__ __forceinline__ bool grid_reduce(double (&v)[N], double* part, GridBar* bar, int nb, int* status, Mid mid) {
     __shared__ double sh[N][32];
@@ -129,71 +129,6 @@ template <int N>
 __device__ __forceinline__ bool grid_reduce(double (&v)[N], double* part, GridBar* bar, int nb, int* status) {
     return grid_reduce<N>(v, part, bar, nb, status, [] {});
 }
-
-// Sum of three per-block partial arrays part[0..nb), part[nb..2nb),
-// part[2nb..3nb), returned to every thread of every block.  All threads load
-// (one L2 round trip when nb <= blockDim) and reduce with a fixed tree, so
-// every block obtains the same bits.
-__device__ __forceinline__ double3 grid_sum3(const double* part, int nb) {
-    __shared__ double3 red3[32];
-    __shared__ double3 res3;
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-        a += __ldcg(part + t);
-        b += __ldcg(part + nb + t);
-        c += __ldcg(part + 2 * nb + t);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) red3[wid] = make_double3(a, b, c);
-    __syncthreads();
-    if (wid == 0) {
-        double3 r = lane < int(blockDim.x >> 5) ? red3[lane] : make_double3(0.0, 0.0, 0.0);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            r.x += __shfl_down_sync(0xffffffffu, r.x, o);
-            r.y += __shfl_down_sync(0xffffffffu, r.y, o);
-            r.z += __shfl_down_sync(0xffffffffu, r.z, o);
-        }
-        if (lane == 0) res3 = r;
-    }
-    __syncthreads();
-    double3 r = res3;
-    __syncthreads();
-    return r;
-}
-
-// Block sum of three doubles; result valid in thread 0.
-__device__ __forceinline__ double3 block_sum3(double a, double b, double c) {
-    __shared__ double3 sh3[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh3[wid] = make_double3(a, b, c);
-    __syncthreads();
-    double3 r = make_double3(0.0, 0.0, 0.0);
-    if (wid == 0) {
-        r = lane < int(blockDim.x >> 5) ? sh3[lane] : make_double3(0.0, 0.0, 0.0);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            r.x += __shfl_down_sync(0xffffffffu, r.x, o);
-            r.y += __shfl_down_sync(0xffffffffu, r.y, o);
-            r.z += __shfl_down_sync(0xffffffffu, r.z, o);
-        }
-    }
-    __syncthreads();
-    return r;
-}
-
 
 }  // namespace
 }  // namespace fp
