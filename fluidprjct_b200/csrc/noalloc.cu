@@ -23,6 +23,14 @@
 //     the stream is synchronised before the mutex is released), and calls
 //     from several host threads, on any streams, are serialised in-process
 //     (separate processes have separate contexts, each with its own array);
+//   * the solve is one cooperative launch (k_csr_cg) of up to one block per SM
+//     on the caller's stream.  It starts when all of its blocks fit on the GPU
+//     together, so a resident kernel of the host that holds the SMs delays it
+//     until that kernel ends, where a solve of separate kernels could run on
+//     whatever SMs were free; a resident kernel that waits for the solution
+//     would wait for good.  Hosts with such a kernel keep SMs free for it: a
+//     system of n rows needs ceil(n / 512) blocks of 512 threads, at most one
+//     per SM;
 //   * each call clears the scratch it relies on before use: the control
 //     block, the product vector, the first direction; x starts at zero;
 //   * the first call on each device, with that device current, looks up the

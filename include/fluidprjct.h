@@ -329,7 +329,11 @@ int fp_pressure_solve(fp_solver* s, const float* rhs, float* x, int64_t n, int* 
  * FP64 vectors: the known-answer path of test.cu:223-395.  Host arrays.
  * FP_OK also when CG stops at max_iters or breaks down: check *relres against
  * tol.  FP_ERR_TIMEOUT: a grid-barrier wait of the solver gave up (after about
- * a minute).  x, *iters and *relres are written only with FP_OK. */
+ * a minute).  x, *iters and *relres are written only with FP_OK.
+ * The solve is one cooperative kernel on the legacy default stream, of one
+ * block per 512 rows and at most one per SM: it starts once all its blocks fit
+ * on the GPU at the same time, so it waits for kernels that hold the SMs, and
+ * must not be waited for by one that keeps running. */
 int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double* vals, const double* b, double* x,
                        double tol, int max_iters, int* iters, double* relres);
 
@@ -347,6 +351,10 @@ int fp_solve_csr_upper(int n, const int* offsets, const int* cols, const double*
  *   - FP_ERR_TIMEOUT: a grid-barrier wait of the solver gave up (after about a
  *     minute); *iters and *relres are then unchanged, x is an unfinished
  *     iterate;
+ *   - the solve is one cooperative kernel on stream, of one block per 512 rows
+ *     and at most one per SM: it starts once all its blocks fit on the GPU at
+ *     the same time, so it waits for kernels of other streams that hold the
+ *     SMs, and such a kernel must not wait for it in turn;
  *   - the call is synchronous (it reads its result back and drains its
  *     stream before returning), so it must not be issued on a stream that is
  *     being captured;

@@ -615,3 +615,17 @@ def test_body_force_of_every_face_in_the_box(body, tmp_path):
     else:
         assert not got[3:].any()
     s.close()
+
+
+def test_csr_solve_of_two_million_rows():
+    """As test_csr_solve_sizes, beyond the allocation-free call's range: 28 rows and more a thread."""
+    from fluidprjct_b200 import capi
+    n = (1 << 21) + 77
+    rng = np.random.default_rng(3)
+    off, cols, vals, rows = _spd_upper(n, rng)
+    xt = rng.standard_normal(n)
+    b = np.bincount(rows, vals * xt[cols], n)
+    up = rows != cols
+    b += np.bincount(cols[up], (vals * xt[rows])[up], n)
+    x, it, rr = capi.solve_csr_upper(off, cols, vals, b, tol=1e-12, max_iters=500)
+    assert rr <= 1e-12 and np.linalg.norm(x - xt) <= 1e-11 * np.linalg.norm(xt)
