@@ -162,13 +162,31 @@ def event_timer(stream_ptr):
     return st, (lambda: torch.cuda.Event(enable_timing=True))
 
 
-def step_bytes(np_, nc, nf, iters, outer=1):
+def step_bytes(np_, nc, solve):
     """Algorithmic HBM bytes of one whole step (FP32 values, uint8 labels,
     each array read or written once per phase): label 12 Np + 2 Nc, P2G
-    24 Np + 24 Nc, RHS 17 Nc, PCG 41 Nf per iteration + 17 Nf per outer
-    refinement, projection 29 Nc, G2P + advection 48 Np + 24 Nc; in all
-    84 Np + 96 Nc + 41 Nf iters + 17 Nf outer."""
-    return 84.0 * np_ + 96.0 * nc + 41.0 * nf * iters + 17.0 * nf * outer
+    24 Np + 24 Nc, RHS 17 Nc, the pressure solve's bytes, projection 29 Nc,
+    G2P + advection 48 Np + 24 Nc; in all 84 Np + 96 Nc + the solve."""
+    return 84.0 * np_ + 96.0 * nc + solve
+
+
+def pcg_bytes(nc, nf, iters, outer, fp64, sms=148):
+    """Bytes that the plain or mixed PCG moves through memory (kernels_pcg.cu;
+    vectors of 8 bytes, or 4 inside the refinement), each array once per pass.
+    With at most 512 FLUID cells per CTA a cell's r, w and s are written and
+    read as a neighbour's once per iteration.  With more, only u is; x, r, p, s
+    and w stay in the CTA's 200 KB of shared memory, and cells beyond it move
+    those too (11 accesses, and the index and diagonal twice).  The FP64
+    residual and the solution take 17 bytes per cell and outer loop."""
+    e = 8 if fp64 else 4
+    nb = max(1, min(sms, -(-nc // 1024)))
+    chunk = -(-nf // nb)
+    if chunk <= 512:
+        per = 6.0 * e * nf
+    else:
+        cap = (200 * 1024 // (5 * e + 5)) & ~15
+        per = 2.0 * e * nf + (11.0 * e + 10.0) * nb * max(0, chunk - cap)
+    return per * iters + 17.0 * nf * outer
 
 
 def algorithmic_bytes(np_, nc, nf):
@@ -262,9 +280,10 @@ def run_ours(args, rank, local, world):
                 "~20 grid barriers per iteration and L2 latency (the working set stays in L2), not by HBM")
     else:
         kernel = "k_pcg_mixed" if "mixed" in args.solver else "k_pcg64"
-        solve_bytes = [41.0 * p["num_fluid_cells"] * p["pcg_iters"] + 17.0 * p["num_fluid_cells"] * p["outer_iters"]
+        solve_bytes = [pcg_bytes(nc, p["num_fluid_cells"], p["pcg_iters"], p["outer_iters"], "mixed" not in args.solver)
                        for p in per]
-        note = "41 B per fluid cell per iteration + 17 B per fluid cell; working set is L2-resident at 128^3"
+        note = (f"{1e3 * sum(solve_ms) / max(1, sum(iters)):.2f} us per iteration; bound by grid barriers and L2 "
+                "latency, not by HBM: most vectors stay in registers or shared memory and the rest in L2")
     peak, peak_kind = load_peaks()
     solve_gbs = sum(solve_bytes) / (sum(solve_ms) / 1000.0) / 1e9
     traffic = load_traffic()
@@ -282,7 +301,7 @@ def run_ours(args, rank, local, world):
         "project": dict(bw("project", phase_ms["t_project"]), kernel="k_project"),
         "g2p+advect": dict(bw("g2p_advect", phase_ms["t_advect"]), kernel="k_g2p_advect"),
     }
-    sb = statistics.mean(step_bytes(np_, nc, p["num_fluid_cells"], p["pcg_iters"], p["outer_iters"]) for p in per)
+    sb = step_bytes(np_, nc, statistics.mean(solve_bytes))
     step_gbs = sb / (ms_step / 1000.0) / 1e9
     # DRAM traffic of one captured launch, per iteration of that launch, times
     # the timed solves' mean iterations: the same unit as the algorithmic bytes
@@ -320,7 +339,7 @@ def run_ours(args, rank, local, world):
            "clocks": clk, "gpu_launches": int(launches), "roofline": roofline, "phases": phases,
            "roofline_step": {"bound": "hbm", "algorithmic_bytes": round(sb), "achieved": round(step_gbs, 1),
                              "peak": peak, "unit": "GB/s", "frac": round(step_gbs / peak, 4),
-                             "note": "84 Np + 96 Nc + 41 Nf iters + 17 Nf outer bytes per step over ms_per_step"}}
+                             "note": "84 Np + 96 Nc + the solve's bytes per step over ms_per_step"}}
 
     # ---- PCG time-to-1e-6 of each solver on the same scene, all from x = 0 (the
     # learned one from its network guess), and MG warm-started as in the step ----
