@@ -262,6 +262,16 @@ int load_net(fp_solver* s) {
     return FP_OK;
 }
 
+// The zero state of the plain PCG's padded grids between solves (where the
+// solver has them).
+cudaError_t pcg_zero(fp_solver* s) {
+    cudaError_t e = cudaSuccess;
+    const PressureBufs& pb = s->pb;
+    for (void* a : {pb.R[0], pb.R[1], pb.Wv[0], pb.Wv[1], pb.S[0], pb.S[1], pb.invd, static_cast<void*>(pb.xd)})
+        if (a && e == cudaSuccess) e = cudaMemsetAsync(a, 0, sizeof(double) * size_t(s->padded), s->st);
+    return e;
+}
+
 // The zero state of the multigrid work grids between solves.
 cudaError_t mg_zero(const MgBufs& m, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
@@ -308,13 +318,18 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
         readback_views(rb, pb.out, pb.red, pb.nf);
     }
     ck(dalloc(&pb.fidx, nc)); ck(dalloc(&pb.diag, nc)); ck(dalloc(&pb.b, nc));
-    ck(dalloc(&pb.bin, nc));
     const size_t pbytes = sizeof(double) * size_t(s->padded), cbytes = sizeof(double) * size_t(nc);
-    for (int i = 0; i < 2; ++i) {
-        ck(dalloc_bytes(&pb.R[i], pbytes)); ck(dalloc_bytes(&pb.Wv[i], pbytes)); ck(dalloc_bytes(&pb.S[i], pbytes));
+    // The plain PCG's vectors, 92 bytes per cell: every solver but the multigrid
+    // one, which has vectors of its own and no fallback, may run it.
+    const bool plain = s->cfg.solver != FP_SOLVER_PCG_MG;
+    if (plain) {
+        ck(dalloc(&pb.bin, nc));
+        for (int i = 0; i < 2; ++i) {
+            ck(dalloc_bytes(&pb.R[i], pbytes)); ck(dalloc_bytes(&pb.Wv[i], pbytes)); ck(dalloc_bytes(&pb.S[i], pbytes));
+        }
+        ck(dalloc_bytes(&pb.invd, pbytes)); ck(dalloc_bytes(&pb.P, cbytes)); ck(dalloc_bytes(&pb.X, cbytes));
+        ck(dalloc(&pb.x64, nc)); ck(dalloc(&pb.xd, s->padded));
     }
-    ck(dalloc_bytes(&pb.invd, pbytes)); ck(dalloc_bytes(&pb.P, cbytes)); ck(dalloc_bytes(&pb.X, cbytes));
-    ck(dalloc(&pb.x64, nc)); ck(dalloc(&pb.xd, s->padded));
     ck(dalloc(&pb.part, size_t(6) * std::max(maxb, 1024)));
     ck(dalloc(&pb.bar, 1));
     pb.tile_sums = s->d_tiles;
@@ -348,12 +363,7 @@ int alloc_grid(fp_solver* s, int W, int H, int D) {
     ck(cudaMemsetAsync(s->d_p, 0, sizeof(float) * nc, s->st));
     ck(cudaMemsetAsync(s->d_bodymark, 0, nc, s->st));
     ck(cudaMemsetAsync(s->d_counts, 0, sizeof(int) * (nc + 1), s->st));
-    for (int i = 0; i < 2; ++i) {
-        ck(cudaMemsetAsync(pb.R[i], 0, pbytes, s->st)); ck(cudaMemsetAsync(pb.Wv[i], 0, pbytes, s->st));
-        ck(cudaMemsetAsync(pb.S[i], 0, pbytes, s->st));
-    }
-    ck(cudaMemsetAsync(pb.invd, 0, pbytes, s->st));
-    ck(cudaMemsetAsync(pb.xd, 0, sizeof(double) * size_t(s->padded), s->st));
+    ck(pcg_zero(s));
     ck(cudaMemsetAsync(pb.bar, 0, sizeof(GridBar), s->st));
     // No FLUID list until the first pressure set-up: the count starts at 0, so
     // FP_GRID_RHS read before any step densifies nothing (an all-zero grid).
@@ -591,10 +601,7 @@ int solve_tail(fp_solver* s, int inner_total, int outer, int dev_status, float p
     if (status == FP_ERR_TIMEOUT) {
         // a solve that gave up mid-way leaves its work grids (MG: the level-0
         // codes too) non-zero; restore the zero state the next solve relies on
-        const size_t pbytes = sizeof(double) * size_t(s->padded);
-        for (void* a : {s->pb.R[0], s->pb.R[1], s->pb.Wv[0], s->pb.Wv[1], s->pb.S[0], s->pb.S[1], s->pb.invd,
-                        static_cast<void*>(s->pb.xd)})
-            cudaMemsetAsync(a, 0, pbytes, s->st);
+        pcg_zero(s);
         mg_zero(s->mg, s->st);
     }
     if (status == FP_ERR_TIMEOUT) return s->fail(status, "PCG grid barrier timed out");

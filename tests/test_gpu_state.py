@@ -85,3 +85,19 @@ def test_state_snapshot_resumes_the_run(O, tmp_path):
         assert e.value.code == capi.FP_ERR_IO
     for x in (a, b, c):
         x.close()
+
+
+def test_device_memory_per_cell_of_the_multigrid_solver():
+    """The multigrid solver's grids take at most 200 bytes per cell: labels 3, counts and offsets 8, faces 24, pairs 24,
+    pressure and scratch 12, the system 13, 11 for the level grids and 57 for the Krylov vectors, quads and the FP64
+    iterate, 152 in all, and the padding and granularity of 45 allocations."""
+    import torch
+    from fluidprjct_b200 import capi
+    n = 192
+    for size in (16, n):  # the small one loads the kernels
+        s = capi.Solver(dx=1.0 / size, dt=0.002, solver="pcg_mg", output_format=capi.OUT_NONE)
+        free0 = torch.cuda.mem_get_info()[0]
+        s.set_labels(np.full((size, size, size), 2, np.uint8))
+        used = free0 - torch.cuda.mem_get_info()[0]
+        s.close()
+    assert used <= 200 * n ** 3, used / n ** 3
