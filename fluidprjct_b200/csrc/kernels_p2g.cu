@@ -22,8 +22,8 @@
 // return at once.  A second, elementwise kernel divides, saves and adds
 // gravity, and zeroes the pair array for the next step.
 //
-// Bound by the L1 data pipe (three quarters busy: a lane's 16-byte loads lie a
-// cell's particles apart) and by the latency of those loads, so by occupancy.
+// Bound by the L1 data pipe (81 % busy: a lane's 16-byte loads lie a cell's
+// particles apart) and by the latency of those loads, so by occupancy.
 // Staging a slab's particles in shared memory for all three components halved
 // the pipe's work but took a third more instructions (152 us at 128^3).  The
 // accumulate kernel takes 131 us for the 128^3 dam break (3.8 M particles), 319

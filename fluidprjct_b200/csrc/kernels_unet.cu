@@ -23,12 +23,14 @@ constexpr int THREADS = 256;
 // with cp.async.  A CTA keeps the sums of its TPC taps over its bricks in
 // registers and writes one partial; the partials are added in a fixed order.
 //
-// Bound by ldmatrix: a brick's operands pass through it once per tap.  A warp's
-// unit is a tap, 16 input and 16 COG output channels: one x4 load of x serves 2
-// COG MMAs, and g's are loaded once per 16 voxels for all the warp's units, where
-// a warp that took 16 x 8 tiles one by one loaded both for each (x4 and x2 per
-// MMA).  Two buffers, where two CTAs of them fit an SM, let a brick's loads run
-// during the one before.  1.31 ms per 128^3 training step, against 3.07.
+// Bound by latency: the 18 warps of an SM wait for ldmatrix (its shared-memory
+// pipe is 56 to 60 % busy), for the MMA before on the same sums and for the
+// block; the tensor pipe is 40 to 43 % busy.  A warp's unit is a tap, 16 input
+// and 16 COG output channels: one x4 load of x serves 2 COG MMAs, and g's are
+// loaded once per 16 voxels for all the warp's units, where a warp that took
+// 16 x 8 tiles one by one loaded both for each (x4 and x2 per MMA).  Two buffers,
+// where two CTAs of them fit an SM, let a brick's loads run during the one
+// before.  1.31 ms per 128^3 training step, against 3.07.
 //
 // Each sum keeps its order, brick by brick and 16 voxels at a time, one MMA after
 // the other: FP32 accumulation of the tensor cores is not exact, and a training
