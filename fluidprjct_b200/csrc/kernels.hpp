@@ -258,8 +258,9 @@ int csr_cg_solve(int n, const int* offsets, const int* cols, const double* vals,
 // Returns the number of launches.
 int launch_extrapolate_unknown(float* v, int nx, int ny, int depth, int front_stride, int* mark, cudaStream_t st);
 // Faces of component axis (0 u, 1 v, 2 w) with no FLUID side, depth waves.
+// guard: as in launch_project.
 int launch_extrapolate_from_fluid(float* v, int axis, const uint8_t* labels, Dims g, int depth, int* mark,
-                                  cudaStream_t st);
+                                  const int* guard, cudaStream_t st);
 
 // -------- scene generation (kernels_scene.cu) --------
 void launch_seabed_labels(uint8_t* labels, int W, int H, int D, double dx, double level, double bed_base,

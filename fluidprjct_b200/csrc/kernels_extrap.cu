@@ -58,7 +58,10 @@ __global__ void k_ext_front(int* __restrict__ mark, int nx, int ny, int nz, int 
             }
 }
 
-__global__ void k_ext_average(float* __restrict__ v, const int* __restrict__ mark, int nx, int ny, int nz, int wave) {
+// guard: the status word of the solve whose projected faces these are, or null; faces of a failed one stay as they are.
+__global__ void k_ext_average(float* __restrict__ v, const int* __restrict__ mark, int nx, int ny, int nz, int wave,
+                              const int* __restrict__ guard) {
+    if (solve_failed(guard)) return;
     const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c >= int64_t(nx) * ny * nz || mark[c] != wave) return;
     const int i = int(c % nx), j = int((c / nx) % ny), k = int(c / (int64_t(nx) * ny));
@@ -83,11 +86,12 @@ __global__ void k_ext_average(float* __restrict__ v, const int* __restrict__ mar
 
 unsigned blocks(int64_t n) { return unsigned((n + 255) / 256); }
 
-void run_waves(float* v, int* mark, int nx, int ny, int nz, int depth, int front_stride, cudaStream_t st) {
+void run_waves(float* v, int* mark, int nx, int ny, int nz, int depth, int front_stride, const int* guard,
+               cudaStream_t st) {
     const int64_t n = int64_t(nx) * ny * nz;
     for (int w = 1; w <= depth; ++w) {
         k_ext_front<<<blocks(n), 256, 0, st>>>(mark, nx, ny, nz, w, front_stride);
-        k_ext_average<<<blocks(n), 256, 0, st>>>(v, mark, nx, ny, nz, w);
+        k_ext_average<<<blocks(n), 256, 0, st>>>(v, mark, nx, ny, nz, w, guard);
     }
 }
 
@@ -96,15 +100,15 @@ void run_waves(float* v, int* mark, int nx, int ny, int nz, int depth, int front
 int launch_extrapolate_unknown(float* v, int nx, int ny, int depth, int front_stride, int* mark, cudaStream_t st) {
     const int64_t n = int64_t(nx) * ny;
     k_ext_known_value<<<blocks(n), 256, 0, st>>>(v, n, mark);
-    run_waves(v, mark, nx, ny, 1, depth, front_stride, st);
+    run_waves(v, mark, nx, ny, 1, depth, front_stride, nullptr, st);
     return 1 + 2 * depth;
 }
 
 int launch_extrapolate_from_fluid(float* v, int axis, const uint8_t* labels, Dims g, int depth, int* mark,
-                                  cudaStream_t st) {
+                                  const int* guard, cudaStream_t st) {
     const int nx = g.W + (axis == 0), ny = g.H + (axis == 1), nz = g.D + (axis == 2);
     k_ext_known_fluid<<<blocks(int64_t(nx) * ny * nz), 256, 0, st>>>(labels, g, axis, mark);
-    run_waves(v, mark, nx, ny, nz, depth, nx, st);
+    run_waves(v, mark, nx, ny, nz, depth, nx, guard, st);
     return 1 + 2 * depth;
 }
 

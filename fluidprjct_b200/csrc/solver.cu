@@ -757,13 +757,13 @@ int r2_extrapolate(fp_solver* s, bool after_g2p) {
 }
 
 // Default scheme: cfg.extrapolate layers into faces with no FLUID side.
-int extrapolate_3d(fp_solver* s) {
+int extrapolate_3d(fp_solver* s, bool guarded = false) {
     int rc = ext_alloc(s);
     if (rc) return rc;
     float* comp[3] = {s->d_u, s->d_v, s->d_w};
     for (int a = 0; a < (s->D > 1 ? 3 : 2); ++a)
         s->launches += launch_extrapolate_from_fluid(comp[a], a, s->d_labels, s->g, s->cfg.extrapolate, s->d_extmark,
-                                                     s->st);
+                                                     guarded ? &s->pb.out->status : nullptr, s->st);
     return FP_OK;
 }
 
@@ -963,7 +963,7 @@ int one_step(fp_solver* s, bool finish = true) {
     NvtxRange adv_range("g2p+advect");
     if (s->cfg.extrapolate > 0) {
         phase_g2p_advect(s, 1, 0, true);
-        rc = extrapolate_3d(s);
+        rc = extrapolate_3d(s, true);
         if (rc != FP_OK) return fail_after(rc);
         phase_g2p_advect(s, 0, 1, true);
     } else {

@@ -169,3 +169,29 @@ def test_ref2d_timers_of_a_call_that_fails_in_its_second_step():
     s.step(2)
     assert s.stats()["step"] == 4 and timers() != first
     s.close()
+
+
+@pytest.mark.parametrize("solver", ["pcg_mg", "pcg", "pcg_mixed"])
+def test_timed_out_solve_with_extrapolation_leaves_the_faces_of_p2g(O, solver):
+    """The face grids after a step whose solve gave up hold that step's P2G output, also where velocities are
+    extrapolated after the projection (P2G's sums may differ in their last bits)."""
+    from fluidprjct_b200 import capi, scenes
+    n, dx = 40, 1.0 / 40
+    lab = scenes.box_3d(n, n, n, dx, 0.5, 0.5, 2.0)
+    pos = O.seed3d(lab, dx, 8, 2)
+    vel = np.random.default_rng(2).uniform(-0.5, 0.5, pos.shape).astype(np.float32)
+    kw = dict(dx=dx, dt=0.002, solver=solver, output_format=capi.OUT_NONE)
+    s, t = capi.Solver(extrapolate=3, **kw), capi.Solver(**kw)
+    for a in (s, t):
+        a.set_labels(lab)
+        a.set_particles(pos, vel)
+    s.set_wait_limit(1)
+    with pytest.raises(capi.FluidError) as e:
+        s.step(1)
+    assert e.value.code == capi.FP_ERR_TIMEOUT
+    for ph in (capi.PHASE_LABEL, capi.PHASE_P2G, capi.PHASE_SAVE, capi.PHASE_FORCES):
+        t.phase(ph)
+    for g in (capi.GRID_U, capi.GRID_V, capi.GRID_W):
+        assert np.abs(s.grid(g) - t.grid(g)).max() <= 1e-5, g
+    s.close()
+    t.close()
